@@ -211,10 +211,10 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   extern __shared__ __align__(16) double csm[];
   double *sA = csm, *sB = csm + CT * CLD, *sP = csm + 2 * CT * CLD;
   const int G = gridDim.x;
-  const unsigned nb = (unsigned)G;
+  GridBarrier bar(T.bar, (unsigned)G, T.err, T.bar_ns);
   // tile 0's diagonal block
   if (blockIdx.x == 0) potrf_tile(tile_at(T, 0, 0), T.Linv, T.err, sA, sB, sP);
-  if (!grid_barrier(T.bar, nb, T.err, T.bar_ns)) return;
+  if (!bar.sync()) return;
   // With the inverse, X = L^-1 is formed in the same loop: tile row J of X
   // in phase T of column J (X_Jj = Linv_J R_Jj, its R final after the
   // updates of the earlier columns), and its updates R_Kj -= L_KJ X_Jj in
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
       __syncthreads();
       for_frag([&](int j, int e, int r, int c) { gt[r * CT + c] = acc[j][e]; });
     }
-    if (!grid_barrier(T.bar, nb, T.err, T.bar_ns)) return;
+    if (!bar.sync()) return;
     // U: A_IK -= L_IJ L_KJ^T (items 0 .. nu - 1); the tile (J+1, J+1) is
     // then factored by the CTA of item 0, which takes no other item when
     // there are other CTAs.  With the inverse also R_Kj -= L_KJ X_Jj, K > J,
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
     }
     if (m == 0 && J + 1 < T.nt && blockIdx.x == (J + 1) % G)
       potrf_tile(tile_at(T, J + 1, J + 1), T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
-    if (!grid_barrier(T.bar, nb, T.err, T.bar_ns)) return;
+    if (!bar.sync()) return;
   }
   if (!T.want_inverse) return;
   const int nt = T.nt;

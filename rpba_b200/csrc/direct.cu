@@ -161,9 +161,10 @@ __device__ void tile_gemv_set(const double *Li, double *yj, bool trans, double *
 __global__ void __launch_bounds__(ST) k_env_solve(SolveArgs A) {
   __shared__ double sv[T], sp[ST];
   const int G = gridDim.x, nt = A.nt;
+  GridBarrier bar(A.bar, (unsigned)G, A.err, A.bar_ns);
   // forward: L y = b
   if (blockIdx.x == 0) tile_gemv_set(A.Linv, A.y, false, sv, sp);
-  if (!grid_barrier(A.bar, G, A.err, A.bar_ns)) return;
+  if (!bar.sync()) return;
   for (int J = 0; J < nt - 1; ++J) {
     const int m = A.hrow[J] - J;
     for (int t = blockIdx.x; t < m; t += G) {
@@ -173,11 +174,11 @@ __global__ void __launch_bounds__(ST) k_env_solve(SolveArgs A) {
     }
     if (m == 0 && blockIdx.x == (J + 1) % G)
       tile_gemv_set(A.Linv + (size_t)(J + 1) * TS, A.y + (size_t)(J + 1) * T, false, sv, sp);
-    if (!grid_barrier(A.bar, G, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
   }
   // backward: L^T x = y
   if (blockIdx.x == 0) tile_gemv_set(A.Linv + (size_t)(nt - 1) * TS, A.y + (size_t)(nt - 1) * T, true, sv, sp);
-  if (!grid_barrier(A.bar, G, A.err, A.bar_ns)) return;
+  if (!bar.sync()) return;
   for (int J = nt - 1; J > 0; --J) {
     const int m = J - A.fcol[J];
     for (int t = blockIdx.x; t < m; t += G) {
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(ST) k_env_solve(SolveArgs A) {
     }
     if (m == 0 && blockIdx.x == (J - 1) % G)
       tile_gemv_set(A.Linv + (size_t)(J - 1) * TS, A.y + (size_t)(J - 1) * T, true, sv, sp);
-    if (!grid_barrier(A.bar, G, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
   }
 }
 

@@ -132,6 +132,7 @@ __device__ float warp_seq(const float *v, int i, int i_end, float s) {
 __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
   const int G = gridDim.x, c = blockIdx.x, tid = threadIdx.x;
   const int n = A.n;
+  GridBarrier bar(A.bar, (unsigned)G, A.err);
   __shared__ Xf s_x[ES_T];  // per-thread composites of the current run
   __shared__ Xf s_w[ES_T / 32];  // per-warp composites
   __shared__ long long s_cR[2 * ES_MAXG], s_cM[2 * ES_MAXG];  // the chunks' composites
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
       A.ctl->i = isfinite(s) ? i : n;
     }
   }
-  if (!grid_barrier(A.bar, G, A.err)) return;
+  if (!bar.sync()) return;
 
   for (int seg = 0;; ++seg) {
     const float s = __ldcg(&A.ctl->s);
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
         A.Tc[2 * c + p] = cx.q[p];
       }
     }
-    if (!grid_barrier(A.bar, G, A.err)) return;
+    if (!bar.sync()) return;
 
     // phase B (every CTA, one thread): walk the chunk composites in order
     // from the run's start state; find the first chunk that crosses, the
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
         }
       }
     }
-    if (!grid_barrier(A.bar, G, A.err)) return;
+    if (!bar.sync()) return;
     // a new run that starts in the zero/subnormal range is continued in sequence
     if (c == 0 && tid < 32) {
       float s2 = __ldcg(&A.ctl->s);
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
         A.ctl->i = i2;
       }
     }
-    if (!grid_barrier(A.bar, G, A.err)) return;
+    if (!bar.sync()) return;
   }
   if (c == 0 && tid == 0) *A.out = __ldcg(&A.ctl->s);
 }

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
   const int gwarp = blockIdx.x * PCG_W + warp, nwarps = gridDim.x * PCG_W;
   const int grp = lane / 9, rr = lane % 9, gbase = grp * 9;
   const int G = gridDim.x;
+  GridBarrier bar(A.bar, (unsigned)G + A.bar_extra, A.err, A.bar_ns);
   __shared__ double sh[PCG_W + 1][4];
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
   BT *stage0 = (BT *)pcg_dyn + (size_t)warp * 2 * P1_ELEMS;
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
     cta_sum<1, PCG_W>(v, sh);
     if (threadIdx.x == 0) A.red2[4 * blockIdx.x] = v[0];
   }
-  if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+  if (!bar.sync()) return;
   double erthk;
   {
     double v[1];
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
       }
     cta_sum<1, PCG_W>(pdq, sh);
     if (threadIdx.x == 0) A.red1[4 * blockIdx.x] = pdq[0];
-    if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
     double edtAdk;
     {
       double v[1];
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
         }
         __syncthreads();
       }
-      if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+      if (!bar.sync()) return;
       for (int a = blockIdx.x; a < A.nagg; a += G) {
         double z[CO_M];
 #pragma unroll
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
       A.red2[4 * blockIdx.x + 1] = p2[1];
       A.red2[4 * blockIdx.x + 2] = p2[2];
     }
-    if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
     double g3[3];
     grid_sum<3, PCG_W>(A.red2, G, g3, sh);
     const double meandr = g3[0], er1th1 = g3[1];
@@ -671,6 +672,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * P32_W + warp, nwarps = gridDim.x * P32_W;
   const int G = gridDim.x;
+  GridBarrier bar(A.bar, (unsigned)G + A.bar_extra, A.err, A.bar_ns);
   __shared__ double sh[P32_W + 1][4];
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
   unsigned char *stg = pcg_dyn + (size_t)warp * STG_BYTES;
@@ -693,7 +695,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
     cta_sum<1, P32_W>(v, sh);
     if (threadIdx.x == 0) A.red2[4 * blockIdx.x] = v[0];
   }
-  if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+  if (!bar.sync()) return;
   double erthk;
   {
     double v[1];
@@ -716,7 +718,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         A.d32[(size_t)row * 12 + lane] = (float)dk;
       }
     if (blockIdx.x == 0 && threadIdx.x < 2) A.ctr[threadIdx.x] = 0u;
-    if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
     // ---- phase 1
     {
       auto grab = [&]() -> long long {
@@ -892,7 +894,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       }
     }
 
-    if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
     double edtAdk;
     {
       // d^T A d: every CTA sums the chunks' shares in the same fixed order
@@ -1004,7 +1006,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         if (lane == 31) A.rowc[(size_t)row * RC_S + CO_M] = d2;
         t = tn;
       }
-      if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+      if (!bar.sync()) return;
       // 2a': per aggregate, its rows' restrictions and shares of dr^2 in a
       // fixed order (warp w: rows w, w + P32_W, ...; then the warps in order)
       for (int a = blockIdx.x; a < A.nagg; a += G) {
@@ -1024,7 +1026,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         }
         __syncthreads();
       }
-      if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+      if (!bar.sync()) return;
       for (int a = blockIdx.x; a < A.nagg; a += G) {
         double z[CO_M];
 #pragma unroll
@@ -1071,7 +1073,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       A.red2[4 * blockIdx.x + 1] = p2[1];
       A.red2[4 * blockIdx.x + 2] = p2[2];
     }
-    if (!grid_barrier(A.bar, G + A.bar_extra, A.err, A.bar_ns)) return;
+    if (!bar.sync()) return;
     double g3[3];
     grid_sum<3, P32_W>(A.red2, G, g3, sh);
     const double meandr = g3[0], er1th1 = g3[1];
