@@ -32,8 +32,10 @@ namespace {
 
 constexpr int CT = 64;                  // tile edge
 constexpr int CLD = 68;                 // shared leading dimension: conflict-free fragment loads
-constexpr int CTH = 256;                // threads per CTA (8 warps)
+constexpr int CTH = 512;                // threads per CTA (16 warps)
 constexpr int TS = CT * CT;             // doubles per stored tile
+static_assert(CTH == 8 * CT, "tile loads: eight lanes a row");
+constexpr int NF = 4;                   // 8 x 8 fragments per warp
 constexpr size_t CSMEM = (2 * CT * CLD + 4 * CT) * sizeof(double);  // two tiles + partials
 
 struct Tiles {
@@ -63,137 +65,263 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// acc (warp w: rows 8w .. 8w + 7, all 64 columns, 8 fragments of 2) +=
-// sA sB^T over k = 0 .. 63; sA, sB in shared memory with ld CLD.
-__device__ __forceinline__ void gemm_nt(const double *sA, const double *sB, double (&acc)[8][2]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const double *pa = sA + (8 * w + g) * CLD + t;
-  const double *pb = sB + g * CLD + t;
+// acc (warp w: rows 8 (w % 8) .. + 7, columns 32 (w / 8) .. + 31, 4
+// fragments of 2) += sA sB^T over k = 0 .. 63; sA, sB in shared memory with
+// ld CLD.
+__device__ __forceinline__ int frag_row() { return 8 * ((threadIdx.x >> 5) & 7) + ((threadIdx.x & 31) >> 2); }
+__device__ __forceinline__ int frag_col() { return 32 * (threadIdx.x >> 8) + 2 * (threadIdx.x & 3); }
+__device__ __forceinline__ void gemm_nt(const double *sA, const double *sB, double (&acc)[NF][2]) {
+  const int lane = threadIdx.x & 31, t = lane & 3;
+  const double *pa = sA + frag_row() * CLD + t;
+  const double *pb = sB + (32 * (threadIdx.x >> 8) + (lane >> 2)) * CLD + t;
 #pragma unroll 4
   for (int kk = 0; kk < CT / 4; ++kk) {
     const double a = pa[4 * kk];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dmma(acc[j][0], acc[j][1], a, pb[8 * j * CLD + 4 * kk]);
+    for (int j = 0; j < NF; ++j) dmma(acc[j][0], acc[j][1], a, pb[8 * j * CLD + 4 * kk]);
   }
 }
 
 // Global tile (ld 64) -> shared (ld CLD), optionally transposed: every
-// thread's sixteen loads are issued before its first store.
+// thread's four 16-byte loads are issued before its first store.
 __device__ __forceinline__ void load_tile(double *s, const double *g, bool trans) {
-  double v[TS / CTH];
+  const int i = threadIdx.x >> 3, j0 = 2 * (threadIdx.x & 7);
+  double2 v[4];
 #pragma unroll
-  for (int q = 0; q < TS / CTH; ++q) v[q] = __ldcg(g + threadIdx.x + q * CTH);
+  for (int q = 0; q < 4; ++q) v[q] = __ldcg((const double2 *)(g + i * CT + 16 * q + j0));
 #pragma unroll
-  for (int q = 0; q < TS / CTH; ++q) {
-    const int idx = threadIdx.x + q * CTH, i = idx >> 6, j = idx & 63;
-    if (trans)
-      s[j * CLD + i] = v[q];
-    else
-      s[i * CLD + j] = v[q];
+  for (int q = 0; q < 4; ++q) {
+    const int j = 16 * q + j0;
+    if (trans) {
+      s[j * CLD + i] = v[q].x;
+      s[(j + 1) * CLD + i] = v[q].y;
+    } else {
+      *(double2 *)(s + i * CLD + j) = v[q];
+    }
   }
 }
 
-// Tile update gt -= acc (fragment positions): the sixteen old values are
-// loaded before any is written back.
-__device__ __forceinline__ void sub_frag(double *gt, const double (&acc)[8][2]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int r = 8 * w + (lane >> 2), c0 = 2 * (lane & 3);
-  double2 old[8];
+// Tile update gt -= acc (fragment positions): the old values are loaded
+// before any is written back.
+__device__ __forceinline__ void sub_frag(double *gt, const double (&acc)[NF][2]) {
+  double *g = gt + frag_row() * CT + frag_col();
+  double2 old[NF];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) old[j] = __ldcg((const double2 *)(gt + r * CT + 8 * j + c0));
+  for (int j = 0; j < NF; ++j) old[j] = __ldcg((const double2 *)(g + 8 * j));
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
-    *(double2 *)(gt + r * CT + 8 * j + c0) = make_double2(old[j].x - acc[j][0], old[j].y - acc[j][1]);
+  for (int j = 0; j < NF; ++j) *(double2 *)(g + 8 * j) = make_double2(old[j].x - acc[j][0], old[j].y - acc[j][1]);
+}
+// The same with the result left in shared memory (ld CT + 1).
+__device__ __forceinline__ void sub_frag_to(const double *gt, const double (&acc)[NF][2], double *s) {
+  const double *g = gt + frag_row() * CT + frag_col();
+  double *d = s + frag_row() * (CT + 1) + frag_col();
+  double2 old[NF];
+#pragma unroll
+  for (int j = 0; j < NF; ++j) old[j] = __ldcg((const double2 *)(g + 8 * j));
+#pragma unroll
+  for (int j = 0; j < NF; ++j) {
+    d[8 * j] = old[j].x - acc[j][0];
+    d[8 * j + 1] = old[j].y - acc[j][1];
+  }
+}
+__device__ __forceinline__ void store_frag(double *gt, const double (&acc)[NF][2]) {
+  double *g = gt + frag_row() * CT + frag_col();
+#pragma unroll
+  for (int j = 0; j < NF; ++j) *(double2 *)(g + 8 * j) = make_double2(acc[j][0], acc[j][1]);
 }
 
-// Fragment positions of acc[j][e]: row 8w + g, column 8j + 2t + e.
-template <class F>
-__device__ __forceinline__ void for_frag(F f) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int r = 8 * w + (lane >> 2), c0 = 2 * (lane & 3);
+// Factor the diagonal tile in s (lower triangle, ld PLD) and write L_JJ and
+// L_JJ^-1, with all threads of the CTA.
+//
+// The chain of the 64 pivots (a square root, a reciprocal, the next pivot's
+// update: about 160 cycles each) bounds the whole factorisation, so warp 0
+// runs that chain and as little else as it can: the 8 x 8 diagonal block of
+// a panel, held whole in every lane's registers (no exchange between the
+// pivots), then only the next block's eight rows and its update.  Meanwhile
+// warps 1-7 solve the panel's other rows and apply the panel to the columns
+// past it, and warps 8-15 form the panel's rows of the inverse; one block
+// barrier a panel.  Every entry takes its updates in column order, and every
+// inverse entry its four partial sums (terms mm = c + q, c + q + 4, ... in
+// order, then (p0 + p1) + (p2 + p3)), as the unblocked column loop takes
+// them, so the result does not depend on the distribution.
+// A tile takes 35,000 cycles (18 us; 125,000 with one warp factoring panels
+// and the inverse formed after them).
+// s, si: two shared tiles (ld PLD); pp: CT doubles (reciprocal pivots).
+constexpr int PLD = CT + 1, PW = 8;
+
+// Rows [r0, r0 + PW) of the inverse of the factored tile, by warps 8 .. 15:
+// four lanes per column c, lane q its partial sum q.  The terms of earlier
+// blocks' rows first (eight rows' sums side by side), then the block's own
+// rows one after the other.
+__device__ __forceinline__ void inverse_block(int r0, const double *s, double *si, const double *pp) {
+  const int lane = threadIdx.x & 31, c = ((threadIdx.x >> 5) - 8) * 8 + (lane >> 2), q = lane & 3;
+  double u[PW];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    f(j, 0, r, 8 * j + c0);
-    f(j, 1, r, 8 * j + c0 + 1);
+  for (int r = 0; r < PW; ++r) u[r] = 0.;
+  const double *sr = s + r0 * PLD, *sc = si + c;
+#pragma unroll 2
+  for (int mm = c + q; mm < r0; mm += 4) {
+    const double x = sc[mm * PLD];
+#pragma unroll
+    for (int r = 0; r < PW; ++r) u[r] += sr[r * PLD + mm] * x;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < PW; ++r) {
+    const int i = r0 + r;
+    const double p2 = u[r] + __shfl_xor_sync(0xffffffffu, u[r], 1);
+    const double p4 = p2 + __shfl_xor_sync(0xffffffffu, p2, 2);
+    const double rdi = pp[i];
+    const double z = c < i ? -p4 * rdi : (c == i ? rdi : 0.);
+    si[i * PLD + c] = z;  // the column's four lanes write the same value
+    // the term mm = i of the block's later rows, in its partial sum
+    const double zq = c <= i && ((i - c) & 3) == q ? z : 0.;
+#pragma unroll
+    for (int t = r + 1; t < PW; ++t) u[t] += sr[t * PLD + i] * zq;
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void load_potrf_tile(const double *gtile, double *s) {
+  const int t = threadIdx.x;
+  double2 v[TS / CTH / 2];
+#pragma unroll
+  for (int q = 0; q < TS / CTH / 2; ++q) v[q] = __ldcg((const double2 *)gtile + t + q * CTH);
+#pragma unroll
+  for (int q = 0; q < TS / CTH / 2; ++q) {
+    const int e = 2 * (t + q * CTH);
+    s[(e >> 6) * PLD + (e & 63)] = v[q].x;
+    s[(e >> 6) * PLD + (e & 63) + 1] = v[q].y;
   }
 }
 
-// Factor the diagonal tile in place and write L_JJ and L_JJ^-1, with all
-// threads of the CTA.  Factor: panels of eight columns; warp 0 factors a
-// panel (per column the pivot's square root, the column scaled by its
-// reciprocal, the panel's later columns updated; warp barriers only), then
-// all threads apply the panel to the trailing triangle, each entry's eight
-// updates in column order, as in the unblocked column loop; two block
-// barriers a panel.  Inverse:
-// four lanes of one warp per column c, rows i in order (lane q takes the
-// terms mm = c + q, c + q + 4, ... of entry (i, c), the partial sums added as
-// (p0 + p1) + (p2 + p3), times the row's reciprocal pivot), warp barriers
-// only.  s, si: two shared tiles (ld CT + 1); pp: CT doubles of scratch
-// (the reciprocal pivots).
+// x (a row's eight entries of a panel) solved by the panel's diagonal block:
+// entry j takes the updates k = 0 .. j - 1 in order, then its pivot.
+template <class F, class G>
+__device__ __forceinline__ void panel_row_solve(double (&x)[PW], F rd, G l) {
+#pragma unroll
+  for (int k = 0; k < PW; ++k) {
+    x[k] *= rd(k);
+#pragma unroll
+    for (int j = k + 1; j < PW; ++j) x[j] -= x[k] * l(j, k);
+  }
+}
+
 __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, double *si, double *pp) {
-  constexpr int LD = CT + 1, PW = 8;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   __syncthreads();
-  {
-    double v[TS / CTH];
-#pragma unroll
-    for (int q = 0; q < TS / CTH; ++q) v[q] = __ldcg(gtile + t + q * CTH);
-#pragma unroll
-    for (int q = 0; q < TS / CTH; ++q) s[((t + q * CTH) >> 6) * LD + ((t + q * CTH) & 63)] = v[q];
-  }
-  __syncthreads();
+  double d[PW][PW], rd[PW];  // warp 0: the current diagonal block (lower), its reciprocal pivots
+#pragma unroll 1
   for (int k0 = 0; k0 < CT; k0 += PW) {
+    const int kp = k0 - PW;  // the previous panel
     if (w == 0) {
-      for (int k = k0; k < k0 + PW; ++k) {
-        const double d = s[k * LD + k];
-        const double dk = sqrt(d > 0. ? d : 1.), rdk = 1. / dk;
-        if (lane == 0 && !(d > 0.)) atomicOr(err, 4);
-        for (int i = k + 1 + lane; i < CT; i += 32) s[i * LD + k] *= rdk;
-        __syncwarp();
-        if (lane == 0) s[k * LD + k] = dk;
-        // the panel's later columns j (k < j < k0 + PW), rows i >= j
-        for (int j = k + 1; j < k0 + PW; ++j) {
-          const double ljk = s[j * LD + k];
-          for (int i = j + lane; i < CT; i += 32) s[i * LD + j] -= s[i * LD + k] * ljk;
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    // trailing triangle (rows and columns >= k0 + PW): the panel's updates
-    for (int i = k0 + PW + w; i < CT; i += CTH / 32)
-      for (int j = k0 + PW + lane; j <= i; j += 32) {
-        double v = s[i * LD + j];
+      if (k0 > 0) {
+        // this block's rows of the previous panel (lane: row lane % 8), then
+        // its diagonal block's update (lane: two entries of that row)
+        const int i = k0 + (lane & 7);
+        double x[PW];
 #pragma unroll
-        for (int k = k0; k < k0 + PW; ++k) v -= s[i * LD + k] * s[j * LD + k];
-        s[i * LD + j] = v;
+        for (int j = 0; j < PW; ++j) x[j] = s[i * PLD + kp + j];
+        panel_row_solve(x, [&](int k) { return rd[k]; }, [&](int j, int k) { return d[j][k]; });
+        __syncwarp();
+        // (every store below is made by all the lanes that hold the value)
+#pragma unroll
+        for (int j = 0; j < PW; ++j) s[i * PLD + kp + j] = x[j];
+        __syncwarp();
+        asm volatile("bar.arrive 1, 256;" ::: "memory");
+        const int j0 = k0 + 2 * (lane >> 3);
+        double y0 = s[i * PLD + j0], y1 = s[i * PLD + j0 + 1];
+#pragma unroll
+        for (int k = 0; k < PW; ++k) {
+          y0 -= x[k] * s[j0 * PLD + kp + k];
+          y1 -= x[k] * s[(j0 + 1) * PLD + kp + k];
+        }
+        s[i * PLD + j0] = y0;
+        s[i * PLD + j0 + 1] = y1;
+        __syncwarp();
       }
+#pragma unroll
+      for (int i = 0; i < PW; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) d[i][j] = s[(k0 + i) * PLD + k0 + j];
+      bool bad = false;
+#pragma unroll
+      for (int k = 0; k < PW; ++k) {
+        const double p = d[k][k];
+        bad = bad || !(p > 0.);
+        const double dk = sqrt(p > 0. ? p : 1.), rdk = 1. / dk;
+        rd[k] = rdk;
+        d[k][k] = dk;
+#pragma unroll
+        for (int i = k + 1; i < PW; ++i) d[i][k] *= rdk;
+#pragma unroll
+        for (int j = k + 1; j < PW; ++j)
+#pragma unroll
+          for (int i = j; i < PW; ++i) d[i][j] -= d[i][k] * d[j][k];
+      }
+      if (bad && lane == 0) atomicOr(err, 4);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < PW; ++i) {
+        pp[k0 + i] = rd[i];
+#pragma unroll
+        for (int j = 0; j <= i; ++j) s[(k0 + i) * PLD + k0 + j] = d[i][j];
+      }
+    } else if (k0 > 0) {
+      if (w < 8) {
+        // the previous panel's rows past this block (warps 1 and 2)
+        const int i = k0 + PW + (w - 1) * 32 + lane;
+        if (i < CT) {
+          double x[PW];
+#pragma unroll
+          for (int j = 0; j < PW; ++j) x[j] = s[i * PLD + kp + j];
+          panel_row_solve(x, [&](int k) { return pp[kp + k]; },
+                          [&](int j, int k) { return s[(kp + j) * PLD + kp + k]; });
+#pragma unroll
+          for (int j = 0; j < PW; ++j) s[i * PLD + kp + j] = x[j];
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        // and its update of the columns j >= k0 (rows past this block):
+        // lane: rows lane, lane + 32, the columns dealt to the seven warps
+        double l[2][PW];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int k = 0; k < PW; ++k) l[h][k] = s[(lane + 32 * h) * PLD + kp + k];
+#pragma unroll 2
+        for (int j = k0 + w - 1; j < CT; j += 7) {
+          double m[PW];
+#pragma unroll
+          for (int k = 0; k < PW; ++k) m[k] = s[j * PLD + kp + k];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int row = lane + 32 * h;
+            if (row >= j && row >= k0 + PW) {
+              double y = s[row * PLD + j];
+#pragma unroll
+              for (int k = 0; k < PW; ++k) y -= l[h][k] * m[k];
+              s[row * PLD + j] = y;
+            }
+          }
+        }
+      } else {
+        inverse_block(kp, s, si, pp);
+      }
+    }
     __syncthreads();
   }
-  if (t < CT) pp[t] = 1. / s[t * LD + t];
-  __syncthreads();
-  {
-    const int c = t >> 2, q = t & 3;  // column c (0..63), partial q
-    for (int i = 0; i < CT; ++i) {
-      double acc = 0.;
-      if (c < i)
-        for (int mm = c + q; mm < i; mm += 4) acc += s[i * LD + mm] * si[mm * LD + c];
-      const double a1 = __shfl_down_sync(0xffffffffu, acc, 1);
-      const double p01 = acc + a1;  // lanes q = 0 and 2: (p0 + p1), (p2 + p3)
-      const double p23 = __shfl_down_sync(0xffffffffu, p01, 2);
-      if (q == 0) {
-        const double rdi = pp[i];
-        si[i * LD + c] = c < i ? -(p01 + p23) * rdi : (c == i ? rdi : 0.);
-      }
-      __syncwarp();
+  if (w >= 8)
+    inverse_block(CT - PW, s, si, pp);
+  else
+    for (int idx = t; idx < TS; idx += CTH / 2) {
+      const int i = idx >> 6, j = idx & 63;
+      gtile[idx] = j <= i ? s[i * PLD + j] : 0.;
     }
-  }
   __syncthreads();
-  for (int idx = t; idx < TS; idx += CTH) {
-    const int i = idx >> 6, j = idx & 63;
-    gtile[idx] = j <= i ? s[i * LD + j] : 0.;
-    ginv[idx] = si[i * LD + j];
+#pragma unroll
+  for (int q = 0; q < TS / CTH; ++q) {
+    const int idx = t + q * CTH;
+    ginv[idx] = si[(idx >> 6) * PLD + (idx & 63)];
   }
   __syncthreads();
 }
@@ -213,7 +341,10 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   const int G = gridDim.x;
   GridBarrier bar(T.bar, (unsigned)G, T.err, T.bar_ns);
   // tile 0's diagonal block
-  if (blockIdx.x == 0) potrf_tile(tile_at(T, 0, 0), T.Linv, T.err, sA, sB, sP);
+  if (blockIdx.x == 0) {
+    load_potrf_tile(tile_at(T, 0, 0), sA);
+    potrf_tile(tile_at(T, 0, 0), T.Linv, T.err, sA, sB, sP);
+  }
   if (!bar.sync()) return;
   // With the inverse, X = L^-1 is formed in the same loop: tile row J of X
   // in phase T of column J (X_Jj = Linv_J R_Jj, its R final after the
@@ -239,10 +370,10 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
         load_tile(sB, gt, true);  // R^T: the product Linv R as Linv (R^T)^T
       }
       __syncthreads();
-      double acc[8][2] = {};
+      double acc[NF][2] = {};
       gemm_nt(sA, sB, acc);
       __syncthreads();
-      for_frag([&](int j, int e, int r, int c) { gt[r * CT + c] = acc[j][e]; });
+      store_frag(gt, acc);
     }
     if (!bar.sync()) return;
     // U: A_IK -= L_IJ L_KJ^T (items 0 .. nu - 1); the tile (J+1, J+1) is
@@ -269,17 +400,23 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
         gt = T.X + tri(K, j) * TS;
       }
       __syncthreads();
-      double acc[8][2] = {};
+      double acc[NF][2] = {};
       gemm_nt(sA, sB, acc);
-      sub_frag(gt, acc);
       if (t == 0) {
+        // the tile goes on to its factorisation without leaving the CTA
         __syncthreads();
+        sub_frag_to(gt, acc, sA);
         potrf_tile(gt, T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
+      } else {
+        sub_frag(gt, acc);
       }
       if (G > 1 && blockIdx.x == 0) break;  // CTA 0: item 0 and the factor only
     }
-    if (m == 0 && J + 1 < T.nt && blockIdx.x == (J + 1) % G)
+    if (m == 0 && J + 1 < T.nt && blockIdx.x == (J + 1) % G) {
+      __syncthreads();
+      load_potrf_tile(tile_at(T, J + 1, J + 1), sA);
       potrf_tile(tile_at(T, J + 1, J + 1), T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
+    }
     if (!bar.sync()) return;
   }
   if (!T.want_inverse) return;
@@ -289,7 +426,7 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   for (long long t = blockIdx.x; t < no; t += G) {
     int bi, bk;
     tri_item(t, bi, bk);
-    double acc[8][2] = {};
+    double acc[NF][2] = {};
     for (int mt = bi; mt < nt; ++mt) {
       __syncthreads();
       load_tile(sA, T.X + tri(mt, bi) * TS, true);
@@ -297,8 +434,7 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
       __syncthreads();
       gemm_nt(sA, sB, acc);
     }
-    double *ga = T.Ainv + tri(bi, bk) * TS;
-    for_frag([&](int j, int e, int r, int c) { ga[r * CT + c] = acc[j][e]; });
+    store_frag(T.Ainv + tri(bi, bk) * TS, acc);
   }
 }
 
