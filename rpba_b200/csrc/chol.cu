@@ -10,14 +10,20 @@
 // envelope reaches column J.
 //
 // Right-looking, per tile column J:
-//   P  the diagonal tile is factored (one warp, shared memory) and inverted:
-//      L_JJ and L_JJ^-1 (Linv[J]);
+//   P  the diagonal tile is factored and inverted: L_JJ and L_JJ^-1
+//      (Linv[J]), potrf_tile;
 //   T  every tile below it: L_IJ = A_IJ L_JJ^-T, a tile product;
 //   U  the trailing tiles: A_IK -= L_IJ L_KJ^T for J < K <= I <= hrow[J].
-// Phases are separated by bounded grid barriers; the tiles of a phase are
-// dealt to the CTAs round robin.  The factorisation of tile J + 1 is done by
-// the CTA that applies its last update (in phase U of column J), so P costs
-// no barrier of its own.  A non-positive pivot sets bit 4 of the error word.
+// The chain P(J), T of tile (J + 1, J), U of tile (J + 1, J + 1), P(J + 1)
+// bounds the launch, so CTA 0 runs that chain alone, the tiles passing
+// through its shared memory, and the other CTAs the rest of T and U of
+// column J meanwhile (dealt round robin).  Two bounded grid barriers a
+// column: between the others' T and U (CTA 0 arrives once its tile of T is
+// stored and does not wait), and at the column's end.  A non-positive pivot
+// sets bit 4 of the error word.
+// Measured on the aerial system (26,991 unknowns, 422 tile columns, band of
+// 21 to 33 tiles): 13.9 ms with every CTA in step (two full barriers a
+// column, CTA 0's tile reloaded in each phase), 10.6 ms so.
 //
 // For a dense matrix the same launch can go on to the inverse:
 //   X  = L^-1, right-looking by tile rows: X_Ij = Linv_I R_Ij (j <= I), then
@@ -144,7 +150,7 @@ __device__ __forceinline__ void store_frag(double *gt, const double (&acc)[NF][2
 // inverse entry its four partial sums (terms mm = c + q, c + q + 4, ... in
 // order, then (p0 + p1) + (p2 + p3)), as the unblocked column loop takes
 // them, so the result does not depend on the distribution.
-// A tile takes 35,000 cycles (18 us; 125,000 with one warp factoring panels
+// A tile takes 31,800 cycles (16.5 us; 125,000 with one warp factoring panels
 // and the inverse formed after them).
 // s, si: two shared tiles (ld PLD); pp: CT doubles (reciprocal pivots).
 constexpr int PLD = CT + 1, PW = 8;
@@ -197,20 +203,19 @@ __device__ __forceinline__ void load_potrf_tile(const double *gtile, double *s) 
 
 // x (a row's eight entries of a panel) solved by the panel's diagonal block:
 // entry j takes the updates k = 0 .. j - 1 in order, then its pivot.
-template <class F, class G>
-__device__ __forceinline__ void panel_row_solve(double (&x)[PW], F rd, G l) {
+// (l: the block, ld PLD; rd: its reciprocal pivots)
+__device__ __forceinline__ void panel_row_solve(double (&x)[PW], const double *rd, const double *l) {
 #pragma unroll
   for (int k = 0; k < PW; ++k) {
-    x[k] *= rd(k);
+    x[k] *= rd[k];
 #pragma unroll
-    for (int j = k + 1; j < PW; ++j) x[j] -= x[k] * l(j, k);
+    for (int j = k + 1; j < PW; ++j) x[j] -= x[k] * l[j * PLD + k];
   }
 }
 
 __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, double *si, double *pp) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   __syncthreads();
-  double d[PW][PW], rd[PW];  // warp 0: the current diagonal block (lower), its reciprocal pivots
 #pragma unroll 1
   for (int k0 = 0; k0 < CT; k0 += PW) {
     const int kp = k0 - PW;  // the previous panel
@@ -222,7 +227,7 @@ __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, dou
         double x[PW];
 #pragma unroll
         for (int j = 0; j < PW; ++j) x[j] = s[i * PLD + kp + j];
-        panel_row_solve(x, [&](int k) { return rd[k]; }, [&](int j, int k) { return d[j][k]; });
+        panel_row_solve(x, pp + kp, s + kp * PLD + kp);
         __syncwarp();
         // (every store below is made by all the lanes that hold the value)
 #pragma unroll
@@ -240,6 +245,7 @@ __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, dou
         s[i * PLD + j0 + 1] = y1;
         __syncwarp();
       }
+      double d[PW][PW], rd[PW];  // the diagonal block (lower), its reciprocal pivots
 #pragma unroll
       for (int i = 0; i < PW; ++i)
 #pragma unroll
@@ -275,8 +281,7 @@ __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, dou
           double x[PW];
 #pragma unroll
           for (int j = 0; j < PW; ++j) x[j] = s[i * PLD + kp + j];
-          panel_row_solve(x, [&](int k) { return pp[kp + k]; },
-                          [&](int j, int k) { return s[(kp + j) * PLD + kp + k]; });
+          panel_row_solve(x, pp + kp, s + kp * PLD + kp);
 #pragma unroll
           for (int j = 0; j < PW; ++j) s[i * PLD + kp + j] = x[j];
         }
@@ -293,15 +298,19 @@ __device__ void potrf_tile(double *gtile, double *ginv, int *err, double *s, dou
           double m[PW];
 #pragma unroll
           for (int k = 0; k < PW; ++k) m[k] = s[j * PLD + kp + k];
+          // (rows that take no update are computed and not stored: no branch
+          // between the two rows' chains)
+          double y[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) y[h] = s[(lane + 32 * h) * PLD + j];
+#pragma unroll
+          for (int k = 0; k < PW; ++k)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) y[h] -= l[h][k] * m[k];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int row = lane + 32 * h;
-            if (row >= j && row >= k0 + PW) {
-              double y = s[row * PLD + j];
-#pragma unroll
-              for (int k = 0; k < PW; ++k) y -= l[h][k] * m[k];
-              s[row * PLD + j] = y;
-            }
+            if (row >= j && row >= k0 + PW) s[row * PLD + j] = y[h];
           }
         }
       } else {
@@ -340,8 +349,11 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   double *sA = csm, *sB = csm + CT * CLD, *sP = csm + 2 * CT * CLD;
   const int G = gridDim.x;
   GridBarrier bar(T.bar, (unsigned)G, T.err, T.bar_ns);
+  GridBarrier sub(T.bar + 1, (unsigned)G, T.err, T.bar_ns);
+  const bool lead = blockIdx.x == 0, solo = G == 1;
+  const int me = solo ? 0 : (int)blockIdx.x - 1, others = solo ? 1 : G - 1;
   // tile 0's diagonal block
-  if (blockIdx.x == 0) {
+  if (lead) {
     load_potrf_tile(tile_at(T, 0, 0), sA);
     potrf_tile(tile_at(T, 0, 0), T.Linv, T.err, sA, sB, sP);
   }
@@ -354,68 +366,89 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   const int nxj = T.want_inverse ? 1 : 0;
   for (int J = 0; J < T.nt; ++J) {
     const int h = T.hrow[J], m = h - J;
+    const int own = m > 0 ? 1 : 0;  // item 0 of T and of U is CTA 0's
     // T: L_IJ = A_IJ L_JJ^-T (items 0 .. m - 1); X_Jj = Linv_J R_Jj (items
     // m .. m + J with the inverse)
-    const int ntt = m + nxj * (J + 1);
-    for (int t = blockIdx.x; t < ntt; t += G) {
+    if (lead && own) {
       __syncthreads();
-      double *gt;
-      if (t < m) {
-        gt = tile_at(T, J + 1 + t, J);
-        load_tile(sA, gt, false);
-        load_tile(sB, T.Linv + (size_t)J * TS, false);
-      } else {
-        gt = T.X + tri(J, t - m) * TS;
-        load_tile(sA, T.Linv + (size_t)J * TS, false);
-        load_tile(sB, gt, true);  // R^T: the product Linv R as Linv (R^T)^T
-      }
+      load_tile(sA, tile_at(T, J + 1, J), false);
+      load_tile(sB, T.Linv + (size_t)J * TS, false);
       __syncthreads();
       double acc[NF][2] = {};
       gemm_nt(sA, sB, acc);
+      store_frag(tile_at(T, J + 1, J), acc);
       __syncthreads();
-      store_frag(gt, acc);
+#pragma unroll
+      for (int j = 0; j < NF; ++j)
+        *(double2 *)(sA + frag_row() * CLD + frag_col() + 8 * j) = make_double2(acc[j][0], acc[j][1]);
     }
-    if (!bar.sync()) return;
-    // U: A_IK -= L_IJ L_KJ^T (items 0 .. nu - 1); the tile (J+1, J+1) is
-    // then factored by the CTA of item 0, which takes no other item when
-    // there are other CTAs.  With the inverse also R_Kj -= L_KJ X_Jj, K > J,
-    // j <= J (items nu .. nu + m (J + 1) - 1).
-    const long long nu = (long long)m * (m + 1) / 2;
-    const long long ntu = nu + (long long)nxj * m * (J + 1);
-    const long long t0 = (G > 1 && blockIdx.x > 0) ? blockIdx.x : 0, dt = (G > 1 && blockIdx.x > 0) ? G - 1 : G;
-    for (long long t = (G > 1 && blockIdx.x == 0) ? 0 : t0; t < ntu; t += dt) {
-      __syncthreads();
-      double *gt;
-      if (t < nu) {
-        int bi, bk;
-        tri_item(t, bi, bk);
-        load_tile(sA, tile_at(T, J + 1 + bi, J), false);
-        load_tile(sB, tile_at(T, J + 1 + bk, J), false);
-        gt = tile_at(T, J + 1 + bi, J + 1 + bk);
-      } else {
-        const long long u = t - nu;
-        const int K = J + 1 + (int)(u / (J + 1)), j = (int)(u % (J + 1));
-        load_tile(sA, tile_at(T, K, J), false);
-        load_tile(sB, T.X + tri(J, j) * TS, true);
-        gt = T.X + tri(K, j) * TS;
-      }
-      __syncthreads();
-      double acc[NF][2] = {};
-      gemm_nt(sA, sB, acc);
-      if (t == 0) {
-        // the tile goes on to its factorisation without leaving the CTA
+    const int ntt = m + nxj * (J + 1);
+    if (!lead || solo)
+      for (int t = own + me; t < ntt; t += others) {
         __syncthreads();
-        sub_frag_to(gt, acc, sA);
-        potrf_tile(gt, T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
-      } else {
+        double *gt;
+        if (t < m) {
+          gt = tile_at(T, J + 1 + t, J);
+          load_tile(sA, gt, false);
+          load_tile(sB, T.Linv + (size_t)J * TS, false);
+        } else {
+          gt = T.X + tri(J, t - m) * TS;
+          load_tile(sA, T.Linv + (size_t)J * TS, false);
+          load_tile(sB, gt, true);  // R^T: the product Linv R as Linv (R^T)^T
+        }
+        __syncthreads();
+        double acc[NF][2] = {};
+        gemm_nt(sA, sB, acc);
+        __syncthreads();
+        store_frag(gt, acc);
+      }
+    // U: A_IK -= L_IJ L_KJ^T (items 0 .. nu - 1).  With the inverse also
+    // R_Kj -= L_KJ X_Jj, K > J, j <= J (items nu .. nu + m (J + 1) - 1).
+    if (!lead || solo) {
+      if (!sub.sync()) return;
+      const long long nu = (long long)m * (m + 1) / 2;
+      const long long ntu = nu + (long long)nxj * m * (J + 1);
+      for (long long t = own + me; t < ntu; t += others) {
+        __syncthreads();
+        double *gt;
+        if (t < nu) {
+          int bi, bk;
+          tri_item(t, bi, bk);
+          load_tile(sA, tile_at(T, J + 1 + bi, J), false);
+          load_tile(sB, tile_at(T, J + 1 + bk, J), false);
+          gt = tile_at(T, J + 1 + bi, J + 1 + bk);
+        } else {
+          const long long u = t - nu;
+          const int K = J + 1 + (int)(u / (J + 1)), j = (int)(u % (J + 1));
+          load_tile(sA, tile_at(T, K, J), false);
+          load_tile(sB, T.X + tri(J, j) * TS, true);
+          gt = T.X + tri(K, j) * TS;
+        }
+        __syncthreads();
+        double acc[NF][2] = {};
+        gemm_nt(sA, sB, acc);
         sub_frag(gt, acc);
       }
-      if (G > 1 && blockIdx.x == 0) break;  // CTA 0: item 0 and the factor only
+    } else {
+      sub.arrive();
     }
-    if (m == 0 && J + 1 < T.nt && blockIdx.x == (J + 1) % G) {
+    if (lead && J + 1 < T.nt) {
+      // the next diagonal tile: its last update from the tile of T in sA
+      double *gt = tile_at(T, J + 1, J + 1);
       __syncthreads();
-      load_potrf_tile(tile_at(T, J + 1, J + 1), sA);
-      potrf_tile(tile_at(T, J + 1, J + 1), T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
+      if (own) {
+        if (solo) {
+          load_tile(sA, tile_at(T, J + 1, J), false);
+          __syncthreads();
+        }
+        double acc[NF][2] = {};
+        gemm_nt(sA, sA, acc);
+        __syncthreads();
+        sub_frag_to(gt, acc, sA);
+      } else {
+        load_potrf_tile(gt, sA);
+      }
+      potrf_tile(gt, T.Linv + (size_t)(J + 1) * TS, T.err, sA, sB, sP);
     }
     if (!bar.sync()) return;
   }

@@ -45,6 +45,16 @@ struct GridBarrier {
                                          unsigned long long limit_ns_ = BAR_TIMEOUT_NS)
       : cnt(cnt_), nblocks(nblocks_), err(err_), limit_ns(limit_ns_), target(0) {}
 
+  // Arrival without the wait, for a CTA that needs none of the others'
+  // results yet (it must not call sync() on the same barrier).
+  __device__ __forceinline__ void arrive() {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      fence_gpu();
+      red_add_gpu(cnt, 1u);
+    }
+  }
+
   __device__ __forceinline__ bool sync() {
     __syncthreads();
     int bad = 0;
