@@ -158,6 +158,7 @@ struct DirectWork {
   double *tiles = nullptr;         // [ntiles][64 * 64] lower envelope, then L
   double *Linv = nullptr;          // [nt][64 * 64] inverses of the diagonal tiles
   double *y = nullptr;             // [nt * 64] right-hand side / solution, factor order
+  ulonglong2 *pub = nullptr;       // [2][nt * 64] the substitutions' finished entries, with flags
   long long *toff = nullptr;       // [nt] first tile of each tile row
   int *fcol = nullptr, *hrow = nullptr;  // [nt] first tile column of a row, last tile row of a column
   int *pos = nullptr;              // [nimg] first unknown of each camera in factor order
