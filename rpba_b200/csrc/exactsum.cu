@@ -11,7 +11,7 @@
 // binade each element acts on the parity p of the running integer sum as a
 // two-state transform  p -> (increment r(p), new parity q(p)), and a run of
 // elements is the composition of their transforms, an associative operation:
-// a grid-wide scan of per-thread and per-CTA composites gives every prefix
+// scans of per-thread, per-warp and per-CTA composites give every prefix
 // without a sequential pass, ties included.  A run ends only at the first
 // element k with S + R_(k-1) + floor(v_k/u) >= 2^24 (the sum leaves the
 // binade); that element is added with a real float addition and a new run
@@ -22,10 +22,21 @@
 // window in the same binade), so the steps together read the input about
 // twice instead of once per binade.
 //
+// A step is latency: a scan over the window's composites, the search for the
+// crossing element, and in the grid form one barrier and one published word.
+// So the first ES_SOLO elements are summed by one CTA (its steps are two
+// block barriers each), inputs up to that length by a kernel of one CTA, not
+// cooperative; longer ones go on with one CTA per SM.  Measured (18 to 20
+// sums a solve): 5.4k terms 82 -> 25 us, 30k 115 -> 43 us, 0.87M 277 ->
+// 112 us, 28M 704 -> 242 us; before, the first 2,048 elements were added
+// at 25 cycles each, a step took four grid barriers, and one thread walked
+// the chunks' composites.
+//
 // The first HEAD elements and any stretch where s is zero or subnormal are
 // added by one warp in plain sequence.  Inputs must be finite and >= 0.
 #include <cuda.h>
 
+#include <climits>
 #include <mutex>
 
 #include "../../include/rpba_b200.h"
@@ -36,304 +47,437 @@ namespace rpba {
 
 namespace {
 
-constexpr int ES_T = 256;
-constexpr int HEAD = 2048;
-constexpr long long RCLAMP = 1ll << 30;  // n * RCLAMP < 2^61 for n < 2^31
+constexpr int ES_T = 1024;
+constexpr int ES_W = ES_T / 32;
+constexpr int HEAD = 512;        // elements added in plain sequence
+constexpr int ES_SEQ = 1024;     // elements per sequential block at most
+constexpr int ES_WMIN = 2048;    // smallest window of a run step
+constexpr int ES_SOLO = 65536;   // elements one CTA sums (a solo step past it costs more than a grid step)
+constexpr int ES_MAXG = 256;     // CTAs at most (eight composites a lane)
 constexpr int MAX_SEGMENTS = 512;
-constexpr int ES_WMIN = 65536;  // smallest window of a run step
-constexpr int ES_MAXG = 512;    // CTAs at most (their composites are staged in shared memory)
-
-struct EsCtl {
-  float s;    // running sum before element i
-  int i;      // next element
-};
+// Increments saturate here: a run crosses its binade long before (at 2^24),
+// and nothing past the first crossing is used.
+constexpr int SAT = 1 << 26;
+constexpr int TOP = 1 << 24;
 
 // Composite transform of a run of elements for incoming parity 0 and 1:
-// total increment R, outgoing parity q, and M = max over the run of
-// (increment before the element + floor(v/u)), the crossing test.
+// total increment R, M = max over the run of (increment before the element +
+// floor(v/u)), the crossing test (-1: no element), and the outgoing parities
+// (bit p of q).
 struct Xf {
-  long long R[2], M[2];
-  int q[2];
+  int R0, R1, M0, M1;
+  unsigned q;
 };
-__device__ __forceinline__ Xf xf_identity() {
+__device__ __forceinline__ Xf xf_identity() { return Xf{0, 0, -1, -1, 2u}; }
+// a then b
+__device__ __forceinline__ Xf xf_then(const Xf &a, const Xf &b) {
+  const bool m0 = a.q & 1u, m1 = a.q & 2u;
+  const int bM0 = m0 ? b.M1 : b.M0, bM1 = m1 ? b.M1 : b.M0;
   Xf x;
-  for (int p = 0; p < 2; ++p) {
-    x.R[p] = 0;
-    x.M[p] = LLONG_MIN;
-    x.q[p] = p;
+  x.R0 = min(a.R0 + (m0 ? b.R1 : b.R0), SAT);
+  x.R1 = min(a.R1 + (m1 ? b.R1 : b.R0), SAT);
+  x.M0 = max(a.M0, bM0 < 0 ? -1 : min(a.R0 + bM0, SAT));
+  x.M1 = max(a.M1, bM1 < 0 ? -1 : min(a.R1 + bM1, SAT));
+  x.q = ((b.q >> (m0 ? 1 : 0)) & 1u) | (((b.q >> (m1 ? 1 : 0)) & 1u) << 1);
+  return x;
+}
+__device__ __forceinline__ Xf xf_up(const Xf &a, int o) {
+  Xf x;
+  x.R0 = __shfl_up_sync(0xffffffffu, a.R0, o);
+  x.R1 = __shfl_up_sync(0xffffffffu, a.R1, o);
+  x.M0 = __shfl_up_sync(0xffffffffu, a.M0, o);
+  x.M1 = __shfl_up_sync(0xffffffffu, a.M1, o);
+  x.q = __shfl_up_sync(0xffffffffu, a.q, o);
+  return x;
+}
+// Inclusive scan over the warp's lanes, in lane order.
+__device__ __forceinline__ Xf xf_scan(Xf x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Xf u = xf_up(x, o);
+    if (lane >= o) x = xf_then(u, x);
   }
   return x;
 }
-// a then b
-__device__ __forceinline__ Xf xf_then(const Xf &a, const Xf &b) {
-  Xf x;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const bool m = a.q[p] != 0;  // b's state entered with parity a.q[p] (selects: no indexing)
-    const long long bR = m ? b.R[1] : b.R[0], bM = m ? b.M[1] : b.M[0];
-    x.R[p] = a.R[p] + bR;
-    x.q[p] = m ? b.q[1] : b.q[0];
-    x.M[p] = bM == LLONG_MIN ? a.M[p] : max(a.M[p], a.R[p] + bM);
+__device__ __forceinline__ Xf xf_exclusive(const Xf &incl, int lane) {
+  const Xf u = xf_up(incl, 1);
+  return lane == 0 ? xf_identity() : u;
+}
+
+// The binade of a normal s: unit u, v -> v / u as two exact float factors
+// (powers of two whose product can be outside the float range), S = s / u.
+struct Binade {
+  float s1, s2;
+  int S;
+  double u;
+};
+__device__ __forceinline__ Binade binade_of(float s) {
+  Binade b;
+  int E;
+  frexpf(s, &E);
+  E -= 1;  // s in [2^E, 2^(E+1))
+  const int k = 23 - E, k1 = k / 2;
+  b.s1 = ldexpf(1.f, k1);
+  b.s2 = ldexpf(1.f, k - k1);
+  b.S = (int)((s * b.s1) * b.s2);
+  b.u = ldexp(1.0, E - 23);
+  return b;
+}
+__device__ __forceinline__ float binade_value(const Binade &b, int S) { return (float)((double)S * b.u); }
+
+// floor(v/u), rne(v/u) away from ties, and whether v/u is a tie; past the
+// saturation (or not a number) the element crosses in any case.
+__device__ __forceinline__ void classify(float v, const Binade &b, int &fl, int &r, bool &tie) {
+  const float f = (v * b.s1) * b.s2;
+  if (!(f < (float)SAT)) {
+    fl = r = SAT;
+    tie = false;
+    return;
   }
+  const float ff = floorf(f), fr = f - ff;
+  fl = (int)ff;
+  tie = fr == 0.5f;
+  r = fl + (fr > 0.5f ? 1 : 0);
+}
+
+// Apply one element to a composite (both incoming parities).
+__device__ __forceinline__ void xf_push(Xf &x, int fl, int r, bool tie) {
+  const int r0 = tie ? fl + (((int)(x.q & 1u) + fl) & 1) : r;
+  const int r1 = tie ? fl + (((int)(x.q >> 1) + fl) & 1) : r;
+  x.M0 = max(x.M0, min(x.R0 + fl, SAT));
+  x.M1 = max(x.M1, min(x.R1 + fl, SAT));
+  x.R0 = min(x.R0 + r0, SAT);
+  x.R1 = min(x.R1 + r1, SAT);
+  x.q ^= (unsigned)(r0 & 1) | ((unsigned)(r1 & 1) << 1);
+}
+
+// Composite of v[lo, hi): 16-byte loads of whole aligned groups.
+__device__ __forceinline__ Xf xf_range(const float *__restrict__ v, int lo, int hi, bool aligned, const Binade &b) {
+  Xf x = xf_identity();
+  auto push = [&](float a) {
+    int fl, r;
+    bool tie;
+    classify(a, b, fl, r, tie);
+    xf_push(x, fl, r, tie);
+  };
+  int k = lo;
+  if (aligned) {
+    for (; k < hi && (k & 3); ++k) push(__ldg(v + k));
+#pragma unroll 2
+    for (; k + 4 <= hi; k += 4) {
+      const float4 a = __ldg((const float4 *)(v + k));
+      push(a.x);
+      push(a.y);
+      push(a.z);
+      push(a.w);
+    }
+  }
+  for (; k < hi; ++k) push(__ldg(v + k));
   return x;
+}
+
+// Adds v[k..) onto the state (R, q) up to the element that crosses, then that
+// element with a float addition.
+__device__ __forceinline__ void cross_element(const float *__restrict__ v, int lo, int hi, int n, const Binade &b,
+                                              int R, int q, float &s, int &i) {
+  for (int k = lo; k < hi; ++k) {
+    int fl, r;
+    bool tie;
+    classify(__ldg(v + k), b, fl, r, tie);
+    if (b.S + R + fl >= TOP) {
+      s = __fadd_rn(binade_value(b, b.S + R), __ldg(v + k));
+      i = isfinite(s) ? k + 1 : n;
+      return;
+    }
+    const int rr = tie ? fl + ((q + fl) & 1) : r;
+    R += rr;
+    q = (q + rr) & 1;
+  }
+}
+
+struct __align__(16) EsShared {
+  float buf[ES_SEQ];  // first: read 16 bytes at a time
+  Xf w[ES_W];         // the warps' composites
+  float s;
+  int i;
+  int R, q;           // grid step: the state before the chunk that crosses
+  int cx;             // grid step: the chunk that crosses, or -1
+};
+
+// v[i, i + cnt) added in plain sequence onto s by warp 0 (cnt <= ES_SEQ); the
+// values are staged in shared memory, so the chain is the additions alone.
+// Valid in warp 0.
+__device__ __forceinline__ float seq_block(const float *__restrict__ v, int i, int cnt, float s, float *buf) {
+  __syncthreads();
+  for (int j = threadIdx.x; j < cnt; j += blockDim.x) buf[j] = __ldg(v + i + j);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int j = 0;
+#pragma unroll 4
+    for (; j + 4 <= cnt; j += 4) {
+      const float4 a = *(const float4 *)(buf + j);
+      s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
+    }
+    for (; j < cnt; ++j) s = __fadd_rn(s, buf[j]);
+  }
+  return s;
+}
+
+// The window [i0, wend) cut into `parts` pieces at multiples of four, and
+// thread tid's range of piece `part`.
+__device__ __forceinline__ void thread_range(int i0, int wend, int part, int parts, int &lo, int &hi) {
+  const int base = i0 & ~3;
+  const int per = (((wend - base + parts - 1) / parts + ES_T - 1) / ES_T + 3) & ~3;
+  const long long a = (long long)base + ((long long)part * ES_T + threadIdx.x) * per;
+  lo = (int)max((long long)i0, min(a, (long long)wend));
+  hi = (int)min(a + per, (long long)wend);
+}
+
+// Sums from the front until at least `stop` elements are taken (or n) and s
+// is normal; the state is left in sh.s, sh.i.
+__device__ void es_solo(const float *__restrict__ v, int n, int stop, bool aligned, EsShared &sh) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float s = 0.f;
+  int i = 0;
+  for (int seg = 0;; ++seg) {
+    // plain sequence: the head, the zero and subnormal range, and past
+    // MAX_SEGMENTS steps (far more than sums of real data take) the rest
+    while (i < n && (i < HEAD || !(s >= 1.17549435e-38f) || seg >= MAX_SEGMENTS)) {
+      const int cnt = min(n - i, i < HEAD ? HEAD - i : ES_SEQ);
+      const float t = seq_block(v, i, cnt, s, sh.buf);
+      if (tid == 0) sh.s = t;
+      __syncthreads();
+      s = sh.s;
+      i = isfinite(s) ? i + cnt : n;
+    }
+    if (i >= n || i >= stop) break;
+    const Binade b = binade_of(s);
+    const int p0 = b.S & 1;
+    const int wend = (int)min((long long)n, (long long)i + max(i, ES_WMIN));
+    int lo, hi;
+    thread_range(i, wend, 0, 1, lo, hi);
+    const Xf tx = xf_range(v, lo, hi, aligned, b);
+    const Xf incl = xf_scan(tx, lane);
+    if (lane == 31) sh.w[warp] = incl;
+    __syncthreads();
+    // every warp: the state before each warp, and the first that crosses
+    const Xf wx = sh.w[lane];
+    const Xf wi = xf_scan(wx, lane), we = xf_exclusive(wi, lane);
+    const int Re = p0 ? we.R1 : we.R0, qe = (we.q >> p0) & 1u;
+    const int Mw = qe ? wx.M1 : wx.M0;
+    const unsigned hit = __ballot_sync(0xffffffffu, Mw >= 0 && b.S + Re + Mw >= TOP);
+    if (hit == 0) {
+      const int R = p0 ? wi.R1 : wi.R0;
+      s = binade_value(b, b.S + __shfl_sync(0xffffffffu, R, 31));
+      i = wend;
+    } else {
+      const int cw = __ffs(hit) - 1;
+      const int Rw = __shfl_sync(0xffffffffu, Re, cw), qw = __shfl_sync(0xffffffffu, qe, cw);
+      if (warp == cw) {
+        const Xf ex = xf_exclusive(incl, lane);
+        const int R = Rw + (qw ? ex.R1 : ex.R0), q = (ex.q >> qw) & 1u;
+        const int M = q ? tx.M1 : tx.M0;
+        const unsigned h2 = __ballot_sync(0xffffffffu, M >= 0 && b.S + R + M >= TOP);
+        if (lane == __ffs(h2) - 1) {
+          float sn = s;
+          int in = n;
+          cross_element(v, lo, hi, n, b, R, q, sn, in);
+          sh.s = sn;
+          sh.i = in;
+        }
+      }
+      __syncthreads();
+      s = sh.s;
+      i = sh.i;
+    }
+    __syncthreads();  // sh is free
+  }
+  __syncthreads();
+  if (tid == 0) {
+    sh.s = s;
+    sh.i = i;
+  }
+  __syncthreads();
+}
+
+// One CTA: the whole sum.
+__global__ void __launch_bounds__(ES_T) k_exact_sum_solo(const float *v, int n, float *out) {
+  __shared__ EsShared sh;
+  es_solo(v, n, n, ((unsigned long long)v & 15ull) == 0, sh);
+  if (threadIdx.x == 0) *out = sh.s;
 }
 
 struct EsArgs {
   const float *v;
   int n;
   float *out;
-  long long *Rc, *Mc;  // per CTA composite: R[2], M[2]
-  int *Tc;             // per CTA composite: q[2]
-  EsCtl *ctl;
-  unsigned *bar;
+  int *comp;                // [2][ES_MAXG][8] the CTAs' composites, by step parity
+  unsigned *bar;            // the barrier counter; zero before the launch, as pub
+  unsigned long long *pub;  // [2] the published state: (s, tag), (i, tag), tag = step + 1
   int *err;
 };
 
-__device__ __forceinline__ void classify(float v, double scale, long long &fl, long long &r, bool &tie) {
-  const double f = (double)v * scale;
-  if (f >= (double)RCLAMP) {
-    fl = r = RCLAMP;
-    tie = false;
-    return;
-  }
-  const double ff = floor(f);
-  const double fr = f - ff;
-  fl = (long long)ff;
-  tie = fr == 0.5;
-  r = fl + (fr > 0.5 ? 1 : 0);
+// A state published by one CTA to all (each 8-byte word carries its tag).
+__device__ __forceinline__ void es_publish(const EsArgs &A, float s, int i, unsigned tag) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(A.pub),
+               "l"((unsigned long long)__float_as_uint(s) | ((unsigned long long)tag << 32))
+               : "memory");
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(A.pub + 1),
+               "l"((unsigned long long)(unsigned)i | ((unsigned long long)tag << 32))
+               : "memory");
 }
-
-// Apply one element to a composite (in place, both incoming parities).
-__device__ __forceinline__ void xf_push(Xf &x, long long fl, long long r, bool tie) {
-  for (int p = 0; p < 2; ++p) {
-    const long long m = x.R[p] + fl;
-    if (m > x.M[p]) x.M[p] = m;
-    const long long rr = tie ? fl + ((x.q[p] + fl) & 1) : r;
-    x.R[p] += rr;
-    x.q[p] = (int)((x.q[p] + rr) & 1);
-  }
-}
-
-// Sequential float additions of v[i..i_end) onto s by one warp.
-__device__ float warp_seq(const float *v, int i, int i_end, float s) {
-  const int lane = threadIdx.x & 31;
-  for (int base = i; base < i_end; base += 32) {
-    const int idx = base + lane;
-    const float x = idx < i_end ? v[idx] : 0.f;
-#pragma unroll 8
-    for (int l = 0; l < 32; ++l) {
-      const float t = __shfl_sync(0xffffffffu, x, l);
-      if (base + l < i_end) s = __fadd_rn(s, t);
-    }
-  }
-  return s;
-}
-
-__global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
-  const int G = gridDim.x, c = blockIdx.x, tid = threadIdx.x;
-  const int n = A.n;
-  GridBarrier bar(A.bar, (unsigned)G, A.err);
-  __shared__ Xf s_x[ES_T];  // per-thread composites of the current run
-  __shared__ Xf s_w[ES_T / 32];  // per-warp composites
-  __shared__ long long s_cR[2 * ES_MAXG], s_cM[2 * ES_MAXG];  // the chunks' composites
-  __shared__ unsigned char s_cT[2 * ES_MAXG];
-  __shared__ long long s_rtot, s_R;
-  __shared__ int s_cx, s_qx, s_tcross, s_q;
-
-  if (c == 0 && tid < 32) {
-    float s = warp_seq(A.v, 0, min(n, HEAD), 0.f);
-    int i = min(n, HEAD);
-    // leave the zero / subnormal range one element at a time
-    while (i < n && !(s >= 1.17549435e-38f) && isfinite(s)) {
-      s = __fadd_rn(s, A.v[i]);
-      ++i;
-    }
-    if (tid == 0) {
-      A.ctl->s = s;
-      A.ctl->i = isfinite(s) ? i : n;
-    }
-  }
-  if (!bar.sync()) return;
-
-  for (int seg = 0;; ++seg) {
-    const float s = __ldcg(&A.ctl->s);
-    const int i0 = __ldcg(&A.ctl->i);
-    if (i0 >= n) break;
-    if (seg >= MAX_SEGMENTS) {
-      // far more steps (binade changes and windows) than sums of real data
-      // take: finish in plain sequence, still exact
-      if (c == 0 && tid < 32) {
-        const float sr = warp_seq(A.v, i0, n, s);
-        if (tid == 0) A.ctl->s = sr;
+// Bounded wait for the state with this tag (thread 0 polls); false in every
+// thread when it ran out.
+__device__ __forceinline__ bool es_receive(const EsArgs &A, unsigned tag, EsShared &sh) {
+  int bad = 0;
+  if (threadIdx.x == 0) {
+    unsigned long long a, b, t0 = 0;
+    for (unsigned n = 1;; ++n) {
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(A.pub) : "memory");
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(A.pub + 1) : "memory");
+      if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag) break;
+      if ((n & 15u) == 0 && ld_relaxed_gpu((const unsigned *)A.err) != 0) {
+        bad = 1;
+        break;
       }
+      if ((n & 63u) == 0) {
+        const unsigned long long t = gtimer();
+        if (t0 == 0)
+          t0 = t;
+        else if (t - t0 > BAR_TIMEOUT_NS)
+          atomicOr(A.err, 2);
+      }
+    }
+    sh.s = __uint_as_float((unsigned)a);
+    sh.i = (int)(unsigned)b;
+  }
+  return __syncthreads_or(bad) == 0;
+}
+
+// One CTA per SM.  Step k: every CTA's chunk composite, barrier, every CTA
+// walks the composites (warp 0, a scan); without a crossing all know the next
+// state, otherwise the crossing CTA finds the element and publishes it.
+__global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
+  const int G = gridDim.x, c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = A.n;
+  const bool aligned = ((unsigned long long)A.v & 15ull) == 0;
+  GridBarrier bar(A.bar, (unsigned)G, A.err);
+  __shared__ EsShared sh;
+  unsigned tag = 1;
+  if (c == 0) {
+    es_solo(A.v, n, ES_SOLO, aligned, sh);
+    if (tid == 0) es_publish(A, sh.s, sh.i, tag);
+  }
+  if (!es_receive(A, tag, sh)) return;
+  float s = sh.s;
+  int i = sh.i;
+  __syncthreads();
+  for (unsigned step = 0; i < n; ++step) {
+    if (step >= MAX_SEGMENTS) {
+      // finish in plain sequence, still exact
+      if (c == 0)
+        for (; i < n; i += ES_SEQ) s = seq_block(A.v, i, min(n - i, ES_SEQ), s, sh.buf);
       break;
     }
-    int E;
-    frexpf(s, &E);
-    E -= 1;  // s in [2^E, 2^(E+1))
-    const double u = ldexp(1.0, E - 23);
-    const double scale = ldexp(1.0, 23 - E);
-    const long long S = (long long)((double)s * scale);
-    const int p0 = (int)(S & 1);
-    const long long TOP = 1ll << 24;
-
-    // The step's window: the elements from i0 on, as many again as the sum
-    // has taken so far (at least ES_WMIN).  The sum leaves its binade when it
-    // doubles, so the crossing is inside the window unless the terms shrink;
-    // a window without a crossing ends the step at its last element, the sum
-    // still in the same binade, and the next step takes the next window.
-    // The window is cut into G chunks (CTA c: chunk c).
-    const int wend = (int)min((long long)n, (long long)i0 + max((long long)i0, (long long)ES_WMIN));
-    const int chunk = (wend - i0 + G - 1) / G;
-    const int lo = min(wend, i0 + c * chunk), hi = min(wend, lo + chunk);
-    const int per = (chunk + ES_T - 1) / ES_T;
-    // phase A: composite of each thread's contiguous sub-range of this
-    // chunk, then of the chunk
-    const int a0 = max(lo, i0);
-    const int t_lo = lo + tid * per, t_hi = min(hi, t_lo + per);
-    Xf tx = xf_identity();
-    for (int k = max(t_lo, a0); k < t_hi; ++k) {
-      long long fl, r;
-      bool tie;
-      classify(A.v[k], scale, fl, r, tie);
-      xf_push(tx, fl, r, tie);
-    }
-    s_x[tid] = tx;  // kept for the crossing chunk's walk
-    // the chunk's composite: each warp's thread composites combined in a
-    // tree that keeps lane order ((x0 x1)(x2 x3))..., then the warps' in
-    // order (the composition is exact integer arithmetic and associative)
+    ++tag;
+    const Binade b = binade_of(s);
+    const int p0 = b.S & 1;
+    const int wend = (int)min((long long)n, 2ll * (long long)i);
+    int lo, hi;
+    thread_range(i, wend, c, G, lo, hi);
+    const Xf tx = xf_range(A.v, lo, hi, aligned, b);
+    const Xf incl = xf_scan(tx, lane);
+    if (lane == 31) sh.w[warp] = incl;
+    __syncthreads();
+    int *comp = A.comp + (size_t)(step & 1u) * ES_MAXG * 8;
+    Xf wx, we;  // every warp: the warps' composites and the ones before them
     {
-      const int lane = tid & 31;
-      Xf wx = tx;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        Xf ot;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          ot.R[p] = __shfl_down_sync(0xffffffffu, wx.R[p], o);
-          ot.M[p] = __shfl_down_sync(0xffffffffu, wx.M[p], o);
-          ot.q[p] = __shfl_down_sync(0xffffffffu, wx.q[p], o);
-        }
-        if ((lane & (2 * o - 1)) == 0) wx = xf_then(wx, ot);
-      }
-      if (lane == 0) s_w[tid >> 5] = wx;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      Xf cx = s_w[0];
-      for (int w = 1; w < ES_T / 32; ++w) cx = xf_then(cx, s_w[w]);
-      for (int p = 0; p < 2; ++p) {
-        A.Rc[2 * c + p] = cx.R[p];
-        A.Mc[2 * c + p] = cx.M[p];
-        A.Tc[2 * c + p] = cx.q[p];
+      wx = sh.w[lane];
+      const Xf wi = xf_scan(wx, lane);
+      we = xf_exclusive(wi, lane);
+      if (warp == 0 && lane == 31) {
+        *(int4 *)(comp + 8 * c) = make_int4(wi.R0, wi.R1, wi.M0, wi.M1);
+        comp[8 * c + 4] = (int)wi.q;
       }
     }
     if (!bar.sync()) return;
-
-    // phase B (every CTA, one thread): walk the chunk composites in order
-    // from the run's start state; find the first chunk that crosses, the
-    // state at its start, and the state at the end
-    // (the composites are first copied to shared memory by all threads,
-    // independent loads, so the walk's dependent steps are shared loads)
-    for (int j = tid; j < 2 * G; j += ES_T) {
-      s_cR[j] = __ldcg(A.Rc + j);
-      s_cM[j] = __ldcg(A.Mc + j);
-      s_cT[j] = (unsigned char)__ldcg(A.Tc + j);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      long long R = 0;
-      int q = p0, cxq = INT_MAX;
-      long long Rx = 0;
-      int qx = 0;
-      for (int cc = 0; cc < G; ++cc) {
-        const long long Mq = s_cM[2 * cc + q];
-        if (Mq != LLONG_MIN && S + R + Mq >= TOP) {
-          cxq = cc;
-          Rx = R;
-          qx = q;
-          break;
+    if (warp == 0) {
+      // lane: the composites of chunks per * lane .. + per - 1
+      const int per = (G + 31) / 32;
+      Xf cx[ES_MAXG / 32];
+      Xf x = xf_identity();
+#pragma unroll
+      for (int j = 0; j < ES_MAXG / 32; ++j) {
+        const int cc = per * lane + j;
+        cx[j] = xf_identity();
+        if (j < per && cc < G) {
+          const int4 a = __ldcg((const int4 *)(comp + 8 * cc));
+          cx[j] = Xf{a.x, a.y, a.z, a.w, (unsigned)__ldcg(comp + 8 * cc + 4)};
         }
-        R += s_cR[2 * cc + q];
-        q = s_cT[2 * cc + q];
+        x = xf_then(x, cx[j]);
       }
-      s_cx = cxq;
-      s_rtot = cxq == INT_MAX ? R : Rx;
-      s_qx = qx;
-    }
-    __syncthreads();
-    const int cxi = s_cx;
-    if (cxi == INT_MAX) {
-      if (c == 0 && tid == 0) {
-        A.ctl->s = (float)((double)(S + s_rtot) * u);
-        A.ctl->i = wend;
-      }
-    } else if (c == cxi) {
-      // the crossing chunk: thread 0 finds the first crossing thread range,
-      // whose thread then finds the element and adds it with a float addition
-      if (tid == 0) {
-        long long R = s_rtot;
-        int q = s_qx;
-        int tx_first = ES_T;
-        for (int t = 0; t < ES_T; ++t) {
-          const Xf &x = s_x[t];
-          if (x.M[q] != LLONG_MIN && S + R + x.M[q] >= TOP) {
-            tx_first = t;
-            break;
+      const Xf xi = xf_scan(x, lane), xe = xf_exclusive(xi, lane);
+      const int Re = p0 ? xe.R1 : xe.R0, qe = (xe.q >> p0) & 1u;
+      const int M = qe ? x.M1 : x.M0;
+      const unsigned hit = __ballot_sync(0xffffffffu, M >= 0 && b.S + Re + M >= TOP);
+      if (hit == 0) {
+        if (lane == 31) {
+          sh.cx = -1;
+          sh.R = p0 ? xi.R1 : xi.R0;
+        }
+      } else if (lane == __ffs(hit) - 1) {
+        int R = Re, q = qe, at = -1;
+#pragma unroll
+        for (int j = 0; j < ES_MAXG / 32; ++j) {
+          const int Mj = q ? cx[j].M1 : cx[j].M0;
+          if (at < 0) {
+            if (Mj >= 0 && b.S + R + Mj >= TOP) {
+              at = per * lane + j;
+            } else {
+              R += q ? cx[j].R1 : cx[j].R0;
+              q = (cx[j].q >> q) & 1u;
+            }
           }
-          R += x.R[q];
-          q = x.q[q];
         }
-        s_tcross = tx_first;
-        s_R = R;
-        s_q = q;
+        sh.cx = at;
+        sh.R = R;
+        sh.q = q;
       }
+    }
+    __syncthreads();
+    if (sh.cx < 0) {
+      s = binade_value(b, b.S + sh.R);
+      i = wend;
       __syncthreads();
-      if (tid == s_tcross) {
-        long long R = s_R;
-        int q = s_q;
-        for (int k = max(t_lo, a0); k < t_hi; ++k) {
-          long long fl, r;
-          bool tie;
-          classify(A.v[k], scale, fl, r, tie);
-          if (S + R + fl >= TOP) {
-            const float sb = (float)((double)(S + R) * u);
-            const float sn = __fadd_rn(sb, A.v[k]);
-            A.ctl->s = sn;
-            A.ctl->i = isfinite(sn) ? k + 1 : n;
-            break;
-          }
-          const long long rr = tie ? fl + ((q + fl) & 1) : r;
-          R += rr;
-          q = (int)((q + rr) & 1);
+      continue;
+    }
+    if (sh.cx == c) {
+      const int R0 = sh.R, q0 = sh.q;
+      // the first warp of the chunk that crosses, its first thread, the element
+      const int Re = R0 + (q0 ? we.R1 : we.R0), qe = (we.q >> q0) & 1u;
+      const int Mw = qe ? wx.M1 : wx.M0;
+      const unsigned hit = __ballot_sync(0xffffffffu, Mw >= 0 && b.S + Re + Mw >= TOP);
+      const int cw = __ffs(hit) - 1;
+      const int Rw = __shfl_sync(0xffffffffu, Re, cw), qw = __shfl_sync(0xffffffffu, qe, cw);
+      if (warp == cw) {
+        const Xf ex = xf_exclusive(incl, lane);
+        const int R = Rw + (qw ? ex.R1 : ex.R0), q = (ex.q >> qw) & 1u;
+        const int M = q ? tx.M1 : tx.M0;
+        const unsigned h2 = __ballot_sync(0xffffffffu, M >= 0 && b.S + R + M >= TOP);
+        if (lane == __ffs(h2) - 1) {
+          float sn = s;
+          int in = n;
+          cross_element(A.v, lo, hi, n, b, R, q, sn, in);
+          es_publish(A, sn, in, tag);
         }
       }
     }
-    if (!bar.sync()) return;
-    // a new run that starts in the zero/subnormal range is continued in sequence
-    if (c == 0 && tid < 32) {
-      float s2 = __ldcg(&A.ctl->s);
-      int i2 = __ldcg(&A.ctl->i);
-      bool moved = false;
-      while (i2 < n && !(s2 >= 1.17549435e-38f)) {
-        s2 = __fadd_rn(s2, A.v[i2]);
-        ++i2;
-        moved = true;
-      }
-      if (moved && tid == 0) {
-        A.ctl->s = s2;
-        A.ctl->i = i2;
-      }
-    }
-    if (!bar.sync()) return;
+    if (!es_receive(A, tag, sh)) return;
+    s = sh.s;
+    i = sh.i;
+    __syncthreads();
   }
-  if (c == 0 && tid == 0) *A.out = __ldcg(&A.ctl->s);
-}
-
-// Sequential float sum by one warp, for short arrays.
-__global__ void k_warp_sum(const float *v, int n, float *out) {
-  const float s = warp_seq(v, 0, n, 0.f);
-  if (threadIdx.x == 0) *out = s;
+  if (c == 0 && tid == 0) *A.out = s;
 }
 
 }  // namespace
@@ -342,32 +486,31 @@ int exact_sum_max_grid(int device) {
   int nsm = 0, per = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact_sum, ES_T, 0);
-  if (per < 1) per = 1;
-  const int g = nsm * (per < 2 ? per : 2);
+  const int g = per < 1 ? 1 : nsm;
   return g < ES_MAXG ? g : ES_MAXG;
 }
 
+size_t exact_sum_comp_ints() { return 2 * (size_t)ES_MAXG * 8; }
+
+bool exact_sum_is_cooperative(int n) { return n > ES_SOLO; }
+
 void launch_exact_sum(const float *v, int n, float *out, const ExactSumWork &W, cudaStream_t s) {
-  if (n <= 4 * HEAD) {
-    k_warp_sum<<<1, 32, 0, s>>>(v, n, out);
+  if (!exact_sum_is_cooperative(n)) {
+    k_exact_sum_solo<<<1, ES_T, 0, s>>>(v, n, out);
     return;
   }
-  int G = (n + 4095) / 4096;
-  if (G > W.max_grid) G = W.max_grid;
-  if (G < 1) G = 1;
   EsArgs A;
   A.v = v;
   A.n = n;
   A.out = out;
-  A.Rc = W.Rc;
-  A.Mc = W.Mc;
-  A.Tc = W.Tc;
-  A.ctl = (EsCtl *)W.ctl;
+  A.comp = W.comp;
   A.bar = W.bar;
+  A.pub = (unsigned long long *)(W.bar + 2);
   A.err = W.err;
-  RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, 2 * sizeof(unsigned), s));
+  RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, ES_BAR_WORDS * sizeof(unsigned), s));
   void *args[] = {&A};
-  RPBA_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)k_exact_sum, dim3(G), dim3(ES_T), args, 0, s));
+  RPBA_CUDA_CHECK(
+      cudaLaunchCooperativeKernel((const void *)k_exact_sum, dim3(W.max_grid), dim3(ES_T), args, 0, s));
 }
 
 }  // namespace rpba
@@ -380,27 +523,18 @@ void launch_exact_sum(const float *v, int n, float *out, const ExactSumWork &W, 
 // (a stray cudaMalloc breaks its accounting or fails when the pool owns the
 // whole device), or a latency-critical loop that cannot absorb the
 // device-wide synchronisation cudaFree implies.  For them this entry point
-// keeps its scratch -- the per-CTA run sums, the run control word and the
-// grid-barrier counters of k_exact_sum -- in one statically sized device
+// keeps its scratch -- the CTAs' composites, the published state and the
+// grid-barrier counter of k_exact_sum -- in one statically sized device
 // array that every GPU loading the library holds until the process exits
-// (about 20 KB).  Its size caps the grid at NA_MAX_CTAS CTAs; inputs up to
-// NA_MAX_N elements are accepted on any device (with fewer resident CTAs,
-// each CTA takes a longer chunk).
+// (about 16 KB).  Its size caps the grid at ES_MAXG CTAs; inputs up to
+// NA_MAX_N elements are accepted on any device.
 using namespace rpba;
 
 namespace {
 
-constexpr int NA_MAX_CTAS = 512;
-static_assert(NA_MAX_CTAS <= ES_MAXG, "k_exact_sum stages at most ES_MAXG chunk composites");
-constexpr int NA_CHUNK = 8192;  // elements per CTA when the grid allows it
-constexpr long long NA_MAX_N = (long long)NA_MAX_CTAS * NA_CHUNK;  // 4,194,304
-constexpr size_t NA_OFF_RC = 0;
-// two entries per CTA (one per incoming parity)
-constexpr size_t NA_OFF_MC = NA_OFF_RC + sizeof(long long) * 2 * NA_MAX_CTAS;
-constexpr size_t NA_OFF_TC = NA_OFF_MC + sizeof(long long) * 2 * NA_MAX_CTAS;
-constexpr size_t NA_OFF_CTL = NA_OFF_TC + sizeof(int) * 2 * NA_MAX_CTAS;
-constexpr size_t NA_OFF_BAR = NA_OFF_CTL + 16;
-constexpr size_t NA_OFF_ERR = NA_OFF_BAR + 16;
+constexpr long long NA_MAX_N = 4194304;  // a fixed limit of the entry point
+constexpr size_t NA_OFF_BAR = 2 * (size_t)ES_MAXG * 8 * sizeof(int);  // after the composites
+constexpr size_t NA_OFF_ERR = NA_OFF_BAR + ES_BAR_WORDS * sizeof(unsigned);
 constexpr size_t NA_BYTES = NA_OFF_ERR + 16;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
@@ -474,35 +608,30 @@ extern "C" int32_t rpba_float_sequential_sum_noalloc(const float *d_v, int64_t n
   // until the sum is written, *d_out holds a NaN (all bits set): a grid
   // barrier that runs out leaves it there
   if (cudaMemsetAsync(d_out, 0xff, sizeof(float), s) != cudaSuccess) return RPBA_ERR_CUDA;
-  if (ni <= 4 * HEAD) {
+  if (!exact_sum_is_cooperative(ni)) {
     void *wargs[] = {(void *)&d_v, (void *)&ni, (void *)&d_out};
-    return cudaLaunchKernel((const void *)k_warp_sum, dim3(1), dim3(32), wargs, 0, s) == cudaSuccess ? RPBA_OK
-                                                                                                      : RPBA_ERR_CUDA;
+    return cudaLaunchKernel((const void *)k_exact_sum_solo, dim3(1), dim3(ES_T), wargs, 0, s) == cudaSuccess
+               ? RPBA_OK
+               : RPBA_ERR_CUDA;
   }
   int nsm = 0, per = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_exact_sum, ES_T, 0) != cudaSuccess || nsm * per < 1)
     return RPBA_ERR_CUDA;
-  // every CTA must be resident (cooperative launch) and own a slot of the
-  // array: past either limit the CTAs take longer chunks
-  int G = (ni + NA_CHUNK - 1) / NA_CHUNK;
-  if (G > NA_MAX_CTAS) G = NA_MAX_CTAS;
-  if (G > nsm * per) G = nsm * per;
+  // every CTA must be resident (cooperative launch) and own a slot of the array
+  const int G = nsm < ES_MAXG ? nsm : ES_MAXG;
   EsArgs A;
   A.v = d_v;
   A.n = ni;
   A.out = d_out;
-  A.Rc = (long long *)(base + NA_OFF_RC);
-  A.Mc = (long long *)(base + NA_OFF_MC);
-  A.Tc = (int *)(base + NA_OFF_TC);
-  A.ctl = (EsCtl *)(base + NA_OFF_CTL);
+  A.comp = (int *)base;
   A.bar = (unsigned *)(base + NA_OFF_BAR);
+  A.pub = (unsigned long long *)(A.bar + 2);
   A.err = (int *)(base + NA_OFF_ERR);
-  // the array keeps the previous call's contents: the barrier counters and
-  // the error word must start at zero; the rest is written before it is read
-  if (cudaMemsetAsync(A.bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess ||
-      cudaMemsetAsync(A.err, 0, sizeof(int), s) != cudaSuccess)
-    return RPBA_ERR_CUDA;
+  // the array keeps the previous call's contents: the barrier counter, the
+  // published state and the error word must start at zero; the rest is
+  // written before it is read
+  if (cudaMemsetAsync(A.bar, 0, NA_BYTES - NA_OFF_BAR, s) != cudaSuccess) return RPBA_ERR_CUDA;
   void *args[] = {&A};
   if (cudaLaunchCooperativeKernel((const void *)k_exact_sum, dim3(G), dim3(ES_T), args, 0, s) != cudaSuccess)
     return RPBA_ERR_CUDA;

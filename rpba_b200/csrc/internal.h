@@ -138,15 +138,17 @@ void launch_delete_compact(const DevLSA &L, const int *oidx, const int *pidx, co
                            int *pt_off_n, int *pt_id_n, double *X_n, cudaStream_t s);
 
 // ---- exact sequential float sums (exactsum.cu)
+constexpr int ES_BAR_WORDS = 6;  // barrier counter, padding, published state (two 8-byte words)
 struct ExactSumWork {
-  long long *Rc, *Mc;
-  int *Tc;
-  void *ctl;
-  unsigned *bar;
+  int *comp;      // [exact_sum_comp_ints()] the CTAs' composites
+  unsigned *bar;  // [ES_BAR_WORDS], 8-byte aligned
   int *err;
   int max_grid;
 };
 int exact_sum_max_grid(int device);
+size_t exact_sum_comp_ints();
+// whether a sum of n terms is a cooperative launch (else one ordinary CTA)
+bool exact_sum_is_cooperative(int n);
 void launch_exact_sum(const float *v, int n, float *out, const ExactSumWork &W, cudaStream_t s);
 
 // ---- dense direct solve (direct.cu)

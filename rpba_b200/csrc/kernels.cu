@@ -117,39 +117,37 @@ __global__ void k_gcp_cost(DevLSA L, const double *__restrict__ XM, float *out) 
   out[p] = t;
 }
 
-// Sequential float sum in array order: the reference accumulates its cost
-// and weight sums in float, one observation after the other
-// (rbacore.cpp:1327, 727, 881).  One warp; every lane carries the same
-// running sum, so the result is bitwise that of the sequential loop.
-__global__ void k_seq_sum(const float *__restrict__ v, int n, float *out) {
-  const int lane = threadIdx.x;
-  constexpr int U = 8;
+// Sequential float sum in array order, terms of either sign: the reference
+// accumulates its prior costs in float, one point after the other
+// (rbacore.cpp:1677-1729).  Warp 0 runs the chain of additions on values the
+// other warps stage in shared memory a block ahead (16-byte broadcast loads,
+// so the chain is the additions alone); with the values passed by shuffle a
+// term took 25 cycles.
+constexpr int SS_T = 256, SS_B = 2048;
+__global__ void __launch_bounds__(SS_T) k_seq_sum(const float *__restrict__ v, int n, float *out) {
+  __shared__ __align__(16) float buf[2][SS_B];
+  const int tid = threadIdx.x;
+  for (int j = tid; j < SS_B; j += SS_T)
+    if (j < n) buf[0][j] = v[j];
+  __syncthreads();
   float s = 0.f;
-  float cur[U], nxt[U];
-#pragma unroll
-  for (int j = 0; j < U; ++j) {
-    const int idx = j * 32 + lane;
-    cur[j] = idx < n ? v[idx] : 0.f;
-  }
-  for (int base = 0; base < n; base += 32 * U) {
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      const int idx = base + 32 * U + j * 32 + lane;
-      nxt[j] = idx < n ? v[idx] : 0.f;
-    }
-    const int lim = n - base;
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-#pragma unroll 8
-      for (int l = 0; l < 32; ++l) {
-        const float t = __shfl_sync(0xffffffffu, cur[j], l);
-        if (j * 32 + l < lim) s = __fadd_rn(s, t);
+  for (int base = 0, b = 0; base < n; base += SS_B, b ^= 1) {
+    if (tid < 32) {
+      const int cnt = min(SS_B, n - base);
+      int j = 0;
+#pragma unroll 4
+      for (; j + 4 <= cnt; j += 4) {
+        const float4 a = *(const float4 *)(buf[b] + j);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a.x), a.y), a.z), a.w);
       }
+      for (; j < cnt; ++j) s = __fadd_rn(s, buf[b][j]);
+    } else {
+      for (int j = tid - 32; j < SS_B; j += SS_T - 32)
+        if (base + SS_B + j < n) buf[b ^ 1][j] = v[base + SS_B + j];
     }
-#pragma unroll
-    for (int j = 0; j < U; ++j) cur[j] = nxt[j];
+    __syncthreads();
   }
-  if (lane == 0) *out = s;
+  if (tid == 0) *out = s;
 }
 
 // ---------------------------------------------------------- point pass
@@ -1135,7 +1133,7 @@ void launch_cost(const DevLSA &L, const double *XM, bool srmv, cudaStream_t s) {
 }
 
 void launch_seq_sum(const float *v, int n, float *out, cudaStream_t s) {
-  k_seq_sum<<<1, 32, 0, s>>>(v, n, out);
+  k_seq_sum<<<1, SS_T, 0, s>>>(v, n, out);
 }
 
 void launch_point_pass(const DevLSA &L, double multfact1, cudaStream_t s) {

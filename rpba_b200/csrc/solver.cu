@@ -377,11 +377,12 @@ struct rpba_handle {
   std::mutex *coop = nullptr;
   struct CoopLock {
     rpba_handle *H;
-    explicit CoopLock(rpba_handle *h) : H(h) {
-      if (H->coop) H->coop->lock();
+    bool on;
+    explicit CoopLock(rpba_handle *h, bool cooperative = true) : H(h), on(h->coop && cooperative) {
+      if (on) H->coop->lock();
     }
     ~CoopLock() {
-      if (H->coop) {
+      if (on) {
         cudaStreamSynchronize(H->s);
         H->coop->unlock();
       }
@@ -390,7 +391,7 @@ struct rpba_handle {
 
   float seq_sum(const float *v, int n) {
     {
-      CoopLock lk(this);
+      CoopLock lk(this, exact_sum_is_cooperative(n));
       prof.next_bytes = 4. * n;  // each element read once
       PROF("seq_sum", 1, launch_exact_sum(v, n, sums, ES, s));
     }
@@ -464,11 +465,8 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   }
   {
     H->ES.max_grid = exact_sum_max_grid(H->dev);
-    H->ES.Rc = dalloc<long long>(2 * (size_t)H->ES.max_grid, own);
-    H->ES.Mc = dalloc<long long>(2 * (size_t)H->ES.max_grid, own);
-    H->ES.Tc = dalloc<int>(2 * (size_t)H->ES.max_grid, own);
-    H->ES.ctl = dalloc<char>(16, own);
-    H->ES.bar = dalloc<unsigned>(2, own);
+    H->ES.comp = dalloc<int>(exact_sum_comp_ints(), own);
+    H->ES.bar = dalloc<unsigned>(ES_BAR_WORDS, own);
     H->ES.err = dalloc<int>(4, own);
     RPBA_CUDA_CHECK(cudaMemsetAsync(H->ES.err, 0, 4 * sizeof(int), H->s));
   }
@@ -1104,7 +1102,7 @@ int rpba_handle::adjust() {
       PROF("decode", 1, launch_decode(L, L.XPMn, s));
       PROF("cost", 1, launch_cost(L, L.XPMn, true, s));
       {
-        CoopLock lk(this);
+        CoopLock lk(this, exact_sum_is_cooperative(L.nobs));
         prof.next_bytes = 4. * L.nobs;
         PROF("seq_sum", 1, launch_exact_sum(L.o_cost, L.nobs, sums, ES, s));
       }
@@ -1238,7 +1236,7 @@ int rpba_handle::adjust_gcp_step() {
   PROF("cost", 1, launch_cost(L, L.XPMn, true, s));
   launch_gcp_cost(L, L.XPMn, aoterm + 2 * (size_t)np, s);
   {
-    CoopLock lk(this);
+    CoopLock lk(this, exact_sum_is_cooperative(L.nobs));
     prof.next_bytes = 4. * L.nobs;
     PROF("seq_sum", 1, launch_exact_sum(L.o_cost, L.nobs, sums, ES, s));
   }
@@ -1650,11 +1648,8 @@ int32_t rpba_float_sequential_sum(const float *v, int64_t n, int32_t device, flo
     cudaStream_t s = 0;
     ExactSumWork W{};
     W.max_grid = exact_sum_max_grid(a->dev);
-    W.Rc = dalloc<long long>(2 * (size_t)W.max_grid, own);
-    W.Mc = dalloc<long long>(2 * (size_t)W.max_grid, own);
-    W.Tc = dalloc<int>(2 * (size_t)W.max_grid, own);
-    W.ctl = dalloc<char>(16, own);
-    W.bar = dalloc<unsigned>(2, own);
+    W.comp = dalloc<int>(exact_sum_comp_ints(), own);
+    W.bar = dalloc<unsigned>(ES_BAR_WORDS, own);
     W.err = dalloc<int>(1, own);
     float *dv = dalloc<float>(std::max(a->n, 1), own), *dout = dalloc<float>(1, own);
     RPBA_CUDA_CHECK(cudaMemset(W.err, 0, sizeof(int)));
