@@ -60,15 +60,15 @@ struct DevLSA {
   const int2 *contrib; // (obs in the row camera, obs in the column camera)
   const int *rowoff;   // [nimg + 1]
   const int2 *ent;     // (column camera, block index | 0x80000000 if transposed)
-  // SpMV work items: runs of <= 3 entries of one row.  In the FP32 form the
-  // items cover each row's diagonal and normal entries only: the SpMV reads
-  // every off-diagonal block once and forms both of its products.
+  // SpMV work items of the FP64 form: runs of <= 3 entries of one row (the
+  // FP32 form reads every off-diagonal block once, in storage order)
   int nitems;
   const int *row_item_off;  // [nimg + 1]
-  const int4 *item_meta;    // (row, first entry, end entry, 0)
-  const int2 *rowspan;      // [nimg] (diagonal entry, end entry) of each row
+  const int2 *item_rec;     // [nitems][4] FP64 form: (row | entries << 16, first entry), then the entries
   float *tpart;             // [nboff * 16] FP32 form: transposed block products, column order
-  const int4 *bidx;         // FP32 form: (row, column, transposed slot, 0) of every block, storage order
+  // (row, column, ...) of every block in storage order: its transposed slot in
+  // the FP32 form, its normal and its transposed entry in the FP64 form
+  const int4 *bidx;
   const int *firstN;        // [nimg + 1] first off-diagonal block of every row
   const int *firstT;        // [nimg + 1] first transposed slot of every row (blocks in its column)
   int *err;            // device error word
@@ -273,7 +273,7 @@ void learned_adam(float *W, float *m, float *v, const float *grad, float lr, int
 
 // ---- PCG (pcg.cu)
 struct PcgWork {
-  double *r, *d, *q, *h, *x, *xbest, *Cinv, *partials, *part;
+  double *r, *d, *q, *h, *x, *xbest, *Cinv, *part;
   // FP32 form: d^k in FP32 ([nimg * 12]), and the SpMV's row sums of the
   // diagonal blocks, of the rows' first runs, and of the chunk runs that
   // start inside a row ([nimg * 9], [nimg * 9], [groups * 9]); per chunk its
@@ -284,7 +284,8 @@ struct PcgWork {
   double *rowc;   // [nimg * 12] with the coarse space: per row P_k^T r and its share of |dr|^2
   double *drs;  // [nimg * 9] 1 / sqrt of the camera blocks' diagonal entries (learned features)
   float *feat;  // [nimg * 20] the learned preconditioner's features per camera row
-  unsigned *bar;
+  double *prod;   // FP64 form: [entries * 9] both products of every block, entry order
+  unsigned *bar;  // [pcg_bar_bytes] grid-barrier word and the exchanges' sums
   int *iters;
 };
 // A PCG solve is pcg_prepare (the preconditioner and the start vectors;
@@ -299,6 +300,7 @@ int pcg_prepare(const DevLSA &L, const PcgWork &W, int mode, const float *weight
 int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStream_t s, int mode, double tol,
                 const CoarseWork *coarse);
 int pcg_max_grid(int device);
+size_t pcg_bar_bytes();
 
 // ---- structure (structure.cu)
 struct StructWork {
@@ -312,7 +314,7 @@ struct StructWork {
   int *bcnt, *boff;
   int *nrun;
   int *cntN, *cntT, *firstN, *firstT, *rowtmp;
-  int4 *bidx;  // FP32 form: (row, column, transposed slot, 0) of every block in storage order
+  int4 *bidx;  // (row, column, ...) of every block in storage order, see DevLSA
   unsigned *tkey, *tkey2;
   int *tidx, *tidx2;
   int2 *contrib;
@@ -321,8 +323,7 @@ struct StructWork {
   int *iota, *iota2;
   unsigned *ckey, *ckey2;
   int *row_items, *row_item_off;
-  int4 *item_meta;
-  int2 *rowspan;
+  int2 *item_rec;
 };
 size_t structure_cub_bytes(int nobs, long long npairs, int nimg);
 // PointXXvIn on the device (structure.cu): the caller's block in device

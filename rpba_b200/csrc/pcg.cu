@@ -35,13 +35,12 @@ constexpr int pcg_warps() {
 
 struct PcgArgs {
   const void *blocks;  // BT[(nimg + nboff) * 81]
-  const int2 *ent;
-  const int *rowoff;
   const int *row_item_off;
-  const int4 *item_meta;  // (row, first entry, end entry, 0)
-  const int2 *rowspan;    // (diagonal entry, end entry) of each row
+  const int2 *item_rec;   // [nitems][4] (row | entries << 16, first entry), up to three entries
+  double *prod;           // FP64 symmetric form: the product of every entry, 9 values each, entry order
   float *tpart;           // FP32 form: transposed products of the off-diagonal blocks
-  // FP32 form (k_pcg32): (row, column) of every block in storage order, the
+  // (row, column) of every block in storage order, with its transposed slot
+  // (FP32 form) or its two entries (FP64 form: normal, transposed); the
   // first off-diagonal block of every row, d^k in FP32 (12 floats a camera),
   // and the phase-1 row sums (diagonal, row head, warp-run head)
   const int4 *bidx;
@@ -55,10 +54,10 @@ struct PcgArgs {
   const double *Cinv;
   double *r, *h, *x, *xbest, *D0, *D1;
   double *part;        // [nitems * 9] SpMV partial rows
-  double *red1, *red2; // [gridDim * 4] per-CTA partial sums of phase 1 / phase 2
-                       // (separate, so a fast CTA never overwrites a slot that
-                       // a slow CTA is still reading)
-  unsigned *bar;
+  // per-CTA sums of phase 1 and of phase 2, [N][XMAXG] (separate, so a fast
+  // CTA never overwrites a slot that a slow CTA is still reading)
+  double *red1, *red2;
+  unsigned *bar;       // [0]: GridBarrier, [1]: the exchanges
   int *err;
   int *iters;
   // grid barriers wait for G + bar_extra arrivals, at most bar_ns each
@@ -66,6 +65,7 @@ struct PcgArgs {
   unsigned bar_extra;
   unsigned long long bar_ns;
   int row0, row1, nitems, msize;
+  int stream_once;  // FP64 symmetric form: the blocks exceed L2
   int mode;     // 0: reference stop rule; 1: relative preconditioned residual
   double tol2;  // mode 1: stop when r^T M^-1 r <= tol2 * (r0^T M^-1 r0)
   // two-level preconditioner (coarse.cu): rows are owned per aggregate
@@ -76,144 +76,213 @@ struct PcgArgs {
   double *rowc;  // FP32 form: per row its restriction P_k^T r1 (CO_M) and its share of dr^2, stride RC_S
 };
 
-// Deterministic CTA sum of up to three values; valid in every thread.
+// Sum of N values over the CTAs with the barrier between the phases in it:
+// each CTA's sum is stored, all CTAs arrive and wait, and every CTA reads all
+// the sums.  All writes a CTA made before the call are visible to all CTAs
+// after it.  The order of the additions is fixed: lanes of a warp
+// (butterfly), warps (butterfly over the W warps' sums), CTAs (lane l takes
+// l, l + 32, ...; butterfly), so every CTA gets the same values.  Bounded like
+// GridBarrier's wait: false in every thread when it ran out.  (Every CTA
+// polling the others' tagged sums themselves instead saves the read, but 148
+// CTAs polling 148 slots took 14,000 cycles where this takes 5,000.)
+constexpr int XMAXG = 256;  // CTAs at most
 template <int N, int W>
-__device__ __forceinline__ void cta_sum(double (&v)[N], double (*sh)[4]) {
+struct Exchange {
+  double warp[W][N];
+  double cta[XMAXG * N];
+};
+template <int N, int W>
+__device__ __forceinline__ bool exchange_sum(GridBarrier &bar, double *red, double (&v)[N], Exchange<N, W> &X) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
 #pragma unroll
   for (int j = 0; j < N; ++j)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0)
 #pragma unroll
-    for (int j = 0; j < N; ++j) sh[warp][j] = v[j];
+    for (int j = 0; j < N; ++j) X.warp[warp][j] = v[j];
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      double t = lane < W ? sh[lane][j] : 0.;
+      double t = lane < W ? X.warp[lane][j] : 0.;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) sh[W][j] = t;
+      if (lane == 0) red[j * XMAXG + blockIdx.x] = t;
     }
   }
+  // (thread 0 wrote the CTA's sums; every other write of the CTA came before
+  // the block barrier above)
+  if (!bar.sync_after_block()) return false;
+  if (threadIdx.x < G)
+#pragma unroll
+    for (int j = 0; j < N; ++j) X.cta[j * XMAXG + threadIdx.x] = __ldcg(red + j * XMAXG + threadIdx.x);
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < N; ++j) v[j] = sh[W][j];
-  __syncthreads();
-}
-
-// Sum of the per-CTA partials (stride 4) in a fixed order; every CTA gets
-// the same values.
-template <int N, int W>
-__device__ __forceinline__ void grid_sum(const double *red, int G, double (&v)[N], double (*sh)[4]) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {
+  for (int j = 0; j < N; ++j) {
+    double t = 0.;
+    for (int i = lane; i < G; i += 32) t += X.cta[j * XMAXG + i];
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double t = 0.;
-      for (int i = lane; i < G; i += 32) t += __ldcg(red + 4 * i + j);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) sh[W][j] = t;
-    }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    v[j] = t;
   }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < N; ++j) v[j] = sh[W][j];
-  __syncthreads();
+  return true;
 }
 
-// Asynchronous global -> shared copies of one element (the blocks are
-// constant during the launch, so the L1-allocating form is safe).
-template <class BT>
-__device__ __forceinline__ void cp_async_elem(BT *dst, const BT *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(BT) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src));
+// ---- mbarriers and bulk copies (1-D TMA, one destination CTA)
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// global -> shared bulk copy completing on `bar` (one destination: this
+// CTA's own shared memory; the source is this GPU's own memory)
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+// the same with an L2 policy; policy 0: none
+__device__ __forceinline__ void bulk_load_hint(void *dst, const void *src, unsigned bytes, unsigned long long *bar,
+                                               unsigned long long policy) {
+  if (policy == 0) {
+    bulk_load(dst, src, bytes, bar);
+    return;
+  }
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n" ::
+          "r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
+// Bounded wait on the stage's mbarrier (the copies of this CTA's own
+// memory end in microseconds; the limit only keeps a fault from hanging).
+__device__ __forceinline__ bool stage_wait(const PcgArgs &A, unsigned long long *bar, unsigned parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = gtimer();
+  while (!mbar_try_wait(bar, parity)) {
+    if (gtimer() - t0 > A.bar_ns) return false;
+  }
+  return true;
 }
 
-// Phase-1 software pipeline: each warp has two work items in flight.  The
-// next item's three blocks are copied to a shared-memory stage (cp.async),
-// and its d^k values (column and row) are loaded into registers, while the
-// current item is multiplied.
-constexpr int P1_ELEMS = 3 * 81;
-// Dynamic shared memory: the FP64 form's stages
-template <class BT>
+// Phase 1 of the FP64 form: q-partials p = sum of B d^k over the (at most
+// three) entries of every work item, and d^T A d.  A warp's items (gwarp,
+// gwarp + nwarps, ...) are the same in every iteration, and so are the
+// blocks.  Two forms with the same operations in the same order per entry
+// and per item:
+//  direct     at most P1_SLOTS items a warp: their blocks and records stay in
+//             shared memory for the whole solve; a 9-lane group forms each
+//             entry's product and the warp the item's sum.
+//  symmetric  more: phase 1a reads every block once, in storage order, by
+//             1-D TMA bulk copies of 32 blocks into P1S_N stages a CTA (a
+//             stage with one group keeps it for the whole solve); two warps
+//             a stage, a lane a block, form B d_col and B^T d_row and store
+//             them at their entries' places (vectors copied in and products
+//             written through shared memory in whole 72-byte pieces); a grid
+//             barrier; phase 1b sums every item's products.  Half the block
+//             traffic of reading each block from both sides, in copies of
+//             20 KB, for one more barrier.
+// The threads have 64 registers each and the stages leave L1 some 20 KB, so
+// spilled registers cost L2 trips: a spill of 50 to 100 bytes was worth 10 to
+// 30%.  Iteration, before (each block read from both sides, 8-byte copies two
+// items ahead, the records through two dependent loads) and now: 50 cameras
+// 14.0 -> 10.0 us (direct), 3,000 cameras and 27,000 blocks 24.0 -> 17.3 us,
+// 1,370 cameras and 371,000 blocks 137 -> 115 us (symmetric).
+constexpr int P1_SLOTS = 3;
+constexpr unsigned P1_PIECE = 656;  // a block's 648 bytes from the 16-byte boundary at or below it
+constexpr unsigned P1_WARP_BYTES = P1_SLOTS * (3 * P1_PIECE + 32) + 648 + 8;  // blocks, records, C of a row, mbarrier
+static_assert(P1_WARP_BYTES % 16 == 0, "16-byte aligned pieces");
+constexpr int P1S_N = 7;                                  // stages per CTA (two warps each)
+constexpr unsigned P1S_BLK = 32 * 648 + 16;               // a group's blocks
+constexpr unsigned P1S_IDX = 32 * 16;                     // and their indices
+constexpr unsigned P1S_BUF = 32 * 9 * 8;                  // a warp's 32 h or d^(k-1), or products
+constexpr unsigned P1S_STAGE = P1S_BLK + P1S_IDX + 4 * P1S_BUF + 16;  // + the mbarrier
+static_assert(P1S_BLK % 16 == 0 && P1S_STAGE % 16 == 0, "16-byte aligned stage parts");
+template <bool SYM>
 constexpr size_t pcg_smem_bytes() {
-  return sizeof(BT) * (size_t)pcg_warps<BT>() * 2 * P1_ELEMS;
+  return SYM ? (size_t)P1S_N * P1S_STAGE : (size_t)pcg_warps<double>() * P1_WARP_BYTES;
 }
-struct P1Item {
-  int it, row, ne;  // item, its row, entries (0 past the end)
-  int2 en;          // this lane's entry (group grp)
-  double dc;        // d^k[col][rr] of this lane's entry
-  double dk;        // d^k[row][lane] (lanes < 9)
-};
 
-template <class BT>
-__device__ __forceinline__ void p1_issue(const PcgArgs &A, int it, BT *stage, const double *dprev, double beta,
-                                         int lane, int grp, int rr, P1Item &I) {
-  I.it = it;
-  I.ne = 0;
-  I.row = 0;
-  I.en = make_int2(0, 0);
-  I.dc = 0.;
-  I.dk = 0.;
-  if (it < A.nitems) {
-    const int4 m = A.item_meta[it];
-    I.row = m.x;
-    I.ne = m.z - m.y;
-    if (lane < 27 && grp < I.ne) {
-      I.en = A.ent[m.y + grp];
-      const size_t j = (size_t)I.en.x * 9 + rr;
-      I.dc = __ldcg(A.h + j) + beta * __ldcg(dprev + j);
-    }
-    if (lane < 9) {
-      const size_t i = (size_t)I.row * 9 + lane;
-      I.dk = __ldcg(A.h + i) + beta * __ldcg(dprev + i);
-    }
-    const int b0 = __shfl_sync(0xffffffffu, I.en.y, 0) & 0x7fffffff;
-    const int b1 = __shfl_sync(0xffffffffu, I.en.y, 9) & 0x7fffffff;
-    const int b2 = __shfl_sync(0xffffffffu, I.en.y, 18) & 0x7fffffff;
-    const BT *blocks = (const BT *)A.blocks;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = lane + 32 * q;
-      if (e < P1_ELEMS) {
-        const int g = e / 81, off = e - g * 81;
-        if (g < I.ne) {
-          const int b = g == 0 ? b0 : (g == 1 ? b1 : b2);
-          cp_async_elem(stage + e, blocks + (size_t)b * 81 + off);
-        }
-      }
-    }
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Groups of 32 blocks in storage order: the diagonal blocks of the system's
+// rows, then the off-diagonal blocks.
+struct Grp64 {
+  long long start;
+  int n;
+  bool diag;
+};
+__device__ __forceinline__ Grp64 group64(const PcgArgs &A, int g) {
+  const int gd = (A.row1 - A.row0 + 31) / 32;
+  Grp64 q;
+  if (g < gd) {
+    q.start = A.row0 + 32ll * g;
+    q.n = (int)min(32ll, A.row1 - q.start);
+    q.diag = true;
+  } else {
+    const long long o = 32ll * (g - gd);
+    q.start = A.row1 + o;
+    q.n = (int)min(32ll, A.nboff - o);
+    q.diag = false;
   }
-  cp_async_commit();
+  return q;
+}
+__device__ __forceinline__ void group64_issue(const PcgArgs &A, int g, unsigned char *stg, unsigned long long *mbar,
+                                              unsigned long long policy) {
+  const Grp64 q = group64(A, g);
+  const unsigned long long src = (unsigned long long)A.blocks + (unsigned long long)q.start * 648u;
+  const unsigned mis = (unsigned)(src & 15ull), nb = (mis + (unsigned)q.n * 648u + 15u) & ~15u;
+  mbar_expect_tx(mbar, nb + (unsigned)q.n * 16u);
+  bulk_load_hint(stg, (const void *)(src - mis), nb, mbar, policy);
+  bulk_load(stg + P1S_BLK, A.bidx + q.start, (unsigned)q.n * 16u, mbar);
 }
 
 // q of one row (valid in lanes < 9) from the phase-1 partials of the FP64
 // form: one partial per item, the three 9-lane groups taking every third
-// item (four loads in flight), in a fixed order.
-__device__ __forceinline__ double row_q(const PcgArgs &A, int row, int lane, int grp, int rr) {
-  const int t0 = A.row_item_off[row], t1 = A.row_item_off[row + 1];
+// item, in a fixed order (four running sums of a group, items t, t + 3, t + 6,
+// t + 9 of every twelve; the last, incomplete twelve onto the first sum); the
+// loads of two twelves are in flight before they are added.
+__device__ __forceinline__ double row_q(const PcgArgs &A, int t0, int t1, int lane, int grp, int rr) {
   double qg = 0.;
   if (lane < 27) {
     double q0 = 0., q1 = 0., q2 = 0., q3 = 0.;
     int t = t0 + grp;
+    const double *p = A.part + rr;
+#pragma unroll 2
     for (; t + 9 < t1; t += 12) {
-      q0 += __ldcg(A.part + (size_t)t * 9 + rr);
-      q1 += __ldcg(A.part + (size_t)(t + 3) * 9 + rr);
-      q2 += __ldcg(A.part + (size_t)(t + 6) * 9 + rr);
-      q3 += __ldcg(A.part + (size_t)(t + 9) * 9 + rr);
+      double u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = __ldcg(p + (size_t)(t + 3 * j) * 9);
+      q0 += u[0];
+      q1 += u[1];
+      q2 += u[2];
+      q3 += u[3];
     }
-    for (; t < t1; t += 3) q0 += __ldcg(A.part + (size_t)t * 9 + rr);
+    double u[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) u[j] = t + 3 * j < t1 ? __ldcg(p + (size_t)(t + 3 * j) * 9) : 0.;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (t + 3 * j < t1) q0 += u[j];
     qg = (q0 + q1) + (q2 + q3);
   }
   const double qa = __shfl_down_sync(0xffffffffu, qg, 9);
@@ -221,7 +290,7 @@ __device__ __forceinline__ double row_q(const PcgArgs &A, int row, int lane, int
   return qg + qa + qb;
 }
 
-// Iteration k (two grid barriers):
+// Iteration k (two grid barriers, three in the symmetric form):
 //  phase 1  q-partials of A d^k per work item (<= 3 blocks of one row), with
 //           d^k = h^k + beta^(k-1) d^(k-1) formed on the fly; partial d^T q
 //  phase 2  per row: q = sum of its items' partials, x += alpha d,
@@ -232,41 +301,100 @@ __device__ __forceinline__ double row_q(const PcgArgs &A, int row, int lane, int
 //           (kept in hj), and the aggregate's restriction P^T r1 is formed
 //  phase 2b per aggregate: z = A_c^-1[aggregate rows] (P^T r1), then
 //           h1 = hj + P z and the two dot products
-// BT: the storage type of the reduced camera system's blocks, double (the
-// FP32 form has its own kernel, k_pcg32 below).
-template <bool CO, class BT>
-__global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
-  static_assert(sizeof(BT) == 8, "k_pcg is the FP64 form");
-  constexpr int PCG_T = pcg_threads<BT>(), PCG_W = pcg_warps<BT>();
+template <bool CO, bool SYM>
+__global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
+  constexpr int PCG_T = pcg_threads<double>(), PCG_W = pcg_warps<double>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * PCG_W + warp, nwarps = gridDim.x * PCG_W;
   const int grp = lane / 9, rr = lane % 9, gbase = grp * 9;
   const int G = gridDim.x;
   GridBarrier bar(A.bar, (unsigned)G + A.bar_extra, A.err, A.bar_ns);
-  __shared__ double sh[PCG_W + 1][4];
+  __shared__ Exchange<1, PCG_W> X1;
+  __shared__ Exchange<3, PCG_W> X2;
+  // scalars of the recurrence by iteration parity (every thread computes the
+  // same values, thread 0 stores them): r^T h, its start value, the smallest
+  // and the first increment
+  __shared__ double sc[2][4];
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
-  BT *stage0 = (BT *)pcg_dyn + (size_t)warp * 2 * P1_ELEMS;
-  BT *stage1 = stage0 + P1_ELEMS;
+  // this warp's items
+  const int T = gwarp < A.nitems ? (A.nitems - 1 - gwarp) / nwarps + 1 : 0;
+  // direct form: blocks, records, C of the warp's first row, mbarrier;
+  // symmetric form: a stream warp's stage and its groups gs, gs + gstep, ...
+  unsigned char *stg = pcg_dyn + (SYM ? (size_t)(warp >> 1) * P1S_STAGE : (size_t)warp * P1_WARP_BYTES);
+  int2 *recs = (int2 *)(stg + P1_SLOTS * 3 * P1_PIECE);
+  double *Cs = (double *)(recs + 4 * P1_SLOTS);
+  unsigned long long *mbar =
+      SYM ? (unsigned long long *)(stg + P1S_STAGE - 16) : (unsigned long long *)(Cs + 81);
+  const int ng = (A.row1 - A.row0 + 31) / 32 + (A.nboff + 31) / 32;
+  const int gs = (warp >> 1) * G + (int)blockIdx.x, gstep = P1S_N * G;
+  const bool stream = SYM && warp < 2 * P1S_N && gs < ng;
+  const bool keep = ng <= gstep;  // every stage's only group stays
+  unsigned parity = 0;
+  bool ok = true;  // false: a copy that never completed (bounded wait)
+  unsigned long long policy = 0;
+  if constexpr (SYM) {
+    if (stream) {
+      // blocks that do not fit L2 beside the products should not evict them
+      if (A.stream_once)
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(policy));
+      if (lane == 0 && (warp & 1) == 0) {
+        mbar_init(mbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        group64_issue(A, gs, stg, mbar, policy);
+      }
+    }
+    __syncthreads();  // the mbarriers are initialised
+  } else {
+    if (lane < 4 * T) recs[lane] = __ldg(A.item_rec + 4 * ((size_t)gwarp + (size_t)(lane >> 2) * nwarps) + (lane & 3));
+    __syncwarp();
+    if (lane == 0 && T > 0) {
+      mbar_init(mbar, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+      int np = 0;
+      for (int t = 0; t < T; ++t) np += recs[4 * t].x >> 16;
+      mbar_expect_tx(mbar, (unsigned)np * P1_PIECE);
+      for (int t = 0; t < T; ++t)
+        for (int g = 0; g < (recs[4 * t].x >> 16); ++g)
+          bulk_load(stg + (3 * t + g) * P1_PIECE,
+                    (const unsigned char *)A.blocks +
+                        (((size_t)(recs[4 * t + 1 + g].y & 0x7fffffff) * 648u) & ~(size_t)15),
+                    P1_PIECE, mbar);
+    }
+    __syncwarp();
+  }
+  // the copies in flight end before the CTA does
+  bool landed = false;
+  auto drain = [&]() {
+    if (SYM ? stream : (T > 0 && !landed)) stage_wait(A, mbar, parity);
+  };
+  // the warp's first row of phase 2: its items and preconditioner block
+  const int rowa = A.row0 + gwarp;
+  const bool has_row = !CO && rowa < A.row1;
+  const int ta0 = has_row ? A.row_item_off[rowa] : 0, ta1 = has_row ? A.row_item_off[rowa + 1] : 0;
+  if (!SYM && has_row)
+    for (int e = lane; e < 81; e += 32) Cs[e] = __ldg(A.Cinv + (size_t)rowa * 81 + e);
   // r^T h of the start vectors
   {
-    double v[1] = {0.};
+    double v[3] = {0., 0., 0.};
     for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
       if (lane < 9) {
         const size_t i = (size_t)row * 9 + lane;
         v[0] += A.r[i] * A.h[i];
       }
-    cta_sum<1, PCG_W>(v, sh);
-    if (threadIdx.x == 0) A.red2[4 * blockIdx.x] = v[0];
+    if (!exchange_sum<3, PCG_W>(bar, A.red2, v, X2)) {
+      drain();
+      return;
+    }
+    if (threadIdx.x == 0) {
+      sc[0][0] = sc[0][1] = v[0];
+      sc[0][2] = sc[0][3] = 1.e50;
+    }
   }
-  if (!bar.sync()) return;
-  double erthk;
-  {
-    double v[1];
-    grid_sum<1, PCG_W>(A.red2, G, v, sh);
-    erthk = v[0];
+  if (!SYM && T > 0) {
+    ok = stage_wait(A, mbar, 0u);
+    landed = true;
   }
-  double meandrold = 1.e50, meandr0 = 1.e50, beta_prev = 0.;
-  const double erthk0 = erthk;
+  double beta_prev = 0.;
   bool converged = false;
   int k;
   for (k = 0; k < A.msize; ++k) {
@@ -274,46 +402,171 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
     double *dcur = (k & 1) ? A.D1 : A.D0;
     // ---- phase 1
     double pdq[1] = {0.};
-      {
-        P1Item cur, nxt;
-        p1_issue<BT>(A, gwarp, stage0, dprev, beta_prev, lane, grp, rr, cur);
-        p1_issue<BT>(A, gwarp + nwarps, stage1, dprev, beta_prev, lane, grp, rr, nxt);
-        for (int t = 0; cur.it < A.nitems; ++t) {
-          BT *st = (t & 1) ? stage1 : stage0;
-          cp_async_wait<1>();
+    if constexpr (SYM) {
+      // 1a: both products of every block; the even warp of a stage B d_col,
+      // the odd one B^T d_row
+      if (stream) {
+        const int tr = warp & 1;
+        double *buf = (double *)(stg + P1S_BLK + P1S_IDX + tr * 2 * P1S_BUF), *bufd = buf + 32 * 9;
+        const int4 *idx = (const int4 *)(stg + P1S_BLK);
+        for (int g = gs; g < ng; g += gstep) {
+          const Grp64 q = group64(A, g);
+          if (!keep || k == 0) ok = stage_wait(A, mbar, parity) && ok;
+          const unsigned mis = (unsigned)(((unsigned long long)A.blocks + (unsigned long long)q.start * 648u) & 15ull);
+          if (!(tr && q.diag)) {
+            // the 32 vectors d^k = h + beta d^(k-1): all the copies of both
+            // parts in flight, three vectors an instruction
+#pragma unroll
+            for (int m = 0; m < 11; ++m) {
+              const int v = 3 * m + grp;
+              if (lane < 27 && v < q.n) {
+                const size_t o = (size_t)(tr ? idx[v].x : idx[v].y) * 9 + rr;
+                cp_async8(buf + v * 9 + rr, A.h + o);
+                cp_async8(bufd + v * 9 + rr, dprev + o);
+              }
+            }
+            cp_async_wait_all();
+            __syncwarp();
+            const double *B = (const double *)(stg + mis + 648 * lane);
+            double dv[9];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) dv[j] = buf[lane * 9 + j] + beta_prev * bufd[lane * 9 + j];
+            if (q.diag && lane < q.n)  // d^k of every row
+#pragma unroll
+              for (int j = 0; j < 9; ++j) dcur[(size_t)idx[lane].x * 9 + j] = dv[j];
+            __syncwarp();
+            if (lane < q.n) {
+              if (!tr) {
+#pragma unroll 3
+                for (int i = 0; i < 9; ++i) {
+                  double acc = 0.;
+#pragma unroll
+                  for (int j = 0; j < 9; ++j) acc += B[i * 9 + j] * dv[j];
+                  buf[lane * 9 + i] = acc;
+                }
+              } else {
+#pragma unroll 3
+                for (int j = 0; j < 9; ++j) {
+                  double acc = 0.;
+#pragma unroll
+                  for (int i = 0; i < 9; ++i) acc += B[i * 9 + j] * dv[i];
+                  buf[lane * 9 + j] = acc;
+                }
+              }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 11; ++m) {
+              const int v = 3 * m + grp;
+              if (lane < 27 && v < q.n) A.prod[(size_t)(tr ? idx[v].w : idx[v].z) * 9 + rr] = buf[v * 9 + rr];
+            }
+          }
+          if (!keep) {
+            // both warps are done with the stage: the next group, or the
+            // first one for the next iteration
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
+            parity ^= 1u;
+            if (lane == 0 && !tr) {
+              fence_proxy_async();
+              group64_issue(A, g + gstep < ng ? g + gstep : gs, stg, mbar, policy);
+            }
+          }
           __syncwarp();
-          const bool act = lane < 27 && grp < cur.ne;
-          const bool tr = cur.en.y < 0;
-          const BT *B = st + grp * 81;
+        }
+      }
+      // the items' records of 1b (constant) ahead of the barrier
+      int2 m[4];
+      auto load_recs = [&](int t) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          m[j] = t + j < T ? __ldg(A.item_rec + 4 * ((size_t)gwarp + (size_t)(t + j) * nwarps)) : make_int2(0, 0);
+      };
+      load_recs(0);
+      if (!ok && lane == 0) atomicOr(A.err, 2);
+      if (!bar.sync()) {
+        drain();
+        return;
+      }
+      // 1b: the items' sums, four items' loads in flight beside the next
+      // four's records
+      for (int t = 0; t < T; t += 4) {
+        double u[4], dk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          u[j] = lane < 27 && grp < (m[j].x >> 16) ? __ldcg(A.prod + (size_t)(m[j].y + grp) * 9 + rr) : 0.;
+          dk[j] = lane < 9 && t + j < T ? __ldcg(dcur + (size_t)(m[j].x & 0xffff) * 9 + lane) : 0.;
+        }
+        if (t + 4 < T) load_recs(t + 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double a1 = __shfl_down_sync(0xffffffffu, u[j], 9);
+          const double a2 = __shfl_down_sync(0xffffffffu, u[j], 18);
+          if (lane < 9 && t + j < T) {
+            const double p = u[j] + a1 + a2;
+            A.part[((size_t)gwarp + (size_t)(t + j) * nwarps) * 9 + lane] = p;
+            pdq[0] += dk[j] * p;
+          }
+        }
+      }
+    } else {
+      double hc[P1_SLOTS], dc[P1_SLOTS], hk[P1_SLOTS], dk[P1_SLOTS];
+#pragma unroll
+      for (int t = 0; t < P1_SLOTS; ++t) {
+        hc[t] = dc[t] = hk[t] = dk[t] = 0.;
+        if (t < T) {
+          const int meta = recs[4 * t].x;
+          if (lane < 27 && grp < (meta >> 16)) {
+            const size_t j = (size_t)recs[4 * t + 1 + grp].x * 9 + rr;
+            hc[t] = __ldcg(A.h + j);
+            dc[t] = __ldcg(dprev + j);
+          }
+          if (lane < 9) {
+            const size_t i = (size_t)(meta & 0xffff) * 9 + lane;
+            hk[t] = __ldcg(A.h + i);
+            dk[t] = __ldcg(dprev + i);
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < P1_SLOTS; ++t)
+        if (t < T) {
+          const int en = recs[4 * t + 1 + (grp < 3 ? grp : 0)].y;
+          const bool act = lane < 27 && grp < (recs[4 * t].x >> 16);
+          const bool tr = en < 0;
+          const double *B = (const double *)(stg + (3 * t + (grp < 3 ? grp : 0)) * P1_PIECE + ((en & 1) << 3));
+          const double cdc = hc[t] + beta_prev * dc[t];
           double acc = 0.;
-  #pragma unroll
+#pragma unroll
           for (int c = 0; c < 9; ++c) {
-            const double xc = __shfl_sync(0xffffffffu, cur.dc, (lane < 27 ? gbase : 0) + c);
-            if (act) acc += (double)B[tr ? c * 9 + rr : rr * 9 + c] * xc;
+            const double xc = __shfl_sync(0xffffffffu, cdc, (lane < 27 ? gbase : 0) + c);
+            if (act) acc += B[tr ? c * 9 + rr : rr * 9 + c] * xc;
           }
           const double a1 = __shfl_down_sync(0xffffffffu, acc, 9);
           const double a2 = __shfl_down_sync(0xffffffffu, acc, 18);
           if (lane < 9) {
             const double p = acc + a1 + a2;
-            A.part[(size_t)cur.it * 9 + lane] = p;
-            pdq[0] += cur.dk * p;
+            A.part[((size_t)gwarp + (size_t)t * nwarps) * 9 + lane] = p;
+            const double dkv = hk[t] + beta_prev * dk[t];
+            pdq[0] += dkv * p;
           }
-          __syncwarp();
-          cur = nxt;
-          p1_issue<BT>(A, cur.it + nwarps, st, dprev, beta_prev, lane, grp, rr, nxt);
         }
-        cp_async_wait<0>();
-        __syncwarp();
-      }
-    cta_sum<1, PCG_W>(pdq, sh);
-    if (threadIdx.x == 0) A.red1[4 * blockIdx.x] = pdq[0];
-    if (!bar.sync()) return;
-    double edtAdk;
-    {
-      double v[1];
-      grid_sum<1, PCG_W>(A.red1, G, v, sh);
-      edtAdk = v[0];
+      if (!ok && lane == 0) atomicOr(A.err, 2);
     }
+    // this warp's vectors of its first row, ahead of the exchange
+    // (symmetric form: d^k itself, stored in phase 1a)
+    double hva = 0., dpa = 0., xva = 0., rva = 0.;
+    if (has_row && lane < 9) {
+      const size_t i = (size_t)rowa * 9 + lane;
+      hva = __ldcg(A.h + i);
+      dpa = __ldcg((SYM ? dcur : dprev) + i);
+      xva = A.x[i];
+      rva = A.r[i];
+    }
+    if (!exchange_sum<1, PCG_W>(bar, A.red1, pdq, X1)) {
+      drain();
+      return;
+    }
+    const double edtAdk = pdq[0], erthk = sc[k & 1][0];
     double alpha;
     if (fabs(erthk) < 1.e-20 || fabs(erthk) > 1.e20)
       alpha = 0.;
@@ -322,25 +575,32 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
     // ---- phase 2
     double p2[3] = {0., 0., 0.};
     if constexpr (!CO) {
-      for (int row = A.row0 + gwarp; row < A.row1; row += nwarps) {
+      for (int row = rowa; row < A.row1; row += nwarps) {
+        const bool first = row == rowa;
         const size_t i = (size_t)row * 9 + (lane < 9 ? lane : 0);
         double r1v = 0., hv = 0.;
-        const double q = row_q(A, row, lane, grp, rr);
+        const int t0 = first ? ta0 : A.row_item_off[row], t1 = first ? ta1 : A.row_item_off[row + 1];
+        const double q = row_q(A, t0, t1, lane, grp, rr);
         if (lane < 9) {
-          hv = __ldcg(A.h + i);
-          const double dk = hv + beta_prev * __ldcg(dprev + i);
-          dcur[i] = dk;
-          A.x[i] = A.x[i] + alpha * dk;
+          hv = first ? hva : __ldcg(A.h + i);
+          double dk;
+          if constexpr (SYM) {
+            dk = first ? dpa : __ldcg(dcur + i);
+          } else {
+            dk = hv + beta_prev * (first ? dpa : __ldcg(dprev + i));
+            dcur[i] = dk;
+          }
+          A.x[i] = (first ? xva : A.x[i]) + alpha * dk;
           const double dr = alpha * q;
-          r1v = A.r[i] - dr;
+          r1v = (first ? rva : A.r[i]) - dr;
           p2[0] += dr * dr;
         }
-        const double *C = A.Cinv + (size_t)row * 81;
+        const double *C = !SYM && first ? Cs : A.Cinv + (size_t)row * 81;
         double h1v = 0.;
 #pragma unroll
         for (int c = 0; c < 9; ++c) {
           const double rc = __shfl_sync(0xffffffffu, r1v, c);
-          if (lane < 9) h1v += __ldg(C + lane * 9 + c) * rc;
+          if (lane < 9) h1v += C[lane * 9 + c] * rc;
         }
         if (lane < 9) {
           A.r[i] = r1v;
@@ -359,11 +619,15 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
           const int row = A.agg_rows[t];
           const size_t i = (size_t)row * 9 + (lane < 9 ? lane : 0);
           double r1v = 0.;
-          const double q = row_q(A, row, lane, grp, rr);
+          const double q = row_q(A, A.row_item_off[row], A.row_item_off[row + 1], lane, grp, rr);
           if (lane < 9) {
-            const double hv = __ldcg(A.h + i);
-            const double dk = hv + beta_prev * __ldcg(dprev + i);
-            dcur[i] = dk;
+            double dk;
+            if constexpr (SYM) {
+              dk = __ldcg(dcur + i);
+            } else {
+              dk = __ldcg(A.h + i) + beta_prev * __ldcg(dprev + i);
+              dcur[i] = dk;
+            }
             A.x[i] = __ldcg(A.x + i) + alpha * dk;
             const double dr = alpha * q;
             r1v = __ldcg(A.r + i) - dr;
@@ -392,7 +656,10 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
         }
         __syncthreads();
       }
-      if (!bar.sync()) return;
+      if (!bar.sync()) {
+        drain();
+        return;
+      }
       for (int a = blockIdx.x; a < A.nagg; a += G) {
         double z[CO_M];
 #pragma unroll
@@ -433,24 +700,19 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
         __syncthreads();
       }
     }
-    cta_sum<3, PCG_W>(p2, sh);
-    if (threadIdx.x == 0) {
-      A.red2[4 * blockIdx.x] = p2[0];
-      A.red2[4 * blockIdx.x + 1] = p2[1];
-      A.red2[4 * blockIdx.x + 2] = p2[2];
+    if (!exchange_sum<3, PCG_W>(bar, A.red2, p2, X2)) {
+      drain();
+      return;
     }
-    if (!bar.sync()) return;
-    double g3[3];
-    grid_sum<3, PCG_W>(A.red2, G, g3, sh);
+    const double(&g3)[3] = p2;
     const double meandr = g3[0], er1th1 = g3[1];
-    if (k == 0) meandr0 = meandr;
+    const double erthk0 = sc[k & 1][1], meandrold = sc[k & 1][2], meandr0 = k == 0 ? meandr : sc[k & 1][3];
     // mode 0 keeps the iterate with the smallest increment (the reference's
     // exivold); mode 1 keeps the latest finite one and stops, unconverged,
     // at a breakdown (a non-finite residual or increment)
     const bool finite = isfinite(g3[0]) && isfinite(g3[2]);
     const bool improved = (A.mode == 1 && finite) || meandr < meandrold;
     if (improved) {
-      meandrold = meandr;
       for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
         if (lane < 9) A.xbest[(size_t)row * 9 + lane] = __ldcg(A.x + (size_t)row * 9 + lane);
     }
@@ -460,11 +722,17 @@ __global__ void __launch_bounds__(pcg_threads<BT>(), 1) k_pcg(PcgArgs A) {
       converged = true;
       break;
     }
-    double beta = fabs(er1th1) < 1.e-10 ? 0. : er1th1 / erthk;
+    double beta = fabs(er1th1) < 1.e-10 ? 0. : er1th1 / sc[k & 1][0];
     if (beta < 0.) beta = 0.;
     beta_prev = beta;
-    erthk = g3[2];
+    if (threadIdx.x == 0) {
+      sc[(k + 1) & 1][0] = g3[2];
+      sc[(k + 1) & 1][1] = erthk0;
+      sc[(k + 1) & 1][2] = improved ? meandr : meandrold;
+      sc[(k + 1) & 1][3] = meandr0;
+    }
   }
+  drain();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     A.iters[0] = k < A.msize ? k + 1 : A.msize;
     A.iters[1] = converged ? 1 : 0;
@@ -520,33 +788,6 @@ constexpr int STG_BYTES = STG_BLK + STG_IDX + 16;  // + the mbarrier
 constexpr size_t P32_SMEM = (size_t)P32_W * STG_BYTES;
 static_assert(STG_BLK % 16 == 0 && STG_IDX % 16 == 0, "16-byte aligned stage parts");
 
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// global -> shared bulk copy completing on `bar` (one destination: this
-// CTA's own shared memory; the source is this GPU's own memory)
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
 // Group g of the stream: its first block (storage index), its block count
 // and, for an off-diagonal group, the first block's off-diagonal index.
 struct Grp32 {
@@ -593,17 +834,6 @@ __device__ __forceinline__ void group_issue(const PcgArgs &A, const Grp32 &q, un
   mbar_expect_tx(bar, nb_bytes + ni_bytes);
   bulk_load(stg, (const unsigned char *)(blocks + q.start * 81) - mb, nb_bytes, bar);
   bulk_load(stg + STG_BLK, A.bidx + q.start, ni_bytes, bar);
-}
-
-// Bounded wait on the stage's mbarrier (the copies of this CTA's own
-// memory end in microseconds; the limit only keeps a fault from hanging).
-__device__ __forceinline__ bool stage_wait(const PcgArgs &A, unsigned long long *bar, unsigned parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
-  while (!mbar_try_wait(bar, parity)) {
-    if (gtimer() - t0 > A.bar_ns) return false;
-  }
-  return true;
 }
 
 // FP32 d^k of camera c (12-float stride) into v[0..8].  The loads may hit
@@ -673,7 +903,8 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
   const int gwarp = blockIdx.x * P32_W + warp, nwarps = gridDim.x * P32_W;
   const int G = gridDim.x;
   GridBarrier bar(A.bar, (unsigned)G + A.bar_extra, A.err, A.bar_ns);
-  __shared__ double sh[P32_W + 1][4];
+  __shared__ Exchange<3, P32_W> X2;
+  __shared__ double sh[P32_W + 1];
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
   unsigned char *stg = pcg_dyn + (size_t)warp * STG_BYTES;
   unsigned long long *mbar = (unsigned long long *)(stg + STG_BLK + STG_IDX);
@@ -685,21 +916,15 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
   const long long gd = (A.row1 - A.row0 + GB - 1) / GB, go = ((long long)A.nboff + GB - 1) / GB;
   const long long ng = gd + go, ch = A.chunk, nch = (ng + ch - 1) / ch;
   // r^T h of the start vectors
+  double erthk;
   {
-    double v[1] = {0.};
+    double v[3] = {0., 0., 0.};
     for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
       if (lane < 9) {
         const size_t i = (size_t)row * 9 + lane;
         v[0] += A.r[i] * A.h[i];
       }
-    cta_sum<1, P32_W>(v, sh);
-    if (threadIdx.x == 0) A.red2[4 * blockIdx.x] = v[0];
-  }
-  if (!bar.sync()) return;
-  double erthk;
-  {
-    double v[1];
-    grid_sum<1, P32_W>(A.red2, G, v, sh);
+    if (!exchange_sum<3, P32_W>(bar, A.red2, v, X2)) return;
     erthk = v[0];
   }
   double meandrold = 1.e50, meandr0 = 1.e50, beta_prev = 0.;
@@ -904,16 +1129,11 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       for (long long i = threadIdx.x; i < nch; i += P32_T) v += __ldcg(A.pdqc + i);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) sh[warp][0] = v;
+      if (lane == 0) sh[warp] = v;
       __syncthreads();
-      if (threadIdx.x == 0) {
-        double t = 0.;
-        for (int w = 0; w < P32_W; ++w) t += sh[w][0];
-        sh[P32_W][0] = t;
-      }
-      __syncthreads();
-      edtAdk = sh[P32_W][0];
-      __syncthreads();
+      double t = 0.;
+      for (int w = 0; w < P32_W; ++w) t += sh[w];
+      edtAdk = t;
     }
     double alpha;
     if (fabs(erthk) < 1.e-20 || fabs(erthk) > 1.e20)
@@ -1067,15 +1287,8 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         __syncthreads();
       }
     }
-    cta_sum<3, P32_W>(p2, sh);
-    if (threadIdx.x == 0) {
-      A.red2[4 * blockIdx.x] = p2[0];
-      A.red2[4 * blockIdx.x + 1] = p2[1];
-      A.red2[4 * blockIdx.x + 2] = p2[2];
-    }
-    if (!bar.sync()) return;
-    double g3[3];
-    grid_sum<3, P32_W>(A.red2, G, g3, sh);
+    if (!exchange_sum<3, P32_W>(bar, A.red2, p2, X2)) return;
+    const double(&g3)[3] = p2;
     const double meandr = g3[0], er1th1 = g3[1];
     if (k == 0) meandr0 = meandr;
     const bool finite = isfinite(g3[0]) && isfinite(g3[2]);
@@ -1134,10 +1347,13 @@ __global__ void k_pcg_setup(DevLSA L, PcgWork W) {
 
 // the phase-1 stages of the FP64 form live in dynamic shared memory (124 KB)
 void pcg_set_smem() {
-  cudaFuncSetAttribute(k_pcg<false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)pcg_smem_bytes<double>());
-  cudaFuncSetAttribute(k_pcg<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)pcg_smem_bytes<double>());
+  auto set = [](auto k, size_t bytes) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  set(k_pcg<false, false>, pcg_smem_bytes<false>());
+  set(k_pcg<true, false>, pcg_smem_bytes<false>());
+  set(k_pcg<false, true>, pcg_smem_bytes<true>());
+  set(k_pcg<true, true>, pcg_smem_bytes<true>());
   cudaFuncSetAttribute(k_pcg32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P32_SMEM);
   cudaFuncSetAttribute(k_pcg32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P32_SMEM);
 }
@@ -1150,21 +1366,27 @@ void pcg_set_smem() {
 constexpr int PCG32_CHUNK = 4;
 
 int pcg_max_grid(int device) {
-  int nsm = 0, per = 0, per2 = 0;
+  int nsm = 0, per = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   pcg_set_smem();
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg<false, double>, pcg_threads<double>(),
-                                                pcg_smem_bytes<double>());
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_pcg<true, double>, pcg_threads<double>(),
-                                                pcg_smem_bytes<double>());
-  per = std::min(per, per2);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_pcg32<false>, P32_T, P32_SMEM);
-  per = std::min(per, per2);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_pcg32<true>, P32_T, P32_SMEM);
-  per = std::min(per, per2);
+  per = 1 << 30;
+  auto fit = [&](auto k, int threads, size_t smem) {
+    int p = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k, threads, smem);
+    per = std::min(per, p);
+  };
+  fit(k_pcg<false, false>, pcg_threads<double>(), pcg_smem_bytes<false>());
+  fit(k_pcg<true, false>, pcg_threads<double>(), pcg_smem_bytes<false>());
+  fit(k_pcg<false, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
+  fit(k_pcg<true, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
+  fit(k_pcg32<false>, P32_T, P32_SMEM);
+  fit(k_pcg32<true>, P32_T, P32_SMEM);
   if (per < 1) per = 1;
-  return nsm * per;
+  return std::min(nsm * per, XMAXG - 1);
 }
+
+// barrier word (and padding), then the CTAs' sums of the two exchanges
+size_t pcg_bar_bytes() { return 16 + 4 * (size_t)XMAXG * sizeof(double); }
 
 // Returns 0; throws CudaError on launch errors.  The iteration count is
 // left in W.iters.
@@ -1199,11 +1421,9 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   if (g < 1) g = 1;
   PcgArgs A;
   A.blocks = L.blocks32 ? (const void *)L.blocks32 : (const void *)L.blocks;
-  A.ent = L.ent;
-  A.rowoff = L.rowoff;
   A.row_item_off = L.row_item_off;
-  A.item_meta = L.item_meta;
-  A.rowspan = L.rowspan;
+  A.item_rec = L.item_rec;
+  A.prod = W.prod;
   A.tpart = L.tpart;
   A.bidx = L.bidx;
   A.firstN = L.firstN;
@@ -1225,9 +1445,9 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.D0 = W.q;
   A.D1 = W.d;
   A.part = W.part;
-  A.red1 = W.partials;
-  A.red2 = W.partials + 4 * (size_t)grid;
   A.bar = W.bar;
+  A.red1 = (double *)(W.bar + 4);
+  A.red2 = A.red1 + XMAXG;
   A.err = L.err;
   A.iters = W.iters;
   A.bar_extra = L.bar_extra;
@@ -1235,6 +1455,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.row0 = L.begini;
   A.row1 = L.nimg;
   A.nitems = L.nitems;
+  A.stream_once = ((double)nrows + L.nboff) * 648. > 6.4e7;
   A.msize = msize;
   A.mode = mode;
   A.tol2 = tol * tol;
@@ -1246,7 +1467,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.Ainv = co ? coarse->Ainv : nullptr;
   A.rc = co ? coarse->rc : nullptr;
   A.hj = co ? coarse->hj : nullptr;
-  RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, 2 * sizeof(unsigned), s));
+  RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, 4 * sizeof(unsigned), s));
   void *args[] = {&A};
   const void *fn;
   size_t smem;
@@ -1256,8 +1477,11 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
     smem = P32_SMEM;
     nthreads = P32_T;
   } else {
-    fn = co ? (const void *)k_pcg<true, double> : (const void *)k_pcg<false, double>;
-    smem = pcg_smem_bytes<double>();
+    const int nw = g * pcg_warps<double>();
+    const bool sym = L.nitems > P1_SLOTS * nw;
+    fn = co ? (sym ? (const void *)k_pcg<true, true> : (const void *)k_pcg<true, false>)
+            : (sym ? (const void *)k_pcg<false, true> : (const void *)k_pcg<false, false>);
+    smem = sym ? pcg_smem_bytes<true>() : pcg_smem_bytes<false>();
     nthreads = pcg_threads<double>();
   }
   pcg_set_smem();

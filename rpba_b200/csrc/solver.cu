@@ -301,7 +301,7 @@ struct rpba_handle {
     if (nb <= blocks_cap && cur) return;
     const int cap = std::max(nb, 1);
     if (cur) {
-      for (void *p : {cur, (void *)S.ent, (void *)S.item_meta, (void *)W.part, (void *)L.tpart, (void *)S.bidx,
+      for (void *p : {cur, (void *)S.ent, (void *)S.item_rec, (void *)W.part, (void *)W.prod, (void *)L.tpart, (void *)S.bidx,
                       (void *)W.pw, (void *)W.pdqc}) {
         if (!p) continue;
         auto it = std::find(owned_async.begin(), owned_async.end(), p);
@@ -319,18 +319,21 @@ struct rpba_handle {
       // FP32 PCG's bulk copies round their sizes up to 16 bytes
       L.blocks32 = dalloc<float>((size_t)(nimg + cap) * BS32 + 16, owned);
       L.tpart = dalloc<float>((size_t)cap * 16 + 16, owned);
-      S.bidx = dalloc<int4>((size_t)nimg + cap + 4, owned);
       // phase-1 chunks of the FP32 PCG: at most one per group of 32 blocks
       const size_t groups = ((size_t)nimg + cap) / 32 + 4;
       W.pw = dalloc<double>(9 * groups, owned);
       W.pdqc = dalloc<double>(groups, owned);
     } else
-      L.blocks = dalloc<double>((size_t)(nimg + cap) * BS64, owned);
+      L.blocks = dalloc<double>((size_t)(nimg + cap) * BS64 + 2, owned);  // slack: the PCG's bulk copies round up
+    S.bidx = dalloc<int4>((size_t)nimg + cap + 4, owned);
     S.ent = dalloc<int2>((size_t)nimg + 2 * (size_t)cap, owned);
-    // SpMV work items: at most ceil(entries / 3) per row
-    const size_t items = (size_t)nimg + ((size_t)nimg + 2 * (size_t)cap) / 3 + 1;
-    S.item_meta = dalloc<int4>(items, owned);
-    W.part = dalloc<double>(items * 9, owned);
+    if (!mixed) {
+      // SpMV work items: at most ceil(entries / 3) per row
+      const size_t items = (size_t)nimg + ((size_t)nimg + 2 * (size_t)cap) / 3 + 1;
+      S.item_rec = dalloc<int2>(4 * items, owned);
+      W.part = dalloc<double>(items * 9, owned);
+      W.prod = dalloc<double>(((size_t)nimg + 2 * (size_t)cap) * 9, owned);
+    }
     blocks_cap = cap;
   }
 
@@ -777,7 +780,6 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   S.iota = dalloc<int>(no, own);
   S.row_items = dalloc<int>(n + 1, own);
   S.row_item_off = dalloc<int>(n + 1, own);
-  S.rowspan = dalloc<int2>(n + 1, own);
   S.ckey = dalloc<unsigned>(no, own);
   S.ckey2 = dalloc<unsigned>(no, own);
   H->ES.err = L.err;  // a barrier timeout in a sum surfaces in the LSA's error word
@@ -794,8 +796,7 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   W.x = dalloc<double>(nv, own);
   W.xbest = dalloc<double>(nv, own);
   W.Cinv = dalloc<double>(81 * (size_t)n, own);
-  W.partials = dalloc<double>(8 * (size_t)H->pcg_grid, own);
-  W.bar = dalloc<unsigned>(2, own);
+  W.bar = (unsigned *)dalloc<char>(pcg_bar_bytes(), own);
   W.iters = dalloc<int>(2, own);
   if (o->precision == RPBA_PREC_MIXED) {
     W.d32 = dalloc<float>(12 * (size_t)n + 4, own);

@@ -118,48 +118,62 @@ __global__ void k_fill_transposed(const unsigned *bkey, const int *tidx_sorted, 
   ent[pos] = make_int2(row, (int)((unsigned)(nimg + b) | 0x80000000u));
 }
 
-// Work items of the SpMV: each row's entry list cut into runs of <= 3 (the
-// symmetric form: from the row's diagonal entry on, the transposed entries
-// before it are served by their blocks' rows).  rowspan: (diagonal entry,
-// end entry) of every row.
-__global__ void k_row_items(const int *rowoff, const int *cntT, int nimg, int begini, int sym, int *cnt,
-                            int2 *rowspan) {
+// Work items of the FP64 SpMV: each row's entry list cut into runs of <= 3.
+__global__ void k_row_items(const int *rowoff, int nimg, int begini, int *cnt) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k > nimg) return;
-  const int first = k < nimg ? rowoff[k] + (sym ? cntT[k] : 0) : 0;
-  cnt[k] = (k < nimg && k >= begini) ? (rowoff[k + 1] - first + 2) / 3 : 0;
-  if (k < nimg) rowspan[k] = make_int2(rowoff[k] + cntT[k], rowoff[k + 1]);
+  cnt[k] = (k < nimg && k >= begini) ? (rowoff[k + 1] - rowoff[k] + 2) / 3 : 0;
 }
 
-__global__ void k_fill_items(const int *rowoff, const int *cntT, const int *row_item_off, int nimg, int begini,
-                             int sym, int4 *meta) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nimg || k < begini) return;
-  const int end = rowoff[k + 1], first = rowoff[k] + (sym ? cntT[k] : 0);
-  for (int t = row_item_off[k], j = 0; t < row_item_off[k + 1]; ++t, ++j) {
-    const int e0 = first + 3 * j;
-    meta[t] = make_int4(k, e0, min(e0 + 3, end), 0);
+// An item's record: its row, its number of entries, its first entry and the
+// entries themselves, in one aligned 32-byte piece.  One thread per (item, word);
+// item t of row k is found by bisection of the rows' first items.
+__global__ void k_fill_items(const int *rowoff, const int *row_item_off, const int2 *ent, int nimg, int nitems,
+                             int2 *rec) {
+  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long t = gid >> 2;
+  if (t >= nitems) return;
+  int lo = 0, hi = nimg;  // the last row whose first item is <= t
+  while (hi - lo > 1) {
+    const int m = (lo + hi) / 2;
+    if (row_item_off[m] <= t)
+      lo = m;
+    else
+      hi = m;
   }
+  const int e0 = rowoff[lo] + 3 * (int)(t - row_item_off[lo]), ne = min(3, rowoff[lo + 1] - e0);
+  const int w = (int)(gid & 3);
+  rec[gid] = w == 0 ? make_int2(lo | (ne << 16), e0) : (w <= ne ? ent[e0 + w - 1] : make_int2(0, 0));
 }
 
-// (row, column, transposed slot) of every block of the reduced camera
-// system in storage order: the diagonal blocks, then the off-diagonal blocks
-// (key row * n + col); the slot of an off-diagonal block is its position in
-// column order (the sorted transposed keys), -1 for a diagonal block
-__global__ void k_fill_bidx(const unsigned *bkey, int nb, int nimg, int4 *bidx) {
+// (row, column, ...) of every block of the reduced camera system in storage
+// order: the diagonal blocks, then the off-diagonal blocks (key row * n +
+// col).  FP32 form: then the transposed slot, an off-diagonal block's
+// position in column order (the sorted transposed keys), -1 for a diagonal
+// block.  FP64 form: its entry in its row and, off the diagonal, in its
+// column's row.
+__global__ void k_fill_bidx(const unsigned *bkey, int nb, int nimg, const int *rowoff, const int *cntT,
+                            const int *firstN, int fp64, int4 *bidx) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)nimg + nb) return;
   if (i < nimg) {
-    bidx[i] = make_int4((int)i, (int)i, -1, 0);
+    bidx[i] = make_int4((int)i, (int)i, fp64 ? rowoff[i] + cntT[i] : -1, 0);
   } else {
-    const unsigned key = bkey[i - nimg];
-    bidx[i] = make_int4((int)(key / (unsigned)nimg), (int)(key % (unsigned)nimg), 0, 0);
+    const int b = (int)(i - nimg);
+    const unsigned key = bkey[b];
+    const int row = (int)(key / (unsigned)nimg), col = (int)(key % (unsigned)nimg);
+    bidx[i] = make_int4(row, col, fp64 ? rowoff[row] + cntT[row] + 1 + (b - firstN[row]) : 0, 0);
   }
 }
-__global__ void k_fill_slots(const int *tidx_sorted, int nb, int nimg, int4 *bidx) {
+__global__ void k_fill_slots(const int *tidx_sorted, int nb, int nimg, const int *rowoff, const int *firstT,
+                             int fp64, int4 *bidx) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nb) return;
-  bidx[nimg + tidx_sorted[q]].z = q;
+  int4 &b = bidx[nimg + tidx_sorted[q]];
+  if (fp64)
+    b.w = rowoff[b.y] + (q - firstT[b.y]);
+  else
+    b.z = q;
 }
 
 __global__ void k_fill_diag(int nimg, const int *rowoff, const int *cntT, int2 *ent) {
@@ -256,27 +270,26 @@ void build_bsr(DevLSA &L, StructWork &S, cudaStream_t s) {
     k_fill_transposed<<<nblk(nb, 256), 256, 0, s>>>(S.bkey, S.tidx2, nb, n, S.rowoff, S.firstT, S.ent);
   }
   k_fill_diag<<<nblk(n, 256), 256, 0, s>>>(n, S.rowoff, S.cntT, S.ent);
-  const int sym = L.blocks32 ? 1 : 0;
-  k_row_items<<<nblk(n + 1, 256), 256, 0, s>>>(S.rowoff, S.cntT, n, L.begini, sym, S.row_items, S.rowspan);
-  bytes = S.cub_bytes;
-  RPBA_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(S.cub_tmp, bytes, S.row_items, S.row_item_off, n + 1, s));
-  int nitems = 0;
-  RPBA_CUDA_CHECK(cudaMemcpyAsync(&nitems, S.row_item_off + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RPBA_CUDA_CHECK(cudaStreamSynchronize(s));
-  k_fill_items<<<nblk(n, 256), 256, 0, s>>>(S.rowoff, S.cntT, S.row_item_off, n, L.begini, sym, S.item_meta);
-  if (L.blocks32) {
-    k_fill_bidx<<<nblk((long long)n + nb, 256), 256, 0, s>>>(S.bkey, nb, n, S.bidx);
-    if (nb > 0) k_fill_slots<<<nblk(nb, 256), 256, 0, s>>>(S.tidx2, nb, n, S.bidx);
-    L.bidx = S.bidx;
-    L.firstN = S.firstN;
-    L.firstT = S.firstT;
+  L.nitems = 0;
+  if (!L.blocks32) {
+    k_row_items<<<nblk(n + 1, 256), 256, 0, s>>>(S.rowoff, n, L.begini, S.row_items);
+    bytes = S.cub_bytes;
+    RPBA_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(S.cub_tmp, bytes, S.row_items, S.row_item_off, n + 1, s));
+    RPBA_CUDA_CHECK(cudaMemcpyAsync(&L.nitems, S.row_item_off + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+    RPBA_CUDA_CHECK(cudaStreamSynchronize(s));
+    if (L.nitems > 0)
+      k_fill_items<<<nblk(4ll * L.nitems, 256), 256, 0, s>>>(S.rowoff, S.row_item_off, S.ent, n, L.nitems, S.item_rec);
   }
+  const int fp64 = L.blocks32 ? 0 : 1;
+  k_fill_bidx<<<nblk((long long)n + nb, 256), 256, 0, s>>>(S.bkey, nb, n, S.rowoff, S.cntT, S.firstN, fp64, S.bidx);
+  if (nb > 0) k_fill_slots<<<nblk(nb, 256), 256, 0, s>>>(S.tidx2, nb, n, S.rowoff, S.firstT, fp64, S.bidx);
+  L.bidx = S.bidx;
+  L.firstN = S.firstN;
+  L.firstT = S.firstT;
   L.rowoff = S.rowoff;
   L.ent = S.ent;
-  L.nitems = nitems;
   L.row_item_off = S.row_item_off;
-  L.item_meta = S.item_meta;
-  L.rowspan = S.rowspan;
+  L.item_rec = S.item_rec;
 }
 
 // ---- PointXXvIn (rbacore.cpp:1918-1974) on the device: the track-ordered
