@@ -51,6 +51,7 @@ struct PcgArgs {
   double *pdqc;               // per chunk: its share of d^T A d
   unsigned *ctr;              // next chunk of phase 1
   int chunk;                  // groups per phase-1 chunk
+  int g0;                     // CTAs whose rows' sums are added (SMALL)
   const double *Cinv;
   double *r, *h, *x, *xbest, *D0, *D1;
   double *part;        // [nitems * 9] SpMV partial rows
@@ -848,8 +849,34 @@ __device__ __forceinline__ void load_d32(const float *d32, int c, float (&v)[9])
   v[8] = e.x;
 }
 
+// The butterfly sums (lanes xor 16, 8, 4, 2, 1) of M <= 16 values over the
+// warp: value j ends in lanes 2 j and 2 j + 1.  Each step passes on the half
+// of the values its partner keeps, 16 exchanges instead of 5 M; every value
+// is added in the order of the full butterfly (a + b = b + a), so the result
+// is the same to the bit.
+template <int M>
+__device__ __forceinline__ double butterfly_scatter(const double (&v)[M], int lane) {
+  double w[8];
+  {
+    const bool up = lane & 16;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double lo = j < M ? v[j < M ? j : 0] : 0., hi = j + 8 < M ? v[j + 8 < M ? j + 8 : 0] : 0.;
+      w[j] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, 16);
+    }
+  }
+#pragma unroll
+  for (int o = 8, n = 4; o > 1; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < n) w[j] = (up ? w[j + n] : w[j]) + __shfl_xor_sync(0xffffffffu, up ? w[j] : w[j + n], o);
+  }
+  return w[0] + __shfl_xor_sync(0xffffffffu, w[0], 1);
+}
+
 // q of one row in lanes < 9 (FP32 form).
-__device__ __forceinline__ double row_q32(const PcgArgs &A, int row, long long gd, int lane) {
+__device__ __forceinline__ double row_q32(const PcgArgs &A, int row, long long gd, long long ch, int lane) {
   // the row's run of transposed products (slots firstT[row] ..
   // firstT[row + 1]): one slot per lane (three 16-byte loads), and the sums
   // of the phase-1 chunks that start strictly inside the row's off-diagonal
@@ -874,21 +901,14 @@ __device__ __forceinline__ double row_q32(const PcgArgs &A, int row, long long g
     acc[8] += (double)c.x;
   }
   if (f1 > f0) {
-    const long long ch = A.chunk, glo = gd + f0 / GB + 1, ghi = gd + (f1 - 1) / GB;
+    const long long glo = gd + f0 / GB + 1, ghi = gd + (f1 - 1) / GB;
     for (long long c = (glo + ch - 1) / ch + lane; c * ch <= ghi; c += 32) {
       const double *w = A.pw + (size_t)c * 9;
 #pragma unroll
       for (int j = 0; j < 9; ++j) acc[j] += __ldcg(w + j);
     }
   }
-#pragma unroll
-  for (int j = 0; j < 9; ++j)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-  double q = 0.;
-#pragma unroll
-  for (int j = 0; j < 9; ++j)
-    if (lane == j) q = acc[j];
+  double q = __shfl_sync(0xffffffffu, butterfly_scatter<9>(acc, lane), 2 * (lane < 9 ? lane : 0));
   if (lane < 9) {
     const size_t i = (size_t)row * 9 + lane;
     q += __ldcg(A.pdiag + i);
@@ -897,7 +917,83 @@ __device__ __forceinline__ double row_q32(const PcgArgs &A, int row, long long g
   return q;
 }
 
-template <bool CO>
+// Both products of the lane's block of the group in the stage: y = B d_col
+// and, off the diagonal, t = B^T d_row; pdq += d_row^T y (+ d_col^T t).
+__device__ __forceinline__ void group_products(const PcgArgs &A, const Grp32 &q, const unsigned char *stg, int lane,
+                                               bool act, int4 &rc, float (&y)[9], float (&t)[9], double &pdq) {
+  const unsigned mb = blk_misalign((const float *)A.blocks, q.start);
+  float dc[9], dr[9];
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    y[j] = 0.f;
+    t[j] = 0.f;
+  }
+  if (act) {
+    rc = *(const int4 *)(stg + STG_BLK + 16 * lane);
+    load_d32(A.d32, rc.y, dc);
+    load_d32(A.d32, rc.x, dr);
+    const float *B = (const float *)(stg + mb + 324 * lane);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      float yi = 0.f;
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        const float b = B[i * 9 + j];
+        yi = fmaf(b, dc[j], yi);
+        t[j] = fmaf(b, dr[i], t[j]);
+      }
+      y[i] = yi;
+    }
+    double s = 0.;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) s += (double)dr[i] * (double)y[i];
+    if (!q.diag)
+#pragma unroll
+      for (int j = 0; j < 9; ++j) s += (double)dc[j] * (double)t[j];
+    pdq += s;
+  }
+}
+// The transposed product to its slot (column order).
+__device__ __forceinline__ void store_transposed(const PcgArgs &A, int slot, const float (&t)[9]) {
+  float4 *dst = (float4 *)(A.tpart + (size_t)slot * TP_STRIDE);
+  __stcg(dst, make_float4(t[0], t[1], t[2], t[3]));
+  __stcg(dst + 1, make_float4(t[4], t[5], t[6], t[7]));
+  __stcg(dst + 2, make_float4(t[8], 0.f, 0.f, 0.f));
+  __stcg(dst + 3, make_float4(0.f, 0.f, 0.f, 0.f));
+}
+// Inclusive scan of y over the lanes of equal row (rows non-decreasing in
+// lane order; inactive lanes carry distinct negative rows).
+__device__ __forceinline__ void segment_scan(int row, float (&y)[9], int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ru = __shfl_up_sync(0xffffffffu, row, o);
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const float vu = __shfl_up_sync(0xffffffffu, y[j], o);
+      if (lane >= o && ru == row) y[j] += vu;
+    }
+  }
+}
+
+// SMALL: systems of at most one group per warp.  Four warps (a quad) take a
+// chunk, a group each, which stays in the warp's stage for the whole solve;
+// the quads are dealt over the CTAs.  Sums that lie inside a group are
+// written by the lane that ends them; a row's run across the quad's groups is
+// put together by the quad's first warp from its pieces in shared memory, in
+// the order and precision of the one-warp form (a group inside the row in
+// FP64 per lane, the others by the FP32 scan), so that both forms give the
+// same bits.  With the coarse space an aggregate's CTA takes its rows itself
+// and sums their restrictions (2a and 2a' in one).  Such a system is latency:
+// with a chunk's groups one after the other in a warp, on as few CTAs as hold
+// the chunks, 3,000 cameras (944 groups) took 117,000 cycles an iteration,
+// 44,000 of them in phase 1; now 42,000 (57.0 -> 20.7 ms a solve).
+struct Quad {
+  float y[4][32 * 9];  // a group inside a row: every lane's product; else the first and last segments' sums
+  double s[4][32];     // the lanes' shares of d^T A d
+  int flags[4], row[4];
+};
+constexpr int QF_OFF = 1, QF_INSIDE = 2, QF_NEXT = 4, QF_HEAD = 8;
+template <bool CO, bool SMALL>
 __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * P32_W + warp, nwarps = gridDim.x * P32_W;
@@ -912,18 +1008,48 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
   if (lane == 0) mbar_init(mbar, 1);
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   __syncwarp();
-  const float *blocks = (const float *)A.blocks;
   const long long gd = (A.row1 - A.row0 + GB - 1) / GB, go = ((long long)A.nboff + GB - 1) / GB;
   const long long ng = gd + go, ch = A.chunk, nch = (ng + ch - 1) / ch;
+  // rows whose contributions to the sums a warp adds (the sums' order): with
+  // SMALL the first g0 CTAs, those the one-warp form would take
+  const int nrw = SMALL ? (int)A.g0 * P32_W : nwarps, row_a = SMALL && gwarp >= nrw ? A.row1 : A.row0 + gwarp;
+  // SMALL: the quad's chunk and the warp's group of it
+  __shared__ Quad quads[SMALL ? P32_W / 4 : 1];
+  Quad &Q = quads[SMALL ? warp >> 2 : 0];
+  const int qp = warp & 3, qc = (warp >> 2) * G + (int)blockIdx.x;
+  const bool has_group = SMALL && qc < nch && 4ll * qc + qp < ng;
+  int qrow_prev = -1, qrow_next = -1;  // the rows next to the group in its chunk
+  if constexpr (SMALL) {
+    if (lane == 0) Q.flags[qp] = 0;
+    Q.s[qp][lane] = 0.;
+    if (has_group) {
+      const long long g = 4ll * qc + qp;
+      const Grp32 q = group_of(g, (int)gd, A.row0, A.row1, A.nboff);
+      if (lane == 0) group_issue(A, q, stg, mbar);
+      if (!q.diag) {
+        const int r0 = A.bidx[q.start].x, r1 = A.bidx[q.start + q.n - 1].x;
+        if (qp > 0 && g - 1 >= gd) qrow_prev = A.bidx[q.start - 1].x;
+        if (qp < 3 && g + 1 < ng) qrow_next = A.bidx[q.start + q.n].x;
+        if (lane == 0) {
+          Q.row[qp] = r1;
+          Q.flags[qp] = QF_OFF | (r0 == r1 && r0 == qrow_prev ? QF_INSIDE : 0) | (r1 == qrow_next ? QF_NEXT : 0) |
+                        (r0 != r1 || qrow_prev >= 0 || q.boff == (long long)A.firstN[r1] ? QF_HEAD : 0);
+        }
+      }
+    }
+  }
   // r^T h of the start vectors
   double erthk;
   {
     double v[3] = {0., 0., 0.};
-    for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
+    for (int row = row_a; row < A.row1; row += nrw)
       if (lane < 9) {
         const size_t i = (size_t)row * 9 + lane;
         v[0] += A.r[i] * A.h[i];
       }
+    // (the group's copy ends before the kernel can)
+    const bool landed = !has_group || stage_wait(A, mbar, 0u);
+    if (!landed && lane == 0) atomicOr(A.err, 2);
     if (!exchange_sum<3, P32_W>(bar, A.red2, v, X2)) return;
     erthk = v[0];
   }
@@ -935,17 +1061,112 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
     const double *dprev = (k & 1) ? A.D0 : A.D1;
     double *dcur = (k & 1) ? A.D1 : A.D0;
     // ---- phase D: d^k for every row, FP64 and FP32
-    for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
+    for (int row = A.row0 + (SMALL ? warp * G + (int)blockIdx.x : gwarp); row < A.row1; row += nwarps)
       if (lane < 9) {
         const size_t i = (size_t)row * 9 + lane;
         const double dk = __ldcg(A.h + i) + beta_prev * __ldcg(dprev + i);
         dcur[i] = dk;
         A.d32[(size_t)row * 12 + lane] = (float)dk;
       }
-    if (blockIdx.x == 0 && threadIdx.x < 2) A.ctr[threadIdx.x] = 0u;
+    if (!SMALL && blockIdx.x == 0 && threadIdx.x < 2) A.ctr[threadIdx.x] = 0u;
     if (!bar.sync()) return;
     // ---- phase 1
-    {
+    if constexpr (SMALL) {
+      if (has_group) {
+        const Grp32 q = group_of(4ll * qc + qp, (int)gd, A.row0, A.row1, A.nboff);
+        const bool act = lane < q.n;
+        int4 rc = make_int4(-1 - lane, -1, 0, 0);
+        float y[9], t[9];
+        double pdq = 0.;
+        group_products(A, q, stg, lane, act, rc, y, t, pdq);
+        Q.s[qp][lane] = pdq;
+        if (q.diag) {
+          if (act) {
+            double *dst = A.pdiag + (size_t)rc.x * 9;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) dst[i] = (double)y[i];
+          }
+        } else {
+          if (act) store_transposed(A, rc.z, t);
+          if (Q.flags[qp] & QF_INSIDE) {
+#pragma unroll
+            for (int j = 0; j < 9; ++j) Q.y[qp][lane * 9 + j] = act ? y[j] : 0.f;
+          } else {
+            const int row = rc.x;
+            segment_scan(row, y, lane);
+            const int rnext = __shfl_down_sync(0xffffffffu, row, 1), r0 = __shfl_sync(0xffffffffu, row, 0);
+            const bool last = lane == q.n - 1;
+            if (act && (last || rnext != row)) {
+              const bool first = row == r0;
+              const bool piece_p = first && row == qrow_prev, piece_n = last && row == qrow_next;
+              if (piece_p || piece_n) {
+                // (both only if the group lies inside the row)
+                float *dst = Q.y[qp] + (piece_n ? 16 : 0);
+#pragma unroll
+                for (int j = 0; j < 9; ++j) dst[j] = y[j];
+              } else {
+                // a segment starts the row unless it is the chunk's first and
+                // the row began before the chunk
+                const bool head = !first || qrow_prev >= 0 || q.boff == (long long)__ldg(A.firstN + row);
+                double *dst = head ? A.prow + (size_t)row * 9 : A.pw + (size_t)qc * 9;
+#pragma unroll
+                for (int j = 0; j < 9; ++j) dst[j] = (double)y[j];
+              }
+            }
+          }
+        }
+      }
+      if (qc < nch) {
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");
+        if (qp == 0) {
+          // rows that run on from one group of the chunk to the next
+          bool open = false, head = false;
+          int row = -1;
+          double racc = 0.;
+#pragma unroll 1
+          for (int p = 0; p < 4; ++p) {
+            const int f = Q.flags[p];
+            if (!(f & QF_OFF)) continue;
+            if (open) {
+              if (f & QF_INSIDE) {
+                // the lanes' sums over the groups inside the row, folded at its end
+                double l[9];
+#pragma unroll
+                for (int j = 0; j < 9; ++j) l[j] = 0.;
+                for (; p < 4 && (Q.flags[p] & QF_INSIDE); ++p) {
+#pragma unroll
+                  for (int j = 0; j < 9; ++j) l[j] += (double)Q.y[p][lane * 9 + j];
+                  if (!(Q.flags[p] & QF_NEXT)) {
+                    open = false;
+                    break;
+                  }
+                }
+                racc += __shfl_sync(0xffffffffu, butterfly_scatter<9>(l, lane), 2 * (lane < 9 ? lane : 0));
+                if (open && p < 4) racc += lane < 9 ? (double)Q.y[p][lane] : 0.;  // its last, partial group
+              } else {
+                racc += lane < 9 ? (double)Q.y[p][lane] : 0.;
+              }
+              open = false;
+              if (lane < 9) (head ? A.prow + (size_t)row * 9 : A.pw + (size_t)qc * 9)[lane] = racc;
+              if (p >= 4) break;
+            }
+            const int g = Q.flags[p];
+            if ((g & QF_NEXT) && !(g & QF_INSIDE)) {
+              open = true;
+              head = g & QF_HEAD;
+              row = Q.row[p];
+              racc = lane < 9 ? (double)Q.y[p][16 + lane] : 0.;
+            }
+          }
+          double pdq = 0.;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) pdq += Q.s[p][lane];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) pdq += __shfl_xor_sync(0xffffffffu, pdq, o);
+          if (lane == 0) A.pdqc[qc] = pdq;
+        }
+      }
+    } else {
       auto grab = [&]() -> long long {
         unsigned c = 0;
         if (lane == 0) c = atomicAdd(A.ctr, 1u);
@@ -969,16 +1190,11 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
 #pragma unroll
       for (int j = 0; j < 9; ++j) lacc[j] = 0.;
       auto fold_lanes = [&]() {
-        double v = 0.;
+        const double v = butterfly_scatter<9>(lacc, lane);
 #pragma unroll
-        for (int j = 0; j < 9; ++j) {
-          double a = lacc[j];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-          if (lane == j) v = a;
-          lacc[j] = 0.;
-        }
-        racc += v;
+        for (int j = 0; j < 9; ++j) lacc[j] = 0.;
+        const double vl = __shfl_sync(0xffffffffu, v, 2 * (lane < 9 ? lane : 0));
+        racc += lane < 9 ? vl : 0.;
       };
       if (c < nch && lane == 0) group_issue(A, group_of(c * ch, (int)gd, A.row0, A.row1, A.nboff), stg, mbar);
       bool ok = true;
@@ -994,39 +1210,10 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           break;
         }
         parity ^= 1u;
-        const unsigned mb = blk_misalign(blocks, q.start);
         const bool act = lane < q.n;
         int4 rc = make_int4(-1 - lane, -1, 0, 0);
-        float dc[9], dr[9], y[9], t[9];
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-          y[j] = 0.f;
-          t[j] = 0.f;
-        }
-        if (act) {
-          rc = *(const int4 *)(stg + STG_BLK + 16 * lane);
-          load_d32(A.d32, rc.y, dc);
-          load_d32(A.d32, rc.x, dr);
-          const float *B = (const float *)(stg + mb + 324 * lane);
-#pragma unroll
-          for (int i = 0; i < 9; ++i) {
-            float yi = 0.f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-              const float b = B[i * 9 + j];
-              yi = fmaf(b, dc[j], yi);
-              t[j] = fmaf(b, dr[i], t[j]);
-            }
-            y[i] = yi;
-          }
-          double s = 0.;
-#pragma unroll
-          for (int i = 0; i < 9; ++i) s += (double)dr[i] * (double)y[i];
-          if (!q.diag)
-#pragma unroll
-            for (int j = 0; j < 9; ++j) s += (double)dc[j] * (double)t[j];
-          pdq += s;
-        }
+        float y[9], t[9];
+        group_products(A, q, stg, lane, act, rc, y, t, pdq);
         // the stage's blocks are read: the next group's copies may land
         // (the next group of this chunk, or the first of the next chunk)
         __syncwarp();
@@ -1044,13 +1231,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           continue;
         }
         // the transposed product to the block's slot (column order)
-        if (act) {
-          float4 *dst = (float4 *)(A.tpart + (size_t)rc.z * TP_STRIDE);
-          __stcg(dst, make_float4(t[0], t[1], t[2], t[3]));
-          __stcg(dst + 1, make_float4(t[4], t[5], t[6], t[7]));
-          __stcg(dst + 2, make_float4(t[8], 0.f, 0.f, 0.f));
-          __stcg(dst + 3, make_float4(0.f, 0.f, 0.f, 0.f));
-        }
+        if (act) store_transposed(A, rc.z, t);
         const int row = rc.x;
         // a group inside the open row (most groups: a row has hundreds of
         // blocks): every lane adds its product to its own FP64 running sum
@@ -1064,15 +1245,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         // then a segmented scan of the group's products (rows non-decreasing
         // in lane order; inactive lanes carry distinct negative rows)
         fold_lanes();
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int ru = __shfl_up_sync(0xffffffffu, row, o);
-#pragma unroll
-          for (int j = 0; j < 9; ++j) {
-            const float vu = __shfl_up_sync(0xffffffffu, y[j], o);
-            if (lane >= o && ru == row) y[j] += vu;
-          }
-        }
+        segment_scan(row, y, lane);
         const int rnext = __shfl_down_sync(0xffffffffu, row, 1);
         const bool end = act && (lane == q.n - 1 || rnext != row);
         unsigned ends = __ballot_sync(0xffffffffu, end);
@@ -1143,10 +1316,10 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
     // ---- phase 2
     double p2[3] = {0., 0., 0.};
     if constexpr (!CO) {
-      for (int row = A.row0 + gwarp; row < A.row1; row += nwarps) {
+      for (int row = row_a; row < A.row1; row += nrw) {
         const size_t i = (size_t)row * 9 + (lane < 9 ? lane : 0);
         double r1v = 0., hv = 0.;
-        const double q = row_q32(A, row, gd, lane);
+        const double q = row_q32(A, row, gd, ch, lane);
         if (lane < 9) {
           hv = __ldcg(A.h + i);
           const double dk = __ldcg(dcur + i);
@@ -1178,16 +1351,10 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       // Every load of a row that does not depend on q is issued before the
       // row's walk: lanes 0..8 hold row `lane` of C_k, lanes 16..25 column
       // `lane - 16` of P_k (9 doubles a lane either way).
-      const int nrows = A.row1 - A.row0;
-      auto grab_row = [&]() -> int {
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(A.ctr + 1, 1u);
-        return (int)__shfl_sync(0xffffffffu, t, 0);
-      };
       const bool cl = lane < 9, pl = lane >= 16 && lane < 16 + CO_M;
-      for (int t = grab_row(); t < nrows;) {
-        const int row = A.row1 - 1 - t;
-        const int tn = grab_row();  // the next row, taken one ahead
+      // one row; returns lanes 16 .. 25 the restriction, lane 31 (all lanes)
+      // the share of dr^2 in d2
+      auto take_row = [&](int row, double &d2) -> double {
         const size_t i = (size_t)row * 9 + (cl ? lane : 0);
         double cp[9];
         {
@@ -1202,8 +1369,9 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           xv = __ldcg(A.x + i);
           rv = __ldcg(A.r + i);
         }
-        const double q = row_q32(A, row, gd, lane);
-        double r1v = 0., d2 = 0.;
+        const double q = row_q32(A, row, gd, ch, lane);
+        double r1v = 0.;
+        d2 = 0.;
         if (cl) {
           A.x[i] = xv + alpha * dk;
           const double dr = alpha * q;
@@ -1222,6 +1390,45 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           A.r[i] = r1v;
           A.hj[i] = acc;
         }
+        return acc;
+      };
+      if constexpr (SMALL) {
+        // an aggregate's rows by its CTA's warps (warp w: rows w, w + P32_W,
+        // ...), then its restriction and share of dr^2, the warps in order
+        for (int a = blockIdx.x; a < A.nagg; a += G) {
+          const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
+          double v = 0.;  // lanes 16 .. 25, and 31
+          for (int t = t0 + warp; t < t1; t += P32_W) {
+            double d2;
+            const double acc = take_row(A.agg_rows[t], d2);
+            if (pl) v += acc;
+            if (lane == 31) v += d2;
+          }
+          if (pl) shr[warp][lane - 16] = v;
+          if (lane == 31) shr[warp][CO_M] = v;
+          __syncthreads();
+          if (threadIdx.x <= CO_M) {
+            double sum = 0.;
+            for (int w = 0; w < P32_W; ++w) sum += shr[w][threadIdx.x];
+            if (threadIdx.x < CO_M)
+              A.rc[a * CO_M + threadIdx.x] = sum;
+            else
+              A.rowc[a] = sum;  // joins the aggregates' sum in 2b, in the one-warp form's order
+          }
+          __syncthreads();
+        }
+      } else {
+      const int nrows = A.row1 - A.row0;
+      auto grab_row = [&]() -> int {
+        unsigned t = 0;
+        if (lane == 0) t = atomicAdd(A.ctr + 1, 1u);
+        return (int)__shfl_sync(0xffffffffu, t, 0);
+      };
+      for (int t = grab_row(); t < nrows;) {
+        const int row = A.row1 - 1 - t;
+        const int tn = grab_row();  // the next row, taken one ahead
+        double d2;
+        const double acc = take_row(row, d2);
         if (pl) A.rowc[(size_t)row * RC_S + lane - 16] = acc;
         if (lane == 31) A.rowc[(size_t)row * RC_S + CO_M] = d2;
         t = tn;
@@ -1246,8 +1453,10 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         }
         __syncthreads();
       }
+      }
       if (!bar.sync()) return;
-      for (int a = blockIdx.x; a < A.nagg; a += G) {
+      // z of an aggregate: its rows of A_c^-1 with the restrictions, a warp's share
+      auto z_share = [&](int a) -> double {
         double z[CO_M];
 #pragma unroll
         for (int j = 0; j < CO_M; ++j) z[j] = 0.;
@@ -1256,11 +1465,82 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
 #pragma unroll
           for (int j = 0; j < CO_M; ++j) z[j] += __ldg(A.Ainv + (size_t)(a * CO_M + j) * A.nc + i) * rv;
         }
+        return butterfly_scatter<CO_M>(z, lane);
+      };
+      if constexpr (SMALL) {
+        // the g0 CTAs of the one-warp form, whose shares of the sums they add:
+        // ZB aggregates at a time, a warp's rows of them in threes (lanes 9 s
+        // + j), their terms added in the rows' order
+        constexpr int ZB = 4;
+        __shared__ double shr4[ZB][P32_W][CO_M + 1], shz4[ZB][CO_M];
+        const int G2 = A.g0, sub = lane / 9, jr = lane - 9 * sub;
+        for (int a0 = (int)blockIdx.x < G2 ? (int)blockIdx.x : A.nagg; a0 < A.nagg; a0 += ZB * G2) {
+#pragma unroll 1
+          for (int b = 0; b < ZB && a0 + b * G2 < A.nagg; ++b) {
+            const double zs = z_share(a0 + b * G2);
+            if ((lane & 1) == 0 && lane < 2 * CO_M) shr4[b][warp][lane >> 1] = zs;
+          }
+          __syncthreads();
+          if (threadIdx.x < ZB * CO_M) {
+            const int b = threadIdx.x / CO_M, j = threadIdx.x - CO_M * b;
+            if (a0 + b * G2 < A.nagg) {
+              double sum = 0.;
+              for (int w = 0; w < P32_W; ++w) sum += shr4[b][w][j];
+              shz4[b][j] = sum;
+            }
+          }
+          if (threadIdx.x == CO_M)
+            for (int b = 0; b < ZB && a0 + b * G2 < A.nagg; ++b) p2[0] += __ldcg(A.rowc + a0 + b * G2);
+          __syncthreads();
+          // a place in the warp's list of rows: aggregate b, row t of it
+          int b = 0, t = __ldg(A.agg_off + a0) + warp, t1 = __ldg(A.agg_off + a0 + 1);
+          auto settle = [&]() {
+            while (t >= t1 && ++b < ZB && a0 + b * G2 < A.nagg) {
+              t = __ldg(A.agg_off + a0 + b * G2) + warp;
+              t1 = __ldg(A.agg_off + a0 + b * G2 + 1);
+            }
+          };
+          settle();
+          for (int s = 0; s < sub && t < t1; ++s) {
+            t += P32_W;
+            settle();
+          }
+          while (__any_sync(0xffffffffu, t < t1)) {
+            const bool act = t < t1 && sub < 3;
+            double r1v = 0., dh = 0., h1v = 0.;
+            if (act) {
+              const int row = __ldg(A.agg_rows + t);
+              const size_t i = (size_t)row * 9 + jr;
+              const double *Pk = A.P + (size_t)row * (9 * CO_M) + jr * CO_M;
+              h1v = __ldcg(A.hj + i);
 #pragma unroll
-        for (int j = 0; j < CO_M; ++j) {
+              for (int j = 0; j < CO_M; ++j) h1v += __ldg(Pk + j) * shz4[b][j];
+              const double hv = __ldcg(A.h + i);
+              r1v = __ldcg(A.r + i);
+              dh = h1v - hv;
+              A.h[i] = h1v;
+            }
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) z[j] += __shfl_xor_sync(0xffffffffu, z[j], o);
-          if (lane == 0) shr[warp][j] = z[j];
+            for (int s = 0; s < 3; ++s) {
+              const int src = lane < 9 ? 9 * s + lane : lane;
+              const double rs = __shfl_sync(0xffffffffu, r1v, src), ds = __shfl_sync(0xffffffffu, dh, src),
+                           hs = __shfl_sync(0xffffffffu, h1v, src);
+              if (lane < 9) {
+                p2[1] += rs * ds;
+                p2[2] += rs * hs;
+              }
+            }
+            for (int s = 0; s < 3 && t < t1; ++s) {
+              t += P32_W;
+              settle();
+            }
+          }
+        }
+      } else {
+      for (int a = blockIdx.x; a < A.nagg; a += G) {
+        {
+          const double zs = z_share(a);
+          if ((lane & 1) == 0 && lane < 2 * CO_M) shr[warp][lane >> 1] = zs;
         }
         __syncthreads();
         if (threadIdx.x < CO_M) {
@@ -1286,6 +1566,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         }
         __syncthreads();
       }
+      }
     }
     if (!exchange_sum<3, P32_W>(bar, A.red2, p2, X2)) return;
     const double(&g3)[3] = p2;
@@ -1295,7 +1576,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
     const bool improved = (A.mode == 1 && finite) || meandr < meandrold;
     if (improved) {
       meandrold = meandr;
-      for (int row = A.row0 + gwarp; row < A.row1; row += nwarps)
+      for (int row = row_a; row < A.row1; row += nrw)
         if (lane < 9) A.xbest[(size_t)row * 9 + lane] = __ldcg(A.x + (size_t)row * 9 + lane);
     }
     if (A.mode == 0 && meandr * 1.e5 < meandr0) break;
@@ -1354,8 +1635,10 @@ void pcg_set_smem() {
   set(k_pcg<true, false>, pcg_smem_bytes<false>());
   set(k_pcg<false, true>, pcg_smem_bytes<true>());
   set(k_pcg<true, true>, pcg_smem_bytes<true>());
-  cudaFuncSetAttribute(k_pcg32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P32_SMEM);
-  cudaFuncSetAttribute(k_pcg32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P32_SMEM);
+  set(k_pcg32<false, false>, P32_SMEM);
+  set(k_pcg32<true, false>, P32_SMEM);
+  set(k_pcg32<false, true>, P32_SMEM);
+  set(k_pcg32<true, true>, P32_SMEM);
 }
 
 
@@ -1379,8 +1662,10 @@ int pcg_max_grid(int device) {
   fit(k_pcg<true, false>, pcg_threads<double>(), pcg_smem_bytes<false>());
   fit(k_pcg<false, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
   fit(k_pcg<true, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
-  fit(k_pcg32<false>, P32_T, P32_SMEM);
-  fit(k_pcg32<true>, P32_T, P32_SMEM);
+  fit(k_pcg32<false, false>, P32_T, P32_SMEM);
+  fit(k_pcg32<true, false>, P32_T, P32_SMEM);
+  fit(k_pcg32<false, true>, P32_T, P32_SMEM);
+  fit(k_pcg32<true, true>, P32_T, P32_SMEM);
   if (per < 1) per = 1;
   return std::min(nsm * per, XMAXG - 1);
 }
@@ -1407,12 +1692,21 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   const bool co = coarse && coarse->nagg > 0;
   const int nrows = L.nimg - L.begini;
   if (nrows <= 0) return 0;
-  int g;
+  int g, g0 = 0;
+  bool small32 = false;
   if (L.blocks32) {
     // FP32 form: groups of 32 blocks (the diagonal blocks of the system's
     // rows, then the off-diagonal blocks), at least one group per warp
     const long long ng = (nrows + GB - 1) / GB + ((long long)L.nboff + GB - 1) / GB;
-    g = (int)std::min<long long>((ng + P32_W - 1) / P32_W, grid);
+    // at least one group per warp (g0); a system of at most one group per
+    // warp of the whole grid is spread further: a chunk, and with the coarse
+    // space an aggregate, per CTA (a barrier over 148 CTAs instead of 58 costs
+    // 500 cycles, a second chunk or aggregate on an SM thousands)
+    g0 = (int)std::min<long long>((ng + P32_W - 1) / P32_W, grid);
+    small32 = ng <= (long long)grid * P32_W && PCG32_CHUNK == 4;
+    g = g0;
+    if (small32) g = (int)std::max<long long>(std::max<long long>(g, (ng + 3) / 4), co ? coarse->nagg : 0);
+    g = (int)std::min<long long>(g, grid);
   } else {
     const int wpc = pcg_warps<double>();
     g = (L.nitems + wpc - 1) / wpc;
@@ -1437,6 +1731,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.ctr = W.ctr;
   A.rowc = W.rowc;
   A.chunk = PCG32_CHUNK;
+  A.g0 = g0;
   A.Cinv = W.Cinv;
   A.r = W.r;
   A.h = W.h;
@@ -1473,7 +1768,8 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   size_t smem;
   int nthreads;
   if (L.blocks32) {
-    fn = co ? (const void *)k_pcg32<true> : (const void *)k_pcg32<false>;
+    fn = co ? (small32 ? (const void *)k_pcg32<true, true> : (const void *)k_pcg32<true, false>)
+            : (small32 ? (const void *)k_pcg32<false, true> : (const void *)k_pcg32<false, false>);
     smem = P32_SMEM;
     nthreads = P32_T;
   } else {
