@@ -14,7 +14,7 @@
 namespace rpba {
 
 // Per-observation linearisation record (doubles):
-//   [0..17]  Bc (2 x 9 camera Jacobian, row major)
+//   [0..17]  Bc (2 x 9 camera Jacobian, column major: pairs (Bc[0][j], Bc[1][j]))
 //   [18..23] G  = W Jp (2 x 3); in the FP32 form H = G L^-T, V = L L^T
 //   [24..25] e  = W d
 //   [26..28] M  = W - G V^-1 G^T  (M00, M01, M11)

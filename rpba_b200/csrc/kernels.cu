@@ -40,6 +40,23 @@ struct Store<float> {
   static constexpr int BS = BS32;
 };
 
+template <class T>
+struct Pair2;
+template <>
+struct Pair2<float> {
+  using type = float2;
+};
+template <>
+struct Pair2<double> {
+  using type = double2;
+};
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Compensated (Kahan) accumulation for the FP32 form; plain in FP64.
 template <class T>
 struct Acc {
@@ -203,10 +220,8 @@ __global__ void k_point(DevLSA L, double multfact1) {
     T *r = Store<T>::rec(L) + (size_t)o * REC;
     const bool cam_active = k >= L.begini;
 #pragma unroll
-    for (int j = 0; j < RPBA_P; ++j) {
-      r[j] = cam_active ? Bc[0][j] : T(0);
-      r[9 + j] = cam_active ? Bc[1][j] : T(0);
-    }
+    for (int j = 0; j < RPBA_P; ++j)
+      *(double2 *)(r + 2 * j) = cam_active ? make_double2(Bc[0][j], Bc[1][j]) : make_double2(0., 0.);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       r[18 + j] = G[0][j];
@@ -326,8 +341,8 @@ __global__ void k_point32(DevLSA L, double multfact1) {
     float v[28];
 #pragma unroll
     for (int j = 0; j < RPBA_P; ++j) {
-      v[j] = cam_active ? Bc[0][j] : 0.f;
-      v[9 + j] = cam_active ? Bc[1][j] : 0.f;
+      v[2 * j] = cam_active ? Bc[0][j] : 0.f;
+      v[2 * j + 1] = cam_active ? Bc[1][j] : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -476,12 +491,12 @@ __global__ void __launch_bounds__(CAM_T) k_camera(DevLSA L, double multfact1) {
     }
     if (tid < 45) {
       for (int ob = 0; ob < nb; ++ob) {
-        const T b0i = s[ob][ei], b1i = s[ob][9 + ei], b0j = s[ob][ej], b1j = s[ob][9 + ej];
+        const T b0i = s[ob][2 * ei], b1i = s[ob][2 * ei + 1], b0j = s[ob][2 * ej], b1j = s[ob][2 * ej + 1];
         const T M00 = s[ob][18], M01 = s[ob][19], M11 = s[ob][20];
         acc.add(b0i * (M00 * b0j + M01 * b1j) + b1i * (M01 * b0j + M11 * b1j));
       }
     } else if (tid < 54) {
-      for (int ob = 0; ob < nb; ++ob) acc.add(s[ob][ei] * s[ob][21] + s[ob][9 + ei] * s[ob][22]);
+      for (int ob = 0; ob < nb; ++ob) acc.add(s[ob][2 * ei] * s[ob][21] + s[ob][2 * ei + 1] * s[ob][22]);
     }
     __syncthreads();
   }
@@ -505,179 +520,183 @@ __global__ void __launch_bounds__(CAM_T) k_camera(DevLSA L, double multfact1) {
 // ----------------------------------------------------------- pair pass
 // Off-diagonal blocks: S_kl = - sum_p W_pk V_p^-1 W_pl^T over the points
 // seen by both cameras (rbacore.cpp:1362-1390), with W_po = Bc^T G.  One
-// warp per block sums its contributions in a fixed order.  FP64 form; the
-// FP32 form is k_pair32.
+// warp per block sums its contributions in a fixed order (the FP32 form in
+// chunks of 32, each added into a compensated sum).  Both forms take a chunk
+// (PairGeom::CH) in three steps: the records by 16-byte asynchronous copies
+// into shared memory; a lane (FP64: two) a contribution, the 2 x 2 product N
+// of the points' part -- FP32 G V^-1 G^T = H H^T of the whitened records --
+// and with it one side's Bc, in place; then lanes 0..26 add every
+// contribution to three entries each, (i, 3 g .. 3 g + 2).
+// What bounds it are instructions (FP64: the FP64 units) and the bytes that
+// shared memory hands to registers (FP32: eight values a lane and
+// contribution, 79% of the cycles), not HBM.  With N formed by every lane and
+// the records staged through registers one contribution ahead the FP32 form
+// took twice the instructions: 5.5M blocks, 28M observations 11.9 -> 8.9 ms
+// a launch; FP64, 365,000 blocks 2.72 -> 1.50 ms, 33,000 blocks of a chain
+// 1.09 -> 0.44 ms, 66 blocks (latency) 94 -> 33 us.  Two stages in flight were
+// no faster but for the smallest (33 -> 29 us), fewer registers (7 or 8 CTAs
+// an SM) slower by their spills in the FP64 form.
 template <class T>
-__global__ void k_pair(DevLSA L) {
-  static_assert(sizeof(T) == 8, "the FP32 form is k_pair32");
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int wl = threadIdx.x >> 5;
-  __shared__ T sm[8][64];
+struct PairGeom {
+  static constexpr bool F32 = sizeof(T) == 4;
+  static constexpr int CH = F32 ? 32 : 16;     // contributions per stage
+  static constexpr int V16 = 16 / sizeof(T);   // values per 16-byte piece
+  static constexpr int PR = 24 / V16;          // pieces of a record's Bc and G (H)
+  static constexpr int PP = F32 ? 0 : 5;       // and of the point's V^-1
+  static constexpr int PC = 2 * PR + PP;
+  // values per contribution: an odd number of 16-byte pieces, so that the
+  // lanes of a quarter warp meet no bank twice
+  static constexpr int ST = F32 ? 52 : 58;
+  static constexpr int STAGE_BYTES = CH * (ST * (int)sizeof(T) + (F32 ? 8 : 16));
+};
+constexpr int PAIR_W = 4;  // warps per CTA
+
+template <class T>
+__global__ void __launch_bounds__(32 * PAIR_W, sizeof(T) == 4 ? 6 : 5) k_pair(DevLSA L) {
+  using Ge = PairGeom<T>;
+  constexpr bool F32 = Ge::F32;
+  constexpr int CH = Ge::CH, ST = Ge::ST, PR = Ge::PR, PC = Ge::PC, V16 = Ge::V16;
+  const int wid = blockIdx.x * PAIR_W + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (wid >= L.nboff) return;
-  T *s = sm[wl];
-  Acc<T> acc[3];
+  __shared__ __align__(16) unsigned char stages[PAIR_W * Ge::STAGE_BYTES];
+  unsigned char *mine = stages + (size_t)(threadIdx.x >> 5) * Ge::STAGE_BYTES;
   const T *rec = Store<T>::rec(L), *ptv = Store<T>::ptV(L);
-  // values of one contribution: 24 of the row camera's observation (Bc 18,
-  // G 6), 24 of the column camera's and V^-1 (9) of the point
-  constexpr int NV = 57;
-  auto fetch = [&](int ox, int oy, int p, T &v0, T &v1) {
-    v0 = lane < 24 ? rec[(size_t)ox * REC + lane] : rec[(size_t)oy * REC + lane - 24];
-    const int i1 = lane + 32;
-    v1 = i1 < 48 ? rec[(size_t)oy * REC + i1 - 24] : (i1 < NV ? ptv[(size_t)p * PREC + i1 - 48] : T(0));
-  };
   const int cb = L.boff[wid], ce = L.boff[wid + 1];
-  for (int c0 = cb; c0 < ce; c0 += 32) {
-    // the next (up to) 32 contributions' observation pairs and points, one
-    // per lane; the record values of contribution j + 1 are fetched while j
-    // is accumulated
-    const int n = min(32, ce - c0);
-    int2 pr = make_int2(0, 0);
-    int pp = 0;
-    if (lane < n) {
-      pr = L.contrib[c0 + lane];
-      pp = L.o_pt[pr.x];
+  // the contributions of the chunk at c0, one per lane, and its points
+  auto pair_of = [&](int c0) { return lane < CH && c0 + lane < ce ? __ldg(L.contrib + c0 + lane) : make_int2(0, 0); };
+  auto point_of = [&](int2 pr, int c0) { return !F32 && lane < CH && c0 + lane < ce ? __ldg(L.o_pt + pr.x) : 0; };
+  // copy the chunk's records to the stage
+  auto issue = [&](int c0, int2 pr, int pp) {
+    int *si = (int *)(mine + CH * ST * (int)sizeof(T));
+    const int n = min(CH, ce - c0);
+    if (lane < CH) {
+      if constexpr (F32)
+        ((int2 *)si)[lane] = pr;
+      else
+        ((int4 *)si)[lane] = make_int4(pr.x, pr.y, pp, 0);
     }
-    T v0, v1;
-    fetch(__shfl_sync(0xffffffffu, pr.x, 0), __shfl_sync(0xffffffffu, pr.y, 0), __shfl_sync(0xffffffffu, pp, 0),
-          v0, v1);
-    for (int j = 0; j < n; ++j) {
-      s[lane] = v0;
-      if (lane + 32 < NV) s[lane + 32] = v1;
-      if (j + 1 < n)
-        fetch(__shfl_sync(0xffffffffu, pr.x, j + 1), __shfl_sync(0xffffffffu, pr.y, j + 1),
-              __shfl_sync(0xffffffffu, pp, j + 1), v0, v1);
-      __syncwarp();
-      // N = G_s V^-1 G_t^T (2 x 2)
-      const T *Gs = s + 18, *Gt = s + 42, *Vi = s + 48;
-      T GV[2][3], N[2][2];
+    __syncwarp();
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+    for (int m = 0; m < (CH * PC + 31) / 32; ++m) {
+      if (32 * m >= n * PC) break;
+      const int t = lane + 32 * m;
+      if (t < n * PC) {
+        const int c = t / PC, e = t - c * PC, w = F32 || e < 2 * PR ? e / PR : 2, f = (e - w * PR) * V16;
+        const int o = si[(F32 ? 2 : 4) * c + w];
+        const T *src = w < 2 ? rec + (size_t)o * REC + f : ptv + (size_t)o * PREC + f;
+        cp_async16((T *)mine + c * ST + 24 * w + f, src);
+      }
+    }
+  };
+  const int i = lane < 27 ? lane / 3 : 0, g = lane < 27 ? lane - 3 * (lane / 3) : 0;
+  T ks[3] = {T(0), T(0), T(0)}, kc[3] = {T(0), T(0), T(0)};
+  // contributions two chunks ahead, points one chunk ahead
+  int2 pr1 = pair_of(cb), pr2 = pair_of(cb + CH);
+  int pp1 = point_of(pr1, cb);
+  issue(cb, pr1, pp1);
+  pp1 = point_of(pr2, cb + CH);
+  pr1 = pr2;
+  pr2 = pair_of(cb + 2 * CH);
+  T *b = (T *)mine;
+  for (int c0 = cb; c0 < ce; c0 += CH) {
+    const int n = min(CH, ce - c0);
+    cp_async_wait_all();
+    __syncwarp();
+    if constexpr (F32) {
+      // a lane a contribution: U = Bc_k^T N, N = H_k H_l^T, in place of Bc_k
+      float *r = (float *)b + lane * ST;
+      if (lane < n) {
+        float x[24];
 #pragma unroll
-        for (int b = 0; b < 3; ++b)
-          GV[a][b] = Gs[a * 3] * Vi[b] + Gs[a * 3 + 1] * Vi[3 + b] + Gs[a * 3 + 2] * Vi[6 + b];
+        for (int v = 0; v < 6; ++v) *(float4 *)(x + 4 * v) = *(const float4 *)(r + 4 * v);
+        const float2 y0 = *(const float2 *)(r + 42);
+        const float4 y1 = *(const float4 *)(r + 44);
+        const float n00 = x[18] * y0.x + x[19] * y0.y + x[20] * y1.x;
+        const float n01 = x[18] * y1.y + x[19] * y1.z + x[20] * y1.w;
+        const float n10 = x[21] * y0.x + x[22] * y0.y + x[23] * y1.x;
+        const float n11 = x[21] * y1.y + x[22] * y1.z + x[23] * y1.w;
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+        for (int k = 0; k < 9; ++k) {
+          const float b0 = x[2 * k], b1 = x[2 * k + 1];
+          x[2 * k] = b0 * n00 + b1 * n10;
+          x[2 * k + 1] = b0 * n01 + b1 * n11;
+        }
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-          N[a][b] = GV[a][0] * Gt[b * 3] + GV[a][1] * Gt[b * 3 + 1] + GV[a][2] * Gt[b * 3 + 2];
+        for (int v = 0; v < 4; ++v) *(float4 *)(r + 4 * v) = *(const float4 *)(x + 4 * v);
+        *(float2 *)(r + 16) = make_float2(x[16], x[17]);
+      }
+    } else {
+      // two lanes a contribution: T = N Bc_l, N = G_k V^-1 G_l^T, in place
+      // of Bc_l (one lane columns 0 .. 4, the other the rest)
+      double *r = (double *)b + (lane & 15) * ST;
+      if ((lane & 15) < n) {
+        double Gs[6], Gt[6], Vi[10];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const int e = lane + 32 * q;
-        if (e < 81) {
-          const int i = e / 9, jj = e % 9;
-          const T bt0 = s[24 + jj], bt1 = s[24 + 9 + jj];
-          const T t0 = N[0][0] * bt0 + N[0][1] * bt1;
-          const T t1 = N[1][0] * bt0 + N[1][1] * bt1;
-          acc[q].add(-(s[i] * t0 + s[9 + i] * t1));
+        for (int v = 0; v < 3; ++v) {
+          *(double2 *)(Gs + 2 * v) = *(const double2 *)(r + 18 + 2 * v);
+          *(double2 *)(Gt + 2 * v) = *(const double2 *)(r + 42 + 2 * v);
+        }
+#pragma unroll
+        for (int v = 0; v < 5; ++v) *(double2 *)(Vi + 2 * v) = *(const double2 *)(r + 48 + 2 * v);
+        double GV[2][3], N[2][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            GV[a][c] = Gs[a * 3] * Vi[c] + Gs[a * 3 + 1] * Vi[3 + c] + Gs[a * 3 + 2] * Vi[6 + c];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            N[a][c] = GV[a][0] * Gt[c * 3] + GV[a][1] * Gt[c * 3 + 1] + GV[a][2] * Gt[c * 3 + 2];
+        const int k0 = lane < 16 ? 0 : 5;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          if (k0 + k < 9) {
+            double2 *q = (double2 *)(r + 24 + 2 * (k0 + k));
+            const double2 bt = *q;
+            *q = make_double2(N[0][0] * bt.x + N[0][1] * bt.y, N[1][0] * bt.x + N[1][1] * bt.y);
+          }
         }
       }
-      __syncwarp();
     }
-  }
-  T *B = Store<T>::blocks(L) + (size_t)(L.nimg + wid) * Store<T>::BS;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const int e = lane + 32 * q;
-    if (e < 81) __stcs(B + e, (T)acc[q].value());  // streaming: keep L2 for the records
-  }
-}
-
-// FP32 form of the pair pass (whitened records): S_kl -= sum Bc_k^T (H_k
-// H_l^T) Bc_l over the block's contributions.  One warp per block; per
-// contribution the warp stages the row camera's and the column camera's
-// record (Bc 18 and H 6 floats each, coalesced 4-byte loads, the next
-// contribution's loads in flight) in shared memory in the order the lanes
-// read them: lanes 0..26 own the three entries (i, 3 (lane % 3) .. + 2) of
-// block row i = lane / 3, and each forms N = H_k H_l^T itself (two 16-byte
-// and two 8-byte broadcast loads, 12 FMAs), U_i = (Bc_k[0][i], Bc_k[1][i]) N
-// (one 8-byte load) and its three entries from the three (Bc_l[0][j],
-// Bc_l[1][j]) pairs (one 16-byte and one 8-byte load): twelve shared-memory
-// or global instructions per contribution.  Each lane sums a chunk of up to
-// 32 contributions in FP32, in order, and adds the chunk into a compensated
-// (Kahan) sum, so the entry is deterministic.
-// Staging layout (floats): row record: pairs (Bc[0][j], Bc[1][j]) at 2 j,
-// H at 20..25; column record: the pairs of j = 3 g .. 3 g + 2 at 28 + 8 g
-// (16-byte aligned groups), H at 52..57.
-constexpr int PS = 60;  // floats per warp
-__device__ __forceinline__ int pair_slot_x(int e) {
-  return e < 9 ? 2 * e : (e < 18 ? 2 * (e - 9) + 1 : e + 2);
-}
-__device__ __forceinline__ int pair_slot_y(int e) {
-  if (e < 18) {
-    const int r = e < 9 ? 0 : 1, j = e - 9 * r;
-    return 28 + 8 * (j / 3) + 2 * (j % 3) + r;
-  }
-  return 52 + (e - 18);
-}
-__global__ void __launch_bounds__(256) k_pair32(DevLSA L) {
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int wl = threadIdx.x >> 5;
-  __shared__ __align__(16) float sm[8][PS];
-  __shared__ int2 spr[8][32];
-  if (wid >= L.nboff) return;
-  float *s = sm[wl];
-  int2 *sp = spr[wl];
-  const float *rec = L.rec32;
-  const int i = lane < 27 ? lane / 3 : 0, g = lane < 27 ? lane - 3 * (lane / 3) : 0;
-  // destinations of this lane's two record values: v0 = float `lane` of the
-  // row record (lane < 24) or float lane - 24 of the column record; v1 =
-  // float lane + 8 of the column record (lane < 16)
-  const int d0 = lane < 24 ? pair_slot_x(lane) : pair_slot_y(lane - 24);
-  const int d1 = pair_slot_y(lane < 16 ? lane + 8 : 8);
-  float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f};
-  auto fetch = [&](int ox, int oy, float &v0, float &v1) {
-    v0 = lane < 24 ? rec[(size_t)ox * REC + lane] : rec[(size_t)oy * REC + lane - 24];
-    v1 = lane < 16 ? rec[(size_t)oy * REC + lane + 8] : 0.f;
-  };
-  const int cb = L.boff[wid], ce = L.boff[wid + 1];
-  for (int c0 = cb; c0 < ce; c0 += 32) {
-    const int n = min(32, ce - c0);
-    if (lane < n) sp[lane] = L.contrib[c0 + lane];
     __syncwarp();
-    float v0, v1;
-    {
-      const int2 q = sp[0];
-      fetch(q.x, q.y, v0, v1);
-    }
-    float part[3] = {0.f, 0.f, 0.f};
-    for (int j = 0; j < n; ++j) {
-      s[d0] = v0;
-      if (lane < 16) s[d1] = v1;
-      if (j + 1 < n) {
-        const int2 q = sp[j + 1];
-        fetch(q.x, q.y, v0, v1);
-      }
-      __syncwarp();
-      const float4 hx = *(const float4 *)(s + 20), hy = *(const float4 *)(s + 52);
-      const float2 hx2 = *(const float2 *)(s + 24), hy2 = *(const float2 *)(s + 56);
-      const float n00 = hx.x * hy.x + hx.y * hy.y + hx.z * hy.z;
-      const float n01 = hx.x * hy.w + hx.y * hy2.x + hx.z * hy2.y;
-      const float n10 = hx.w * hy.x + hx2.x * hy.y + hx2.y * hy.z;
-      const float n11 = hx.w * hy.w + hx2.x * hy2.x + hx2.y * hy2.y;
-      const float2 bx = *(const float2 *)(s + 2 * i);
-      const float4 ya = *(const float4 *)(s + 28 + 8 * g);
-      const float2 yb = *(const float2 *)(s + 32 + 8 * g);
-      const float u0 = bx.x * n00 + bx.y * n10, u1 = bx.x * n01 + bx.y * n11;
-      part[0] -= u0 * ya.x + u1 * ya.y;
-      part[1] -= u0 * ya.z + u1 * ya.w;
-      part[2] -= u0 * yb.x + u1 * yb.y;
-      __syncwarp();
-    }
+    // every lane its three entries (i, 3 g .. 3 g + 2), in the contributions' order
+    T part[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const float y = part[q] - kc[q];
-      const float t = ks[q] + y;
-      kc[q] = (t - ks[q]) - y;
-      ks[q] = t;
+    for (int q = 0; q < 3; ++q) part[q] = F32 ? T(0) : ks[q];
+    const T *pa = b + 2 * i, *pc = b + 24 + 6 * g;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const typename Pair2<T>::type a = *(const typename Pair2<T>::type *)(pa + j * ST);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const typename Pair2<T>::type c = *(const typename Pair2<T>::type *)(pc + j * ST + 2 * q);
+        part[q] -= a.x * c.x + a.y * c.y;
+      }
     }
-    __syncwarp();  // sp is rewritten by the next chunk
+    __syncwarp();
+    if constexpr (F32) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const float y = part[q] - kc[q];
+        const float t = ks[q] + y;
+        kc[q] = (t - ks[q]) - y;
+        ks[q] = t;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) ks[q] = part[q];
+    }
+    if (c0 + CH < ce) issue(c0 + CH, pr1, pp1);
+    pp1 = point_of(pr2, c0 + 2 * CH);
+    pr1 = pr2;
+    pr2 = pair_of(c0 + 3 * CH);
   }
   if (lane < 27) {
-    float *B = L.blocks32 + (size_t)(L.nimg + wid) * BS32 + i * 9 + 3 * g;
+    T *B = Store<T>::blocks(L) + (size_t)(L.nimg + wid) * Store<T>::BS + i * 9 + 3 * g;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) __stcs(B + q, (float)((double)ks[q] - (double)kc[q]));  // keep L2 for the records
+    for (int q = 0; q < 3; ++q) __stcs(B + q, F32 ? (T)((double)ks[q] - (double)kc[q]) : ks[q]);  // keep L2 for the records
   }
 }
 
@@ -709,13 +728,17 @@ __global__ void k_backsub(DevLSA L, const double *__restrict__ xsol) {
       }
     } else {
 #pragma unroll
-      for (int a = 0; a < 24; ++a) r[a] = rp[a];
+      for (int a = 0; a < 24; a += 2) {
+        const double2 q = __ldg((const double2 *)(rp + a));
+        r[a] = q.x;
+        r[a + 1] = q.y;
+      }
     }
     T s0 = 0., s1 = 0.;
 #pragma unroll
     for (int a = 0; a < 9; ++a) {
-      s0 += r[a] * (T)dc[a];
-      s1 += r[9 + a] * (T)dc[a];
+      s0 += r[2 * a] * (T)dc[a];
+      s1 += r[2 * a + 1] * (T)dc[a];
     }
     a0 += r[18] * s0 + r[21] * s1;
     a1 += r[19] * s0 + r[22] * s1;
@@ -1156,9 +1179,9 @@ void launch_camera_pass(const DevLSA &L, double multfact1, cudaStream_t s) {
 void launch_pair_pass(const DevLSA &L, cudaStream_t s) {
   if (L.nboff <= 0) return;
   if (L.rec32)
-    k_pair32<<<nblk((long long)L.nboff * 32, 256), 256, 0, s>>>(L);
+    k_pair<float><<<nblk(L.nboff, PAIR_W), 32 * PAIR_W, 0, s>>>(L);
   else
-    k_pair<double><<<nblk((long long)L.nboff * 32, 256), 256, 0, s>>>(L);
+    k_pair<double><<<nblk(L.nboff, PAIR_W), 32 * PAIR_W, 0, s>>>(L);
 }
 
 void launch_backsub(const DevLSA &L, const double *xsol, cudaStream_t s) {
