@@ -286,13 +286,6 @@ __device__ __forceinline__ void lu_inverse9(int n, const double *A, double *Ai) 
   for (int i = n; i < 9; ++i) Ai[i * 9 + i] = 1.;
 }
 
-// lu_inverse9 by one warp: the same operations in the same order (the
-// compiler may contract them into FMAs differently, so the last bits can
-// differ), with row r of the factor in lane r's registers (r < 9) and
-// column col of the inverse solved by lane col.  `row` holds row `lane` of
-// the input (lanes < 9; anything in the other lanes); every lane of the warp
-// calls it; lanes < n write their column of the inverse to Ai (Ai may be the
-// input's storage: nothing is read from memory).
 // Step k of lu_inverse9_warp's factorisation (k a compile-time constant, so
 // that the rows stay in registers).
 template <int k>
@@ -334,13 +327,15 @@ __device__ __forceinline__ void lu9_warp_factor(int n, double (&row)[9], int &pe
   (lu9_warp_step<K>(n, row, perm, lane), ...);
 }
 
-// lu_inverse9 by one warp: the same operations in the same order (the
-// compiler may contract them into FMAs differently, so the last bits can
-// differ), with row r of the factor in lane r's registers (r < 9) and
+// lu_inverse9 by one warp: the same operations in the same order, with row r of the factor in lane r's registers (r < 9) and
 // column col of the inverse solved by lane col.  `row` holds row `lane` of
 // the input (lanes < 9; anything in the other lanes); every lane of the warp
 // calls it; lanes < 9 write their column of the inverse to Ai (Ai may be the
 // input's storage: nothing is read from memory).
+// SAME: the same bits as lu_inverse9 too.  Left to itself the compiler forms
+// the first step of row 0's back substitution, 1 - u y, in two roundings
+// (its start value is known to be 0 or 1), where lu_inverse9's is one FMA.
+template <bool SAME = false>
 __device__ __forceinline__ void lu_inverse9_warp(int n, double (&row)[9], double *Ai, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   int perm = lane;
@@ -364,7 +359,7 @@ __device__ __forceinline__ void lu_inverse9_warp(int n, double (&row)[9], double
 #pragma unroll
       for (int j = i + 1; j < 9; ++j) {
         const double u = __shfl_sync(FULL, row[j], i);
-        if (j < n) s -= u * y[j];
+        if (j < n) s = SAME ? __fma_rn(-u, y[j], s) : s - u * y[j];
       }
       y[i] = s / __shfl_sync(FULL, row[i], i);
     }

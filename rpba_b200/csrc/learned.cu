@@ -217,10 +217,10 @@ __global__ void __launch_bounds__(128) k_learned_features(DevLSA L, const double
 // PCG start with the learned preconditioner (replaces k_pcg_setup), one
 // warp per camera row: C_k = diag(s) S_kk^-1 diag(s) with S_kk^-1 from
 // lu_inverse9_warp and s from the network on the row's features
-// (k_learned_features); W == nullptr gives plain block-Jacobi.
+// (k_learned_features).
 __global__ void k_learned_setup(DevLSA L, PcgWork Wk, const float *weights) {
   __shared__ float Ws[NN_WEIGHTS];
-  for (int i = threadIdx.x; i < NN_WEIGHTS; i += blockDim.x) Ws[i] = weights ? bf16r(weights[i]) : 0.f;
+  for (int i = threadIdx.x; i < NN_WEIGHTS; i += blockDim.x) Ws[i] = bf16r(weights[i]);
   __syncthreads();
   const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (k >= L.nimg) return;
@@ -239,9 +239,7 @@ __global__ void k_learned_setup(DevLSA L, PcgWork Wk, const float *weights) {
     lu_inverse9_warp(np, row, C, lane);
   }
   float sc[NN_O];
-#pragma unroll
-  for (int a = 0; a < NN_O; ++a) sc[a] = 1.f;
-  if (weights) {
+  {
     const float fl = lane < NN_F ? Wk.feat[(size_t)k * NN_FS + lane] : 0.f;
     float f[NN_F];
 #pragma unroll
@@ -259,7 +257,7 @@ __global__ void k_learned_setup(DevLSA L, PcgWork Wk, const float *weights) {
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
       double cv = C[a * 9 + c];
-      if (weights && a < np && c < np) {
+      if (a < np && c < np) {
         cv *= (double)sa * (double)sc[c];
         C[a * 9 + c] = cv;
       }
@@ -551,10 +549,8 @@ __global__ void k_rec_uc(DevLSA L, TrainSet T, int row0, int pr, const double *v
 }  // namespace
 
 void learned_pcg_setup(const DevLSA &L, const PcgWork &W, const float *weights, cudaStream_t s) {
-  if (weights) {
-    k_diag_rsqrt<<<(L.nimg * 9 + 255) / 256, 256, 0, s>>>(L, W.drs);
-    k_learned_features<<<(L.nimg + 3) / 4, 128, 0, s>>>(L, W.drs, W.feat);
-  }
+  k_diag_rsqrt<<<(L.nimg * 9 + 255) / 256, 256, 0, s>>>(L, W.drs);
+  k_learned_features<<<(L.nimg + 3) / 4, 128, 0, s>>>(L, W.drs, W.feat);
   k_learned_setup<<<(L.nimg + 7) / 8, 256, 0, s>>>(L, W, weights);
 }
 
