@@ -33,40 +33,69 @@ namespace rpba {
 namespace {
 
 constexpr int CP = CO_M * 9;  // P_k entries
+constexpr int PC_S = CoarseWork::PC_S;
 
-// P_k for the rows of aggregate blockIdx.x (row major, 9 x CO_M).
+// P_k for the rows of aggregate blockIdx.x (row major, 9 x CO_M), and its
+// compact form Pc: columns 0..2 live in rows 0..5 (6 values each) and column
+// 6 in rows 3..5 (3 values); every other column holds a single 1, whose row
+// (15: none) is a nibble of the last word -- column 3 + g nibble g, column
+// 7 + g nibble 3 + g.
 __global__ void k_coarse_P(DevLSA L, CoarseWork C) {
   const int a = blockIdx.x;
   const int t0 = C.agg_off[a], t1 = C.agg_off[a + 1];
-  __shared__ double cen[3], rho_inv;
+  // centre and spread of the cameras, in the rows' order: their positions
+  // come in parallel, a chunk at a time, and one thread a component (the
+  // spread: one thread) adds
+  constexpr int CH = 128;
+  __shared__ double cen[3], rho_inv, pc[CH][3];
+  __shared__ int in[CH];
+  auto stage = [&](int c0) {
+    __syncthreads();
+    const int t = c0 + threadIdx.x;
+    if (threadIdx.x < CH && t < t1) {
+      const int k = C.agg_rows[t];
+      in[threadIdx.x] = k >= 1;
+      for (int j = 0; j < 3; ++j) pc[threadIdx.x][j] = L.camn[k].PC[j];
+    }
+    __syncthreads();
+  };
+  double c = 0.;
+  int n = 0;
+  for (int c0 = t0; c0 < t1; c0 += CH) {
+    stage(c0);
+    if (threadIdx.x < 3)
+      for (int u = 0; u < min(CH, t1 - c0); ++u)
+        if (in[u]) {
+          c += pc[u][threadIdx.x];
+          ++n;
+        }
+  }
+  if (threadIdx.x < 3) cen[threadIdx.x] = c / (n > 0 ? n : 1);
+  double r2 = 0.;
+  for (int c0 = t0; c0 < t1; c0 += CH) {
+    stage(c0);
+    if (threadIdx.x == 0)
+      for (int u = 0; u < min(CH, t1 - c0); ++u)
+        if (in[u])
+          for (int j = 0; j < 3; ++j) {
+            const double d = pc[u][j] - cen[j];
+            r2 += d * d;
+          }
+  }
   if (threadIdx.x == 0) {
-    double c[3] = {0., 0., 0.};
-    int n = 0;
-    for (int t = t0; t < t1; ++t) {
-      const int k = C.agg_rows[t];
-      if (k < 1) continue;
-      for (int j = 0; j < 3; ++j) c[j] += L.camn[k].PC[j];
-      ++n;
-    }
-    for (int j = 0; j < 3; ++j) c[j] /= (n > 0 ? n : 1);
-    double r2 = 0.;
-    for (int t = t0; t < t1; ++t) {
-      const int k = C.agg_rows[t];
-      if (k < 1) continue;
-      for (int j = 0; j < 3; ++j) {
-        const double d = L.camn[k].PC[j] - c[j];
-        r2 += d * d;
-      }
-    }
     const double rho = sqrt(r2 / (n > 0 ? n : 1));
-    for (int j = 0; j < 3; ++j) cen[j] = c[j];
     rho_inv = rho > 0. ? 1. / rho : 0.;
   }
   __syncthreads();
   for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
     const int k = C.agg_rows[t];
     double *P = C.P + (size_t)k * CP;
+    double *Pc = C.Pc + (size_t)k * PC_S;
+    unsigned ones = 0xffffffu;
+    auto one = [&](int nibble, int r) { ones = (ones & ~(15u << (4 * nibble))) | ((unsigned)r << (4 * nibble)); };
     for (int i = 0; i < CP; ++i) P[i] = 0.;
+    for (int i = 0; i < PC_S - 1; ++i) Pc[i] = 0.;
+    Pc[PC_S - 1] = __longlong_as_double(ones);
     if (k < 1) continue;  // camera 0's intrinsics row: block-Jacobi only
     const CamState &cs = L.camn[k];
     for (int r = 0; r < 3; ++r)
@@ -84,12 +113,19 @@ __global__ void k_coarse_P(DevLSA L, CoarseWork C) {
       const int c = comp[q], r = 3 + q;
       for (int j = 0; j < 3; ++j) P[r * CO_M + j] = cr[j][c];
       P[r * CO_M + 3 + c] = 1.;
+      one(c, r);
       P[r * CO_M + 6] = lev[c] * rho_inv;
     }
     int r = 3 + npc;
-    if (L.addmask & 1) P[(r++) * CO_M + 7] = 1.;
-    if (L.addmask & 2) P[(r++) * CO_M + 8] = 1.;
-    if (L.addmask & 4) P[(r++) * CO_M + 9] = 1.;
+    for (int j = 0; j < 3; ++j)
+      if (L.addmask & (1 << j)) {
+        one(3 + j, r);
+        P[(r++) * CO_M + 7 + j] = 1.;
+      }
+    for (int j = 0; j < 3; ++j)
+      for (int q = 0; q < 6; ++q) Pc[6 * j + q] = P[q * CO_M + j];
+    for (int q = 0; q < 3; ++q) Pc[18 + q] = P[(3 + q) * CO_M + 6];
+    Pc[PC_S - 1] = __longlong_as_double(ones);
   }
 }
 
@@ -116,85 +152,97 @@ __global__ void k_entry_keys(DevLSA L, CoarseWork C, unsigned *key, int *val) {
 }
 
 // Step 2, one warp per run.  Per entry (l, S_kl) the warp stages S_kl in the
-// run's orientation (row p of k, column q of l) and P_l^T in shared memory,
-// the global loads of the next entry already in flight; lane (j, s) < 30
-// then owns Y[3 s .. 3 s + 2][j] and reads row p of S and column j of P_l as
-// 16-byte pairs.  Each Y entry sums q = 0 .. npl - 1 per entry, the entries
-// in run order (the same operations in the same order as a lane per Y entry
-// reading both operands from global memory).
+// run's orientation (row p of k, column q of l) in shared memory, the next
+// entry's block and P_l already in flight.  Lane (p, g) < 27 owns Y[p][j],
+// j = g, 3 + g, 6 (g = 0) and 7 + g, and adds the products in the order of q
+// that a full row times a full column has; only P_l's nonzero rows (Pc) are
+// multiplied -- the others add 0 -- and its ones added: 11 instead of 27
+// operations a lane, eight instead of 36 values from shared memory, which
+// bounded the full product (5.5M FP32 blocks: 3.8 ms, now 2.2).
 constexpr int RS_T = 256, RS_W = RS_T / 32;
-__global__ void __launch_bounds__(RS_T) k_coarse_runs(DevLSA L, CoarseWork C, int nruns) {
-  __shared__ __align__(16) double Ssh[RS_W][90];   // S_kl[p][q] at 10 p + q
-  __shared__ __align__(16) double Psh[RS_W][100];  // P_l[q][j] at 10 j + q
+template <bool F32>
+__global__ void __launch_bounds__(RS_T, 3) k_coarse_runs(DevLSA L, CoarseWork C, int nruns) {
+  __shared__ __align__(16) double Ssh[RS_W][2][90];  // S_kl[p][q] at 10 p + q
   __shared__ double Ysh[RS_W][9 * CO_M];
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   if (r >= nruns) return;
-  double *Ss = Ssh[wl], *Ps = Psh[wl];
   const int k = (int)(C.run_key[r] / (unsigned)C.nagg);
   const int npk = L.camparv[k + 1] - L.camparv[k];
-  const int jc = lane % 10, s3 = lane < 30 ? lane / 10 : 0;
-  double y[3] = {0., 0., 0.};
+  const int p = lane < 27 ? lane / 3 : 0, g = lane < 27 ? lane - 3 * (lane / 3) : 0;
+  double yg = 0., y3 = 0., y6 = 0., y7 = 0.;
   const int t0 = C.run_off[r], t1 = C.run_off[r + 1];
-  int2 en = make_int2(0, 0);
-  double sv[3], pv[3];
+  // the entries' positions, 32 at a time, one per lane
+  int2 enl = make_int2(0, 0);
+  float sf[3];
+  double sd[3], pc[10];
+  bool tr = false;
   auto fetch = [&](int t) {
-    en = L.ent[C.ent_sorted[t]];
-    const size_t B = (size_t)(en.y & 0x7fffffff);
-    const double *Pl = C.P + (size_t)en.x * CP;
+    const int u = (t - t0) & 31;
+    if (u == 0 && t + lane < t1) enl = __ldg(L.ent + __ldg(C.ent_sorted + t + lane));
+    const int l = __shfl_sync(0xffffffffu, enl.x, u), y = __shfl_sync(0xffffffffu, enl.y, u);
+    tr = y < 0;
+    const size_t B = (size_t)(y & 0x7fffffff);
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const int e = lane + 32 * m;
-      sv[m] = e < 81 ? blk_at(L, B, e) : 0.;
-      pv[m] = e < CP ? __ldg(Pl + e) : 0.;
+      if constexpr (F32)
+        sf[m] = e < 81 ? __ldg(L.blocks32 + B * BS32 + e) : 0.f;
+      else
+        sd[m] = e < 81 ? __ldg(L.blocks + B * BS64 + e) : 0.;
+    }
+    const double *Pl = C.Pc + (size_t)l * PC_S;
+#pragma unroll
+    for (int h = 0; h < 3; ++h) {
+      const double2 v = __ldg((const double2 *)(Pl + 6 * g) + h);
+      pc[2 * h] = v.x;
+      pc[2 * h + 1] = v.y;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double2 v = __ldg((const double2 *)(Pl + 18) + h);
+      pc[6 + 2 * h] = v.x;
+      pc[7 + 2 * h] = v.y;
     }
   };
   if (t0 < t1) fetch(t0);
   for (int t = t0; t < t1; ++t) {
-    const bool tr = en.y < 0;
-    const int l = en.x;
+    double *Ss = Ssh[wl][t & 1];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const int e = lane + 32 * m;
       if (e < 81) {
         const int i = e / 9, c = e - 9 * (e / 9);
-        Ss[tr ? c * 10 + i : i * 10 + c] = sv[m];
-      }
-      if (e < CP) {
-        const int q = e / CO_M, j = e - CO_M * (e / CO_M);
-        Ps[j * 10 + q] = pv[m];
+        Ss[tr ? c * 10 + i : i * 10 + c] = F32 ? (double)sf[m] : sd[m];
       }
     }
-    const int npl = L.camparv[l + 1] - L.camparv[l];
+    double q[9];
+#pragma unroll
+    for (int h = 0; h < 9; ++h) q[h] = pc[h];
+    const unsigned ones = (unsigned)__double2loint(pc[9]);
     __syncwarp();
     if (t + 1 < t1) fetch(t + 1);
-    double pc[10];
+    double sr[6];
 #pragma unroll
-    for (int h = 0; h < 5; ++h) {
-      const double2 v = *(const double2 *)(Ps + jc * 10 + 2 * h);
-      pc[2 * h] = v.x;
-      pc[2 * h + 1] = v.y;
+    for (int h = 0; h < 3; ++h) {
+      const double2 v = *(const double2 *)(Ss + p * 10 + 2 * h);
+      sr[2 * h] = v.x;
+      sr[2 * h + 1] = v.y;
     }
+    const unsigned r3 = (ones >> (4 * g)) & 15u, r7 = (ones >> (12 + 4 * g)) & 15u;
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int p = 3 * s3 + u;
-      double sr[10];
+    for (int h = 0; h < 6; ++h) yg += sr[h] * q[h];
 #pragma unroll
-      for (int h = 0; h < 5; ++h) {
-        const double2 v = *(const double2 *)(Ss + p * 10 + 2 * h);
-        sr[2 * h] = v.x;
-        sr[2 * h + 1] = v.y;
-      }
-      if (lane < 30 && p < npk) {
-#pragma unroll
-        for (int q = 0; q < 9; ++q)
-          if (q < npl) y[u] += sr[q] * pc[q];
-      }
-    }
-    __syncwarp();
+    for (int h = 0; h < 3; ++h) y6 += sr[3 + h] * q[6 + h];
+    if (r3 < 9u) y3 += Ss[p * 10 + r3];
+    if (r7 < 9u) y7 += Ss[p * 10 + r7];
   }
-  if (lane < 30)
-#pragma unroll
-    for (int u = 0; u < 3; ++u) Ysh[wl][(3 * s3 + u) * CO_M + jc] = y[u];
+  double *Y = Ysh[wl];
+  if (lane < 27) {
+    Y[p * CO_M + g] = yg;
+    Y[p * CO_M + 3 + g] = y3;
+    Y[p * CO_M + 7 + g] = y7;
+    if (g == 0) Y[p * CO_M + 6] = y6;
+  }
   __syncwarp();
   const double *Pk = C.P + (size_t)k * CP;
 #pragma unroll
@@ -202,7 +250,7 @@ __global__ void __launch_bounds__(RS_T) k_coarse_runs(DevLSA L, CoarseWork C, in
     const int o = lane + 32 * m, i = o / CO_M, j = o % CO_M;
     if (o < CO_M * CO_M) {
       double z = 0.;
-      for (int p = 0; p < npk; ++p) z += Pk[p * CO_M + i] * Ysh[wl][p * CO_M + j];
+      for (int pp = 0; pp < npk; ++pp) z += Pk[pp * CO_M + i] * Y[pp * CO_M + j];
       C.Z[(size_t)r * CO_M * CO_M + o] = z;
     }
   }
@@ -264,17 +312,33 @@ __global__ void k_coarse_diag(CoarseWork C) {
   C.dsc[i] = d > 0. ? 1. / sqrt(d) : 1.;
 }
 
-// rc_a = sum_{k in a} P_k^T r_k (rows in order)
+// rc_a = sum_{k in a} P_k^T r_k (rows in order), lane j component j.  One
+// chain of sums; four rows' values are loaded before they are added (each
+// row's loads in turn: 120 us for 93 rows an aggregate, now 87).
 __global__ void k_coarse_restrict(CoarseWork C, const double *r) {
-  const int a = blockIdx.x, j = threadIdx.x;
-  if (j >= CO_M) return;
+  const int a = blockIdx.x, j = min((int)threadIdx.x, CO_M - 1);
+  const int t0 = C.agg_off[a], t1 = C.agg_off[a + 1];
   double s = 0.;
-  for (int t = C.agg_off[a]; t < C.agg_off[a + 1]; ++t) {
-    const int k = C.agg_rows[t];
-    const double *P = C.P + (size_t)k * CP;
-    for (int c = 0; c < 9; ++c) s += P[c * CO_M + j] * r[(size_t)k * 9 + c];
+  constexpr int U = 4;
+  for (int tb = t0; tb < t1; tb += U) {
+    double p[U][9], v[U][9];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = C.agg_rows[min(tb + u, t1 - 1)];
+      const double *P = C.P + (size_t)k * CP;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) {
+        p[u][c] = __ldg(P + c * CO_M + j);
+        v[u][c] = __ldg(r + (size_t)k * 9 + c);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (tb + u < t1)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) s += p[u][c] * v[u][c];
   }
-  C.rc[a * CO_M + j] = s;
+  if (threadIdx.x < CO_M) C.rc[a * CO_M + j] = s;
 }
 
 // z_a = A_c^-1[a rows] rc; h_k += P_k z_a for the rows of a
@@ -389,6 +453,7 @@ void coarse_build(const DevLSA &L, int max_aggs, CoarseWork &C, std::vector<void
   C.agg_rows = calloc_dev<int>(rows.size(), owned);
   C.row_agg = calloc_dev<int>(nimg, owned);
   C.P = calloc_dev<double>((size_t)nimg * CP, owned);
+  C.Pc = calloc_dev<double>((size_t)nimg * PC_S, owned);
   C.Ac = calloc_dev<double>(nc * nc, owned);
   C.Ainv = calloc_dev<double>(nc * nc, owned);
   C.rc = calloc_dev<double>(nc, owned);
@@ -493,7 +558,11 @@ void coarse_assemble(const DevLSA &L, CoarseWork &C, int structure_version, cuda
   const size_t nn = (size_t)C.nc * C.nc;
   RPBA_CUDA_CHECK(cudaMemsetAsync(C.Ac, 0, sizeof(double) * nn, s));
   if (C.nruns > 0) {
-    k_coarse_runs<<<(C.nruns + RS_T / 32 - 1) / (RS_T / 32), RS_T, 0, s>>>(L, C, C.nruns);
+    const int g = (C.nruns + RS_W - 1) / RS_W;
+    if (L.blocks32)
+      k_coarse_runs<true><<<g, RS_T, 0, s>>>(L, C, C.nruns);
+    else
+      k_coarse_runs<false><<<g, RS_T, 0, s>>>(L, C, C.nruns);
     k_coarse_blocks<<<(C.nsegs + 7) / 8, 256, 0, s>>>(C, C.nsegs);
   }
   k_coarse_fixdiag<<<(C.nc + 255) / 256, 256, 0, s>>>(C);

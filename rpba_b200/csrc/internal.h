@@ -201,6 +201,8 @@ struct CoarseWork {
   int *agg_rows = nullptr;       // rows of the system grouped by aggregate
   int *row_agg = nullptr;        // [nimg] aggregate of a row, -1 outside
   double *P = nullptr;           // [nimg * 9 * CO_M]
+  static constexpr int PC_S = 22;
+  double *Pc = nullptr;          // [nimg * PC_S] its compact form
   double *Ac = nullptr, *Ainv = nullptr;
   double *rc = nullptr;          // [nc] restricted residual
   double *dsc = nullptr;         // [nc] Jacobi scaling of A_c
@@ -282,7 +284,7 @@ struct PcgWork {
   double *pdiag, *prow, *pw, *pdqc;
   unsigned *ctr;  // [2] next phase-1 chunk, next phase-2 row
   double *rowc;   // [nimg * 12] with the coarse space: per row P_k^T r and its share of |dr|^2
-  double *drs;  // [nimg * 9] 1 / sqrt of the camera blocks' diagonal entries (learned features)
+  double *drs;  // [2 * nimg * 9] 1 / sqrt of the camera blocks' diagonal entries (learned features), the same as floats
   float *feat;  // [nimg * 20] the learned preconditioner's features per camera row
   double *prod;   // FP64 form: [entries * 9] both products of every block, entry order
   unsigned *bar;  // [pcg_bar_bytes] grid-barrier word and the exchanges' sums

@@ -39,27 +39,78 @@ constexpr float ALPHA = 1.0f;
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // 1 / sqrt of the diagonal entries of every camera block (0 past the
-// camera's parameter count), for the normalised couplings of the features.
+// camera's parameter count), for the normalised couplings of the features;
+// behind them the same values rounded to float, the columns' factors.
 // The diagonal is damped (+1e-2), so the clamp never binds on a real entry.
 __global__ void k_diag_rsqrt(DevLSA L, double *drs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = i / 9, a = i % 9;
   if (k >= L.nimg) return;
-  drs[i] = (k >= L.begini && a < L.camparv[k + 1] - L.camparv[k]) ? 1. / sqrt(fmax(blk_at(L, (size_t)k, a * 10), 1e-300))
-                                                                   : 0.;
+  const double v = (k >= L.begini && a < L.camparv[k + 1] - L.camparv[k])
+                       ? 1. / sqrt(fmax(blk_at(L, (size_t)k, a * 10), 1e-300))
+                       : 0.;
+  drs[i] = v;
+  drs[L.nimg * 9 + i] = (double)(float)v;
 }
 
-// Features of camera row k (>= begini) of the assembled system, computed by
-// one warp.  Lane l owns the block elements e = l, l + 32, l + 64 of every
-// off-diagonal block of the row (coalesced reads of the 81 values) and keeps
-// their normalised magnitudes in two accumulators, for the block stored as
-// (k, l) and as (l, k); the coupling sum of parameter a is then reduced over
-// the lanes in a fixed butterfly order.  Every lane returns the same f.
-// drs: 1 / sqrt of every camera block's diagonal entries (k_diag_rsqrt).
-__device__ void block_features(const DevLSA &L, const double *__restrict__ drs, int k, int lane, float f[NN_F]) {
+// Coupling sums of camera row k (>= begini) over its entries t0 .. t1 - 1,
+// which are all stored transposed, as (l, k) (TR), or all as (k, l), by one
+// warp.  Lane l owns the block elements e = l, l + 32, l + 64 (coalesced
+// reads of the 81 values) and adds their normalised magnitudes
+// |S_ij| / sqrt(S_ii S_jj) to ac in entry order, in FP64; of a block stored
+// (k, l), element (i, j) couples parameter i of k to j of l, of one stored
+// (l, k), parameter j of k to i of l.  Elements past either camera's
+// parameter count have a zero factor and are left out.  Four entries at a
+// time: their positions, elements and column factors are loaded before any
+// is used, the next four's positions one batch ahead.
+template <bool F32, bool TR>
+__device__ __forceinline__ void couple(const DevLSA &L, const double *__restrict__ drs, int k, int t0, int t1, int lane,
+                                       double (&ac)[3]) {
+  int own[3], oth[3];  // this row's parameter of the element, and the other's
+  double rk[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const int e = lane + 32 * m, i = e / 9, jj = e - 9 * (e / 9);
+    own[m] = TR ? jj : i;
+    oth[m] = TR ? i : jj;
+    rk[m] = e < 81 ? __ldg(drs + (size_t)k * 9 + own[m]) : 0.;
+  }
+  const double *col = drs + (size_t)L.nimg * 9;
+  constexpr int U = 4;
+  auto entry = [&](int t) { return lane < U && t + lane < t1 ? __ldg(L.ent + t + lane) : make_int2(0, 0); };
+  int2 enl = entry(t0);
+  for (int tb = t0; tb < t1; tb += U) {
+    float v[U][3];
+    double rc[U][3];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int x = __shfl_sync(0xffffffffu, enl.x, u);
+      const size_t B = (size_t)(__shfl_sync(0xffffffffu, enl.y, u) & 0x7fffffff);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const int e = lane + 32 * m;
+        const bool in = tb + u < t1 && (m < 2 || e < 81);
+        v[u][m] = !in ? 0.f : (F32 ? __ldg(L.blocks32 + B * BS32 + e) : (float)__ldg(L.blocks + B * BS64 + e));
+        rc[u][m] = in ? __ldg(col + (size_t)x * 9 + oth[m]) : 0.;
+      }
+    }
+    enl = entry(tb + U);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+        if (__double2hiint(rc[u][m]) != 0 && __double2hiint(rk[m]) != 0)
+          ac[m] += fabs((double)v[u][m]) * rk[m] * rc[u][m];
+  }
+}
+
+// The features of camera row k from its coupling sums (an: entries stored
+// (k, l), at: (l, k)), reduced over the lanes of one warp in a fixed
+// butterfly order.  Every lane returns the same f.
+__device__ __forceinline__ void features_of(const DevLSA &L, int k, int lane, const double (&an)[3],
+                                            const double (&at)[3], float f[NN_F]) {
   const int np = L.camparv[k + 1] - L.camparv[k];
   {
-    // f[0..8] first, so that only nine floats stay live through the walk
     double ld[9], mean = 0.;
 #pragma unroll
     for (int a = 0; a < 9; ++a) {
@@ -70,78 +121,15 @@ __device__ void block_features(const DevLSA &L, const double *__restrict__ drs, 
 #pragma unroll
     for (int a = 0; a < 9; ++a) f[a] = a < np ? (float)(ld[a] - mean) : 0.f;
   }
-  // per owned slot: row i, column j of the stored block, and this row's
-  // diagonal entry for either orientation
-  int ei[3], ej[3];
-  double rn[3], rt[3], an[3] = {0., 0., 0.}, at[3] = {0., 0., 0.};
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const int e = lane + 32 * m;
-    ei[m] = e < 81 ? e / 9 : 9;
-    ej[m] = e < 81 ? e % 9 : 9;
-    rn[m] = ei[m] < 9 ? drs[(size_t)k * 9 + ei[m]] : 0.;
-    rt[m] = ej[m] < 9 ? drs[(size_t)k * 9 + ej[m]] : 0.;
-  }
-  // the row's entries eight at a time: their positions, block elements and
-  // column scalings (as floats: features need no more) are all loaded
-  // before any is used (independent loads in flight), then added in entry
-  // order in FP64
-  // (the next batch's entries are loaded one batch ahead, lane u entry u)
-  constexpr int U = 8;
-  const int t0 = L.rowoff[k], t1 = L.rowoff[k + 1];
-  int2 enl = (lane < U && t0 + lane < t1) ? L.ent[t0 + lane] : make_int2(k, k);
-  for (int tb = t0; tb < t1; tb += U) {
-    int2 en[U];
-    int nc[U];
-    float v[U][3], rcv[U][3];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      en[u].x = __shfl_sync(0xffffffffu, enl.x, u);
-      en[u].y = __shfl_sync(0xffffffffu, enl.y, u);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool tr = en[u].y < 0;
-      const size_t B = (size_t)(en[u].y & 0x7fffffff);
-      const double *rc = drs + (size_t)en[u].x * 9;
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const int i = ei[m], j = ej[m];
-        v[u][m] = i < 9 ? (float)blk_at(L, B, i * 9 + j) : 0.f;
-        rcv[u][m] = i < 9 ? (float)__ldg(rc + (tr ? i : j)) : 0.f;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) nc[u] = L.camparv[en[u].x + 1] - L.camparv[en[u].x];
-    {
-      const int tn = tb + U + lane;
-      enl = (lane < U && tn < t1) ? L.ent[tn] : make_int2(k, k);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (en[u].x == k) continue;  // the diagonal block (and the padding past the row)
-      const bool tr = en[u].y < 0;
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const int i = ei[m], j = ej[m];
-        if (i >= 9) continue;
-        // stored (k, col): element (i, j) couples parameter i of k to j of
-        // col; stored (col, k): it couples parameter j of k to i of col; both
-        // normalised by the two diagonal entries, |S_ij| / sqrt(S_ii S_jj)
-        if (!tr) {
-          if (i < np && j < nc[u]) an[m] += fabs((double)v[u][m]) * rn[m] * (double)rcv[u][m];
-        } else {
-          if (j < np && i < nc[u]) at[m] += fabs((double)v[u][m]) * rt[m] * (double)rcv[u][m];
-        }
-      }
-    }
-  }
   double cpl[9];
 #pragma unroll
   for (int a = 0; a < 9; ++a) {
     double v = 0.;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) v += (ei[m] == a ? an[m] : 0.) + (ej[m] == a ? at[m] : 0.);
+    for (int m = 0; m < 3; ++m) {
+      const int e = lane + 32 * m, i = e < 81 ? e / 9 : 9, j = e < 81 ? e % 9 : 9;
+      v += (i == a ? an[m] : 0.) + (j == a ? at[m] : 0.);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     cpl[a] = v;
@@ -150,6 +138,25 @@ __device__ void block_features(const DevLSA &L, const double *__restrict__ drs, 
 #pragma unroll
   for (int a = 0; a < 9; ++a) f[9 + a] = a < np ? (float)log1p(cpl[a]) : 0.f;
   f[18] = (float)(log1p((double)deg) / 4.);
+}
+
+// Coupling sums of row k's entries before (part 0: stored transposed) or
+// behind (part 1) its diagonal entry.
+__device__ __forceinline__ void couple_part(const DevLSA &L, const double *__restrict__ drs, int k, int part, int lane,
+                                            double (&ac)[3]) {
+  const int t0 = L.rowoff[k], td = t0 + L.firstT[k + 1] - L.firstT[k], t1 = L.rowoff[k + 1];
+  ac[0] = ac[1] = ac[2] = 0.;
+  if (L.blocks32) {
+    if (part == 0)
+      couple<true, true>(L, drs, k, t0, td, lane, ac);
+    else
+      couple<true, false>(L, drs, k, td + 1, t1, lane, ac);
+  } else {
+    if (part == 0)
+      couple<false, true>(L, drs, k, t0, td, lane, ac);
+    else
+      couple<false, false>(L, drs, k, td + 1, t1, lane, ac);
+  }
 }
 
 // Network forward: s (per-parameter scaling) and the tanh hidden layer.
@@ -198,15 +205,26 @@ __device__ __forceinline__ void mlp_forward_warp(const float *W, const float f[N
   for (int i = 0; i < NN_O; ++i) s[i] = expf(ALPHA * tanhf(o[i]));
 }
 
-// Features of every camera row >= begini, one warp per row (block_features),
-// to feat[k * NN_FS ..]: a kernel of its own, so that its loads run at the
-// occupancy of a small register count.
+// Features of every camera row >= begini to feat[k * NN_FS ..], a CTA of two
+// warps per row: one for the entries stored transposed, one for the others
+// (two sums, so the order of neither changes).  Bound by the latency of the
+// blocks, all of which are read from both sides (3.6 GB for 5.5M FP32 blocks):
+// with one warp per row, 168 registers and thus 12 warps an SM it took
+// 2.9 ms for them, now 1.7 ms (16 CTAs an SM; 20 or 8 with eight entries at a time were slower).
 constexpr int NN_FS = 20;  // floats per row of feat
-__global__ void __launch_bounds__(128) k_learned_features(DevLSA L, const double *drs, float *feat) {
-  const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (k >= L.nimg || k < L.begini) return;
+__global__ void __launch_bounds__(64, 16) k_learned_features(DevLSA L, const double *drs, float *feat) {
+  __shared__ double sn[3][32];
+  const int k = blockIdx.x + L.begini, lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  double ac[3];
+  couple_part(L, drs, k, part, lane, ac);
+  if (part == 1)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) sn[m][lane] = ac[m];
+  __syncthreads();
+  if (part == 1) return;
+  const double an[3] = {sn[0][lane], sn[1][lane], sn[2][lane]};
   float f[NN_F];
-  block_features(L, drs, k, lane, f);
+  features_of(L, k, lane, an, ac, f);
   float v = 0.f;
 #pragma unroll
   for (int j = 0; j < NN_F; ++j)
@@ -473,7 +491,12 @@ __global__ void k_rec_rows(DevLSA L, TrainSet T, int row0, int sys, const double
   if (k >= L.nimg) return;
   const int r = row0 + (k - L.begini);
   float f[NN_F];
-  block_features(L, drs, k, lane, f);
+  {
+    double at[3], an[3];
+    couple_part(L, drs, k, 0, lane, at);
+    couple_part(L, drs, k, 1, lane, an);
+    features_of(L, k, lane, an, at, f);
+  }
   const int np = L.camparv[k + 1] - L.camparv[k];
   const double *D = L.blocks + (size_t)k * 81;
   double *Sk = Si + (size_t)k * 81;
@@ -550,7 +573,7 @@ __global__ void k_rec_uc(DevLSA L, TrainSet T, int row0, int pr, const double *v
 
 void learned_pcg_setup(const DevLSA &L, const PcgWork &W, const float *weights, cudaStream_t s) {
   k_diag_rsqrt<<<(L.nimg * 9 + 255) / 256, 256, 0, s>>>(L, W.drs);
-  k_learned_features<<<(L.nimg + 3) / 4, 128, 0, s>>>(L, W.drs, W.feat);
+  if (L.nimg > L.begini) k_learned_features<<<L.nimg - L.begini, 64, 0, s>>>(L, W.drs, W.feat);
   k_learned_setup<<<(L.nimg + 7) / 8, 256, 0, s>>>(L, W, weights);
 }
 

@@ -791,7 +791,7 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   W.d = dalloc<double>(nv, own);
   W.q = dalloc<double>(nv, own);
   W.h = dalloc<double>(nv, own);
-  W.drs = dalloc<double>(nv, own);
+  W.drs = dalloc<double>(2 * nv, own);
   W.feat = dalloc<float>(20 * (size_t)n, own);
   W.x = dalloc<double>(nv, own);
   W.xbest = dalloc<double>(nv, own);
