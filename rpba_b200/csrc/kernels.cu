@@ -177,119 +177,9 @@ __global__ void __launch_bounds__(SS_T) k_seq_sum(const float *__restrict__ v, i
 // (rbacore.cpp:1215-1348, 1420-1616): Jacobians of every observation, the
 // point block V = sum Jp^T W Jp and g = sum Jp^T W d, V damped and inverted;
 // the per-observation record for the camera, pair and back-substitution
-// kernels.  FP64 form (T = double); the FP32 form is k_point32.
-template <class T>
-__global__ void k_point(DevLSA L, double multfact1) {
-  static_assert(sizeof(T) == 8, "the FP32 form is k_point32");
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int p = gt / GRP, ln = gt % GRP;
-  // no early exit: the group reductions below shuffle over the full warp
-  const bool valid = p < L.npts;
-  const int t0 = valid ? L.pt_off[p] : 0, t1 = valid ? L.pt_off[p + 1] : 0;
-  double X0 = 0., X1 = 0., X2 = 0.;
-  if (valid) {
-    const double *X = L.XPM + L.nrioff + 3 * p;
-    X0 = X[0];
-    X1 = X[1];
-    X2 = X[2];
-  }
-  const int esvm[2] = {L.gauge[0], L.gauge[1]};
-  T V[9], g[3];
-#pragma unroll
-  for (int j = 0; j < 9; ++j) V[j] = 0.;
-  g[0] = g[1] = g[2] = 0.;
-  for (int o = t0 + ln; o < t1; o += GRP) {
-    const int k = L.o_cam[o];
-    const CamState c = L.camn[k];
-    const float2 xg = L.o_xg[o];
-    ObsEval e;
-    eval_obs(c, X0, X1, X2, xg.x, xg.y, L.defdiff, e);
-    if (e.nan) L.o_s0rmv[o] = 1.e20f;
-    T Bc[2][RPBA_P], Bp[2][3];
-    jacobians<T>(c, e, role_of(L, k), esvm, L.addmask, Bc, Bp);
-    const float4 w = L.o_w[o];
-    const T W0 = w.x, W1 = w.y, W2 = w.z;
-    const T d1 = (T)e.d1, d2 = (T)e.d2;
-    T G[2][3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      G[0][j] = Bp[0][j] * W0 + Bp[1][j] * W2;
-      G[1][j] = Bp[0][j] * W2 + Bp[1][j] * W1;
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-      for (int b = 0; b < 3; ++b) V[a * 3 + b] += G[0][a] * Bp[0][b] + G[1][a] * Bp[1][b];
-      g[a] += G[0][a] * d1 + G[1][a] * d2;
-    }
-    T *r = Store<T>::rec(L) + (size_t)o * REC;
-    const bool cam_active = k >= L.begini;
-#pragma unroll
-    for (int j = 0; j < RPBA_P; ++j)
-      *(double2 *)(r + 2 * j) = cam_active ? make_double2(Bc[0][j], Bc[1][j]) : make_double2(0., 0.);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      r[18 + j] = G[0][j];
-      r[21 + j] = G[1][j];
-    }
-    r[24] = d1 * W0 + d2 * W2;
-    r[25] = d1 * W2 + d2 * W1;
-  }
-#pragma unroll
-  for (int j = 0; j < 9; ++j) V[j] = grp_sum(V[j]);
-#pragma unroll
-  for (int j = 0; j < 3; ++j) g[j] = grp_sum(g[j]);
-  if (L.ao && valid && L.pt_gcp[p] > -1) {
-    // CalcDerivatives3DGCP (rbacore.cpp:1677-1729): the 3-D prior of a
-    // point shared with other partitions, residual gcp - X, B = -I
-    const float *w = L.W3 + 6 * (size_t)L.pt_w3row[p];
-    const double *gx = L.gcpdata + 3 * (size_t)L.pt_gcp[p];
-    const double d1 = gx[0] - X0, d2 = gx[1] - X1, d3 = gx[2] - X2;
-    const double Wm[9] = {w[0], w[3], w[4], w[3], w[1], w[5], w[4], w[5], w[2]};
-#pragma unroll
-    for (int j = 0; j < 9; ++j) V[j] += Wm[j];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) g[r] += (-Wm[r * 3]) * d1 + (-Wm[r * 3 + 1]) * d2 + (-Wm[r * 3 + 2]) * d3;
-  }
-  V[0] = (T)(V[0] * multfact1);
-  V[4] = (T)(V[4] * multfact1);
-  V[8] = (T)(V[8] * multfact1);
-  T Vi[9];
-  inv3<T>(V, Vi);
-  if (ln == 0 && valid) {
-    T *pv = Store<T>::ptV(L) + (size_t)p * PREC;
-#pragma unroll
-    for (int j = 0; j < 9; ++j) pv[j] = Vi[j];
-    pv[9] = g[0];
-    pv[10] = g[1];
-    pv[11] = g[2];
-  }
-  T vg[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) vg[a] = Vi[a * 3] * g[0] + Vi[a * 3 + 1] * g[1] + Vi[a * 3 + 2] * g[2];
-  for (int o = t0 + ln; o < t1; o += GRP) {
-    T *r = Store<T>::rec(L) + (size_t)o * REC;
-    T G[2][3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      G[0][j] = r[18 + j];
-      G[1][j] = r[21 + j];
-    }
-    const float4 w = L.o_w[o];
-    T GV[2][3];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) GV[a][b] = G[a][0] * Vi[b] + G[a][1] * Vi[3 + b] + G[a][2] * Vi[6 + b];
-    r[26] = (T)w.x - (GV[0][0] * G[0][0] + GV[0][1] * G[0][1] + GV[0][2] * G[0][2]);
-    r[27] = (T)w.z - (GV[0][0] * G[1][0] + GV[0][1] * G[1][1] + GV[0][2] * G[1][2]);
-    r[28] = (T)w.y - (GV[1][0] * G[1][0] + GV[1][1] * G[1][1] + GV[1][2] * G[1][2]);
-    r[29] = r[24] - (G[0][0] * vg[0] + G[0][1] * vg[1] + G[0][2] * vg[2]);
-    r[30] = r[25] - (G[1][0] * vg[0] + G[1][1] * vg[1] + G[1][2] * vg[2]);
-  }
-}
-
-// FP32 form of the point pass, whitened.  V and g are summed in FP64 from
+// kernels.
+//
+// FP32 form: whitened.  V and g are summed in FP64 from
 // the FP32-rounded point Jacobians, V = L L^T is factored in FP64, and the
 // record carries H = G L^-T in place of G, so that every Schur product
 // G V^-1 G^T = H H^T is formed from bounded factors (H H^T <= W for each
@@ -300,136 +190,303 @@ __global__ void k_point(DevLSA L, double multfact1) {
 // coordinate of the point unchanged (the factor is that of V without its row
 // and column), and the Schur contribution stays positive semidefinite.
 // Point record: L^-1 (9, row major, zeros above the diagonal), q = L^-1 g.
-__global__ void k_point32(DevLSA L, double multfact1) {
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int p = gt / GRP, ln = gt % GRP;
-  const bool valid = p < L.npts;  // no early exit (full-warp shuffles below)
-  const int t0 = valid ? L.pt_off[p] : 0, t1 = valid ? L.pt_off[p + 1] : 0;
-  double X0 = 0., X1 = 0., X2 = 0.;
-  if (valid) {
-    const double *X = L.XPM + L.nrioff + 3 * p;
-    X0 = X[0];
-    X1 = X[1];
-    X2 = X[2];
-  }
+//
+// A warp takes PT_N consecutive points, whose observations are consecutive
+// too, 32 at a time whichever point they belong to.  Every lane leaves its
+// observation's record and its terms of V and g in shared memory; four lanes
+// a point then sum the terms (eight running sums a point, observations l,
+// l + 8, ... in sum l, then a butterfly) and factor V, and the records are
+// finished and written out 16 bytes a lane along the lines.  Observations
+// before the last 32 wait in global memory.  Bound by the latency of the
+// camera states and of the FP64 divisions and roots at 12 to 16 warps an SM:
+// eight lanes a point, in turns of eight observations, ran 1.9 turns for
+// every four points of a city (the longest of the four decides), each lane
+// writing its own record, 32 lines an instruction.  A launch: FP32, 27.8M
+// observations 3.95 -> 2.8 ms, 868,000 155 -> 97 us; FP64, 2.8M 0.58 -> 0.42
+// ms, 902,000 191 -> 141 us.
+template <class T>
+struct PointGeom {
+  static constexpr bool F32 = sizeof(T) == 4;
+  static constexpr int RS = REC + 16 / (int)sizeof(T);  // values per record in shared memory (odd number of pieces)
+  static constexpr int NC = F32 ? 9 : 12, CS = F32 ? 9 : 13;  // terms of V and g, stride
+  static constexpr int NM = F32 ? 9 : 12;                     // per point: factor and q, or V^-1 and V^-1 g
+  static constexpr int W = F32 ? 4 : 2;                       // warps per CTA (48 KB of shared memory at most)
+};
+constexpr int PT_N = 8;  // points per warp
+template <class T>
+struct PointShared {
+  using Ge = PointGeom<T>;
+  T rec[32 * Ge::RS];
+  double term[32 * Ge::CS], acc[2 * Ge::NC][32], pt[PT_N][Ge::NM];
+};
+
+template <class T>
+__global__ void __launch_bounds__(32 * PointGeom<T>::W, sizeof(T) == 4 ? 4 : 6) k_point(DevLSA L, double multfact1) {
+  using Ge = PointGeom<T>;
+  constexpr bool F32 = Ge::F32;
+  constexpr int RS = Ge::RS, NC = Ge::NC, CS = Ge::CS;
+  constexpr int PR = REC * (int)sizeof(T) / 16;  // pieces of a record
+  extern __shared__ __align__(16) unsigned char pt_dyn[];
+  PointShared<T> &S = ((PointShared<T> *)pt_dyn)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, p0 = (blockIdx.x * Ge::W + (threadIdx.x >> 5)) * PT_N;
+  if (p0 >= L.npts) return;
+  const int pn = min(PT_N, L.npts - p0);
+  T *rec = Store<T>::rec(L);
+  // the lane's point (four lanes each) and the warp's observations
+  const int q = lane >> 2, j = lane & 3;
+  const int base = L.pt_off[p0], end = L.pt_off[p0 + pn];
+  const int t0 = q < pn ? L.pt_off[p0 + q] : end, t1 = q < pn ? L.pt_off[p0 + q + 1] : end;
   const int esvm[2] = {L.gauge[0], L.gauge[1]};
-  double V[6] = {0., 0., 0., 0., 0., 0.};  // V00 V01 V02 V11 V12 V22
-  double g[3] = {0., 0., 0.};
-  for (int o = t0 + ln; o < t1; o += GRP) {
-    const int k = L.o_cam[o];
-    const CamState c = L.camn[k];
-    const float2 xg = L.o_xg[o];
-    ObsEval e;
-    eval_obs(c, X0, X1, X2, xg.x, xg.y, L.defdiff, e);
-    if (e.nan) L.o_s0rmv[o] = 1.e20f;
-    float Bc[2][RPBA_P], Bp[2][3];
-    jacobians<float>(c, e, role_of(L, k), esvm, L.addmask, Bc, Bp);
-    const float4 w = L.o_w[o];
-    const double W0 = w.x, W1 = w.y, W2 = w.z;
-    double G[2][3];
+  T *r = S.rec + lane * RS;
+  // records of the observations wb .. wb + 31: shared memory to global and back
+  auto copy_out = [&](int wb) {
+    __syncwarp();
+    const int n = min(32, end - wb) * PR;
+    float4 *dst = (float4 *)(rec + (size_t)wb * REC);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      G[0][j] = Bp[0][j] * W0 + Bp[1][j] * W2;
-      G[1][j] = Bp[0][j] * W2 + Bp[1][j] * W1;
+    for (int it = 0; it < PR; ++it) {
+      const int i = lane + 32 * it;
+      if (i < n) dst[i] = *(const float4 *)(S.rec + (i / PR) * RS + (i % PR) * (16 / (int)sizeof(T)));
     }
-    V[0] += G[0][0] * Bp[0][0] + G[1][0] * Bp[1][0];
-    V[1] += G[0][0] * Bp[0][1] + G[1][0] * Bp[1][1];
-    V[2] += G[0][0] * Bp[0][2] + G[1][0] * Bp[1][2];
-    V[3] += G[0][1] * Bp[0][1] + G[1][1] * Bp[1][1];
-    V[4] += G[0][1] * Bp[0][2] + G[1][1] * Bp[1][2];
-    V[5] += G[0][2] * Bp[0][2] + G[1][2] * Bp[1][2];
+    __syncwarp();
+  };
+  auto copy_in = [&](int wb) {
+    const float4 *src = (const float4 *)(rec + (size_t)wb * REC);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) g[a] += G[0][a] * e.d1 + G[1][a] * e.d2;
-    // the record's floats 0..25 in 16-byte stores: Bc, then Jp until the
-    // factor is known (replaced by H below), then W d
-    const bool cam_active = k >= L.begini;
-    float v[28];
-#pragma unroll
-    for (int j = 0; j < RPBA_P; ++j) {
-      v[2 * j] = cam_active ? Bc[0][j] : 0.f;
-      v[2 * j + 1] = cam_active ? Bc[1][j] : 0.f;
+    for (int it = 0; it < PR; ++it) {
+      const int i = lane + 32 * it;  // (only the last 32 can be fewer, and they never left)
+      *(float4 *)(S.rec + (i / PR) * RS + (i % PR) * (16 / (int)sizeof(T))) = src[i];
     }
+    __syncwarp();
+  };
+  double va[NC], vb[NC];  // running sums j and j + 4 of the point
+  for (int wb = base; wb < end || wb == base; wb += 32) {
+    const int o = wb + lane;
+    if (o < end) {
+      const int k = L.o_cam[o];
+      const double *X = L.XPM + L.nrioff + 3 * (size_t)L.o_pt[o];
+      const CamState c = L.camn[k];
+      const float2 xg = L.o_xg[o];
+      ObsEval e;
+      eval_obs(c, X[0], X[1], X[2], xg.x, xg.y, L.defdiff, e);
+      if (e.nan) L.o_s0rmv[o] = 1.e20f;
+      T Bc[2][RPBA_P], Bp[2][3];
+      jacobians<T>(c, e, role_of(L, k), esvm, L.addmask, Bc, Bp);
+      const bool cam_active = k >= L.begini;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      v[18 + j] = Bp[0][j];
-      v[21 + j] = Bp[1][j];
+      for (int h = 0; h < RPBA_P; ++h) {
+        typename Pair2<T>::type v;
+        v.x = cam_active ? Bc[0][h] : T(0);
+        v.y = cam_active ? Bc[1][h] : T(0);
+        *(typename Pair2<T>::type *)(r + 2 * h) = v;
+      }
+      const float4 w = L.o_w[o];
+      const double W0 = w.x, W1 = w.y, W2 = w.z;
+      double *t = S.term + lane * CS;
+      double G[2][3];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        G[0][h] = Bp[0][h] * W0 + Bp[1][h] * W2;
+        G[1][h] = Bp[0][h] * W2 + Bp[1][h] * W1;
+      }
+      if constexpr (F32) {
+        t[0] = G[0][0] * Bp[0][0] + G[1][0] * Bp[1][0];
+        t[1] = G[0][0] * Bp[0][1] + G[1][0] * Bp[1][1];
+        t[2] = G[0][0] * Bp[0][2] + G[1][0] * Bp[1][2];
+        t[3] = G[0][1] * Bp[0][1] + G[1][1] * Bp[1][1];
+        t[4] = G[0][1] * Bp[0][2] + G[1][1] * Bp[1][2];
+        t[5] = G[0][2] * Bp[0][2] + G[1][2] * Bp[1][2];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) t[6 + a] = G[0][a] * e.d1 + G[1][a] * e.d2;
+        // Jp until the factor is known (then H)
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+          r[18 + h] = Bp[0][h];
+          r[21 + h] = Bp[1][h];
+        }
+      } else {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+#pragma unroll
+          for (int b = 0; b < 3; ++b) t[a * 3 + b] = G[0][a] * Bp[0][b] + G[1][a] * Bp[1][b];
+          t[9 + a] = G[0][a] * e.d1 + G[1][a] * e.d2;
+        }
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+          r[18 + h] = G[0][h];
+          r[21 + h] = G[1][h];
+        }
+      }
+      r[24] = (T)(e.d1 * W0 + e.d2 * W2);
+      r[25] = (T)(e.d1 * W2 + e.d2 * W1);
     }
-    v[24] = (float)(e.d1 * W0 + e.d2 * W2);
-    v[25] = (float)(e.d1 * W2 + e.d2 * W1);
-    float4 *r4 = (float4 *)(L.rec32 + (size_t)o * REC);
+    __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 6; ++j) r4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    *(float2 *)(r4 + 6) = make_float2(v[24], v[25]);
+    for (int f = 0; f < NC; ++f) {
+      va[f] = wb > base ? S.acc[f][lane] : 0.;
+      vb[f] = wb > base ? S.acc[NC + f][lane] : 0.;
+    }
+    int u = t0 + j;
+    if (u < wb) u += ((wb - u) >> 3) << 3;
+    const int ue = min(t1, wb + 32);
+    for (; u < ue; u += 8) {
+      if (u >= wb) {
+        const double *t = S.term + (u - wb) * CS;
+#pragma unroll
+        for (int f = 0; f < NC; ++f) va[f] += t[f];
+      }
+      if (u + 4 >= wb && u + 4 < ue) {
+        const double *t = S.term + (u + 4 - wb) * CS;
+#pragma unroll
+        for (int f = 0; f < NC; ++f) vb[f] += t[f];
+      }
+    }
+    if (wb + 32 < end) {
+#pragma unroll
+      for (int f = 0; f < NC; ++f) {
+        S.acc[f][lane] = va[f];
+        S.acc[NC + f][lane] = vb[f];
+      }
+      copy_out(wb);
+    }
   }
 #pragma unroll
-  for (int j = 0; j < 6; ++j) V[j] = grp_sum(V[j]);
-#pragma unroll
-  for (int j = 0; j < 3; ++j) g[j] = grp_sum(g[j]);
-  V[0] *= multfact1;
-  V[3] *= multfact1;
-  V[5] *= multfact1;
-  // V = L L^T with guarded pivots; m = L^-1 (lower)
-  auto root = [](double d, double diag) { return (d > 1.e-13 * diag && d > 1.e-60) ? sqrt(d) : 0.; };
-  const double l00 = root(V[0], V[0]);
-  const double i00 = l00 > 0. ? 1. / l00 : 0.;
-  const double l10 = V[1] * i00, l20 = V[2] * i00;
-  const double l11 = root(V[3] - l10 * l10, V[3]);
-  const double i11 = l11 > 0. ? 1. / l11 : 0.;
-  const double l21 = (V[4] - l20 * l10) * i11;
-  const double l22 = root(V[5] - l20 * l20 - l21 * l21, V[5]);
-  const double i22 = l22 > 0. ? 1. / l22 : 0.;
-  double m[6] = {i00, -l10 * i00 * i11, i11, -(l20 * i00 - l21 * l10 * i00 * i11) * i22, -l21 * i11 * i22, i22};
-  // m00 m10 m11 m20 m21 m22; a factor beyond the FP32 range drops the point
-  bool inrange = true;
-#pragma unroll
-  for (int j = 0; j < 6; ++j) inrange = inrange && fabs(m[j]) < 1.e30;
-  if (!inrange)
-#pragma unroll
-    for (int j = 0; j < 6; ++j) m[j] = 0.;
-  const double q0 = m[0] * g[0], q1 = m[1] * g[0] + m[2] * g[1], q2 = m[3] * g[0] + m[4] * g[1] + m[5] * g[2];
-  if (ln == 0 && valid) {
-    float *pv = L.ptV32 + (size_t)p * PREC;
-    pv[0] = (float)m[0];
-    pv[1] = pv[2] = 0.f;
-    pv[3] = (float)m[1];
-    pv[4] = (float)m[2];
-    pv[5] = 0.f;
-    pv[6] = (float)m[3];
-    pv[7] = (float)m[4];
-    pv[8] = (float)m[5];
-    pv[9] = (float)q0;
-    pv[10] = (float)q1;
-    pv[11] = (float)q2;
+  for (int f = 0; f < NC; ++f) {
+    va[f] += vb[f];
+    va[f] += __shfl_xor_sync(0xffffffffu, va[f], 2);
+    va[f] += __shfl_xor_sync(0xffffffffu, va[f], 1);
   }
-  for (int o = t0 + ln; o < t1; o += GRP) {
-    float *r = L.rec32 + (size_t)o * REC;
-    const float4 w = L.o_w[o];
-    const double W0 = w.x, W1 = w.y, W2 = w.z;
-    // floats 16..27 of the record (Jp at 18..23, W d at 24, 25)
-    const float4 ra = *(const float4 *)(r + 16), rb = *(const float4 *)(r + 20), rcv = *(const float4 *)(r + 24);
-    double H[2][3];
-    {
-      const double p00 = ra.z, p01 = ra.w, p02 = rb.x, p10 = rb.y, p11 = rb.z, p12 = rb.w;
-      const double G0[3] = {p00 * W0 + p10 * W2, p01 * W0 + p11 * W2, p02 * W0 + p12 * W2};
-      const double G1[3] = {p00 * W2 + p10 * W1, p01 * W2 + p11 * W1, p02 * W2 + p12 * W1};
-      H[0][0] = m[0] * G0[0];
-      H[0][1] = m[1] * G0[0] + m[2] * G0[1];
-      H[0][2] = m[3] * G0[0] + m[4] * G0[1] + m[5] * G0[2];
-      H[1][0] = m[0] * G1[0];
-      H[1][1] = m[1] * G1[0] + m[2] * G1[1];
-      H[1][2] = m[3] * G1[0] + m[4] * G1[1] + m[5] * G1[2];
+  const int p = p0 + q;
+  T *pv = Store<T>::ptV(L) + (size_t)p * PREC;
+  if constexpr (F32) {
+    double V[6], g[3];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) V[f] = va[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) g[f] = va[6 + f];
+    V[0] *= multfact1;
+    V[3] *= multfact1;
+    V[5] *= multfact1;
+    // V = L L^T with guarded pivots; m = L^-1 (lower)
+    auto root = [](double d, double diag) { return (d > 1.e-13 * diag && d > 1.e-60) ? sqrt(d) : 0.; };
+    const double l00 = root(V[0], V[0]);
+    const double i00 = l00 > 0. ? 1. / l00 : 0.;
+    const double l10 = V[1] * i00, l20 = V[2] * i00;
+    const double l11 = root(V[3] - l10 * l10, V[3]);
+    const double i11 = l11 > 0. ? 1. / l11 : 0.;
+    const double l21 = (V[4] - l20 * l10) * i11;
+    const double l22 = root(V[5] - l20 * l20 - l21 * l21, V[5]);
+    const double i22 = l22 > 0. ? 1. / l22 : 0.;
+    double m[6] = {i00, -l10 * i00 * i11, i11, -(l20 * i00 - l21 * l10 * i00 * i11) * i22, -l21 * i11 * i22, i22};
+    // m00 m10 m11 m20 m21 m22; a factor beyond the FP32 range drops the point
+    bool inrange = true;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) inrange = inrange && fabs(m[f]) < 1.e30;
+    if (!inrange)
+#pragma unroll
+      for (int f = 0; f < 6; ++f) m[f] = 0.;
+    const double q0 = m[0] * g[0], q1 = m[1] * g[0] + m[2] * g[1], q2 = m[3] * g[0] + m[4] * g[1] + m[5] * g[2];
+    if (j == 0 && q < pn) {
+#pragma unroll
+      for (int f = 0; f < 6; ++f) S.pt[q][f] = m[f];
+      S.pt[q][6] = q0;
+      S.pt[q][7] = q1;
+      S.pt[q][8] = q2;
+      ((float4 *)pv)[0] = make_float4((float)m[0], 0.f, 0.f, (float)m[1]);
+      ((float4 *)pv)[1] = make_float4((float)m[2], 0.f, (float)m[3], (float)m[4]);
+      ((float4 *)pv)[2] = make_float4((float)m[5], (float)q0, (float)q1, (float)q2);
     }
-    const double h00 = H[0][0] * H[0][0] + H[0][1] * H[0][1] + H[0][2] * H[0][2];
-    const double h01 = H[0][0] * H[1][0] + H[0][1] * H[1][1] + H[0][2] * H[1][2];
-    const double h11 = H[1][0] * H[1][0] + H[1][1] * H[1][1] + H[1][2] * H[1][2];
-    // floats 16..31 in 16-byte stores: H at 18..23, W - H H^T at 26..28,
-    // W d - H q at 29, 30 (16, 17, 24, 25 rewritten unchanged, 31 zero)
-    float4 *r4 = (float4 *)(r + 16);
-    r4[0] = make_float4(ra.x, ra.y, (float)H[0][0], (float)H[0][1]);
-    r4[1] = make_float4((float)H[0][2], (float)H[1][0], (float)H[1][1], (float)H[1][2]);
-    r4[2] = make_float4(rcv.x, rcv.y, (float)(W0 - h00), (float)(W2 - h01));
-    r4[3] = make_float4((float)(W1 - h11), (float)((double)rcv.x - (H[0][0] * q0 + H[0][1] * q1 + H[0][2] * q2)),
-                        (float)((double)rcv.y - (H[1][0] * q0 + H[1][1] * q1 + H[1][2] * q2)), 0.f);
+  } else {
+    double V[9], g[3];
+#pragma unroll
+    for (int f = 0; f < 9; ++f) V[f] = va[f];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) g[f] = va[9 + f];
+    if (L.ao && q < pn && L.pt_gcp[p] > -1) {
+      // CalcDerivatives3DGCP (rbacore.cpp:1677-1729): the 3-D prior of a
+      // point shared with other partitions, residual gcp - X, B = -I
+      const double *X = L.XPM + L.nrioff + 3 * (size_t)p;
+      const float *w = L.W3 + 6 * (size_t)L.pt_w3row[p];
+      const double *gx = L.gcpdata + 3 * (size_t)L.pt_gcp[p];
+      const double d1 = gx[0] - X[0], d2 = gx[1] - X[1], d3 = gx[2] - X[2];
+      const double Wm[9] = {w[0], w[3], w[4], w[3], w[1], w[5], w[4], w[5], w[2]};
+#pragma unroll
+      for (int f = 0; f < 9; ++f) V[f] += Wm[f];
+#pragma unroll
+      for (int f = 0; f < 3; ++f) g[f] += (-Wm[f * 3]) * d1 + (-Wm[f * 3 + 1]) * d2 + (-Wm[f * 3 + 2]) * d3;
+    }
+    V[0] = V[0] * multfact1;
+    V[4] = V[4] * multfact1;
+    V[8] = V[8] * multfact1;
+    double Vi[9];
+    inv3<double>(V, Vi);
+    if (j == 0 && q < pn) {
+#pragma unroll
+      for (int f = 0; f < 9; ++f) S.pt[q][f] = pv[f] = Vi[f];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        pv[9 + a] = g[a];
+        S.pt[q][9 + a] = Vi[a * 3] * g[0] + Vi[a * 3 + 1] * g[1] + Vi[a * 3 + 2] * g[2];
+      }
+    }
+  }
+  __syncwarp();
+  // the last 32 observations' records are in shared memory, the others return
+  bool here = true;
+  for (int wb = base + ((max(end - base, 1) - 1) / 32) * 32; wb >= base; wb -= 32) {
+    if (!here) copy_in(wb);
+    here = false;
+    const int o = wb + lane;
+    if (o < end) {
+      const double *m = S.pt[L.o_pt[o] - p0];
+      const float4 w = L.o_w[o];
+      if constexpr (F32) {
+        const double W0 = w.x, W1 = w.y, W2 = w.z;
+        const float4 ra = *(const float4 *)(r + 16), rb = *(const float4 *)(r + 20);
+        const float2 e = *(const float2 *)(r + 24);
+        double H[2][3];
+        {
+          const double p00 = ra.z, p01 = ra.w, p02 = rb.x, p10 = rb.y, p11 = rb.z, p12 = rb.w;
+          const double G0[3] = {p00 * W0 + p10 * W2, p01 * W0 + p11 * W2, p02 * W0 + p12 * W2};
+          const double G1[3] = {p00 * W2 + p10 * W1, p01 * W2 + p11 * W1, p02 * W2 + p12 * W1};
+          H[0][0] = m[0] * G0[0];
+          H[0][1] = m[1] * G0[0] + m[2] * G0[1];
+          H[0][2] = m[3] * G0[0] + m[4] * G0[1] + m[5] * G0[2];
+          H[1][0] = m[0] * G1[0];
+          H[1][1] = m[1] * G1[0] + m[2] * G1[1];
+          H[1][2] = m[3] * G1[0] + m[4] * G1[1] + m[5] * G1[2];
+        }
+        const double h00 = H[0][0] * H[0][0] + H[0][1] * H[0][1] + H[0][2] * H[0][2];
+        const double h01 = H[0][0] * H[1][0] + H[0][1] * H[1][1] + H[0][2] * H[1][2];
+        const double h11 = H[1][0] * H[1][0] + H[1][1] * H[1][1] + H[1][2] * H[1][2];
+        // H at 18..23, W - H H^T at 26..28, W d - H q at 29, 30, 31 zero
+        float4 *r4 = (float4 *)(r + 16);
+        r4[0] = make_float4(ra.x, ra.y, (float)H[0][0], (float)H[0][1]);
+        r4[1] = make_float4((float)H[0][2], (float)H[1][0], (float)H[1][1], (float)H[1][2]);
+        r4[2] = make_float4(e.x, e.y, (float)(W0 - h00), (float)(W2 - h01));
+        r4[3] = make_float4((float)(W1 - h11), (float)((double)e.x - (H[0][0] * m[6] + H[0][1] * m[7] + H[0][2] * m[8])),
+                            (float)((double)e.y - (H[1][0] * m[6] + H[1][1] * m[7] + H[1][2] * m[8])), 0.f);
+      } else {
+        double G[2][3], GV[2][3];
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+          G[0][h] = r[18 + h];
+          G[1][h] = r[21 + h];
+        }
+        const double *vg = m + 9;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 3; ++b) GV[a][b] = G[a][0] * m[b] + G[a][1] * m[3 + b] + G[a][2] * m[6 + b];
+        r[26] = (T)w.x - (GV[0][0] * G[0][0] + GV[0][1] * G[0][1] + GV[0][2] * G[0][2]);
+        r[27] = (T)w.z - (GV[0][0] * G[1][0] + GV[0][1] * G[1][1] + GV[0][2] * G[1][2]);
+        r[28] = (T)w.y - (GV[1][0] * G[1][0] + GV[1][1] * G[1][1] + GV[1][2] * G[1][2]);
+        r[29] = r[24] - (G[0][0] * vg[0] + G[0][1] * vg[1] + G[0][2] * vg[2]);
+        r[30] = r[25] - (G[1][0] * vg[0] + G[1][1] * vg[1] + G[1][2] * vg[2]);
+        r[31] = 0.;
+      }
+    }
+    copy_out(wb);
   }
 }
 
@@ -1211,12 +1268,19 @@ void launch_seq_sum(const float *v, int n, float *out, cudaStream_t s) {
   k_seq_sum<<<1, SS_T, 0, s>>>(v, n, out);
 }
 
+template <class T>
+static void point_pass(const DevLSA &L, double multfact1, cudaStream_t s) {
+  constexpr int W = PointGeom<T>::W;
+  static_assert(W * sizeof(PointShared<T>) <= 48 * 1024, "shared memory without an attribute");
+  k_point<T><<<nblk(L.npts, PT_N * W), 32 * W, W * sizeof(PointShared<T>), s>>>(L, multfact1);
+}
+
 void launch_point_pass(const DevLSA &L, double multfact1, cudaStream_t s) {
   if (L.npts <= 0) return;
   if (L.rec32)
-    k_point32<<<nblk((long long)L.npts * GRP, 128), 128, 0, s>>>(L, multfact1);
+    point_pass<float>(L, multfact1, s);
   else
-    k_point<double><<<nblk((long long)L.npts * GRP, 128), 128, 0, s>>>(L, multfact1);
+    point_pass<double>(L, multfact1, s);
 }
 
 void launch_camera_pass(const DevLSA &L, double multfact1, cudaStream_t s) {
