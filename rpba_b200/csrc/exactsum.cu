@@ -27,8 +27,8 @@
 // So the first ES_SOLO elements are summed by one CTA (its steps are two
 // block barriers each), inputs up to that length by a kernel of one CTA, not
 // cooperative; longer ones go on with one CTA per SM.  Measured (18 to 20
-// sums a solve): 5.4k terms 82 -> 25 us, 30k 115 -> 43 us, 0.87M 277 ->
-// 112 us, 28M 704 -> 242 us; before, the first 2,048 elements were added
+// sums a solve): 5.4k terms 82 -> 22 us, 30k 115 -> 37 us, 0.87M 277 ->
+// 102 us, 28M 704 -> 216 us; before, the first 2,048 elements were added
 // at 25 cycles each, a step took four grid barriers, and one thread walked
 // the chunks' composites.
 //
@@ -151,28 +151,64 @@ __device__ __forceinline__ void xf_push(Xf &x, int fl, int r, bool tie) {
   x.q ^= (unsigned)(r0 & 1) | ((unsigned)(r1 & 1) << 1);
 }
 
+// Four elements onto a composite whose two parities have not parted (R0, M0
+// stand for both), unless one of them is a tie or saturates: 10 instead of 25
+// instructions an element.  Increments are not negative, so the saturation of
+// R and M can wait for the end of the group.
+__device__ __forceinline__ bool xf_push4(Xf &x, const float4 &a, const Binade &b) {
+  const float f0 = (a.x * b.s1) * b.s2, f1 = (a.y * b.s1) * b.s2, f2 = (a.z * b.s1) * b.s2, f3 = (a.w * b.s1) * b.s2;
+  const float g0 = floorf(f0), g1 = floorf(f1), g2 = floorf(f2), g3 = floorf(f3);
+  const float h0 = f0 - g0, h1 = f1 - g1, h2 = f2 - g2, h3 = f3 - g3;
+  const bool in = f0 < (float)SAT && f1 < (float)SAT && f2 < (float)SAT && f3 < (float)SAT;
+  if (!in || h0 == 0.5f || h1 == 0.5f || h2 == 0.5f || h3 == 0.5f) return false;
+  const int R0 = x.R0, R1 = R0 + (int)g0 + (h0 > 0.5f), R2 = R1 + (int)g1 + (h1 > 0.5f), R3 = R2 + (int)g2 + (h2 > 0.5f),
+            R4 = R3 + (int)g3 + (h3 > 0.5f);
+  const int M = max(max(R0 + (int)g0, R1 + (int)g1), max(R2 + (int)g2, R3 + (int)g3));
+  x.M0 = max(x.M0, min(M, SAT));
+  x.R0 = min(R4, SAT);
+  if ((R4 - R0) & 1) x.q ^= 3u;
+  return true;
+}
+
 // Composite of v[lo, hi): 16-byte loads of whole aligned groups.
 __device__ __forceinline__ Xf xf_range(const float *__restrict__ v, int lo, int hi, bool aligned, const Binade &b) {
   Xf x = xf_identity();
+  bool parted = false;
   auto push = [&](float a) {
     int fl, r;
     bool tie;
     classify(a, b, fl, r, tie);
+    if (!parted) {
+      x.R1 = x.R0;
+      x.M1 = x.M0;
+      parted = true;
+    }
     xf_push(x, fl, r, tie);
+  };
+  auto push4 = [&](const float4 &a) {
+    if (!parted && xf_push4(x, a, b)) return;
+    push(a.x);
+    push(a.y);
+    push(a.z);
+    push(a.w);
   };
   int k = lo;
   if (aligned) {
     for (; k < hi && (k & 3); ++k) push(__ldg(v + k));
-#pragma unroll 2
-    for (; k + 4 <= hi; k += 4) {
-      const float4 a = __ldg((const float4 *)(v + k));
-      push(a.x);
-      push(a.y);
-      push(a.z);
-      push(a.w);
+    for (; k + 16 <= hi; k += 16) {
+      float4 a[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) a[m] = __ldg((const float4 *)(v + k) + m);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) push4(a[m]);
     }
+    for (; k + 4 <= hi; k += 4) push4(__ldg((const float4 *)(v + k)));
   }
   for (; k < hi; ++k) push(__ldg(v + k));
+  if (!parted) {
+    x.R1 = x.R0;
+    x.M1 = x.M0;
+  }
   return x;
 }
 
@@ -225,9 +261,9 @@ __device__ __forceinline__ float seq_block(const float *__restrict__ v, int i, i
 
 // The window [i0, wend) cut into `parts` pieces at multiples of four, and
 // thread tid's range of piece `part`.
-__device__ __forceinline__ void thread_range(int i0, int wend, int part, int parts, int &lo, int &hi) {
+__device__ __forceinline__ void thread_range(int i0, int wend, int part, int parts, int &lo, int &hi, int least = 4) {
   const int base = i0 & ~3;
-  const int per = (((wend - base + parts - 1) / parts + ES_T - 1) / ES_T + 3) & ~3;
+  const int per = max(least, (((wend - base + parts - 1) / parts + ES_T - 1) / ES_T + 3) & ~3);
   const long long a = (long long)base + ((long long)part * ES_T + threadIdx.x) * per;
   lo = (int)max((long long)i0, min(a, (long long)wend));
   hi = (int)min(a + per, (long long)wend);
@@ -254,26 +290,42 @@ __device__ void es_solo(const float *__restrict__ v, int n, int stop, bool align
     const Binade b = binade_of(s);
     const int p0 = b.S & 1;
     const int wend = (int)min((long long)n, (long long)i + max(i, ES_WMIN));
+    // (a short window goes to the first warps alone, eight elements a thread
+    // at least, and one warp looks for the crossing: 32 warps that all scan
+    // spent most of a step's 4,400 cycles on issuing the scans)
     int lo, hi;
-    thread_range(i, wend, 0, 1, lo, hi);
-    const Xf tx = xf_range(v, lo, hi, aligned, b);
-    const Xf incl = xf_scan(tx, lane);
+    thread_range(i, wend, 0, 1, lo, hi, 8);
+    Xf tx = xf_identity(), incl = tx;
+    if (__any_sync(0xffffffffu, lo < hi)) {
+      tx = xf_range(v, lo, hi, aligned, b);
+      incl = xf_scan(tx, lane);
+    }
     if (lane == 31) sh.w[warp] = incl;
     __syncthreads();
-    // every warp: the state before each warp, and the first that crosses
-    const Xf wx = sh.w[lane];
-    const Xf wi = xf_scan(wx, lane), we = xf_exclusive(wi, lane);
-    const int Re = p0 ? we.R1 : we.R0, qe = (we.q >> p0) & 1u;
-    const int Mw = qe ? wx.M1 : wx.M0;
-    const unsigned hit = __ballot_sync(0xffffffffu, Mw >= 0 && b.S + Re + Mw >= TOP);
-    if (hit == 0) {
-      const int R = p0 ? wi.R1 : wi.R0;
-      s = binade_value(b, b.S + __shfl_sync(0xffffffffu, R, 31));
-      i = wend;
-    } else {
-      const int cw = __ffs(hit) - 1;
-      const int Rw = __shfl_sync(0xffffffffu, Re, cw), qw = __shfl_sync(0xffffffffu, qe, cw);
+    if (warp == 0) {
+      // the state before each warp, and the first that crosses
+      const Xf wx = sh.w[lane];
+      const Xf wi = xf_scan(wx, lane), we = xf_exclusive(wi, lane);
+      const int Re = p0 ? we.R1 : we.R0, qe = (we.q >> p0) & 1u;
+      const int Mw = qe ? wx.M1 : wx.M0;
+      const unsigned hit = __ballot_sync(0xffffffffu, Mw >= 0 && b.S + Re + Mw >= TOP);
+      if (hit == 0) {
+        if (lane == 31) {
+          sh.s = binade_value(b, b.S + (p0 ? wi.R1 : wi.R0));
+          sh.i = wend;
+          sh.cx = -1;
+        }
+      } else if (lane == __ffs(hit) - 1) {
+        sh.cx = lane;
+        sh.R = Re;
+        sh.q = qe;
+      }
+    }
+    __syncthreads();
+    const int cw = sh.cx;
+    if (cw >= 0) {
       if (warp == cw) {
+        const int Rw = sh.R, qw = sh.q;
         const Xf ex = xf_exclusive(incl, lane);
         const int R = Rw + (qw ? ex.R1 : ex.R0), q = (ex.q >> qw) & 1u;
         const int M = q ? tx.M1 : tx.M0;
@@ -287,9 +339,9 @@ __device__ void es_solo(const float *__restrict__ v, int n, int stop, bool align
         }
       }
       __syncthreads();
-      s = sh.s;
-      i = sh.i;
     }
+    s = sh.s;
+    i = sh.i;
     __syncthreads();  // sh is free
   }
   __syncthreads();
