@@ -303,7 +303,7 @@ int32_t rpba_precond_loss_grad(const rpba_precond_set *set, const float *weights
  * d_v and d_out are device pointers on the calling thread's current device;
  * the work is enqueued on `stream` (a cudaStream_t; NULL = legacy default
  * stream) and the call returns without waiting for it.  Scratch lives in one
- * static device array of the library (about 20 KB, held by every GPU that
+ * static device array of the library (about 16 KB, held by every GPU that
  * loads the library until the process exits), which caps n at 4,194,304 on
  * every device: larger n returns RPBA_ERR_TOO_LARGE.  The first call on a
  * device (and the first after cudaDeviceReset or with another context

@@ -4,7 +4,7 @@
 // drop-in form) and the mixed-precision form: FP32 records and blocks with
 // FP32 arithmetic and compensated (Kahan) per-camera and per-pair sums, the
 // point blocks factored in FP64 and the records whitened by the factor
-// (k_point32).  Residuals and the cost stay FP64.
+// (k_point<float>).  Residuals and the cost stay FP64.
 #include <cub/cub.cuh>
 
 #include "internal.h"

@@ -4,9 +4,9 @@
 // the squared step increment drops by 1e5 or after msize iterations,
 // beta = r1^T (h1 - h) / r^T h clamped at 0.
 //
-// One cooperative launch runs the whole solve.  FP64 form (k_pcg): rows
-// (cameras) are owned by warps; a 9x9 block product uses 27 lanes (3 blocks
-// at a time).  The FP32 form (k_pcg32) is described before it.  Dot
+// One cooperative launch runs the whole solve.  The FP64 form is k_pcg, the
+// FP32 form k_pcg32; each has a variant for systems that stay in shared memory
+// (described before them).  Dot
 // products are reduced per CTA and then, after a grid barrier, by every CTA
 // in the same fixed order, so all CTAs take identical decisions.  The grid
 // barrier's wait is bounded: after 2 s it sets an error bit and returns.
@@ -21,8 +21,7 @@ namespace rpba {
 
 namespace {
 
-// Threads per CTA of the FP64 form's persistent kernel: 32 warps, two work
-// items in flight each through shared memory.  (The FP32 form is k_pcg32.)
+// Threads per CTA of the FP64 form's persistent kernel.
 template <class BT>
 constexpr int pcg_threads() {
   return 1024;
