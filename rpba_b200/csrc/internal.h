@@ -125,6 +125,10 @@ void launch_final_cost(const DevLSA &L, double *partials, int nparts, cudaStream
 // GCP mode: the prior cost term of every point at the state XM (0 for a
 // point without a prior), out[0 .. npts)
 void launch_gcp_cost(const DevLSA &L, const double *XM, float *out, cudaStream_t s);
+// *bad (zero before) becomes 1 if a track entry names an image outside
+// [0, n) or a slot outside that image's observations
+void launch_check_tracks(int nt, int n, const int *pt_img, const int *pt_slot, const int *img_off, int *bad,
+                         cudaStream_t s);
 void launch_exteval(int n_points, const int *pt_off, const int *pt_img, const int *pt_slot,
                     const int *img_off, const float *pmat, const float *K, const float *dist,
                     const float *XX, const float *xg, const float *wx, const float *wy,

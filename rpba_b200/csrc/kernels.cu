@@ -1161,6 +1161,14 @@ __global__ void k_final_cost(DevLSA L, double *partials) {
 // ------------------------------------------------------------ Exteval
 // EvalLSA + CalcCorrPointMulti (rpbacore.cpp:778-837, 882-941): one thread
 // per point, float sums in the reference's order within the point.
+__global__ void k_check_tracks(int nt, int n, const int *__restrict__ pt_img, const int *__restrict__ pt_slot,
+                               const int *__restrict__ img_off, int *bad) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nt) return;
+  const int im = pt_img[t], sl = pt_slot[t];
+  if (im < 0 || im >= n || sl < 0 || sl >= img_off[im + 1] - img_off[im]) *bad = 1;
+}
+
 __global__ void k_exteval(int n_points, const int *__restrict__ pt_off, const int *__restrict__ pt_img,
                           const int *__restrict__ pt_slot, const int *__restrict__ img_off,
                           const float *__restrict__ pmat, const float *__restrict__ Kf,
@@ -1347,6 +1355,11 @@ void launch_final_cost(const DevLSA &L, double *partials, int nparts, cudaStream
 
 void launch_gcp_cost(const DevLSA &L, const double *XM, float *out, cudaStream_t s) {
   if (L.npts > 0) k_gcp_cost<<<nblk(L.npts, 256), 256, 0, s>>>(L, XM, out);
+}
+
+void launch_check_tracks(int nt, int n, const int *pt_img, const int *pt_slot, const int *img_off, int *bad,
+                         cudaStream_t s) {
+  if (nt > 0) k_check_tracks<<<nblk(nt, 256), 256, 0, s>>>(nt, n, pt_img, pt_slot, img_off, bad);
 }
 
 void launch_exteval(int n_points, const int *pt_off, const int *pt_img, const int *pt_slot, const int *img_off,

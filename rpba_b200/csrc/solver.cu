@@ -197,8 +197,13 @@ struct rpba_handle {
   std::vector<int32_t> img_off_in;
   rpba_block raw{};  // device copy of the caller's block (Exteval)
   bool raw_uploaded = false;
-  std::vector<float> h_pmat, h_K, h_dist, h_XX, h_xg, h_wx, h_wy, h_wxy;
-  std::vector<int32_t> h_img_off, h_pt_off, h_pt_img, h_pt_slot;
+  std::vector<float> h_pmat, h_K, h_dist, h_XX;
+  // an Exteval handle's block and results on the device
+  struct {
+    float *pmat, *K, *dist, *xg, *wx, *wy, *wxy, *term, *sum;
+    int *img_off, *pt_off, *pt_img, *pt_slot, *red, *bad;
+    double *resid;
+  } ext{};
 
   // GCP mode (the parallel RPBA's per-partition LSA): the scene's camera
   // count (unknowns of the additional parameters), the kept points with a
@@ -448,8 +453,7 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   if (n > 65535) return RPBA_ERR_UNSUPPORTED;
   // host copies of the caller's cameras and points (the output keeps the
   // input values of points the solve does not use); the observations and
-  // tracks only for an Exteval handle, whose rpba_exteval reads them (a
-  // solve handle takes them straight from the caller's arrays to the device)
+  // tracks go straight from the caller's arrays to the device
   H->h_pmat.assign(b->pmat, b->pmat + 12 * n);
   H->h_K.assign(b->K, b->K + 9 * n);
   H->h_dist.assign(b->distpara, b->distpara + 2 * n);
@@ -457,14 +461,31 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   H->d_XXin = dalloc<float>(3 * (size_t)std::max(np, 1), own);
   if (np) RPBA_CUDA_CHECK(cudaMemcpyAsync(H->d_XXin, b->XX, sizeof(float) * 3 * np, cudaMemcpyHostToDevice, H->s));
   if (o->exteval) {
-    H->h_img_off.assign(b->img_obs_off, b->img_obs_off + n + 1);
-    H->h_xg.assign(b->xg, b->xg + 2 * H->n_slots);
-    H->h_wx.assign(b->wx, b->wx + H->n_slots);
-    H->h_wy.assign(b->wy, b->wy + H->n_slots);
-    H->h_wxy.assign(b->wxy, b->wxy + H->n_slots);
-    H->h_pt_off.assign(b->pt_obs_off, b->pt_obs_off + np + 1);
-    H->h_pt_img.assign(b->pt_obs_image, b->pt_obs_image + H->n_track_in);
-    H->h_pt_slot.assign(b->pt_obs_slot, b->pt_obs_slot + H->n_track_in);
+    auto &X = H->ext;
+    const size_t ns = H->n_slots, nt = H->n_track_in;
+    auto up = [&](auto *&d, const void *h, size_t count) {
+      using E = std::remove_reference_t<decltype(*d)>;
+      d = dalloc<E>(count, own);
+      if (count) RPBA_CUDA_CHECK(cudaMemcpyAsync(d, h, sizeof(E) * count, cudaMemcpyHostToDevice, H->s));
+    };
+    up(X.img_off, b->img_obs_off, (size_t)n + 1);
+    up(X.pt_img, b->pt_obs_image, nt);
+    up(X.pt_slot, b->pt_obs_slot, nt);
+    X.bad = dalloc<int>(1, own);
+    RPBA_CUDA_CHECK(cudaMemsetAsync(X.bad, 0, sizeof(int), H->s));
+    launch_check_tracks((int)nt, n, X.pt_img, X.pt_slot, X.img_off, X.bad, H->s);
+    up(X.pt_off, b->pt_obs_off, (size_t)np + 1);
+    up(X.pmat, b->pmat, 12 * (size_t)n);
+    up(X.K, b->K, 9 * (size_t)n);
+    up(X.dist, b->distpara, 2 * (size_t)n);
+    up(X.xg, b->xg, 2 * ns);
+    up(X.wx, b->wx, ns);
+    up(X.wy, b->wy, ns);
+    up(X.wxy, b->wxy, ns);
+    X.resid = dalloc<double>(2 * nt, own);
+    X.term = dalloc<float>(np, own);
+    X.sum = dalloc<float>(1, own);
+    X.red = dalloc<int>(np, own);
   }
   {
     H->ES.max_grid = exact_sum_max_grid(H->dev);
@@ -474,13 +495,10 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
     RPBA_CUDA_CHECK(cudaMemsetAsync(H->ES.err, 0, 4 * sizeof(int), H->s));
   }
   if (o->exteval) {
+    int bad = 0;
+    RPBA_CUDA_CHECK(cudaMemcpyAsync(&bad, H->ext.bad, sizeof(int), cudaMemcpyDeviceToHost, H->s));
     RPBA_CUDA_CHECK(cudaStreamSynchronize(H->s));
-    for (int i = 0; i < H->n_track_in; ++i) {
-      const int im = H->h_pt_img[i];
-      if (im < 0 || im >= n || H->h_pt_slot[i] < 0 || H->h_pt_slot[i] >= H->h_img_off[im + 1] - H->h_img_off[im])
-        return RPBA_ERR_ARG;
-    }
-    return RPBA_OK;
+    return bad ? RPBA_ERR_ARG : RPBA_OK;
   }
 
   // ihw2 / defdiff for iwidth = iheight = 1 (rpba.cpp:264-265, rpbacore.cpp:87-90, rbacore.cpp:48)
@@ -1570,40 +1588,17 @@ int32_t rpba_exteval(rpba_handle *H, double *resid, rpba_report *rep) {
     A *a = (A *)p;
     rpba_handle *H = a->H;
     RPBA_CUDA_CHECK(cudaSetDevice(H->dev));
-    auto &own = H->owned;
-    const int n = H->nimg, np = H->XXnr, ns = H->n_slots, nt = H->n_track_in;
-    float *pm = dalloc<float>(12 * (size_t)n, own), *K = dalloc<float>(9 * (size_t)n, own);
-    float *ds = dalloc<float>(2 * (size_t)n, own), *XX = dalloc<float>(3 * (size_t)std::max(np, 1), own);
-    float *xg = dalloc<float>(2 * (size_t)std::max(ns, 1), own), *wx = dalloc<float>(std::max(ns, 1), own);
-    float *wy = dalloc<float>(std::max(ns, 1), own), *wxy = dalloc<float>(std::max(ns, 1), own);
-    int *io = dalloc<int>(n + 1, own), *po = dalloc<int>(np + 1, own);
-    int *pi = dalloc<int>(std::max(nt, 1), own), *ps = dalloc<int>(std::max(nt, 1), own);
-    double *res = dalloc<double>(2 * (size_t)std::max(nt, 1), own);
-    float *term = dalloc<float>(std::max(np, 1), own), *sum = dalloc<float>(1, own);
-    int *red = dalloc<int>(std::max(np, 1), own);
-    auto up = [&](void *d, const void *h, size_t bytes) {
-      if (bytes) RPBA_CUDA_CHECK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, H->s));
-    };
-    up(pm, H->h_pmat.data(), sizeof(float) * 12 * n);
-    up(K, H->h_K.data(), sizeof(float) * 9 * n);
-    up(ds, H->h_dist.data(), sizeof(float) * 2 * n);
-    up(XX, H->h_XX.data(), sizeof(float) * 3 * np);
-    up(xg, H->h_xg.data(), sizeof(float) * 2 * ns);
-    up(wx, H->h_wx.data(), sizeof(float) * ns);
-    up(wy, H->h_wy.data(), sizeof(float) * ns);
-    up(wxy, H->h_wxy.data(), sizeof(float) * ns);
-    up(io, H->h_img_off.data(), sizeof(int) * (n + 1));
-    up(po, H->h_pt_off.data(), sizeof(int) * (np + 1));
-    up(pi, H->h_pt_img.data(), sizeof(int) * nt);
-    up(ps, H->h_pt_slot.data(), sizeof(int) * nt);
-    launch_exteval(np, po, pi, ps, io, pm, K, ds, XX, xg, wx, wy, wxy, res, term, red, H->s);
-    launch_exact_sum(term, np, sum, H->ES, H->s);
+    const auto &X = H->ext;
+    const int n = H->nimg, np = H->XXnr, nt = H->n_track_in;
+    launch_exteval(np, X.pt_off, X.pt_img, X.pt_slot, X.img_off, X.pmat, X.K, X.dist, H->d_XXin, X.xg, X.wx, X.wy, X.wxy,
+                   X.resid, X.term, X.red, H->s);
+    launch_exact_sum(X.term, np, X.sum, H->ES, H->s);
     std::vector<int> hred(np);
     float s = 0.f;
-    if (np) RPBA_CUDA_CHECK(cudaMemcpyAsync(hred.data(), red, sizeof(int) * np, cudaMemcpyDeviceToHost, H->s));
-    RPBA_CUDA_CHECK(cudaMemcpyAsync(&s, sum, sizeof(float), cudaMemcpyDeviceToHost, H->s));
+    if (np) RPBA_CUDA_CHECK(cudaMemcpyAsync(hred.data(), X.red, sizeof(int) * np, cudaMemcpyDeviceToHost, H->s));
+    RPBA_CUDA_CHECK(cudaMemcpyAsync(&s, X.sum, sizeof(float), cudaMemcpyDeviceToHost, H->s));
     if (a->resid && nt)
-      RPBA_CUDA_CHECK(cudaMemcpyAsync(a->resid, res, sizeof(double) * 2 * nt, cudaMemcpyDeviceToHost, H->s));
+      RPBA_CUDA_CHECK(cudaMemcpyAsync(a->resid, X.resid, sizeof(double) * 2 * nt, cudaMemcpyDeviceToHost, H->s));
     RPBA_CUDA_CHECK(cudaStreamSynchronize(H->s));
     long redundancy = 0, nrobs = 0;
     for (int i = 0; i < np; ++i) {

@@ -306,83 +306,106 @@ int32_t rpba::triangulate_impl(const rpba_block *b, const double *Pd, const floa
   const int nc = b->n_images, np = b->n_points;
   if (nc < 1 || np < 0) return RPBA_ERR_ARG;
   const size_t nslot = (size_t)b->img_obs_off[nc], ntr = (size_t)b->pt_obs_off[np];
-  for (size_t t = 0; t < ntr; ++t) {
-    const int im = b->pt_obs_image[t];
-    if (im < 0 || im >= nc || b->pt_obs_slot[t] < 0 || b->pt_obs_slot[t] >= b->img_obs_off[im + 1] - b->img_obs_off[im])
-      return RPBA_ERR_ARG;
-  }
   try {
     RPBA_CUDA_CHECK(cudaSetDevice(opt->device));
     cudaStream_t s;
     RPBA_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    std::vector<void *> mem;
-    struct Free {
-      std::vector<void *> &m;
+    struct Arena {
+      char *base = nullptr;
       cudaStream_t s;
-      ~Free() {
-        for (void *p : m) cudaFreeAsync(p, s);
+      ~Arena() {
+        if (base) cudaFreeAsync(base, s);
         cudaStreamSynchronize(s);
         cudaStreamDestroy(s);
       }
-    } fr{mem, s};
-    auto dev = [&](size_t bytes) {
-      void *p = nullptr;
-      RPBA_CUDA_CHECK(cudaMallocAsync(&p, bytes ? bytes : 16, s));
-      mem.push_back(p);
-      return p;
-    };
-    auto up = [&](const void *h, size_t bytes) {
-      void *d = dev(bytes);
-      if (bytes) RPBA_CUDA_CHECK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
-      return d;
-    };
-    TriIn I;
-    if (Pd) {
-      I.pmat = (const double *)up(Pd, sizeof(double) * 12 * nc);
-    } else {
-      std::vector<double> P(12 * (size_t)nc);
-      for (size_t i = 0; i < P.size(); ++i) P[i] = (double)b->pmat[i];
-      I.pmat = (const double *)up(P.data(), sizeof(double) * P.size());
-      RPBA_CUDA_CHECK(cudaStreamSynchronize(s));  // P is a local
+    } ar;
+    ar.s = s;
+    TriIn I{};
+    TriScratch S{};
+    TriOut O{};
+    int *bad_d = nullptr, bad = 0;
+    // one allocation for all arrays: the pool gives its memory back at the
+    // call's end, and the driver maps every allocation anew
+    std::vector<std::pair<void **, size_t>> req;
+    auto want = [&](auto *&p, size_t count) { req.push_back({(void **)&p, std::max<size_t>(sizeof(*p) * count, 16)}); };
+    want(I.img_off, (size_t)nc + 1);
+    want(I.pt_img, ntr);
+    want(I.pt_slot, ntr);
+    want(bad_d, 1);
+    want(I.pmat, 12 * (size_t)nc);
+    want(I.K, 9 * (size_t)nc);
+    want(I.dist, 2 * (size_t)nc);
+    want(I.XX, 3 * (size_t)np);
+    want(I.xg, 2 * nslot);
+    want(I.wx, nslot);
+    want(I.wy, nslot);
+    want(I.wxy, nslot);
+    want(I.pt_off, (size_t)np + 1);
+    if (sig0w) want(I.sig0w, nc);
+    want(S.wx, ntr);
+    want(S.wy, ntr);
+    want(S.wxy, ntr);
+    want(S.p1, ntr);
+    want(S.p2, ntr);
+    want(S.p3, ntr);
+    want(S.corr, 2 * ntr);
+    want(S.Bw, 6 * ntr);
+    want(S.del, ntr);
+    want(O.XX, 3 * (size_t)np);
+    want(O.keep, ntr);
+    want(O.conv, np);
+    want(O.sig0v, ntr);
+    want(O.s0, np);
+    want(O.red, np);
+    if (w3d) {
+      want(I.part, nc);
+      want(S.Bxy, 6 * ntr);
+      want(S.dpart, ntr);
+      want(S.wt, 6 * ntr);
+      want(O.w3d, 6 * (size_t)nparts * np);
     }
-    I.K = (const float *)up(b->K, sizeof(float) * 9 * nc);
-    I.dist = (const float *)up(b->distpara, sizeof(float) * 2 * nc);
-    I.XX = (const float *)up(b->XX, sizeof(float) * 3 * np);
-    I.xg = (const float *)up(b->xg, sizeof(float) * 2 * nslot);
-    I.wx = (const float *)up(b->wx, sizeof(float) * nslot);
-    I.wy = (const float *)up(b->wy, sizeof(float) * nslot);
-    I.wxy = (const float *)up(b->wxy, sizeof(float) * nslot);
-    I.sig0w = sig0w ? (const float *)up(sig0w, sizeof(float) * nc) : nullptr;
-    I.img_off = (const int *)up(b->img_obs_off, sizeof(int) * (nc + 1));
-    I.pt_off = (const int *)up(b->pt_obs_off, sizeof(int) * (np + 1));
-    I.pt_img = (const int *)up(b->pt_obs_image, sizeof(int) * ntr);
-    I.pt_slot = (const int *)up(b->pt_obs_slot, sizeof(int) * ntr);
+    auto up256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (auto &q : req) total += up256(q.second);
+    RPBA_CUDA_CHECK(cudaMallocAsync((void **)&ar.base, total, s));
+    total = 0;
+    for (auto &q : req) {
+      *q.first = ar.base + total;
+      total += up256(q.second);
+    }
+    auto up = [&](const void *d, const void *h, size_t bytes) {
+      if (bytes) RPBA_CUDA_CHECK(cudaMemcpyAsync((void *)d, h, bytes, cudaMemcpyHostToDevice, s));
+    };
+    // the tracks first: they are checked on the device (a host loop took as
+    // long as all the copies) while the rest follows
+    up(I.img_off, b->img_obs_off, sizeof(int) * (nc + 1));
+    up(I.pt_img, b->pt_obs_image, sizeof(int) * ntr);
+    up(I.pt_slot, b->pt_obs_slot, sizeof(int) * ntr);
+    RPBA_CUDA_CHECK(cudaMemsetAsync(bad_d, 0, sizeof(int), s));
+    launch_check_tracks((int)ntr, nc, I.pt_img, I.pt_slot, I.img_off, bad_d, s);
+    std::vector<double> P;
+    if (!Pd) {
+      P.assign(b->pmat, b->pmat + 12 * (size_t)nc);
+      Pd = P.data();
+    }
+    up(I.pmat, Pd, sizeof(double) * 12 * nc);
+    up(I.K, b->K, sizeof(float) * 9 * nc);
+    up(I.dist, b->distpara, sizeof(float) * 2 * nc);
+    up(I.XX, b->XX, sizeof(float) * 3 * np);
+    up(I.xg, b->xg, sizeof(float) * 2 * nslot);
+    up(I.wx, b->wx, sizeof(float) * nslot);
+    up(I.wy, b->wy, sizeof(float) * nslot);
+    up(I.wxy, b->wxy, sizeof(float) * nslot);
+    up(I.pt_off, b->pt_obs_off, sizeof(int) * (np + 1));
+    if (sig0w) up(I.sig0w, sig0w, sizeof(float) * nc);
+    if (w3d) up(I.part, part, sizeof(int) * nc);
+    RPBA_CUDA_CHECK(cudaMemcpyAsync(&bad, bad_d, sizeof(int), cudaMemcpyDeviceToHost, s));
+    RPBA_CUDA_CHECK(cudaStreamSynchronize(s));
+    if (bad) return RPBA_ERR_ARG;
     I.np = np;
     I.robustmode = opt->robustmode;
     I.weight_only = opt->weight_only != 0;
-    I.part = w3d ? (const int *)up(part, sizeof(int) * nc) : nullptr;
     I.nparts = w3d ? nparts : 1;
-    TriScratch S;
-    S.wx = (float *)dev(sizeof(float) * ntr);
-    S.wy = (float *)dev(sizeof(float) * ntr);
-    S.wxy = (float *)dev(sizeof(float) * ntr);
-    S.p1 = (float *)dev(sizeof(float) * ntr);
-    S.p2 = (float *)dev(sizeof(float) * ntr);
-    S.p3 = (float *)dev(sizeof(float) * ntr);
-    S.corr = (double *)dev(sizeof(double) * 2 * ntr);
-    S.Bw = (double *)dev(sizeof(double) * 6 * ntr);
-    S.del = (uint8_t *)dev(ntr);
-    S.Bxy = w3d ? (double *)dev(sizeof(double) * 6 * ntr) : nullptr;
-    S.dpart = w3d ? (int *)dev(sizeof(int) * ntr) : nullptr;
-    S.wt = w3d ? (float *)dev(sizeof(float) * 6 * ntr) : nullptr;
-    TriOut O;
-    O.XX = (double *)dev(sizeof(double) * 3 * np);
-    O.keep = (uint8_t *)dev(ntr);
-    O.conv = (uint8_t *)dev(np);
-    O.sig0v = (float *)dev(sizeof(float) * ntr);
-    O.s0 = (double *)dev(sizeof(double) * np);
-    O.red = (int *)dev(sizeof(int) * np);
-    O.w3d = w3d ? (float *)dev(sizeof(float) * 6 * (size_t)nparts * np) : nullptr;
     if (np > 0) k_triangulate<<<(np + 127) / 128, 128, 0, s>>>(I, S, O);
     RPBA_CUDA_CHECK(cudaGetLastError());
     std::vector<double> s0(np);
