@@ -99,12 +99,6 @@ constexpr int BS64 = 81, BS32 = 81;
 __device__ __forceinline__ double blk_at(const DevLSA &L, size_t b, int e) {
   return L.blocks32 ? (double)L.blocks32[b * BS32 + e] : L.blocks[b * BS64 + e];
 }
-__device__ __forceinline__ void load_block(const DevLSA &L, size_t b, double out[81]) {
-  if (L.blocks32)
-    for (int e = 0; e < 81; ++e) out[e] = (double)L.blocks32[b * BS32 + e];
-  else
-    for (int e = 0; e < 81; ++e) out[e] = L.blocks[b * BS64 + e];
-}
 
 // ---- launchers (kernels.cu)
 void launch_cost(const DevLSA &L, const double *XM, bool srmv, cudaStream_t s);
