@@ -493,6 +493,13 @@ int32_t rpba_spd_inverse(const double *A, int32_t n, double *Ainv, int32_t devic
  * reference has no device waits and no counterpart; its error exits are
  * the BA-Error lines of rbacore.cpp:415-424, 470-476 and 541-546. */
 int32_t rpba_debug_barrier_timeout(rpba_handle *h, int32_t extra_ctas, int64_t timeout_ns);
+/* Test hook of single bounded waits: `which` of them runs out after
+ * timeout_ns (1 ms .. 2 s) and its kernel ends with RPBA_ERR_DEVICE_TIMEOUT;
+ * the handle stays usable.  (0, 0) restores normal operation.
+ *   1  the persistent PCG's wait for its bulk copies: the first CTA's stages
+ *      expect 16 bytes more than are copied
+ * No counterpart in the reference. */
+int32_t rpba_debug_wait_fault(rpba_handle *h, int32_t which, int64_t timeout_ns);
 /* Releases a handle and its device memory (`delete LSA1`,
  * rpbacore.cpp:525). */
 void rpba_destroy(rpba_handle *h);

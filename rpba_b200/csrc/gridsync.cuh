@@ -35,7 +35,10 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
 // bit 2 of *err; once *err is set every waiting CTA gives up, sync() returns
 // false in all its threads and the caller leaves the kernel (the first
 // barrier always looks at *err, later ones after a few polls without
-// success; a poll is an L2 round trip).
+// success; a poll is an L2 round trip).  A thread whose own work failed (it
+// has set a bit of *err) passes bad != 0: its CTA arrives, so that nobody waits
+// for it, and leaves, and the others leave at the next barrier at the latest,
+// which this CTA never reaches.
 // Measured (1,024 threads, 148 CTAs, each thread writing between barriers):
 // 2,800 cycles with the release and acquire on the two accesses themselves,
 // 3,460 with fences around them, 1,870 without either; arriving with a
@@ -60,15 +63,14 @@ struct GridBarrier {
     if (threadIdx.x == 0) red_release_gpu(cnt, 1u);
   }
 
-  __device__ __forceinline__ bool sync() {
+  __device__ __forceinline__ bool sync(int bad = 0) {
     __syncthreads();
-    return sync_after_block();
+    return sync_after_block(bad);
   }
 
   // sync() where a block barrier has just ordered the other threads' writes
   // before thread 0.
-  __device__ __forceinline__ bool sync_after_block() {
-    int bad = 0;
+  __device__ __forceinline__ bool sync_after_block(int bad = 0) {
     if (threadIdx.x == 0) {
       const bool look = target == 0;
       target += nblocks;
@@ -76,7 +78,7 @@ struct GridBarrier {
       unsigned long long t0 = 0;
       for (unsigned n = 1;; ++n) {
         if ((int)(ld_acquire_gpu(cnt) - target) >= 0) {
-          if (look) bad = ld_relaxed_gpu((const unsigned *)err) != 0;
+          if (look && ld_relaxed_gpu((const unsigned *)err) != 0) bad = 1;
           break;
         }
         if ((n & 7u) == 0 && ld_relaxed_gpu((const unsigned *)err) != 0) {

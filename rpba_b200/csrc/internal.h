@@ -77,6 +77,7 @@ struct DevLSA {
   // most bar_timeout_ns (0: the default limit).  Both 0 in normal use.
   unsigned bar_extra = 0;
   unsigned long long bar_timeout_ns = 0;
+  int wait_fault = 0;  // the wait that rpba_debug_wait_fault lets run out (0: none)
   // GCP mode of the parallel RPBA's per-partition LSA (ao = 1): every
   // camera free (no scale camera, camera 0 with a full block), and the
   // points shared with other partitions held by 3-D priors.  Per point

@@ -64,6 +64,7 @@ struct PcgArgs {
   // (bar_extra 0 and the default limit outside the timeout test hook)
   unsigned bar_extra;
   unsigned long long bar_ns;
+  unsigned tx_extra;
   int row0, row1, nitems, msize;
   int stream_once;  // FP64 symmetric form: the blocks exceed L2
   int mode;     // 0: reference stop rule; 1: relative preconditioned residual
@@ -82,7 +83,8 @@ struct PcgArgs {
 // after it.  The order of the additions is fixed: lanes of a warp
 // (butterfly), warps (butterfly over the W warps' sums), CTAs (lane l takes
 // l, l + 32, ...; butterfly), so every CTA gets the same values.  Bounded like
-// GridBarrier's wait: false in every thread when it ran out.  (Every CTA
+// GridBarrier's wait, and `bad` as there: false in every thread when it ran
+// out or a thread of the CTA passed bad.  (Every CTA
 // polling the others' tagged sums themselves instead saves the read, but 148
 // CTAs polling 148 slots took 14,000 cycles where this takes 5,000.)
 constexpr int XMAXG = 256;  // CTAs at most
@@ -92,7 +94,8 @@ struct Exchange {
   double cta[XMAXG * N];
 };
 template <int N, int W>
-__device__ __forceinline__ bool exchange_sum(GridBarrier &bar, double *red, double (&v)[N], Exchange<N, W> &X) {
+__device__ __forceinline__ bool exchange_sum(GridBarrier &bar, double *red, double (&v)[N], Exchange<N, W> &X,
+                                             int bad = 0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
 #pragma unroll
   for (int j = 0; j < N; ++j)
@@ -113,7 +116,7 @@ __device__ __forceinline__ bool exchange_sum(GridBarrier &bar, double *red, doub
   }
   // (thread 0 wrote the CTA's sums; every other write of the CTA came before
   // the block barrier above)
-  if (!bar.sync_after_block()) return false;
+  if (!bar.sync_after_block(bad)) return false;
   if (threadIdx.x < G)
 #pragma unroll
     for (int j = 0; j < N; ++j) X.cta[j * XMAXG + threadIdx.x] = __ldcg(red + j * XMAXG + threadIdx.x);
@@ -170,16 +173,21 @@ __device__ __forceinline__ void bulk_load_hint(void *dst, const void *src, unsig
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-// Bounded wait on the stage's mbarrier (the copies of this CTA's own
-// memory end in microseconds; the limit only keeps a fault from hanging).
+// Bounded wait of a whole warp on the stage's mbarrier (the copies of this
+// CTA's own memory end in microseconds; the limit only keeps a fault from
+// hanging): one result for all lanes.
 __device__ __forceinline__ bool stage_wait(const PcgArgs &A, unsigned long long *bar, unsigned parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
-  while (!mbar_try_wait(bar, parity)) {
-    if (gtimer() - t0 > A.bar_ns) return false;
+  bool ok = mbar_try_wait(bar, parity);
+  if (!ok) {
+    const unsigned long long t0 = gtimer();
+    while (!(ok = mbar_try_wait(bar, parity)))
+      if (gtimer() - t0 > A.bar_ns) break;
   }
-  return true;
+  return __all_sync(0xffffffffu, ok);
 }
+// bytes that no copy brings, added to what the stages of CTA 0 expect (0
+// outside the test hook)
+__device__ __forceinline__ unsigned tx_extra(const PcgArgs &A) { return blockIdx.x == 0 ? A.tx_extra : 0u; }
 
 // Phase 1 of the FP64 form: q-partials p = sum of B d^k over the (at most
 // three) entries of every work item, and d^T A d.  A warp's items (gwarp,
@@ -251,7 +259,7 @@ __device__ __forceinline__ void group64_issue(const PcgArgs &A, int g, unsigned 
   const Grp64 q = group64(A, g);
   const unsigned long long src = (unsigned long long)A.blocks + (unsigned long long)q.start * 648u;
   const unsigned mis = (unsigned)(src & 15ull), nb = (mis + (unsigned)q.n * 648u + 15u) & ~15u;
-  mbar_expect_tx(mbar, nb + (unsigned)q.n * 16u);
+  mbar_expect_tx(mbar, nb + (unsigned)q.n * 16u + tx_extra(A));
   bulk_load_hint(stg, (const void *)(src - mis), nb, mbar, policy);
   bulk_load(stg + P1S_BLK, A.bidx + q.start, (unsigned)q.n * 16u, mbar);
 }
@@ -330,7 +338,10 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
   const bool stream = SYM && warp < 2 * P1S_N && gs < ng;
   const bool keep = ng <= gstep;  // every stage's only group stays
   unsigned parity = 0;
-  bool ok = true;  // false: a copy that never completed (bounded wait)
+  // false: a copy that never completed (bounded wait); nothing is taken from
+  // its stage, no other copy is issued to it, and the CTA leaves at the next
+  // grid barrier
+  bool ok = true;
   unsigned long long policy = 0;
   if constexpr (SYM) {
     if (stream) {
@@ -352,7 +363,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
       int np = 0;
       for (int t = 0; t < T; ++t) np += recs[4 * t].x >> 16;
-      mbar_expect_tx(mbar, (unsigned)np * P1_PIECE);
+      mbar_expect_tx(mbar, (unsigned)np * P1_PIECE + tx_extra(A));
       for (int t = 0; t < T; ++t)
         for (int g = 0; g < (recs[4 * t].x >> 16); ++g)
           bulk_load(stg + (3 * t + g) * P1_PIECE,
@@ -411,9 +422,9 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         const int4 *idx = (const int4 *)(stg + P1S_BLK);
         for (int g = gs; g < ng; g += gstep) {
           const Grp64 q = group64(A, g);
-          if (!keep || k == 0) ok = stage_wait(A, mbar, parity) && ok;
+          if (ok && (!keep || k == 0)) ok = stage_wait(A, mbar, parity);
           const unsigned mis = (unsigned)(((unsigned long long)A.blocks + (unsigned long long)q.start * 648u) & 15ull);
-          if (!(tr && q.diag)) {
+          if (ok && !(tr && q.diag)) {
             // the 32 vectors d^k = h + beta d^(k-1): all the copies of both
             // parts in flight, three vectors an instruction
 #pragma unroll
@@ -466,7 +477,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
             // first one for the next iteration
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
             parity ^= 1u;
-            if (lane == 0 && !tr) {
+            if (ok && lane == 0 && !tr) {
               fence_proxy_async();
               group64_issue(A, g + gstep < ng ? g + gstep : gs, stg, mbar, policy);
             }
@@ -483,7 +494,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       };
       load_recs(0);
       if (!ok && lane == 0) atomicOr(A.err, 2);
-      if (!bar.sync()) {
+      if (!bar.sync(!ok)) {
         drain();
         return;
       }
@@ -562,7 +573,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       xva = A.x[i];
       rva = A.r[i];
     }
-    if (!exchange_sum<1, PCG_W>(bar, A.red1, pdq, X1)) {
+    if (!exchange_sum<1, PCG_W>(bar, A.red1, pdq, X1, !ok)) {
       drain();
       return;
     }
@@ -831,7 +842,7 @@ __device__ __forceinline__ void group_issue(const PcgArgs &A, const Grp32 &q, un
   const unsigned mb = blk_misalign(blocks, q.start);
   const unsigned nb_bytes = (mb + (unsigned)q.n * 324u + 15u) & ~15u;
   const unsigned ni_bytes = (unsigned)q.n * 16u;
-  mbar_expect_tx(bar, nb_bytes + ni_bytes);
+  mbar_expect_tx(bar, nb_bytes + ni_bytes + tx_extra(A));
   bulk_load(stg, (const unsigned char *)(blocks + q.start * 81) - mb, nb_bytes, bar);
   bulk_load(stg + STG_BLK, A.bidx + q.start, ni_bytes, bar);
 }
@@ -1048,8 +1059,11 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       }
     // (the group's copy ends before the kernel can)
     const bool landed = !has_group || stage_wait(A, mbar, 0u);
-    if (!landed && lane == 0) atomicOr(A.err, 2);
-    if (!exchange_sum<3, P32_W>(bar, A.red2, v, X2)) return;
+    if (!landed) {
+      if (lane == 0) atomicOr(A.err, 2);
+      stage_wait(A, mbar, 0u);
+    }
+    if (!exchange_sum<3, P32_W>(bar, A.red2, v, X2, !landed)) return;
     erthk = v[0];
   }
   double meandrold = 1.e50, meandr0 = 1.e50, beta_prev = 0.;
@@ -1070,6 +1084,7 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
     if (!SMALL && blockIdx.x == 0 && threadIdx.x < 2) A.ctr[threadIdx.x] = 0u;
     if (!bar.sync()) return;
     // ---- phase 1
+    bool ok = true;
     if constexpr (SMALL) {
       if (has_group) {
         const Grp32 q = group_of(4ll * qc + qp, (int)gd, A.row0, A.row1, A.nboff);
@@ -1196,7 +1211,6 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
         racc += lane < 9 ? vl : 0.;
       };
       if (c < nch && lane == 0) group_issue(A, group_of(c * ch, (int)gd, A.row0, A.row1, A.nboff), stg, mbar);
-      bool ok = true;
       while (c < nch) {
       const long long g0 = c * ch, g1 = min(ng, g0 + ch);
       cur_row = -1;
@@ -1285,13 +1299,13 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       __syncwarp();
       if (!ok) {
         // a copy that never completed: record it, give it one more bounded
-        // wait, and leave after the grid barrier below has failed as well
+        // wait, and leave at the grid barrier below
         if (lane == 0) atomicOr(A.err, 2);
         stage_wait(A, mbar, parity);
       }
     }
 
-    if (!bar.sync()) return;
+    if (!bar.sync(!ok)) return;
     double edtAdk;
     {
       // d^T A d: every CTA sums the chunks' shares in the same fixed order
@@ -1759,6 +1773,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.iters = W.iters;
   A.bar_extra = L.bar_extra;
   A.bar_ns = L.bar_timeout_ns ? L.bar_timeout_ns : BAR_TIMEOUT_NS;
+  A.tx_extra = L.wait_fault == 1 ? 16u : 0u;
   A.row0 = L.begini;
   A.row1 = L.nimg;
   A.nitems = L.nitems;

@@ -2025,6 +2025,15 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *H, int32_t extra_ctas, int64_t t
   return RPBA_OK;
 }
 
+int32_t rpba_debug_wait_fault(rpba_handle *H, int32_t which, int64_t timeout_ns) {
+  if (!H || which < 0 || which > 1 || (which > 0 && (timeout_ns < 1000000 || timeout_ns > 2000000000ll)) ||
+      (which == 0 && timeout_ns != 0))
+    return RPBA_ERR_ARG;
+  H->L.wait_fault = which;
+  H->L.bar_timeout_ns = (unsigned long long)timeout_ns;
+  return RPBA_OK;
+}
+
 void rpba_destroy(rpba_handle *H) { delete H; }
 
 int32_t rpba_partition_count(int32_t n_images, int32_t threads, int32_t exteval) {

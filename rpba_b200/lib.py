@@ -41,7 +41,7 @@ EXPORTS = ("rpba_status_string", "rpba_version", "rpba_input_block", "rpba_block
            "rpba_set_preconditioner", "rpba_precond_loss_grad", "rpba_record_systems", "rpba_solve_batch",
            "rpba_triangulate", "rpba_triangulate_parts", "rpba_partition_images", "rpba_lsa_gcp_step",
            "rpba_calc_plsa_parallel", "rpba_calc_plsa_parallel_hosted", "rpba_calc_plsa_parallel_ranks",
-           "rpba_calc_plsa_parallel_ranks_hosted", "rpba_debug_barrier_timeout",
+           "rpba_calc_plsa_parallel_ranks_hosted", "rpba_debug_barrier_timeout", "rpba_debug_wait_fault",
            "rpba_partition_count", "rpba_spd_inverse",
            "rpba_destroy")
 
@@ -163,6 +163,8 @@ def load():
     L.rpba_partition_count.restype = C.c_int32
     L.rpba_debug_barrier_timeout.argtypes = [C.c_void_p, C.c_int32, C.c_int64]
     L.rpba_debug_barrier_timeout.restype = C.c_int32
+    L.rpba_debug_wait_fault.argtypes = [C.c_void_p, C.c_int32, C.c_int64]
+    L.rpba_debug_wait_fault.restype = C.c_int32
     L.rpba_destroy.argtypes = [C.c_void_p]
     _lib = L
     return L
@@ -559,6 +561,13 @@ class Solver:
         st = load().rpba_debug_barrier_timeout(self.h, int(extra_ctas), int(timeout_ns))
         if st != 0:
             raise RpbaError(st, "rpba_debug_barrier_timeout")
+
+    def debug_wait_fault(self, which: int, timeout_ns: int):
+        """Test hook: bounded wait number `which` (rpba_debug_wait_fault)
+        runs out after `timeout_ns`; (0, 0) restores it."""
+        st = load().rpba_debug_wait_fault(self.h, int(which), int(timeout_ns))
+        if st != 0:
+            raise RpbaError(st, "rpba_debug_wait_fault")
 
     def close(self):
         if self.h:
