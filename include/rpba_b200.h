@@ -498,6 +498,8 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *h, int32_t extra_ctas, int64_t t
  * the handle stays usable.  (0, 0) restores normal operation.
  *   1  the persistent PCG's wait for its bulk copies: the first CTA's stages
  *      expect 16 bytes more than are copied
+ *   2  the exact float sums' wait for the first CTA's state, which it
+ *      withholds (sums of more than 65,536 terms)
  * No counterpart in the reference. */
 int32_t rpba_debug_wait_fault(rpba_handle *h, int32_t which, int64_t timeout_ns);
 /* Releases a handle and its device memory (`delete LSA1`,

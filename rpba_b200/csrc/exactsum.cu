@@ -367,6 +367,8 @@ struct EsArgs {
   unsigned *bar;            // the barrier counter; zero before the launch, as pub
   unsigned long long *pub;  // [2] the published state: (s, tag), (i, tag), tag = step + 1
   int *err;
+  unsigned long long wait_ns;  // limit of every wait
+  bool hold;                   // the first state is not published (test hook)
 };
 
 // A state published by one CTA to all (each 8-byte word carries its tag).
@@ -396,7 +398,7 @@ __device__ __forceinline__ bool es_receive(const EsArgs &A, unsigned tag, EsShar
         const unsigned long long t = gtimer();
         if (t0 == 0)
           t0 = t;
-        else if (t - t0 > BAR_TIMEOUT_NS)
+        else if (t - t0 > A.wait_ns)
           atomicOr(A.err, 2);
       }
     }
@@ -413,12 +415,12 @@ __global__ void __launch_bounds__(ES_T) k_exact_sum(EsArgs A) {
   const int G = gridDim.x, c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = A.n;
   const bool aligned = ((unsigned long long)A.v & 15ull) == 0;
-  GridBarrier bar(A.bar, (unsigned)G, A.err);
+  GridBarrier bar(A.bar, (unsigned)G, A.err, A.wait_ns);
   __shared__ EsShared sh;
   unsigned tag = 1;
   if (c == 0) {
     es_solo(A.v, n, ES_SOLO, aligned, sh);
-    if (tid == 0) es_publish(A, sh.s, sh.i, tag);
+    if (tid == 0 && !A.hold) es_publish(A, sh.s, sh.i, tag);
   }
   if (!es_receive(A, tag, sh)) return;
   float s = sh.s;
@@ -559,6 +561,8 @@ void launch_exact_sum(const float *v, int n, float *out, const ExactSumWork &W, 
   A.bar = W.bar;
   A.pub = (unsigned long long *)(W.bar + 2);
   A.err = W.err;
+  A.wait_ns = W.wait_ns ? W.wait_ns : BAR_TIMEOUT_NS;
+  A.hold = W.hold;
   RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, ES_BAR_WORDS * sizeof(unsigned), s));
   void *args[] = {&A};
   RPBA_CUDA_CHECK(
@@ -680,6 +684,8 @@ extern "C" int32_t rpba_float_sequential_sum_noalloc(const float *d_v, int64_t n
   A.bar = (unsigned *)(base + NA_OFF_BAR);
   A.pub = (unsigned long long *)(A.bar + 2);
   A.err = (int *)(base + NA_OFF_ERR);
+  A.wait_ns = BAR_TIMEOUT_NS;
+  A.hold = false;
   // the array keeps the previous call's contents: the barrier counter, the
   // published state and the error word must start at zero; the rest is
   // written before it is read

@@ -141,8 +141,11 @@ constexpr int ES_BAR_WORDS = 6;  // barrier counter, padding, published state (t
 struct ExactSumWork {
   int *comp;      // [exact_sum_comp_ints()] the CTAs' composites
   unsigned *bar;  // [ES_BAR_WORDS], 8-byte aligned
-  int *err;
+  int *err;       // bit 2: a wait ran out, the sum is not valid
   int max_grid;
+  // test hook: the first state is withheld; limit of the waits (0: the default)
+  bool hold = false;
+  unsigned long long wait_ns = 0;
 };
 int exact_sum_max_grid(int device);
 size_t exact_sum_comp_ints();

@@ -1592,14 +1592,18 @@ int32_t rpba_exteval(rpba_handle *H, double *resid, rpba_report *rep) {
     const int n = H->nimg, np = H->XXnr, nt = H->n_track_in;
     launch_exteval(np, X.pt_off, X.pt_img, X.pt_slot, X.img_off, X.pmat, X.K, X.dist, H->d_XXin, X.xg, X.wx, X.wy, X.wxy,
                    X.resid, X.term, X.red, H->s);
+    RPBA_CUDA_CHECK(cudaMemsetAsync(H->ES.err, 0, sizeof(int), H->s));
     launch_exact_sum(X.term, np, X.sum, H->ES, H->s);
     std::vector<int> hred(np);
     float s = 0.f;
+    int err = 0;
     if (np) RPBA_CUDA_CHECK(cudaMemcpyAsync(hred.data(), X.red, sizeof(int) * np, cudaMemcpyDeviceToHost, H->s));
     RPBA_CUDA_CHECK(cudaMemcpyAsync(&s, X.sum, sizeof(float), cudaMemcpyDeviceToHost, H->s));
+    RPBA_CUDA_CHECK(cudaMemcpyAsync(&err, H->ES.err, sizeof(int), cudaMemcpyDeviceToHost, H->s));
     if (a->resid && nt)
       RPBA_CUDA_CHECK(cudaMemcpyAsync(a->resid, X.resid, sizeof(double) * 2 * nt, cudaMemcpyDeviceToHost, H->s));
     RPBA_CUDA_CHECK(cudaStreamSynchronize(H->s));
+    if (err) return (int)RPBA_ERR_DEVICE_TIMEOUT;
     long redundancy = 0, nrobs = 0;
     for (int i = 0; i < np; ++i) {
       redundancy += hred[i];
@@ -2026,11 +2030,12 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *H, int32_t extra_ctas, int64_t t
 }
 
 int32_t rpba_debug_wait_fault(rpba_handle *H, int32_t which, int64_t timeout_ns) {
-  if (!H || which < 0 || which > 1 || (which > 0 && (timeout_ns < 1000000 || timeout_ns > 2000000000ll)) ||
+  if (!H || which < 0 || which > 2 || (which > 0 && (timeout_ns < 1000000 || timeout_ns > 2000000000ll)) ||
       (which == 0 && timeout_ns != 0))
     return RPBA_ERR_ARG;
   H->L.wait_fault = which;
-  H->L.bar_timeout_ns = (unsigned long long)timeout_ns;
+  H->L.bar_timeout_ns = H->ES.wait_ns = (unsigned long long)timeout_ns;
+  H->ES.hold = which == 2;
   return RPBA_OK;
 }
 

@@ -53,3 +53,34 @@ def test_copy_that_never_completes(scene, precision):
             st_f, _ = F.solve()
             assert st == st_f == 0
             assert _same(S.state(), F.state())
+
+
+def _arc_large():
+    """More than 65,536 points and observations: the sums run on every SM."""
+    from rpba_b200 import scenes
+    return scenes.to_block(scenes.arc_scene(seed=5, n_cams=20, n_pts=66_000))
+
+
+def test_exteval_sum_that_never_comes():
+    import rpba_b200 as rb
+    blk = _arc_large()
+    assert blk.n_points > 65536
+    with rb.Solver(blk, exteval=True) as S, rb.Solver(blk, exteval=True) as F:
+        for _ in range(2):
+            _runs_out(S, 2, S.exteval)
+            res, rep = S.exteval()
+            res_f, rep_f = F.exteval()
+            assert np.array_equal(res, res_f, equal_nan=True)
+            for key in ("exteval_sigma0", "exteval_nrobs", "exteval_redundancy"):
+                assert rep[key] == rep_f[key], key
+
+
+def test_solve_sum_that_never_comes():
+    import rpba_b200 as rb
+    blk = _arc_large()
+    with rb.Solver(blk) as S, rb.Solver(blk) as F:
+        _runs_out(S, 2, S.solve)
+        st, _ = S.solve()
+        st_f, _ = F.solve()
+        assert st == st_f == 0
+        assert _same(S.state(), F.state())
