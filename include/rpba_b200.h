@@ -500,6 +500,8 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *h, int32_t extra_ctas, int64_t t
  *      expect 16 bytes more than are copied
  *   2  the exact float sums' wait for the first CTA's state, which it
  *      withholds (sums of more than 65,536 terms)
+ *   3  the direct solve's wait for the first tile row's entries
+ *   4  the tiled Cholesky's grid barrier: one CTA more than the launch has
  * No counterpart in the reference. */
 int32_t rpba_debug_wait_fault(rpba_handle *h, int32_t which, int64_t timeout_ns);
 /* Releases a handle and its device memory (`delete LSA1`,

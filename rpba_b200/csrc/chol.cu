@@ -56,6 +56,7 @@ struct Tiles {
   int want_inverse;
   unsigned *bar;
   int *err;
+  unsigned bar_extra;  // arrivals that never come (test hook)
   unsigned long long bar_ns;
 };
 
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(CTH, 1) k_chol_tiles(Tiles T) {
   extern __shared__ __align__(16) double csm[];
   double *sA = csm, *sB = csm + CT * CLD, *sP = csm + 2 * CT * CLD;
   const int G = gridDim.x;
-  GridBarrier bar(T.bar, (unsigned)G, T.err, T.bar_ns);
+  GridBarrier bar(T.bar, (unsigned)G + T.bar_extra, T.err, T.bar_ns);
   GridBarrier sub(T.bar + 1, (unsigned)G, T.err, T.bar_ns);
   const bool lead = blockIdx.x == 0, solo = G == 1;
   const int me = solo ? 0 : (int)blockIdx.x - 1, others = solo ? 1 : G - 1;
@@ -533,9 +534,10 @@ int chol_grid() {
 }  // namespace
 
 // Factor the envelope tiles in place (L over A) and write the inverses of
-// the diagonal tiles; one cooperative launch.
+// the diagonal tiles; one cooperative launch.  bar_extra, bar_ns: test hook
+// (0, 0: none, the default limit).
 void tile_cholesky(double *tiles, const long long *toff, const int *fcol, const int *hrow, double *Linv, int nt,
-                   unsigned *bar, int *err, cudaStream_t s) {
+                   unsigned *bar, int *err, cudaStream_t s, unsigned bar_extra, unsigned long long bar_ns) {
   if (nt <= 0) return;
   Tiles T;
   T.L = tiles;
@@ -549,7 +551,8 @@ void tile_cholesky(double *tiles, const long long *toff, const int *fcol, const 
   T.want_inverse = 0;
   T.bar = bar;
   T.err = err;
-  T.bar_ns = BAR_TIMEOUT_NS;
+  T.bar_extra = bar_extra;
+  T.bar_ns = bar_ns ? bar_ns : BAR_TIMEOUT_NS;
   const int g = std::max(1, chol_grid());
   RPBA_CUDA_CHECK(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));
   void *args[] = {&T};
@@ -590,6 +593,7 @@ void spd_inverse_scaled(const double *A, const double *dsc, double eps, int n, d
   T.want_inverse = 1;
   T.bar = bar;
   T.err = err;
+  T.bar_extra = 0;
   T.bar_ns = BAR_TIMEOUT_NS;
   const int g = (int)std::max<long long>(1, std::min<long long>(chol_grid(), ntile));
   RPBA_CUDA_CHECK(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));

@@ -99,6 +99,7 @@ struct SolveArgs {
   unsigned *bar;
   int *err;
   unsigned long long bar_ns;
+  bool hold;  // tile row 0 is not published (test hook)
 };
 
 // A finished entry travels as two 8-byte words, each half of its bits and a
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(ST) k_env_solve(SolveArgs A) {
     __syncthreads();
     if (t < T) {
       const double v = (sp[t] + sp[t + 64]) + (sp[t + 128] + sp[t + 192]);
-      pub_store(fwd + (size_t)J * T + t, v);
+      if (J > 0 || !A.hold) pub_store(fwd + (size_t)J * T + t, v);
       A.y[(size_t)J * T + t] = v;
     }
   }
@@ -430,7 +431,8 @@ void direct_factor(const DevLSA &L, const DirectWork &W, cudaStream_t s) {
   if (nd > 0) k_env_fill_diag<<<(int)((nd + 255) / 256), 256, 0, s>>>(L, W.pos, W.tiles, W.toff, W.fcol);
   const long long no = (long long)L.nboff * 81;
   if (no > 0) k_env_fill_off<<<(int)((no + 255) / 256), 256, 0, s>>>(L, W.bkey, W.pos, W.tiles, W.toff, W.fcol);
-  tile_cholesky(W.tiles, W.toff, W.fcol, W.hrow, W.Linv, W.nt, W.bar, L.err, s);
+  tile_cholesky(W.tiles, W.toff, W.fcol, W.hrow, W.Linv, W.nt, W.bar, L.err, s,
+                L.wait_fault == 4 ? 1u : 0u, L.bar_timeout_ns);
 }
 
 // x = S^-1 b with the factor from direct_factor; b and x padded 9 per camera
@@ -451,7 +453,8 @@ void direct_resolve(const DevLSA &L, const DirectWork &W, const double *b, doubl
   A.nt = W.nt;
   A.bar = W.bar;
   A.err = L.err;
-  A.bar_ns = BAR_TIMEOUT_NS;
+  A.bar_ns = L.bar_timeout_ns ? L.bar_timeout_ns : BAR_TIMEOUT_NS;
+  A.hold = L.wait_fault == 3;
   const int g = std::max(1, std::min(solve_grid(), W.nt));
   RPBA_CUDA_CHECK(cudaMemsetAsync(W.bar, 0, 2 * sizeof(unsigned), s));
   RPBA_CUDA_CHECK(cudaMemsetAsync(W.pub, 0, 2 * (size_t)W.nt * T * sizeof(ulonglong2), s));

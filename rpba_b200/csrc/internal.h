@@ -182,7 +182,7 @@ void direct_resolve(const DevLSA &L, const DirectWork &W, const double *b, doubl
 // Tiled Cholesky of a lower envelope of 64 x 64 tiles in place, with the
 // inverses of the diagonal tiles (chol.cu; one cooperative launch).
 void tile_cholesky(double *tiles, const long long *toff, const int *fcol, const int *hrow, double *Linv, int nt,
-                   unsigned *bar, int *err, cudaStream_t s);
+                   unsigned *bar, int *err, cudaStream_t s, unsigned bar_extra = 0, unsigned long long bar_ns = 0);
 // A^-1 of (D A D + eps I), scaled back by D = diag(dsc), for a dense SPD
 // matrix (row major n x n, lower triangle used): tiled Cholesky and inverse
 // in one cooperative launch on the FP64 tensor cores (chol.cu).  work:

@@ -2030,7 +2030,7 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *H, int32_t extra_ctas, int64_t t
 }
 
 int32_t rpba_debug_wait_fault(rpba_handle *H, int32_t which, int64_t timeout_ns) {
-  if (!H || which < 0 || which > 2 || (which > 0 && (timeout_ns < 1000000 || timeout_ns > 2000000000ll)) ||
+  if (!H || which < 0 || which > 4 || (which > 0 && (timeout_ns < 1000000 || timeout_ns > 2000000000ll)) ||
       (which == 0 && timeout_ns != 0))
     return RPBA_ERR_ARG;
   H->L.wait_fault = which;

@@ -84,3 +84,16 @@ def test_solve_sum_that_never_comes():
         st_f, _ = F.solve()
         assert st == st_f == 0
         assert _same(S.state(), F.state())
+
+
+@pytest.mark.parametrize("which", [3, 4])
+def test_direct_solve_wait(which):
+    """The envelope solve's first row, and the factorisation's barrier."""
+    import rpba_b200 as rb
+    blk = _arc()
+    with rb.Solver(blk, solver=rb.SOLVER_DIRECT) as S, rb.Solver(blk, solver=rb.SOLVER_DIRECT) as F:
+        _runs_out(S, which, S.solve)
+        st, _ = S.solve()
+        st_f, _ = F.solve()
+        assert st == st_f == 0
+        assert _same(S.state(), F.state())
