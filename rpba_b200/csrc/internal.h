@@ -361,6 +361,10 @@ int build_pairs(DevLSA &L, StructWork &S, long long max_pairs, long long *npairs
                 cudaStream_t s);
 void build_bsr(DevLSA &L, StructWork &S, cudaStream_t s);
 cudaError_t cub_exclusive_sum_int(void *tmp, size_t &bytes, const int *in, int *out, int n, cudaStream_t s);
+// Whether every track entry of b names an image and a slot of it (host loop:
+// the calls check on the device, this decides the status of one that failed
+// before that check, so that a bad entry is RPBA_ERR_ARG on a full device too)
+bool tracks_in_range(const rpba_block *b);
 // CalcLSAXMulti for every point of b (triangulate.cu): the cameras Pd in
 // double precision (null: b->pmat), the other arguments as
 // rpba_triangulate_parts (part null: no weight blocks); s0_pt / red_pt

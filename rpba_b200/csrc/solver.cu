@@ -1303,6 +1303,7 @@ int guard(int (*fn)(void *), void *arg) {
     return fn(arg);
   } catch (const CudaError &e) {
     std::fprintf(stderr, "rpba_b200: CUDA error %s at %s\n", cudaGetErrorString(e.code), e.what);
+    cudaGetLastError();  // a failed allocation is not the next call's error
     return RPBA_ERR_CUDA;
   } catch (const std::bad_alloc &) {
     return RPBA_ERR_CUDA;
@@ -1349,12 +1350,13 @@ int32_t rpba_create(rpba_handle **h, const rpba_block *blk, const rpba_options *
     const rpba_block *b;
     const rpba_options *o;
   } a{H, blk, opt};
-  const int st = guard([](void *p) {
+  int st = guard([](void *p) {
     A *a = (A *)p;
     return create_impl(a->H, a->b, a->o);
   }, &a);
   if (st != RPBA_OK) {
     delete H;
+    if (st == RPBA_ERR_CUDA && opt->exteval && !tracks_in_range(blk)) st = RPBA_ERR_ARG;
     return st;
   }
   *h = H;

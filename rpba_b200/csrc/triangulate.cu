@@ -292,6 +292,16 @@ __global__ void k_triangulate(TriIn I, TriScratch S, TriOut O) {
 
 using namespace rpba;
 
+bool rpba::tracks_in_range(const rpba_block *b) {
+  const int nc = b->n_images;
+  for (int t = 0; t < b->pt_obs_off[b->n_points]; ++t) {
+    const int im = b->pt_obs_image[t];
+    if (im < 0 || im >= nc || b->pt_obs_slot[t] < 0 || b->pt_obs_slot[t] >= b->img_obs_off[im + 1] - b->img_obs_off[im])
+      return false;
+  }
+  return true;
+}
+
 // CalcLSAXMulti over all points of b with the cameras Pd (12 doubles per
 // image; null: b->pmat widened to double); s0_pt / red_pt (optional): every
 // point's contribution to sig0io and to the redundancy.
@@ -324,8 +334,9 @@ int32_t rpba::triangulate_impl(const rpba_block *b, const double *Pd, const floa
     TriScratch S{};
     TriOut O{};
     int *bad_d = nullptr, bad = 0;
-    // one allocation for all arrays: the pool gives its memory back at the
-    // call's end, and the driver maps every allocation anew
+    // one allocation for all arrays: while no handle has been made on the
+    // device, its pool gives the memory back at the call's end, and the driver
+    // maps every allocation anew
     std::vector<std::pair<void **, size_t>> req;
     auto want = [&](auto *&p, size_t count) { req.push_back({(void **)&p, std::max<size_t>(sizeof(*p) * count, 16)}); };
     want(I.img_off, (size_t)nc + 1);
@@ -433,7 +444,8 @@ int32_t rpba::triangulate_impl(const rpba_block *b, const double *Pd, const floa
     if (s0_pt) std::memcpy(s0_pt, s0.data(), sizeof(double) * np);
     if (red_pt) std::memcpy(red_pt, red.data(), sizeof(int32_t) * np);
   } catch (const CudaError &) {
-    return RPBA_ERR_CUDA;
+    cudaGetLastError();
+    return tracks_in_range(b) ? RPBA_ERR_CUDA : RPBA_ERR_ARG;
   }
   return RPBA_OK;
 }
