@@ -504,6 +504,12 @@ int32_t rpba_debug_barrier_timeout(rpba_handle *h, int32_t extra_ctas, int64_t t
  *   4  the tiled Cholesky's grid barrier: one CTA more than the launch has
  * No counterpart in the reference. */
 int32_t rpba_debug_wait_fault(rpba_handle *h, int32_t which, int64_t timeout_ns);
+/* Test hook of the persistent PCG's forms, from the handle's next solve on:
+ * 2 streams every block through shared memory, 3 (FP64 only) gathers the
+ * blocks from global memory, also where the system would stay resident;
+ * 0 (and 1) leave the choice to the library.  The form that ran is
+ * "_rcs"."pcg_form" of rpba_kernel_stats.  No counterpart in the reference. */
+int32_t rpba_debug_pcg_form(rpba_handle *h, int32_t form);
 /* Releases a handle and its device memory (`delete LSA1`,
  * rpbacore.cpp:525). */
 void rpba_destroy(rpba_handle *h);

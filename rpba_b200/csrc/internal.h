@@ -64,10 +64,14 @@ struct DevLSA {
   // FP32 form reads every off-diagonal block once, in storage order)
   int nitems;
   const int *row_item_off;  // [nimg + 1]
-  const int2 *item_rec;     // [nitems][4] FP64 form: (row | entries << 16, first entry), then the entries
+  // [nitems][item_words] FP64 form: (row | entries << 16, first entry); with
+  // four words, for the PCG's resident form, the entries behind it
+  const int2 *item_rec;
+  int item_words;
   float *tpart;             // [nboff * 16] FP32 form: transposed block products, column order
   // (row, column, ...) of every block in storage order: its transposed slot in
-  // the FP32 form, its normal and its transposed entry in the FP64 form
+  // the FP32 form, its normal and its transposed entry in the FP64 form (there
+  // for the PCG's streamed form only, build_block_index)
   const int4 *bidx;
   const int *firstN;        // [nimg + 1] first off-diagonal block of every row
   const int *firstT;        // [nimg + 1] first transposed slot of every row (blocks in its column)
@@ -288,7 +292,8 @@ struct PcgWork {
   double *rowc;   // [nimg * 12] with the coarse space: per row P_k^T r and its share of |dr|^2
   double *drs;  // [2 * nimg * 9] 1 / sqrt of the camera blocks' diagonal entries (learned features), the same as floats
   float *feat;  // [nimg * 20] the learned preconditioner's features per camera row
-  double *prod;   // FP64 form: [entries * 9] both products of every block, entry order
+  double *prod;   // FP64 streamed form: [entries * 9] both products of every block, entry order
+  int force_form = 0;  // test hook (rpba_debug_pcg_form)
   unsigned *bar;  // [pcg_bar_bytes] grid-barrier word and the exchanges' sums
   int *iters;
 };
@@ -301,24 +306,32 @@ struct PcgWork {
 // Jacobi part plus the coarse correction P A_c^-1 P^T.
 int pcg_prepare(const DevLSA &L, const PcgWork &W, int mode, const float *weights, const CoarseWork *coarse,
                 cudaStream_t s);
+// pcg_iterate returns the form it launched.
+enum PcgForm { PCG_RESIDENT = 1, PCG_STREAMED = 2, PCG_GATHERED = 3 };
 int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStream_t s, int mode, double tol,
                 const CoarseWork *coarse);
 int pcg_max_grid(int device);
+// most work items that the FP64 PCG's resident form holds
+int pcg_resident_items(int grid);
 size_t pcg_bar_bytes();
 
 // ---- structure (structure.cu)
 struct StructWork {
   void *cub_tmp;
   size_t cub_bytes;
+  // the pairs' keys and values, unsorted and sorted: one piece of pair_bytes
+  // bytes at pval, free between one build_pairs and the next (the FP64 PCG's
+  // streamed form keeps its block index and products there)
   unsigned *pkey, *pkey2;
   unsigned long long *pval, *pval2;
+  size_t pair_bytes;
   int *pcnt, *poff;
   int *ccnt;
   unsigned *bkey;
   int *bcnt, *boff;
   int *nrun;
   int *cntN, *cntT, *firstN, *firstT, *rowtmp;
-  int4 *bidx;  // (row, column, ...) of every block in storage order, see DevLSA
+  int4 *bidx;  // FP32 form: DevLSA's
   unsigned *tkey, *tkey2;
   int *tidx, *tidx2;
   int2 *contrib;
@@ -328,6 +341,7 @@ struct StructWork {
   unsigned *ckey, *ckey2;
   int *row_items, *row_item_off;
   int2 *item_rec;
+  int resident_items;  // systems of at most that many items get four-word records
 };
 size_t structure_cub_bytes(int nobs, long long npairs, int nimg);
 // PointXXvIn on the device (structure.cu): the caller's block in device
@@ -360,6 +374,8 @@ void build_camera_order(DevLSA &L, StructWork &S, cudaStream_t s);
 int build_pairs(DevLSA &L, StructWork &S, long long max_pairs, long long *npairs_out,
                 cudaStream_t s);
 void build_bsr(DevLSA &L, StructWork &S, cudaStream_t s);
+// fills bidx (see DevLSA) after build_bsr
+void build_block_index(DevLSA &L, StructWork &S, int4 *bidx, cudaStream_t s);
 cudaError_t cub_exclusive_sum_int(void *tmp, size_t &bytes, const int *in, int *out, int n, cudaStream_t s);
 // Whether every track entry of b names an image and a slot of it (host loop:
 // the calls check on the device, this decides the status of one that failed

@@ -35,8 +35,9 @@ constexpr int pcg_warps() {
 struct PcgArgs {
   const void *blocks;  // BT[(nimg + nboff) * 81]
   const int *row_item_off;
-  const int2 *item_rec;   // [nitems][4] (row | entries << 16, first entry), up to three entries
-  double *prod;           // FP64 symmetric form: the product of every entry, 9 values each, entry order
+  const int2 *item_rec;   // [nitems][4 or 1] (row | entries << 16, first entry), resident form: up to three entries
+  const int2 *ent;        // gathered form: the entries
+  double *prod;           // FP64 streamed form: the product of every entry, 9 values each, entry order
   float *tpart;           // FP32 form: transposed products of the off-diagonal blocks
   // (row, column) of every block in storage order, with its transposed slot
   // (FP32 form) or its two entries (FP64 form: normal, transposed); the
@@ -66,7 +67,7 @@ struct PcgArgs {
   unsigned long long bar_ns;
   unsigned tx_extra;
   int row0, row1, nitems, msize;
-  int stream_once;  // FP64 symmetric form: the blocks exceed L2
+  int stream_once;  // FP64 streamed form: the blocks exceed L2
   int mode;     // 0: reference stop rule; 1: relative preconditioned residual
   double tol2;  // mode 1: stop when r^T M^-1 r <= tol2 * (r0^T M^-1 r0)
   // two-level preconditioner (coarse.cu): rows are owned per aggregate
@@ -192,12 +193,12 @@ __device__ __forceinline__ unsigned tx_extra(const PcgArgs &A) { return blockIdx
 // Phase 1 of the FP64 form: q-partials p = sum of B d^k over the (at most
 // three) entries of every work item, and d^T A d.  A warp's items (gwarp,
 // gwarp + nwarps, ...) are the same in every iteration, and so are the
-// blocks.  Two forms with the same operations in the same order per entry
+// blocks.  Three forms with the same operations in the same order per entry
 // and per item:
-//  direct     at most P1_SLOTS items a warp: their blocks and records stay in
+//  resident   at most P1_SLOTS items a warp: their blocks and records stay in
 //             shared memory for the whole solve; a 9-lane group forms each
 //             entry's product and the warp the item's sum.
-//  symmetric  more: phase 1a reads every block once, in storage order, by
+//  streamed   more: phase 1a reads every block once, in storage order, by
 //             1-D TMA bulk copies of 32 blocks into P1S_N stages a CTA (a
 //             stage with one group keeps it for the whole solve); two warps
 //             a stage, a lane a block, form B d_col and B^T d_row and store
@@ -206,12 +207,15 @@ __device__ __forceinline__ unsigned tx_extra(const PcgArgs &A) { return blockIdx
 //             barrier; phase 1b sums every item's products.  Half the block
 //             traffic of reading each block from both sides, in copies of
 //             20 KB, for one more barrier.
+//  gathered   the resident form's sums with the blocks read from global
+//             memory in every iteration, from both sides: needs no memory for
+//             products, taken only where there is none.
 // The threads have 64 registers each and the stages leave L1 some 20 KB, so
 // spilled registers cost L2 trips: a spill of 50 to 100 bytes was worth 10 to
 // 30%.  Iteration, before (each block read from both sides, 8-byte copies two
 // items ahead, the records through two dependent loads) and now: 50 cameras
-// 14.0 -> 10.0 us (direct), 3,000 cameras and 27,000 blocks 24.0 -> 17.3 us,
-// 1,370 cameras and 371,000 blocks 137 -> 115 us (symmetric).
+// 14.0 -> 10.0 us (resident), 3,000 cameras and 27,000 blocks 24.0 -> 17.3 us,
+// 1,370 cameras and 371,000 blocks 137 -> 115 us (streamed).
 constexpr int P1_SLOTS = 3;
 constexpr unsigned P1_PIECE = 656;  // a block's 648 bytes from the 16-byte boundary at or below it
 constexpr unsigned P1_WARP_BYTES = P1_SLOTS * (3 * P1_PIECE + 32) + 648 + 8;  // blocks, records, C of a row, mbarrier
@@ -222,9 +226,10 @@ constexpr unsigned P1S_IDX = 32 * 16;                     // and their indices
 constexpr unsigned P1S_BUF = 32 * 9 * 8;                  // a warp's 32 h or d^(k-1), or products
 constexpr unsigned P1S_STAGE = P1S_BLK + P1S_IDX + 4 * P1S_BUF + 16;  // + the mbarrier
 static_assert(P1S_BLK % 16 == 0 && P1S_STAGE % 16 == 0, "16-byte aligned stage parts");
-template <bool SYM>
+template <int FORM>
 constexpr size_t pcg_smem_bytes() {
-  return SYM ? (size_t)P1S_N * P1S_STAGE : (size_t)pcg_warps<double>() * P1_WARP_BYTES;
+  return FORM == PCG_STREAMED ? (size_t)P1S_N * P1S_STAGE
+                              : (FORM == PCG_RESIDENT ? (size_t)pcg_warps<double>() * P1_WARP_BYTES : 0);
 }
 
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
@@ -298,7 +303,7 @@ __device__ __forceinline__ double row_q(const PcgArgs &A, int t0, int t1, int la
   return qg + qa + qb;
 }
 
-// Iteration k (two grid barriers, three in the symmetric form):
+// Iteration k (two grid barriers, three in the streamed form):
 //  phase 1  q-partials of A d^k per work item (<= 3 blocks of one row), with
 //           d^k = h^k + beta^(k-1) d^(k-1) formed on the fly; partial d^T q
 //  phase 2  per row: q = sum of its items' partials, x += alpha d,
@@ -309,9 +314,10 @@ __device__ __forceinline__ double row_q(const PcgArgs &A, int t0, int t1, int la
 //           (kept in hj), and the aggregate's restriction P^T r1 is formed
 //  phase 2b per aggregate: z = A_c^-1[aggregate rows] (P^T r1), then
 //           h1 = hj + P z and the two dot products
-template <bool CO, bool SYM>
+template <bool CO, int FORM>
 __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
   constexpr int PCG_T = pcg_threads<double>(), PCG_W = pcg_warps<double>();
+  constexpr bool RES = FORM == PCG_RESIDENT, SYM = FORM == PCG_STREAMED;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * PCG_W + warp, nwarps = gridDim.x * PCG_W;
   const int grp = lane / 9, rr = lane % 9, gbase = grp * 9;
@@ -326,8 +332,8 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
   // this warp's items
   const int T = gwarp < A.nitems ? (A.nitems - 1 - gwarp) / nwarps + 1 : 0;
-  // direct form: blocks, records, C of the warp's first row, mbarrier;
-  // symmetric form: a stream warp's stage and its groups gs, gs + gstep, ...
+  // resident form: blocks, records, C of the warp's first row, mbarrier;
+  // streamed form: a stream warp's stage and its groups gs, gs + gstep, ...
   unsigned char *stg = pcg_dyn + (SYM ? (size_t)(warp >> 1) * P1S_STAGE : (size_t)warp * P1_WARP_BYTES);
   int2 *recs = (int2 *)(stg + P1_SLOTS * 3 * P1_PIECE);
   double *Cs = (double *)(recs + 4 * P1_SLOTS);
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       }
     }
     __syncthreads();  // the mbarriers are initialised
-  } else {
+  } else if constexpr (RES) {
     if (lane < 4 * T) recs[lane] = __ldg(A.item_rec + 4 * ((size_t)gwarp + (size_t)(lane >> 2) * nwarps) + (lane & 3));
     __syncwarp();
     if (lane == 0 && T > 0) {
@@ -376,13 +382,13 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
   // the copies in flight end before the CTA does
   bool landed = false;
   auto drain = [&]() {
-    if (SYM ? stream : (T > 0 && !landed)) stage_wait(A, mbar, parity);
+    if (SYM ? stream : (RES && T > 0 && !landed)) stage_wait(A, mbar, parity);
   };
   // the warp's first row of phase 2: its items and preconditioner block
   const int rowa = A.row0 + gwarp;
   const bool has_row = !CO && rowa < A.row1;
   const int ta0 = has_row ? A.row_item_off[rowa] : 0, ta1 = has_row ? A.row_item_off[rowa + 1] : 0;
-  if (!SYM && has_row)
+  if (RES && has_row)
     for (int e = lane; e < 81; e += 32) Cs[e] = __ldg(A.Cinv + (size_t)rowa * 81 + e);
   // r^T h of the start vectors
   {
@@ -401,7 +407,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       sc[0][2] = sc[0][3] = 1.e50;
     }
   }
-  if (!SYM && T > 0) {
+  if (RES && T > 0) {
     ok = stage_wait(A, mbar, 0u);
     landed = true;
   }
@@ -490,7 +496,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       auto load_recs = [&](int t) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          m[j] = t + j < T ? __ldg(A.item_rec + 4 * ((size_t)gwarp + (size_t)(t + j) * nwarps)) : make_int2(0, 0);
+          m[j] = t + j < T ? __ldg(A.item_rec + (size_t)gwarp + (size_t)(t + j) * nwarps) : make_int2(0, 0);
       };
       load_recs(0);
       if (!ok && lane == 0) atomicOr(A.err, 2);
@@ -519,7 +525,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
           }
         }
       }
-    } else {
+    } else if constexpr (RES) {
       double hc[P1_SLOTS], dc[P1_SLOTS], hk[P1_SLOTS], dk[P1_SLOTS];
 #pragma unroll
       for (int t = 0; t < P1_SLOTS; ++t) {
@@ -562,9 +568,41 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
           }
         }
       if (!ok && lane == 0) atomicOr(A.err, 2);
+    } else {
+      const int gl = grp < 3 ? grp : 0;
+      for (int t = 0; t < T; ++t) {
+        const size_t item = (size_t)gwarp + (size_t)t * nwarps;
+        const int2 m = __ldg(A.item_rec + item);
+        const bool act = lane < 27 && grp < (m.x >> 16);
+        const int2 en = act ? __ldg(A.ent + m.y + grp) : make_int2(0, 0);
+        const bool tr = en.y < 0;
+        const double *B = (const double *)A.blocks + (size_t)(en.y & 0x7fffffff) * 81;
+        double bv[9], cdc = 0.;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) bv[c] = act ? __ldg(B + (tr ? c * 9 + rr : rr * 9 + c)) : 0.;
+        if (act) {
+          const size_t j = (size_t)en.x * 9 + rr;
+          cdc = __ldcg(A.h + j) + beta_prev * __ldcg(dprev + j);
+        }
+        double acc = 0.;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+          const double xc = __shfl_sync(0xffffffffu, cdc, 9 * gl + c);
+          if (act) acc += bv[c] * xc;
+        }
+        const double a1 = __shfl_down_sync(0xffffffffu, acc, 9);
+        const double a2 = __shfl_down_sync(0xffffffffu, acc, 18);
+        if (lane < 9) {
+          const size_t i = (size_t)(m.x & 0xffff) * 9 + lane;
+          const double p = acc + a1 + a2;
+          A.part[item * 9 + lane] = p;
+          const double dkv = __ldcg(A.h + i) + beta_prev * __ldcg(dprev + i);
+          pdq[0] += dkv * p;
+        }
+      }
     }
     // this warp's vectors of its first row, ahead of the exchange
-    // (symmetric form: d^k itself, stored in phase 1a)
+    // (streamed form: d^k itself, stored in phase 1a)
     double hva = 0., dpa = 0., xva = 0., rva = 0.;
     if (has_row && lane < 9) {
       const size_t i = (size_t)rowa * 9 + lane;
@@ -606,7 +644,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
           r1v = (first ? rva : A.r[i]) - dr;
           p2[0] += dr * dr;
         }
-        const double *C = !SYM && first ? Cs : A.Cinv + (size_t)row * 81;
+        const double *C = RES && first ? Cs : A.Cinv + (size_t)row * 81;
         double h1v = 0.;
 #pragma unroll
         for (int c = 0; c < 9; ++c) {
@@ -1654,10 +1692,10 @@ void pcg_set_smem() {
   auto set = [](auto k, size_t bytes) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  set(k_pcg<false, false>, pcg_smem_bytes<false>());
-  set(k_pcg<true, false>, pcg_smem_bytes<false>());
-  set(k_pcg<false, true>, pcg_smem_bytes<true>());
-  set(k_pcg<true, true>, pcg_smem_bytes<true>());
+  set(k_pcg<false, PCG_RESIDENT>, pcg_smem_bytes<PCG_RESIDENT>());
+  set(k_pcg<true, PCG_RESIDENT>, pcg_smem_bytes<PCG_RESIDENT>());
+  set(k_pcg<false, PCG_STREAMED>, pcg_smem_bytes<PCG_STREAMED>());
+  set(k_pcg<true, PCG_STREAMED>, pcg_smem_bytes<PCG_STREAMED>());
   set(k_pcg32<false, false>, P32_SMEM);
   set(k_pcg32<true, false>, P32_SMEM);
   set(k_pcg32<false, true>, P32_SMEM);
@@ -1681,10 +1719,12 @@ int pcg_max_grid(int device) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k, threads, smem);
     per = std::min(per, p);
   };
-  fit(k_pcg<false, false>, pcg_threads<double>(), pcg_smem_bytes<false>());
-  fit(k_pcg<true, false>, pcg_threads<double>(), pcg_smem_bytes<false>());
-  fit(k_pcg<false, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
-  fit(k_pcg<true, true>, pcg_threads<double>(), pcg_smem_bytes<true>());
+  fit(k_pcg<false, PCG_RESIDENT>, pcg_threads<double>(), pcg_smem_bytes<PCG_RESIDENT>());
+  fit(k_pcg<true, PCG_RESIDENT>, pcg_threads<double>(), pcg_smem_bytes<PCG_RESIDENT>());
+  fit(k_pcg<false, PCG_STREAMED>, pcg_threads<double>(), pcg_smem_bytes<PCG_STREAMED>());
+  fit(k_pcg<true, PCG_STREAMED>, pcg_threads<double>(), pcg_smem_bytes<PCG_STREAMED>());
+  fit(k_pcg<false, PCG_GATHERED>, pcg_threads<double>(), 0);
+  fit(k_pcg<true, PCG_GATHERED>, pcg_threads<double>(), 0);
   fit(k_pcg32<false, false>, P32_T, P32_SMEM);
   fit(k_pcg32<true, false>, P32_T, P32_SMEM);
   fit(k_pcg32<false, true>, P32_T, P32_SMEM);
@@ -1692,6 +1732,8 @@ int pcg_max_grid(int device) {
   if (per < 1) per = 1;
   return std::min(nsm * per, XMAXG - 1);
 }
+
+int pcg_resident_items(int grid) { return P1_SLOTS * pcg_warps<double>() * grid; }
 
 // barrier word (and padding), then the CTAs' sums of the two exchanges
 size_t pcg_bar_bytes() { return 16 + 4 * (size_t)XMAXG * sizeof(double); }
@@ -1729,7 +1771,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
     // space an aggregate, per CTA (a barrier over 148 CTAs instead of 58 costs
     // 500 cycles, a second chunk or aggregate on an SM thousands)
     g0 = (int)std::min<long long>((ng + P32_W - 1) / P32_W, grid);
-    small32 = ng <= (long long)grid * P32_W && PCG32_CHUNK == 4;
+    small32 = ng <= (long long)grid * P32_W && PCG32_CHUNK == 4 && W.force_form <= PCG_RESIDENT;
     g = g0;
     if (small32) g = (int)std::max<long long>(std::max<long long>(g, (ng + 3) / 4), co ? coarse->nagg : 0);
     g = (int)std::min<long long>(g, grid);
@@ -1743,6 +1785,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.blocks = L.blocks32 ? (const void *)L.blocks32 : (const void *)L.blocks;
   A.row_item_off = L.row_item_off;
   A.item_rec = L.item_rec;
+  A.ent = L.ent;
   A.prod = W.prod;
   A.tpart = L.tpart;
   A.bidx = L.bidx;
@@ -1793,23 +1836,30 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   void *args[] = {&A};
   const void *fn;
   size_t smem;
-  int nthreads;
+  int nthreads, form;
   if (L.blocks32) {
     fn = co ? (small32 ? (const void *)k_pcg32<true, true> : (const void *)k_pcg32<true, false>)
             : (small32 ? (const void *)k_pcg32<false, true> : (const void *)k_pcg32<false, false>);
     smem = P32_SMEM;
     nthreads = P32_T;
+    form = small32 ? PCG_RESIDENT : PCG_STREAMED;
   } else {
-    const int nw = g * pcg_warps<double>();
-    const bool sym = L.nitems > P1_SLOTS * nw;
-    fn = co ? (sym ? (const void *)k_pcg<true, true> : (const void *)k_pcg<true, false>)
-            : (sym ? (const void *)k_pcg<false, true> : (const void *)k_pcg<false, false>);
-    smem = sym ? pcg_smem_bytes<true>() : pcg_smem_bytes<false>();
+    form = L.item_words == 4 ? PCG_RESIDENT : (W.prod ? PCG_STREAMED : PCG_GATHERED);
+    if (form == PCG_RESIDENT) {
+      fn = co ? (const void *)k_pcg<true, PCG_RESIDENT> : (const void *)k_pcg<false, PCG_RESIDENT>;
+      smem = pcg_smem_bytes<PCG_RESIDENT>();
+    } else if (form == PCG_STREAMED) {
+      fn = co ? (const void *)k_pcg<true, PCG_STREAMED> : (const void *)k_pcg<false, PCG_STREAMED>;
+      smem = pcg_smem_bytes<PCG_STREAMED>();
+    } else {
+      fn = co ? (const void *)k_pcg<true, PCG_GATHERED> : (const void *)k_pcg<false, PCG_GATHERED>;
+      smem = 0;
+    }
     nthreads = pcg_threads<double>();
   }
   pcg_set_smem();
   RPBA_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3(g), dim3(nthreads), args, smem, s));
-  return 0;
+  return form;
 }
 
 }  // namespace rpba

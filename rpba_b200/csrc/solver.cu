@@ -223,6 +223,7 @@ struct rpba_handle {
   std::vector<int> camparv;
   long long max_pairs = 0, npairs_cur = 0, learned_iters = 0;
   int pcg_grid = 1;
+  int pcg_form = 0;  // form of the last PCG (PcgForm), 0: none yet
   bool pcg_pending = false;
 
   // original state (restored by every solve)
@@ -306,8 +307,8 @@ struct rpba_handle {
     if (nb <= blocks_cap && cur) return;
     const int cap = std::max(nb, 1);
     if (cur) {
-      for (void *p : {cur, (void *)S.ent, (void *)S.item_rec, (void *)W.part, (void *)W.prod, (void *)L.tpart, (void *)S.bidx,
-                      (void *)W.pw, (void *)W.pdqc}) {
+      for (void *p : {cur, (void *)S.ent, (void *)S.item_rec, (void *)W.part, (void *)L.tpart, (void *)S.bidx, (void *)W.pw,
+                       (void *)W.pdqc}) {
         if (!p) continue;
         auto it = std::find(owned_async.begin(), owned_async.end(), p);
         if (it != owned_async.end()) {
@@ -325,21 +326,60 @@ struct rpba_handle {
       L.blocks32 = dalloc<float>((size_t)(nimg + cap) * BS32 + 16, owned);
       L.tpart = dalloc<float>((size_t)cap * 16 + 16, owned);
       // phase-1 chunks of the FP32 PCG: at most one per group of 32 blocks
+      S.bidx = dalloc<int4>((size_t)nimg + cap + 4, owned);
       const size_t groups = ((size_t)nimg + cap) / 32 + 4;
       W.pw = dalloc<double>(9 * groups, owned);
       W.pdqc = dalloc<double>(groups, owned);
     } else
       L.blocks = dalloc<double>((size_t)(nimg + cap) * BS64 + 2, owned);  // slack: the PCG's bulk copies round up
-    S.bidx = dalloc<int4>((size_t)nimg + cap + 4, owned);
     S.ent = dalloc<int2>((size_t)nimg + 2 * (size_t)cap, owned);
     if (!mixed) {
       // SpMV work items: at most ceil(entries / 3) per row
       const size_t items = (size_t)nimg + ((size_t)nimg + 2 * (size_t)cap) / 3 + 1;
-      S.item_rec = dalloc<int2>(4 * items, owned);
+      S.item_rec = dalloc<int2>(std::max(items, 4 * std::min(items, (size_t)pcg_resident_items(pcg_grid))), owned);
       W.part = dalloc<double>(items * 9, owned);
-      W.prod = dalloc<double>(((size_t)nimg + 2 * (size_t)cap) * 9, owned);
     }
     blocks_cap = cap;
+  }
+
+  // The FP64 PCG's form for the present structure.  A system that is not
+  // resident is streamed: its block index (16 B a block) and its blocks'
+  // products (72 B an entry) fit the pairs' keys and values (24 B a
+  // contribution) unless a block has fewer than seven contributions on
+  // average; then they get memory of their own, and where there is none left
+  // the blocks are gathered from both sides.
+  int stream_version = -1;
+  char *stream_buf = nullptr;
+  size_t stream_cap = 0;
+  void ensure_stream() {
+    if (L.blocks32 || stream_version == structure_version) return;
+    stream_version = structure_version;
+    W.prod = nullptr;
+    if (L.item_words == 4 || W.force_form == PCG_GATHERED) return;
+    const size_t nidx = (size_t)nimg + L.nboff + 4, need = nidx * sizeof(int4) +
+                        ((size_t)nimg + 2 * (size_t)L.nboff) * 9 * sizeof(double);
+    char *base = (char *)S.pval;
+    if (need > S.pair_bytes) {
+      if (need > stream_cap) {
+        if (stream_buf) {
+          owned_async.erase(std::find(owned_async.begin(), owned_async.end(), (void *)stream_buf));
+          cudaFreeAsync(stream_buf, s);
+        }
+        stream_buf = nullptr;
+        stream_cap = 0;
+        void *p = nullptr;
+        if (cudaMallocAsync(&p, need, s) != cudaSuccess) {
+          cudaGetLastError();
+          return;
+        }
+        owned_async.push_back(p);
+        stream_buf = (char *)p;
+        stream_cap = need;
+      }
+      base = stream_buf;
+    }
+    PROF("structure_bsr", 2, build_block_index(L, S, (int4 *)base, s));
+    W.prod = (double *)(base + nidx * sizeof(int4));
   }
 
   // dense direct-solve buffers, allocated on first use
@@ -773,10 +813,13 @@ static int create_impl(rpba_handle *H, const rpba_block *b, const rpba_options *
   const long long mb = std::min(mp, (long long)n * (n - 1) / 2 + 1);
   S.cub_bytes = structure_cub_bytes(nobs, mp, n);
   S.cub_tmp = dalloc<char>(S.cub_bytes, own);
-  S.pkey = dalloc<unsigned>(mp, own);
-  S.pkey2 = dalloc<unsigned>(mp, own);
-  S.pval = dalloc<unsigned long long>(mp, own);
-  S.pval2 = dalloc<unsigned long long>(mp, own);
+  const size_t bk = (4 * (size_t)mp + 255) & ~(size_t)255, bv = 2 * bk;  // each part aligned
+  S.pair_bytes = 2 * (bk + bv);
+  char *pairs = dalloc<char>(S.pair_bytes, own);
+  S.pval = (unsigned long long *)pairs;
+  S.pval2 = (unsigned long long *)(pairs + bv);
+  S.pkey = (unsigned *)(pairs + 2 * bv);
+  S.pkey2 = (unsigned *)(pairs + 2 * bv + bk);
   S.contrib = dalloc<int2>(mp, own);
   S.pcnt = dalloc<int>(npp + 1, own);
   S.poff = dalloc<int>(npp + 1, own);
@@ -865,7 +908,8 @@ void rpba_handle::structure() {
   PROF("structure_pairs", 3, nb = build_pairs(L, S, max_pairs, &npairs, s));
   npairs_cur = npairs;
   ensure_blocks(nb);
-  PROF("structure_bsr", 6, build_bsr(L, S, s));
+  S.resident_items = W.force_form > PCG_RESIDENT ? 0 : pcg_resident_items(pcg_grid);
+  PROF("structure_bsr", 7, build_bsr(L, S, s));
   if (opt.verbose & 4) {
     char line[160];
     std::snprintf(line, sizeof line, "Structure: cameras %d points %d observations %d pair contributions %lld "
@@ -935,6 +979,7 @@ bool rpba_handle::calc_bundle_sep(double multfact, int nrunknowns) {
         coarse_stale = false;
         fresh = true;
       }
+      ensure_stream();
       const int cap_try = (cw && !fresh) ? std::min(cap, 3 * coarse_ref_iters + 20) : cap;
       {
         CoopLock lk(this);
@@ -942,7 +987,7 @@ bool rpba_handle::calc_bundle_sep(double multfact, int nrunknowns) {
         // set-up kernels: rsqrt, features and set-up with weights (else the
         // set-up alone), the coarse restriction and prolongation
         PROF("pcg_setup", (d_weights ? 3 : 1) + (cw ? 2 : 0), pcg_prepare(L, W, mode, d_weights, cw, s));
-        PROF("pcg", 1, pcg_iterate(L, W, cap_try, pcg_grid, s, mode, opt.pcg_tolerance, cw));
+        PROF("pcg", 1, pcg_form = pcg_iterate(L, W, cap_try, pcg_grid, s, mode, opt.pcg_tolerance, cw));
       }
       RPBA_CUDA_CHECK(cudaMemcpyAsync(it, W.iters, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
       if (cw) RPBA_CUDA_CHECK(cudaMemcpyAsync(it + 2, CW.err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -977,7 +1022,7 @@ bool rpba_handle::calc_bundle_sep(double multfact, int nrunknowns) {
         CoopLock lk(this);
         prof.next_bytes = setup_bytes(false);
         PROF("pcg_setup", 1, pcg_prepare(L, W, 1, nullptr, nullptr, s));
-        PROF("pcg", 1, pcg_iterate(L, W, msize, pcg_grid, s, 1, opt.pcg_tolerance > 0. ? opt.pcg_tolerance : 1e-6,
+        PROF("pcg", 1, pcg_form = pcg_iterate(L, W, msize, pcg_grid, s, 1, opt.pcg_tolerance > 0. ? opt.pcg_tolerance : 1e-6,
                                     nullptr));
       }
       RPBA_CUDA_CHECK(cudaMemcpyAsync(it2, W.iters, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -994,11 +1039,12 @@ bool rpba_handle::calc_bundle_sep(double multfact, int nrunknowns) {
       }
     }
   } else {
+    ensure_stream();
     {
       CoopLock lk(this);
       prof.next_bytes = setup_bytes(false);
       PROF("pcg_setup", 1, pcg_prepare(L, W, 0, nullptr, nullptr, s));
-      PROF("pcg", 1, pcg_iterate(L, W, msize, pcg_grid, s, 0, 0., nullptr));
+      PROF("pcg", 1, pcg_form = pcg_iterate(L, W, msize, pcg_grid, s, 0, 0., nullptr));
     }
     pcg_pending = true;
   }
@@ -1966,9 +2012,12 @@ int32_t rpba_kernel_stats(rpba_handle *H, char *json, size_t cap) {
     first = false;
   }
   // the reduced camera system's size, for per-iteration byte counts
-  char b[160];
-  std::snprintf(b, sizeof b, "%s\"_rcs\": {\"rows\": %d, \"offdiag_blocks\": %d, \"fp32\": %d}", first ? "" : ", ",
-                H->nimg - H->begini, H->L.nboff, H->L.blocks32 ? 1 : 0);
+  // and the form of its last PCG
+  static const char *forms[] = {"none", "resident", "streamed", "gathered"};
+  char b[192];
+  std::snprintf(b, sizeof b,
+                "%s\"_rcs\": {\"rows\": %d, \"offdiag_blocks\": %d, \"fp32\": %d, \"pcg_form\": \"%s\"}",
+                first ? "" : ", ", H->nimg - H->begini, H->L.nboff, H->L.blocks32 ? 1 : 0, forms[H->pcg_form]);
   o += b;
   o += "}";
   const size_t n = std::min(cap - 1, o.size());
@@ -2038,6 +2087,12 @@ int32_t rpba_debug_wait_fault(rpba_handle *H, int32_t which, int64_t timeout_ns)
   H->L.wait_fault = which;
   H->L.bar_timeout_ns = H->ES.wait_ns = (unsigned long long)timeout_ns;
   H->ES.hold = which == 2;
+  return RPBA_OK;
+}
+
+int32_t rpba_debug_pcg_form(rpba_handle *H, int32_t form) {
+  if (!H || form < 0 || form > PCG_GATHERED) return RPBA_ERR_ARG;
+  H->W.force_form = form;
   return RPBA_OK;
 }
 

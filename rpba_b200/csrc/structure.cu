@@ -125,13 +125,14 @@ __global__ void k_row_items(const int *rowoff, int nimg, int begini, int *cnt) {
   cnt[k] = (k < nimg && k >= begini) ? (rowoff[k + 1] - rowoff[k] + 2) / 3 : 0;
 }
 
-// An item's record: its row, its number of entries, its first entry and the
-// entries themselves, in one aligned 32-byte piece.  One thread per (item, word);
-// item t of row k is found by bisection of the rows' first items.
+// An item's record: its row, its number of entries and its first entry, and
+// with four words the entries themselves, in one aligned 32-byte piece.  One
+// thread per (item, word); item t of row k is found by bisection of the rows'
+// first items.
 __global__ void k_fill_items(const int *rowoff, const int *row_item_off, const int2 *ent, int nimg, int nitems,
-                             int2 *rec) {
+                             int words, int2 *rec) {
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long t = gid >> 2;
+  const long long t = words == 4 ? gid >> 2 : gid;
   if (t >= nitems) return;
   int lo = 0, hi = nimg;  // the last row whose first item is <= t
   while (hi - lo > 1) {
@@ -142,7 +143,7 @@ __global__ void k_fill_items(const int *rowoff, const int *row_item_off, const i
       hi = m;
   }
   const int e0 = rowoff[lo] + 3 * (int)(t - row_item_off[lo]), ne = min(3, rowoff[lo + 1] - e0);
-  const int w = (int)(gid & 3);
+  const int w = words == 4 ? (int)(gid & 3) : 0;
   rec[gid] = w == 0 ? make_int2(lo | (ne << 16), e0) : (w <= ne ? ent[e0 + w - 1] : make_int2(0, 0));
 }
 
@@ -277,19 +278,27 @@ void build_bsr(DevLSA &L, StructWork &S, cudaStream_t s) {
     RPBA_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(S.cub_tmp, bytes, S.row_items, S.row_item_off, n + 1, s));
     RPBA_CUDA_CHECK(cudaMemcpyAsync(&L.nitems, S.row_item_off + n, sizeof(int), cudaMemcpyDeviceToHost, s));
     RPBA_CUDA_CHECK(cudaStreamSynchronize(s));
+    L.item_words = L.nitems <= S.resident_items ? 4 : 1;
     if (L.nitems > 0)
-      k_fill_items<<<nblk(4ll * L.nitems, 256), 256, 0, s>>>(S.rowoff, S.row_item_off, S.ent, n, L.nitems, S.item_rec);
+      k_fill_items<<<nblk((long long)L.item_words * L.nitems, 256), 256, 0, s>>>(S.rowoff, S.row_item_off, S.ent, n,
+                                                                                 L.nitems, L.item_words, S.item_rec);
+    L.bidx = nullptr;
+  } else {
+    build_block_index(L, S, S.bidx, s);
   }
-  const int fp64 = L.blocks32 ? 0 : 1;
-  k_fill_bidx<<<nblk((long long)n + nb, 256), 256, 0, s>>>(S.bkey, nb, n, S.rowoff, S.cntT, S.firstN, fp64, S.bidx);
-  if (nb > 0) k_fill_slots<<<nblk(nb, 256), 256, 0, s>>>(S.tidx2, nb, n, S.rowoff, S.firstT, fp64, S.bidx);
-  L.bidx = S.bidx;
   L.firstN = S.firstN;
   L.firstT = S.firstT;
   L.rowoff = S.rowoff;
   L.ent = S.ent;
   L.row_item_off = S.row_item_off;
   L.item_rec = S.item_rec;
+}
+
+void build_block_index(DevLSA &L, StructWork &S, int4 *bidx, cudaStream_t s) {
+  const int n = L.nimg, nb = L.nboff, fp64 = L.blocks32 ? 0 : 1;
+  k_fill_bidx<<<nblk((long long)n + nb, 256), 256, 0, s>>>(S.bkey, nb, n, S.rowoff, S.cntT, S.firstN, fp64, bidx);
+  if (nb > 0) k_fill_slots<<<nblk(nb, 256), 256, 0, s>>>(S.tidx2, nb, n, S.rowoff, S.firstT, fp64, bidx);
+  L.bidx = bidx;
 }
 
 // ---- PointXXvIn (rbacore.cpp:1918-1974) on the device: the track-ordered

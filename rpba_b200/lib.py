@@ -41,7 +41,7 @@ EXPORTS = ("rpba_status_string", "rpba_version", "rpba_input_block", "rpba_block
            "rpba_set_preconditioner", "rpba_precond_loss_grad", "rpba_record_systems", "rpba_solve_batch",
            "rpba_triangulate", "rpba_triangulate_parts", "rpba_partition_images", "rpba_lsa_gcp_step",
            "rpba_calc_plsa_parallel", "rpba_calc_plsa_parallel_hosted", "rpba_calc_plsa_parallel_ranks",
-           "rpba_calc_plsa_parallel_ranks_hosted", "rpba_debug_barrier_timeout", "rpba_debug_wait_fault",
+           "rpba_calc_plsa_parallel_ranks_hosted", "rpba_debug_barrier_timeout", "rpba_debug_wait_fault", "rpba_debug_pcg_form",
            "rpba_partition_count", "rpba_spd_inverse",
            "rpba_destroy")
 
@@ -165,6 +165,8 @@ def load():
     L.rpba_debug_barrier_timeout.restype = C.c_int32
     L.rpba_debug_wait_fault.argtypes = [C.c_void_p, C.c_int32, C.c_int64]
     L.rpba_debug_wait_fault.restype = C.c_int32
+    L.rpba_debug_pcg_form.argtypes = [C.c_void_p, C.c_int32]
+    L.rpba_debug_pcg_form.restype = C.c_int32
     L.rpba_destroy.argtypes = [C.c_void_p]
     _lib = L
     return L
@@ -568,6 +570,13 @@ class Solver:
         st = load().rpba_debug_wait_fault(self.h, int(which), int(timeout_ns))
         if st != 0:
             raise RpbaError(st, "rpba_debug_wait_fault")
+
+    def debug_pcg_form(self, form: int):
+        """Test hook: the PCG's form from the next solve on
+        (rpba_debug_pcg_form; 0: the library's choice)."""
+        st = load().rpba_debug_pcg_form(self.h, int(form))
+        if st != 0:
+            raise RpbaError(st, "rpba_debug_pcg_form")
 
     def close(self):
         if self.h:
