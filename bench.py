@@ -278,7 +278,7 @@ def rooflines(kstats, hbm, peak_kind):
                 "traffic_note": (f"ncu DRAM bytes / algorithmic bytes = {ratio:.3f} from {src}, scaled to "
                                  "this launch's algorithmic bytes") if ratio else None,
                 "algorithmic_bytes_per_launch": alg, "avg_launch_ms": d["ms"] / d["launches"]}
-    if dom == "pcg" and rcs and rcs.get("fp32"):
+    if dom == "pcg" and rcs and rcs.get("fp32") and rcs.get("pcg_form") == "streamed":
         # the library's count per iteration (solver.cu): blocks with their
         # 16 B index, the transposed products' 64 B slots written and read,
         # the per-row vectors; minimal: each block once with an 8 B index

@@ -310,6 +310,8 @@ int pcg_prepare(const DevLSA &L, const PcgWork &W, int mode, const float *weight
 enum PcgForm { PCG_RESIDENT = 1, PCG_STREAMED = 2, PCG_GATHERED = 3 };
 int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStream_t s, int mode, double tol,
                 const CoarseWork *coarse);
+// whether that form reads the system's blocks once a solve
+bool pcg_blocks_stay(const DevLSA &L, int form, int grid);
 int pcg_max_grid(int device);
 // most work items that the FP64 PCG's resident form holds
 int pcg_resident_items(int grid);

@@ -1733,6 +1733,19 @@ int pcg_max_grid(int device) {
   return std::min(nsm * per, XMAXG - 1);
 }
 
+// CTAs of the FP64 form: an item a warp
+static int grid64(int nitems, int grid) {
+  const int wpc = pcg_warps<double>();
+  return std::max(1, std::min((nitems + wpc - 1) / wpc, grid));
+}
+// its groups of 32 blocks, see group64
+static long long groups64(const DevLSA &L) { return (L.nimg - L.begini + 31) / 32 + (L.nboff + 31ll) / 32; }
+
+bool pcg_blocks_stay(const DevLSA &L, int form, int grid) {
+  if (form == PCG_STREAMED && !L.blocks32) return groups64(L) <= (long long)P1S_N * grid64(L.nitems, grid);
+  return form == PCG_RESIDENT;
+}
+
 int pcg_resident_items(int grid) { return P1_SLOTS * pcg_warps<double>() * grid; }
 
 // barrier word (and padding), then the CTAs' sums of the two exchanges
@@ -1776,8 +1789,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
     if (small32) g = (int)std::max<long long>(std::max<long long>(g, (ng + 3) / 4), co ? coarse->nagg : 0);
     g = (int)std::min<long long>(g, grid);
   } else {
-    const int wpc = pcg_warps<double>();
-    g = (L.nitems + wpc - 1) / wpc;
+    g = grid64(L.nitems, grid);
   }
   if (g > grid) g = grid;
   if (g < 1) g = 1;

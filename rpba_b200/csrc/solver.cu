@@ -277,18 +277,27 @@ struct rpba_handle {
     }
   }
 
-  // Algorithmic bytes of one PCG iteration.  FP64 form: every block read from
-  // both sides with its entry (648 + 8 B per side).  FP32 form (symmetric):
-  // every block read once with its index (324 + 16 B), and per off-diagonal
-  // block the transposed product written and read (a 64 B slot each way).  Per camera row: the preconditioner (648 B) and
-  // 22 reads/writes of 9-vectors (72 B each); with the coarse space P_k twice
-  // (720 B each) and the block part of h twice; A_c^-1 stays in L2 and is
-  // not counted.
-  double pcg_bytes_per_iteration(bool coarse) const {
+  // Algorithmic bytes of a PCG solve of `it` iterations, by its form.  Per
+  // block of the rows and off the diagonal once: the block with its index
+  // (FP64 648 + 16 B, FP32 324 + 16 B), in every iteration, or once a solve
+  // where the blocks stay in shared memory; gathered: 656 B (block, entry)
+  // from both sides.  Per iteration also the products that pass through
+  // memory, written and read: FP64 streamed 72 B each of every entry, FP32 a
+  // 64 B slot of every off-diagonal block.  Per camera row: the preconditioner
+  // (648 B) and 22 reads/writes of 9-vectors (72 B each); with the coarse space
+  // P_k twice (720 B each) and the block part of h twice; A_c^-1 stays in L2
+  // and is not counted.
+  double pcg_bytes(double it, bool coarse) const {
     const double Nc = nimg - begini, Nb = L.nboff;
     const double row = 648. + 22. * 72. + (coarse ? 2. * 720. + 2. * 72. : 0.);
-    const double blocks = L.blocks32 ? 340. * (Nc + Nb) + 128. * Nb : 656. * (Nc + 2. * Nb);
-    return blocks + Nc * row;
+    double blocks = (L.blocks32 ? 340. : 664.) * (Nc + Nb), products = 0.;
+    if (L.blocks32)
+      products = 128. * Nb;
+    else if (pcg_form == PCG_STREAMED)
+      products = 144. * (Nc + 2. * Nb);
+    else if (pcg_form == PCG_GATHERED)
+      blocks = 656. * (Nc + 2. * Nb);
+    return blocks * (pcg_blocks_stay(L, pcg_form, pcg_grid) ? 1. : it) + it * (products + Nc * row);
   }
 
   // Algorithmic bytes of the PCG set-up: per camera row its diagonal block,
@@ -996,7 +1005,7 @@ bool rpba_handle::calc_bundle_sep(double multfact, int nrunknowns) {
       if (prof.on)
         for (auto itp = prof.pending.rbegin(); itp != prof.pending.rend(); ++itp)
           if (std::string(itp->name) == "pcg") {
-            itp->bytes = (double)it[0] * pcg_bytes_per_iteration(cw != nullptr);
+            itp->bytes = pcg_bytes(it[0], cw != nullptr);
             break;
           }
       if (fresh) coarse_ref_iters = it[0];
@@ -1184,7 +1193,7 @@ int rpba_handle::adjust() {
       if (prof.on && pcg_pending)
         for (auto it = prof.pending.rbegin(); it != prof.pending.rend(); ++it)
           if (std::string(it->name) == "pcg") {
-            it->bytes = (double)hv.iters * pcg_bytes_per_iteration(false);
+            it->bytes = pcg_bytes(hv.iters, false);
             break;
           }
       pcg_pending = false;
