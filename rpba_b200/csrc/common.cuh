@@ -235,7 +235,8 @@ __device__ __forceinline__ void rectify(double *R, int rs) {
 }
 
 // n x n (n <= 9) inverse by LU with partial pivoting; A, Ai row major with
-// leading dimension 9.
+// leading dimension 9.  (FMAs written out: the compiler's choice of
+// contractions does not enter the bits.)
 __device__ __forceinline__ void lu_inverse9(int n, const double *A, double *Ai) {
   double LU[81];
   int perm[9];
@@ -265,7 +266,7 @@ __device__ __forceinline__ void lu_inverse9(int n, const double *A, double *Ai) 
     for (int r = k + 1; r < n; ++r) {
       const double l = LU[r * 9 + k] / piv;
       LU[r * 9 + k] = l;
-      for (int c = k + 1; c < n; ++c) LU[r * 9 + c] -= l * LU[k * 9 + c];
+      for (int c = k + 1; c < n; ++c) LU[r * 9 + c] = __fma_rn(-l, LU[k * 9 + c], LU[r * 9 + c]);
     }
   }
   for (int i = 0; i < 81; ++i) Ai[i] = 0.;
@@ -273,12 +274,12 @@ __device__ __forceinline__ void lu_inverse9(int n, const double *A, double *Ai) 
     double y[9];
     for (int i = 0; i < n; ++i) {
       double s = perm[i] == col ? 1. : 0.;
-      for (int j = 0; j < i; ++j) s -= LU[i * 9 + j] * y[j];
+      for (int j = 0; j < i; ++j) s = __fma_rn(-LU[i * 9 + j], y[j], s);
       y[i] = s;
     }
     for (int i = n - 1; i >= 0; --i) {
       double s = y[i];
-      for (int j = i + 1; j < n; ++j) s -= LU[i * 9 + j] * y[j];
+      for (int j = i + 1; j < n; ++j) s = __fma_rn(-LU[i * 9 + j], y[j], s);
       y[i] = s / LU[i * 9 + i];
     }
     for (int i = 0; i < n; ++i) Ai[i * 9 + col] = y[i];
@@ -288,7 +289,7 @@ __device__ __forceinline__ void lu_inverse9(int n, const double *A, double *Ai) 
 
 // Step k of lu_inverse9_warp's factorisation (k a compile-time constant, so
 // that the rows stay in registers).
-template <int k>
+template <int k, bool SAME>
 __device__ __forceinline__ void lu9_warp_step(int n, double (&row)[9], int &perm, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   if (k >= n) return;
@@ -317,29 +318,29 @@ __device__ __forceinline__ void lu9_warp_step(int n, double (&row)[9], int &perm
 #pragma unroll
   for (int c = k + 1; c < 9; ++c) {
     const double pk = __shfl_sync(FULL, row[c], k);
-    if (below && c < n) row[c] -= l * pk;
+    if (below && c < n) row[c] = SAME ? __fma_rn(-l, pk, row[c]) : row[c] - l * pk;
   }
 }
 
-template <int... K>
+template <bool SAME, int... K>
 __device__ __forceinline__ void lu9_warp_factor(int n, double (&row)[9], int &perm, int lane,
                                                 std::integer_sequence<int, K...>) {
-  (lu9_warp_step<K>(n, row, perm, lane), ...);
+  (lu9_warp_step<K, SAME>(n, row, perm, lane), ...);
 }
 
-// lu_inverse9 by one warp: the same operations in the same order, with row r of the factor in lane r's registers (r < 9) and
-// column col of the inverse solved by lane col.  `row` holds row `lane` of
+// lu_inverse9 by one warp: the same operations in the same order, with row r
+// of the factor in lane r's registers (r < 9) and column col of the inverse solved by lane col.  `row` holds row `lane` of
 // the input (lanes < 9; anything in the other lanes); every lane of the warp
 // calls it; lanes < 9 write their column of the inverse to Ai (Ai may be the
 // input's storage: nothing is read from memory).
-// SAME: the same bits as lu_inverse9 too.  Left to itself the compiler forms
-// the first step of row 0's back substitution, 1 - u y, in two roundings
-// (its start value is known to be 0 or 1), where lu_inverse9's is one FMA.
+// SAME: the same bits as lu_inverse9 too, every FMA written out as there.
+// (Left to itself the compiler forms the first step of row 0's back
+// substitution, 1 - u y, in two roundings, its start value being 0 or 1.)
 template <bool SAME = false>
 __device__ __forceinline__ void lu_inverse9_warp(int n, double (&row)[9], double *Ai, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   int perm = lane;
-  lu9_warp_factor(n, row, perm, lane, std::make_integer_sequence<int, 9>{});
+  lu9_warp_factor<SAME>(n, row, perm, lane, std::make_integer_sequence<int, 9>{});
   // column `lane` of the inverse: forward then back substitution
   double y[9];
 #pragma unroll
@@ -348,7 +349,10 @@ __device__ __forceinline__ void lu_inverse9_warp(int n, double (&row)[9], double
     if (i < n) {
       double s = __shfl_sync(FULL, perm, i) == lane ? 1. : 0.;
 #pragma unroll
-      for (int j = 0; j < i; ++j) s -= __shfl_sync(FULL, row[j], i) * y[j];
+      for (int j = 0; j < i; ++j) {
+        const double l = __shfl_sync(FULL, row[j], i);
+        s = SAME ? __fma_rn(-l, y[j], s) : s - l * y[j];
+      }
       y[i] = s;
     }
   }

@@ -316,6 +316,9 @@ int pcg_max_grid(int device);
 // most work items that the FP64 PCG's resident form holds
 int pcg_resident_items(int grid);
 size_t pcg_bar_bytes();
+// test of the set-up's 9 x 9 inverse: `count` matrices (device) inverted by one
+// thread and by one warp each
+void lu_inverse9_both(const double *A, int count, int np, double *by_thread, double *by_warp, cudaStream_t s);
 
 // ---- structure (structure.cu)
 struct StructWork {

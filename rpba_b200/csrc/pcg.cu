@@ -1685,7 +1685,25 @@ __global__ void __launch_bounds__(32 * SETUP_W) k_pcg_setup(DevLSA L, PcgWork W)
   }
 }
 
+// Test of lu_inverse9_warp<true>: matrix blockIdx.x inverted by one thread and
+// by the warp.
+__global__ void k_lu_both(const double *A, int np, double *by_thread, double *by_warp) {
+  const int lane = threadIdx.x;
+  const double *a = A + (size_t)blockIdx.x * 81;
+  if (lane == 0) lu_inverse9(np, a, by_thread + (size_t)blockIdx.x * 81);
+  __syncwarp();
+  double row[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) row[c] = lane < 9 ? a[lane * 9 + c] : 0.;
+  lu_inverse9_warp<true>(np, row, by_warp + (size_t)blockIdx.x * 81, lane);
+}
+
 }  // namespace
+
+void lu_inverse9_both(const double *A, int count, int np, double *by_thread, double *by_warp, cudaStream_t s) {
+  k_lu_both<<<count, 32, 0, s>>>(A, np, by_thread, by_warp);
+  RPBA_CUDA_CHECK(cudaGetLastError());
+}
 
 // the phase-1 stages of the FP64 form live in dynamic shared memory (124 KB)
 void pcg_set_smem() {

@@ -2105,6 +2105,39 @@ int32_t rpba_debug_pcg_form(rpba_handle *H, int32_t form) {
   return RPBA_OK;
 }
 
+int32_t rpba_debug_lu_inverse9(const double *A, int32_t count, int32_t np, double *by_thread, double *by_warp,
+                               int32_t device) {
+  if (!A || !by_thread || !by_warp || count < 1 || count > 65536 || np < 1 || np > 9) return RPBA_ERR_ARG;
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= device) return RPBA_ERR_NO_DEVICE;
+  struct Args {
+    const double *A;
+    int count, np;
+    double *t, *w;
+    int device;
+  } args{A, count, np, by_thread, by_warp, device};
+  return guard(
+      [](void *p) -> int {
+        const Args &a = *(const Args *)p;
+        RPBA_CUDA_CHECK(cudaSetDevice(a.device));
+        std::vector<void *> own;
+        struct Free {
+          std::vector<void *> &o;
+          ~Free() {
+            for (void *q : o) cudaFree(q);
+          }
+        } fr{own};
+        const size_t n = 81 * (size_t)a.count, bytes = n * sizeof(double);
+        double *dA = dalloc<double>(n, own), *dt = dalloc<double>(n, own), *dw = dalloc<double>(n, own);
+        RPBA_CUDA_CHECK(cudaMemcpy(dA, a.A, bytes, cudaMemcpyHostToDevice));
+        lu_inverse9_both(dA, a.count, a.np, dt, dw, 0);
+        RPBA_CUDA_CHECK(cudaMemcpy(a.t, dt, bytes, cudaMemcpyDeviceToHost));
+        RPBA_CUDA_CHECK(cudaMemcpy(a.w, dw, bytes, cudaMemcpyDeviceToHost));
+        return (int)RPBA_OK;
+      },
+      &args);
+}
+
 void rpba_destroy(rpba_handle *H) { delete H; }
 
 int32_t rpba_partition_count(int32_t n_images, int32_t threads, int32_t exteval) {
