@@ -514,7 +514,7 @@ int32_t rpba_debug_pcg_form(rpba_handle *h, int32_t form);
  * 9 x 9 matrices (row major, host buffers) whose leading np x np part (1 .. 9)
  * is inverted by one thread and by one warp; the two agree to the bit.  No
  * counterpart in the reference. */
-int32_t rpba_debug_lu_inverse9(const double *A, int32_t count, int32_t np, double *by_thread, double *by_warp,
+int32_t rpba_debug_lu_inverse(const double *A, int32_t count, int32_t np, double *by_thread, double *by_warp,
                                int32_t device);
 /* Releases a handle and its device memory (`delete LSA1`,
  * rpbacore.cpp:525). */

@@ -2105,7 +2105,7 @@ int32_t rpba_debug_pcg_form(rpba_handle *H, int32_t form) {
   return RPBA_OK;
 }
 
-int32_t rpba_debug_lu_inverse9(const double *A, int32_t count, int32_t np, double *by_thread, double *by_warp,
+int32_t rpba_debug_lu_inverse(const double *A, int32_t count, int32_t np, double *by_thread, double *by_warp,
                                int32_t device) {
   if (!A || !by_thread || !by_warp || count < 1 || count > 65536 || np < 1 || np > 9) return RPBA_ERR_ARG;
   int ndev = 0;

@@ -42,7 +42,7 @@ EXPORTS = ("rpba_status_string", "rpba_version", "rpba_input_block", "rpba_block
            "rpba_triangulate", "rpba_triangulate_parts", "rpba_partition_images", "rpba_lsa_gcp_step",
            "rpba_calc_plsa_parallel", "rpba_calc_plsa_parallel_hosted", "rpba_calc_plsa_parallel_ranks",
            "rpba_calc_plsa_parallel_ranks_hosted", "rpba_debug_barrier_timeout", "rpba_debug_wait_fault", "rpba_debug_pcg_form",
-           "rpba_debug_lu_inverse9",
+           "rpba_debug_lu_inverse",
            "rpba_partition_count", "rpba_spd_inverse",
            "rpba_destroy")
 
@@ -169,8 +169,8 @@ def load():
     L.rpba_debug_pcg_form.argtypes = [C.c_void_p, C.c_int32]
     L.rpba_debug_pcg_form.restype = C.c_int32
     dp = C.POINTER(C.c_double)
-    L.rpba_debug_lu_inverse9.argtypes = [dp, C.c_int32, C.c_int32, dp, dp, C.c_int32]
-    L.rpba_debug_lu_inverse9.restype = C.c_int32
+    L.rpba_debug_lu_inverse.argtypes = [dp, C.c_int32, C.c_int32, dp, dp, C.c_int32]
+    L.rpba_debug_lu_inverse.restype = C.c_int32
     L.rpba_destroy.argtypes = [C.c_void_p]
     _lib = L
     return L

@@ -21,7 +21,7 @@ def test_warp_equals_thread(np_):
         A[0, :np_, :np_] = np.eye(np_)[::-1]
     t, w = np.full_like(A, np.nan), np.full_like(A, np.nan)
     dp = C.POINTER(C.c_double)
-    st = rb.load().rpba_debug_lu_inverse9(A.ctypes.data_as(dp), n, np_, t.ctypes.data_as(dp), w.ctypes.data_as(dp), 0)
+    st = rb.load().rpba_debug_lu_inverse(A.ctypes.data_as(dp), n, np_, t.ctypes.data_as(dp), w.ctypes.data_as(dp), 0)
     assert st == 0
     assert np.isfinite(t).all()
     # (by value: the padding's zeros may differ in sign)
