@@ -329,10 +329,11 @@ __device__ __forceinline__ void lu9_warp_factor(int n, double (&row)[9], int &pe
 }
 
 // lu_inverse9 by one warp: the same operations in the same order, with row r
-// of the factor in lane r's registers (r < 9) and column col of the inverse solved by lane col.  `row` holds row `lane` of
-// the input (lanes < 9; anything in the other lanes); every lane of the warp
-// calls it; lanes < 9 write their column of the inverse to Ai (Ai may be the
-// input's storage: nothing is read from memory).
+// of the factor in lane r's registers (r < 9) and column col of the inverse
+// solved by lane col.  `row` holds row `lane` of the input (lanes < 9; anything
+// in the other lanes); every lane of the warp calls it; lanes < 9 write their
+// column of the inverse to Ai (Ai may be the input's storage: nothing is read
+// from memory).
 // SAME: the same bits as lu_inverse9 too, every FMA written out as there.
 // (Left to itself the compiler forms the first step of row 0's back
 // substitution, 1 - u y, in two roundings, its start value being 0 or 1.)

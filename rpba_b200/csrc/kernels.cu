@@ -1158,9 +1158,7 @@ __global__ void k_final_cost(DevLSA L, double *partials) {
   }
 }
 
-// ------------------------------------------------------------ Exteval
-// EvalLSA + CalcCorrPointMulti (rpbacore.cpp:778-837, 882-941): one thread
-// per point, float sums in the reference's order within the point.
+// A track entry that names no observation sets *bad (Exteval, refinement).
 __global__ void k_check_tracks(int nt, int n, const int *__restrict__ pt_img, const int *__restrict__ pt_slot,
                                const int *__restrict__ img_off, int *bad) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1169,6 +1167,9 @@ __global__ void k_check_tracks(int nt, int n, const int *__restrict__ pt_img, co
   if (im < 0 || im >= n || sl < 0 || sl >= img_off[im + 1] - img_off[im]) *bad = 1;
 }
 
+// ------------------------------------------------------------ Exteval
+// EvalLSA + CalcCorrPointMulti (rpbacore.cpp:778-837, 882-941): one thread
+// per point, float sums in the reference's order within the point.
 __global__ void k_exteval(int n_points, const int *__restrict__ pt_off, const int *__restrict__ pt_img,
                           const int *__restrict__ pt_slot, const int *__restrict__ img_off,
                           const float *__restrict__ pmat, const float *__restrict__ Kf,

@@ -6,10 +6,10 @@
 //
 // One cooperative launch runs the whole solve.  The FP64 form is k_pcg, the
 // FP32 form k_pcg32; each has a variant for systems that stay in shared memory
-// (described before them).  Dot
-// products are reduced per CTA and then, after a grid barrier, by every CTA
-// in the same fixed order, so all CTAs take identical decisions.  The grid
-// barrier's wait is bounded: after 2 s it sets an error bit and returns.
+// (described before them).  Dot products are reduced per CTA and then, after a
+// grid barrier, by every CTA in the same fixed order, so all CTAs take
+// identical decisions.  The grid barrier's wait is bounded: after 2 s it sets
+// an error bit and returns.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -21,19 +21,11 @@ namespace rpba {
 
 namespace {
 
-// Threads per CTA of the FP64 form's persistent kernel.
-template <class BT>
-constexpr int pcg_threads() {
-  return 1024;
-}
-template <class BT>
-constexpr int pcg_warps() {
-  return pcg_threads<BT>() / 32;
-}
-
+// Threads and warps per CTA of the FP64 form's persistent kernel.
+constexpr int P64_T = 1024, P64_W = P64_T / 32;
 
 struct PcgArgs {
-  const void *blocks;  // BT[(nimg + nboff) * 81]
+  const void *blocks;  // [(nimg + nboff) * 81] doubles or floats
   const int *row_item_off;
   const int2 *item_rec;   // [nitems][4 or 1] (row | entries << 16, first entry), resident form: up to three entries
   const int2 *ent;        // gathered form: the entries
@@ -229,7 +221,7 @@ static_assert(P1S_BLK % 16 == 0 && P1S_STAGE % 16 == 0, "16-byte aligned stage p
 template <int FORM>
 constexpr size_t pcg_smem_bytes() {
   return FORM == PCG_STREAMED ? (size_t)P1S_N * P1S_STAGE
-                              : (FORM == PCG_RESIDENT ? (size_t)pcg_warps<double>() * P1_WARP_BYTES : 0);
+                              : (FORM == PCG_RESIDENT ? (size_t)P64_W * P1_WARP_BYTES : 0);
 }
 
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
@@ -315,16 +307,15 @@ __device__ __forceinline__ double row_q(const PcgArgs &A, int t0, int t1, int la
 //  phase 2b per aggregate: z = A_c^-1[aggregate rows] (P^T r1), then
 //           h1 = hj + P z and the two dot products
 template <bool CO, int FORM>
-__global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
-  constexpr int PCG_T = pcg_threads<double>(), PCG_W = pcg_warps<double>();
+__global__ void __launch_bounds__(P64_T, 1) k_pcg(PcgArgs A) {
   constexpr bool RES = FORM == PCG_RESIDENT, SYM = FORM == PCG_STREAMED;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gwarp = blockIdx.x * PCG_W + warp, nwarps = gridDim.x * PCG_W;
+  const int gwarp = blockIdx.x * P64_W + warp, nwarps = gridDim.x * P64_W;
   const int grp = lane / 9, rr = lane % 9, gbase = grp * 9;
   const int G = gridDim.x;
   GridBarrier bar(A.bar, (unsigned)G + A.bar_extra, A.err, A.bar_ns);
-  __shared__ Exchange<1, PCG_W> X1;
-  __shared__ Exchange<3, PCG_W> X2;
+  __shared__ Exchange<1, P64_W> X1;
+  __shared__ Exchange<3, P64_W> X2;
   // scalars of the recurrence by iteration parity (every thread computes the
   // same values, thread 0 stores them): r^T h, its start value, the smallest
   // and the first increment
@@ -398,7 +389,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         const size_t i = (size_t)row * 9 + lane;
         v[0] += A.r[i] * A.h[i];
       }
-    if (!exchange_sum<3, PCG_W>(bar, A.red2, v, X2)) {
+    if (!exchange_sum<3, P64_W>(bar, A.red2, v, X2)) {
       drain();
       return;
     }
@@ -611,7 +602,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
       xva = A.x[i];
       rva = A.r[i];
     }
-    if (!exchange_sum<1, PCG_W>(bar, A.red1, pdq, X1, !ok)) {
+    if (!exchange_sum<1, P64_W>(bar, A.red1, pdq, X1, !ok)) {
       drain();
       return;
     }
@@ -659,12 +650,12 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         }
       }
     } else {
-      __shared__ double shr[PCG_W][CO_M];
+      __shared__ double shr[P64_W][CO_M];
       __shared__ double shz[CO_M];
       for (int a = blockIdx.x; a < A.nagg; a += G) {
         const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
         double rcw = 0.;
-        for (int t = t0 + warp; t < t1; t += PCG_W) {
+        for (int t = t0 + warp; t < t1; t += P64_W) {
           const int row = A.agg_rows[t];
           const size_t i = (size_t)row * 9 + (lane < 9 ? lane : 0);
           double r1v = 0.;
@@ -700,7 +691,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         __syncthreads();
         if (threadIdx.x < CO_M) {
           double sum = 0.;
-          for (int w = 0; w < PCG_W; ++w) sum += shr[w][threadIdx.x];
+          for (int w = 0; w < P64_W; ++w) sum += shr[w][threadIdx.x];
           A.rc[a * CO_M + threadIdx.x] = sum;
         }
         __syncthreads();
@@ -713,7 +704,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         double z[CO_M];
 #pragma unroll
         for (int j = 0; j < CO_M; ++j) z[j] = 0.;
-        for (int i = threadIdx.x; i < A.nc; i += PCG_T) {
+        for (int i = threadIdx.x; i < A.nc; i += P64_T) {
           const double rv = __ldcg(A.rc + i);
 #pragma unroll
           for (int j = 0; j < CO_M; ++j) z[j] += __ldg(A.Ainv + (size_t)(a * CO_M + j) * A.nc + i) * rv;
@@ -727,12 +718,12 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         __syncthreads();
         if (threadIdx.x < CO_M) {
           double sum = 0.;
-          for (int w = 0; w < PCG_W; ++w) sum += shr[w][threadIdx.x];
+          for (int w = 0; w < P64_W; ++w) sum += shr[w][threadIdx.x];
           shz[threadIdx.x] = sum;
         }
         __syncthreads();
         const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
-        for (int t = t0 + warp; t < t1; t += PCG_W) {
+        for (int t = t0 + warp; t < t1; t += P64_W) {
           const int row = A.agg_rows[t];
           if (lane < 9) {
             const size_t i = (size_t)row * 9 + lane;
@@ -749,7 +740,7 @@ __global__ void __launch_bounds__(pcg_threads<double>(), 1) k_pcg(PcgArgs A) {
         __syncthreads();
       }
     }
-    if (!exchange_sum<3, PCG_W>(bar, A.red2, p2, X2)) {
+    if (!exchange_sum<3, P64_W>(bar, A.red2, p2, X2)) {
       drain();
       return;
     }
@@ -887,8 +878,9 @@ __device__ __forceinline__ void group_issue(const PcgArgs &A, const Grp32 &q, un
 
 // FP32 d^k of camera c (12-float stride) into v[0..8].  The loads may hit
 // L1: d32 is written in phase D by all CTAs before a grid barrier, whose
-// gpu-scope fence and block barrier order those writes before these loads,
-// and the rows of a cluster keep gathering the same columns.
+// release arrivals, acquiring load (thread 0's) and block barrier order those
+// writes before these loads, and the rows of a cluster keep gathering the
+// same columns.
 __device__ __forceinline__ void load_d32(const float *d32, int c, float (&v)[9]) {
   const float4 *p = (const float4 *)(d32 + (size_t)c * 12);
   const float4 a = __ldca(p), b = __ldca(p + 1), e = __ldca(p + 2);
@@ -1250,89 +1242,89 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
       };
       if (c < nch && lane == 0) group_issue(A, group_of(c * ch, (int)gd, A.row0, A.row1, A.nboff), stg, mbar);
       while (c < nch) {
-      const long long g0 = c * ch, g1 = min(ng, g0 + ch);
-      cur_row = -1;
-      racc = 0.;
-      pdq = 0.;
-      for (long long g = g0; g < g1; ++g) {
-        const Grp32 q = group_of(g, (int)gd, A.row0, A.row1, A.nboff);
-        if (!stage_wait(A, mbar, parity)) {
-          ok = false;
-          break;
-        }
-        parity ^= 1u;
-        const bool act = lane < q.n;
-        int4 rc = make_int4(-1 - lane, -1, 0, 0);
-        float y[9], t[9];
-        group_products(A, q, stg, lane, act, rc, y, t, pdq);
-        // the stage's blocks are read: the next group's copies may land
-        // (the next group of this chunk, or the first of the next chunk)
-        __syncwarp();
-        const long long gn = g + 1 < g1 ? g + 1 : (cn < nch ? cn * ch : -1);
-        if (lane == 0 && gn >= 0) {
-          fence_proxy_async();
-          group_issue(A, group_of(gn, (int)gd, A.row0, A.row1, A.nboff), stg, mbar);
-        }
-        if (q.diag) {
-          if (act) {
-            double *dst = A.pdiag + (size_t)rc.x * 9;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) dst[i] = (double)y[i];
+        const long long g0 = c * ch, g1 = min(ng, g0 + ch);
+        cur_row = -1;
+        racc = 0.;
+        pdq = 0.;
+        for (long long g = g0; g < g1; ++g) {
+          const Grp32 q = group_of(g, (int)gd, A.row0, A.row1, A.nboff);
+          if (!stage_wait(A, mbar, parity)) {
+            ok = false;
+            break;
           }
-          continue;
-        }
-        // the transposed product to the block's slot (column order)
-        if (act) store_transposed(A, rc.z, t);
-        const int row = rc.x;
-        // a group inside the open row (most groups: a row has hundreds of
-        // blocks): every lane adds its product to its own FP64 running sum
-        if (cur_row >= 0 && __all_sync(0xffffffffu, !act || row == cur_row)) {
-          if (act)
+          parity ^= 1u;
+          const bool act = lane < q.n;
+          int4 rc = make_int4(-1 - lane, -1, 0, 0);
+          float y[9], t[9];
+          group_products(A, q, stg, lane, act, rc, y, t, pdq);
+          // the stage's blocks are read: the next group's copies may land
+          // (the next group of this chunk, or the first of the next chunk)
+          __syncwarp();
+          const long long gn = g + 1 < g1 ? g + 1 : (cn < nch ? cn * ch : -1);
+          if (lane == 0 && gn >= 0) {
+            fence_proxy_async();
+            group_issue(A, group_of(gn, (int)gd, A.row0, A.row1, A.nboff), stg, mbar);
+          }
+          if (q.diag) {
+            if (act) {
+              double *dst = A.pdiag + (size_t)rc.x * 9;
 #pragma unroll
-            for (int j = 0; j < 9; ++j) lacc[j] += (double)y[j];
-          continue;
+              for (int i = 0; i < 9; ++i) dst[i] = (double)y[i];
+            }
+            continue;
+          }
+          // the transposed product to the block's slot (column order)
+          if (act) store_transposed(A, rc.z, t);
+          const int row = rc.x;
+          // a group inside the open row (most groups: a row has hundreds of
+          // blocks): every lane adds its product to its own FP64 running sum
+          if (cur_row >= 0 && __all_sync(0xffffffffu, !act || row == cur_row)) {
+            if (act)
+#pragma unroll
+              for (int j = 0; j < 9; ++j) lacc[j] += (double)y[j];
+            continue;
+          }
+          // a row boundary: the lanes' running sums join the open row's sum,
+          // then a segmented scan of the group's products (rows non-decreasing
+          // in lane order; inactive lanes carry distinct negative rows)
+          fold_lanes();
+          segment_scan(row, y, lane);
+          const int rnext = __shfl_down_sync(0xffffffffu, row, 1);
+          const bool end = act && (lane == q.n - 1 || rnext != row);
+          unsigned ends = __ballot_sync(0xffffffffu, end);
+          int seg_first = 0;  // first lane of the segment ending at e
+          while (ends) {
+            const int e = __ffs(ends) - 1;
+            ends &= ends - 1;
+            const int re = __shfl_sync(0xffffffffu, row, e);
+            double sv = 0.;
+#pragma unroll
+            for (int j = 0; j < 9; ++j) {
+              const float tv = __shfl_sync(0xffffffffu, y[j], e);
+              if (lane == j) sv = (double)tv;
+            }
+            if (re == cur_row) {
+              racc += sv;
+            } else {
+              flush();
+              // a segment starts the row unless it is the chunk's first and
+              // the row began before the chunk
+              cur_head = cur_row >= 0 || seg_first > 0 || q.boff + seg_first == (long long)__ldg(A.firstN + re);
+              cur_row = re;
+              racc = sv;
+            }
+            seg_first = e + 1;
+          }
         }
-        // a row boundary: the lanes' running sums join the open row's sum,
-        // then a segmented scan of the group's products (rows non-decreasing
-        // in lane order; inactive lanes carry distinct negative rows)
+        if (!ok) break;
         fold_lanes();
-        segment_scan(row, y, lane);
-        const int rnext = __shfl_down_sync(0xffffffffu, row, 1);
-        const bool end = act && (lane == q.n - 1 || rnext != row);
-        unsigned ends = __ballot_sync(0xffffffffu, end);
-        int seg_first = 0;  // first lane of the segment ending at e
-        while (ends) {
-          const int e = __ffs(ends) - 1;
-          ends &= ends - 1;
-          const int re = __shfl_sync(0xffffffffu, row, e);
-          double sv = 0.;
+        flush();
+        // the chunk's share of d^T A d, summed over its lanes in a fixed order
 #pragma unroll
-          for (int j = 0; j < 9; ++j) {
-            const float tv = __shfl_sync(0xffffffffu, y[j], e);
-            if (lane == j) sv = (double)tv;
-          }
-          if (re == cur_row) {
-            racc += sv;
-          } else {
-            flush();
-            // a segment starts the row unless it is the chunk's first and
-            // the row began before the chunk
-            cur_head = cur_row >= 0 || seg_first > 0 || q.boff + seg_first == (long long)__ldg(A.firstN + re);
-            cur_row = re;
-            racc = sv;
-          }
-          seg_first = e + 1;
-        }
-      }
-      if (!ok) break;
-      fold_lanes();
-      flush();
-      // the chunk's share of d^T A d, summed over its lanes in a fixed order
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) pdq += __shfl_xor_sync(0xffffffffu, pdq, o);
-      if (lane == 0) A.pdqc[c] = pdq;
-      c = cn;
-      cn = c < nch ? grab() : nch;
+        for (int o = 16; o > 0; o >>= 1) pdq += __shfl_xor_sync(0xffffffffu, pdq, o);
+        if (lane == 0) A.pdqc[c] = pdq;
+        c = cn;
+        cn = c < nch ? grab() : nch;
       }
       __syncwarp();
       if (!ok) {
@@ -1469,41 +1461,41 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           __syncthreads();
         }
       } else {
-      const int nrows = A.row1 - A.row0;
-      auto grab_row = [&]() -> int {
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(A.ctr + 1, 1u);
-        return (int)__shfl_sync(0xffffffffu, t, 0);
-      };
-      for (int t = grab_row(); t < nrows;) {
-        const int row = A.row1 - 1 - t;
-        const int tn = grab_row();  // the next row, taken one ahead
-        double d2;
-        const double acc = take_row(row, d2);
-        if (pl) A.rowc[(size_t)row * RC_S + lane - 16] = acc;
-        if (lane == 31) A.rowc[(size_t)row * RC_S + CO_M] = d2;
-        t = tn;
-      }
-      if (!bar.sync()) return;
-      // 2a': per aggregate, its rows' restrictions and shares of dr^2 in a
-      // fixed order (warp w: rows w, w + P32_W, ...; then the warps in order)
-      for (int a = blockIdx.x; a < A.nagg; a += G) {
-        const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
-        double v = 0.;
-        if (lane <= CO_M)
-          for (int t = t0 + warp; t < t1; t += P32_W) v += __ldcg(A.rowc + (size_t)A.agg_rows[t] * RC_S + lane);
-        if (lane <= CO_M) shr[warp][lane] = v;
-        __syncthreads();
-        if (threadIdx.x <= CO_M) {
-          double sum = 0.;
-          for (int w = 0; w < P32_W; ++w) sum += shr[w][threadIdx.x];
-          if (threadIdx.x < CO_M)
-            A.rc[a * CO_M + threadIdx.x] = sum;
-          else
-            p2[0] += sum;
+        const int nrows = A.row1 - A.row0;
+        auto grab_row = [&]() -> int {
+          unsigned t = 0;
+          if (lane == 0) t = atomicAdd(A.ctr + 1, 1u);
+          return (int)__shfl_sync(0xffffffffu, t, 0);
+        };
+        for (int t = grab_row(); t < nrows;) {
+          const int row = A.row1 - 1 - t;
+          const int tn = grab_row();  // the next row, taken one ahead
+          double d2;
+          const double acc = take_row(row, d2);
+          if (pl) A.rowc[(size_t)row * RC_S + lane - 16] = acc;
+          if (lane == 31) A.rowc[(size_t)row * RC_S + CO_M] = d2;
+          t = tn;
         }
-        __syncthreads();
-      }
+        if (!bar.sync()) return;
+        // 2a': per aggregate, its rows' restrictions and shares of dr^2 in a
+        // fixed order (warp w: rows w, w + P32_W, ...; then the warps in order)
+        for (int a = blockIdx.x; a < A.nagg; a += G) {
+          const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
+          double v = 0.;
+          if (lane <= CO_M)
+            for (int t = t0 + warp; t < t1; t += P32_W) v += __ldcg(A.rowc + (size_t)A.agg_rows[t] * RC_S + lane);
+          if (lane <= CO_M) shr[warp][lane] = v;
+          __syncthreads();
+          if (threadIdx.x <= CO_M) {
+            double sum = 0.;
+            for (int w = 0; w < P32_W; ++w) sum += shr[w][threadIdx.x];
+            if (threadIdx.x < CO_M)
+              A.rc[a * CO_M + threadIdx.x] = sum;
+            else
+              p2[0] += sum;
+          }
+          __syncthreads();
+        }
       }
       if (!bar.sync()) return;
       // z of an aggregate: its rows of A_c^-1 with the restrictions, a warp's share
@@ -1588,35 +1580,35 @@ __global__ void __launch_bounds__(P32_T, 1) k_pcg32(PcgArgs A) {
           }
         }
       } else {
-      for (int a = blockIdx.x; a < A.nagg; a += G) {
-        {
-          const double zs = z_share(a);
-          if ((lane & 1) == 0 && lane < 2 * CO_M) shr[warp][lane >> 1] = zs;
-        }
-        __syncthreads();
-        if (threadIdx.x < CO_M) {
-          double sum = 0.;
-          for (int w = 0; w < P32_W; ++w) sum += shr[w][threadIdx.x];
-          shz[threadIdx.x] = sum;
-        }
-        __syncthreads();
-        const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
-        for (int t = t0 + warp; t < t1; t += P32_W) {
-          const int row = A.agg_rows[t];
-          if (lane < 9) {
-            const size_t i = (size_t)row * 9 + lane;
-            const double *Pk = A.P + (size_t)row * (9 * CO_M) + lane * CO_M;
-            double h1v = __ldcg(A.hj + i);
-#pragma unroll
-            for (int j = 0; j < CO_M; ++j) h1v += __ldg(Pk + j) * shz[j];
-            const double hv = __ldcg(A.h + i), r1v = __ldcg(A.r + i);
-            p2[1] += r1v * (h1v - hv);
-            p2[2] += r1v * h1v;
-            A.h[i] = h1v;
+        for (int a = blockIdx.x; a < A.nagg; a += G) {
+          {
+            const double zs = z_share(a);
+            if ((lane & 1) == 0 && lane < 2 * CO_M) shr[warp][lane >> 1] = zs;
           }
+          __syncthreads();
+          if (threadIdx.x < CO_M) {
+            double sum = 0.;
+            for (int w = 0; w < P32_W; ++w) sum += shr[w][threadIdx.x];
+            shz[threadIdx.x] = sum;
+          }
+          __syncthreads();
+          const int t0 = A.agg_off[a], t1 = A.agg_off[a + 1];
+          for (int t = t0 + warp; t < t1; t += P32_W) {
+            const int row = A.agg_rows[t];
+            if (lane < 9) {
+              const size_t i = (size_t)row * 9 + lane;
+              const double *Pk = A.P + (size_t)row * (9 * CO_M) + lane * CO_M;
+              double h1v = __ldcg(A.hj + i);
+#pragma unroll
+              for (int j = 0; j < CO_M; ++j) h1v += __ldg(Pk + j) * shz[j];
+              const double hv = __ldcg(A.h + i), r1v = __ldcg(A.r + i);
+              p2[1] += r1v * (h1v - hv);
+              p2[2] += r1v * h1v;
+              A.h[i] = h1v;
+            }
+          }
+          __syncthreads();
         }
-        __syncthreads();
-      }
       }
     }
     if (!exchange_sum<3, P32_W>(bar, A.red2, p2, X2)) return;
@@ -1705,7 +1697,8 @@ void lu_inverse9_both(const double *A, int count, int np, double *by_thread, dou
   RPBA_CUDA_CHECK(cudaGetLastError());
 }
 
-// the phase-1 stages of the FP64 form live in dynamic shared memory (124 KB)
+// the blocks and stages live in dynamic shared memory (FP64 resident 212,992 B,
+// streamed 213,472 B)
 void pcg_set_smem() {
   auto set = [](auto k, size_t bytes) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -1719,7 +1712,6 @@ void pcg_set_smem() {
   set(k_pcg32<false, true>, P32_SMEM);
   set(k_pcg32<true, true>, P32_SMEM);
 }
-
 
 // Groups of 32 blocks per phase-1 chunk of the FP32 PCG: small enough that
 // the warps finish together, large enough that a chunk's fixed work (its
@@ -1737,12 +1729,12 @@ int pcg_max_grid(int device) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k, threads, smem);
     per = std::min(per, p);
   };
-  fit(k_pcg<false, PCG_RESIDENT>, pcg_threads<double>(), pcg_smem_bytes<PCG_RESIDENT>());
-  fit(k_pcg<true, PCG_RESIDENT>, pcg_threads<double>(), pcg_smem_bytes<PCG_RESIDENT>());
-  fit(k_pcg<false, PCG_STREAMED>, pcg_threads<double>(), pcg_smem_bytes<PCG_STREAMED>());
-  fit(k_pcg<true, PCG_STREAMED>, pcg_threads<double>(), pcg_smem_bytes<PCG_STREAMED>());
-  fit(k_pcg<false, PCG_GATHERED>, pcg_threads<double>(), 0);
-  fit(k_pcg<true, PCG_GATHERED>, pcg_threads<double>(), 0);
+  fit(k_pcg<false, PCG_RESIDENT>, P64_T, pcg_smem_bytes<PCG_RESIDENT>());
+  fit(k_pcg<true, PCG_RESIDENT>, P64_T, pcg_smem_bytes<PCG_RESIDENT>());
+  fit(k_pcg<false, PCG_STREAMED>, P64_T, pcg_smem_bytes<PCG_STREAMED>());
+  fit(k_pcg<true, PCG_STREAMED>, P64_T, pcg_smem_bytes<PCG_STREAMED>());
+  fit(k_pcg<false, PCG_GATHERED>, P64_T, 0);
+  fit(k_pcg<true, PCG_GATHERED>, P64_T, 0);
   fit(k_pcg32<false, false>, P32_T, P32_SMEM);
   fit(k_pcg32<true, false>, P32_T, P32_SMEM);
   fit(k_pcg32<false, true>, P32_T, P32_SMEM);
@@ -1753,8 +1745,7 @@ int pcg_max_grid(int device) {
 
 // CTAs of the FP64 form: an item a warp
 static int grid64(int nitems, int grid) {
-  const int wpc = pcg_warps<double>();
-  return std::max(1, std::min((nitems + wpc - 1) / wpc, grid));
+  return std::max(1, std::min((nitems + P64_W - 1) / P64_W, grid));
 }
 // its groups of 32 blocks, see group64
 static long long groups64(const DevLSA &L) { return (L.nimg - L.begini + 31) / 32 + (L.nboff + 31ll) / 32; }
@@ -1764,7 +1755,7 @@ bool pcg_blocks_stay(const DevLSA &L, int form, int grid) {
   return form == PCG_RESIDENT;
 }
 
-int pcg_resident_items(int grid) { return P1_SLOTS * pcg_warps<double>() * grid; }
+int pcg_resident_items(int grid) { return P1_SLOTS * P64_W * grid; }
 
 // barrier word (and padding), then the CTAs' sums of the two exchanges
 size_t pcg_bar_bytes() { return 16 + 4 * (size_t)XMAXG * sizeof(double); }
@@ -1885,7 +1876,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
       fn = co ? (const void *)k_pcg<true, PCG_GATHERED> : (const void *)k_pcg<false, PCG_GATHERED>;
       smem = 0;
     }
-    nthreads = pcg_threads<double>();
+    nthreads = P64_T;
   }
   pcg_set_smem();
   RPBA_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3(g), dim3(nthreads), args, smem, s));

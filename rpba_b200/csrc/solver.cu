@@ -195,8 +195,6 @@ struct rpba_handle {
   int nimg = 0, XXnr = 0, n_slots = 0, n_track_in = 0;
   std::vector<float> K_in, XX_in;
   std::vector<int32_t> img_off_in;
-  rpba_block raw{};  // device copy of the caller's block (Exteval)
-  bool raw_uploaded = false;
   std::vector<float> h_pmat, h_K, h_dist, h_XX;
   // an Exteval handle's block and results on the device
   struct {
@@ -334,8 +332,8 @@ struct rpba_handle {
       // FP32 PCG's bulk copies round their sizes up to 16 bytes
       L.blocks32 = dalloc<float>((size_t)(nimg + cap) * BS32 + 16, owned);
       L.tpart = dalloc<float>((size_t)cap * 16 + 16, owned);
-      // phase-1 chunks of the FP32 PCG: at most one per group of 32 blocks
       S.bidx = dalloc<int4>((size_t)nimg + cap + 4, owned);
+      // phase-1 chunks of the FP32 PCG: at most one per group of 32 blocks
       const size_t groups = ((size_t)nimg + cap) / 32 + 4;
       W.pw = dalloc<double>(9 * groups, owned);
       W.pdqc = dalloc<double>(groups, owned);
@@ -391,7 +389,6 @@ struct rpba_handle {
     W.prod = (double *)(base + nidx * sizeof(int4));
   }
 
-  // dense direct-solve buffers, allocated on first use
   // coarse space of the learned solver, built once per handle from the
   // cameras of the first linear system (nullptr: none)
   CoarseWork CW{};
