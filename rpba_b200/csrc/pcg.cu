@@ -59,7 +59,7 @@ struct PcgArgs {
   unsigned long long bar_ns;
   unsigned tx_extra;
   int row0, row1, nitems, msize;
-  int stream_once;  // FP64 streamed form: the blocks exceed L2
+  int stream_once;  // FP64 streamed form: blocks read with an evict-first hint
   int mode;     // 0: reference stop rule; 1: relative preconditioned residual
   double tol2;  // mode 1: stop when r^T M^-1 r <= tol2 * (r0^T M^-1 r0)
   // two-level preconditioner (coarse.cu): rows are owned per aggregate
@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(P64_T, 1) k_pcg(PcgArgs A) {
   if constexpr (SYM) {
     if (stream) {
       // blocks that do not fit L2 beside the products should not evict them
+      // (STREAM_ONCE_BYTES)
       if (A.stream_once)
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(policy));
       if (lane == 0 && (warp & 1) == 0) {
@@ -1719,6 +1720,14 @@ void pcg_set_smem() {
 // its barrier: 2 groups 377 us, 4 groups 365 us, 8 groups 379 us).
 constexpr int PCG32_CHUNK = 4;
 
+// Bytes of blocks from which on the FP64 streamed form reads them with an
+// evict-first hint.  With products and index, a quarter on top, the system
+// reaches the 126 MB of L2 at 100 MB of blocks, and the hint keeps the products
+// there.  An iteration without and with it, by size of the blocks: 24 MB 26.6
+// and 26.9 us, 76 MB 52.3 and 52.4, 82 MB 54.8 and 53.4, 123 MB 75.7 and 68.7,
+// 177 MB 98.8 and 90.4, 241 MB 126.7 and 120.4.
+constexpr double STREAM_ONCE_BYTES = 6.4e7;
+
 int pcg_max_grid(int device) {
   int nsm = 0, per = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
@@ -1841,7 +1850,7 @@ int pcg_iterate(const DevLSA &L, const PcgWork &W, int msize, int grid, cudaStre
   A.row0 = L.begini;
   A.row1 = L.nimg;
   A.nitems = L.nitems;
-  A.stream_once = ((double)nrows + L.nboff) * 648. > 6.4e7;
+  A.stream_once = ((double)nrows + L.nboff) * 648. > STREAM_ONCE_BYTES;
   A.msize = msize;
   A.mode = mode;
   A.tol2 = tol * tol;
